@@ -16,6 +16,7 @@ gradient come back). The keys of a case:
 import math
 
 import torch
+import torch.nn.functional as F
 
 import miniworld_b200 as mw
 from miniworld_b200.training import trimul_train
@@ -126,7 +127,8 @@ def _mask(case, gen):
     return torch.rand(b, n, generator=gen, device="cuda") >= 0.1
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """Parameters (fp32), pair tensor, mask, and for a training step the output's gradient and the dropout scale."""
     gen = torch.Generator(device="cuda")
     gen.manual_seed(seed)
     b, n, c = case["b"], case["n"], case["c"]
@@ -136,7 +138,20 @@ def prepare(case, seed):
     for i in range(b):  # (in slabs: the fp32 draw of a large pair tensor is never held whole)
         for r in range(0, n, 256):
             z[i, r : r + 256] = torch.randn(min(256, n - r), n, c, generator=gen, device="cuda") * scale
-    state = {"z": z, "mask": _mask(case, gen)}
+    mask, dy, drop_scale = _mask(case, gen), None, None
+    if case["mode"] == "train":
+        dy = torch.empty_like(z)
+        for i in range(b):
+            dy[i] = torch.randn(n, n, c, generator=gen, device="cuda") * 0.01
+        if case["drop"]:
+            keep = torch.rand(b, 1, n, c, generator=gen, device="cuda") >= 0.25
+            drop_scale = keep.to(torch.bfloat16) / 0.75
+    return params, z, mask, dy, drop_scale
+
+
+def prepare(case, seed):
+    params, z, mask, dy, drop_scale = _inputs(case, seed)
+    state = {"z": z, "mask": mask}
     module = _module(case)
     module.load_state_dict(params)
     module = module.to("cuda")
@@ -146,12 +161,9 @@ def prepare(case, seed):
     state["module"] = module.train()
     state["params"] = dict(module.named_parameters())
     z.requires_grad_(True)
-    state["dy"] = torch.empty_like(z)
-    for i in range(b):
-        state["dy"][i] = torch.randn(n, n, c, generator=gen, device="cuda") * 0.01
-    if case["drop"]:
-        keep = torch.rand(b, 1, n, c, generator=gen, device="cuda") >= 0.25
-        state["drop_scale"] = keep.to(torch.bfloat16) / 0.75
+    state["dy"] = dy
+    if drop_scale is not None:
+        state["drop_scale"] = drop_scale
     state["outgoing"] = {"outgoing": True, "incoming": False}.get(case["op"])
     return state
 
@@ -170,6 +182,64 @@ def run(state):
         y = module(z) if mask is None else module(z, mask)
     grads = torch.autograd.grad(y, [z, *params.values()], state["dy"])
     return {"y": y.detach(), "z": grads[0], **dict(zip(params, grads[1:]))}
+
+
+def _update64(case, p, z, valid, drop_scale):
+    """The published operator on one sample ``z`` [N, N, C] in float64, residual included."""
+    c = case["c"]
+    if case["op"] == "transition":
+        rows = []
+        for zr in z.split(256):
+            x = F.layer_norm(zr, (c,), p["ln_in.weight"], p["ln_in.bias"], 1e-5)
+            h = F.silu(F.linear(x, p["expand_a.weight"])) * F.linear(x, p["expand_b.weight"])
+            rows.append(zr + F.linear(h, p["squeeze.weight"]))
+        return torch.cat(rows)
+    x = F.layer_norm(z, (c,), p["ln_pair.weight"], p["ln_pair.bias"], 1e-5)
+    left = torch.sigmoid(F.linear(x, p["to_left_gate.weight"])) * F.linear(x, p["to_left.weight"])
+    right = torch.sigmoid(F.linear(x, p["to_right_gate.weight"])) * F.linear(x, p["to_right.weight"])
+    if valid is not None:
+        left, right = left * valid[..., None], right * valid[..., None]
+    w = left.shape[-1]
+    out = {"outgoing": w, "incoming": 0, "bidirectional": w // 2}[case["op"]]  # channels contracted over k of (i, k), (j, k)
+    tri = []
+    if out:
+        tri.append(torch.einsum("ikd,jkd->ijd", left[..., :out], right[..., :out]))
+    if out < w:
+        tri.append(torch.einsum("kid,kjd->ijd", left[..., out:], right[..., out:]))
+    del left, right
+    t = F.layer_norm(torch.cat(tri, -1), (w,), p["ln_out.weight"], p["ln_out.bias"], 1e-5)
+    del tri
+    update = torch.sigmoid(F.linear(x, p["to_gate.weight"])) * F.linear(t, p["to_out.weight"])
+    return z + (update if drop_scale is None else update * drop_scale)
+
+
+def exact(case, seed):
+    """What ``run`` returns, from the same inputs in float64 and one sample at a time (samples share the parameters only)."""
+    params, z, mask, dy, drop_scale = _inputs(case, seed)
+    train = case["mode"] == "train"
+    p = {}
+    for key, v in params.items():  # inference rounds the linear weights to bf16 once; the LayerNorms stay fp32
+        p[key] = (v if train or key.startswith("ln_") else v.to(torch.bfloat16)).double().requires_grad_(train)
+    out = {"y": torch.empty(z.shape, dtype=torch.float64, device="cuda")}
+    if train:
+        out["z"] = torch.empty_like(out["y"])
+        out.update({key: torch.zeros_like(v) for key, v in p.items()})
+    for i in range(case["b"]):
+        valid = None
+        if mask is not None:
+            valid = mask[i] if mask.dim() == 3 else mask[i][:, None] & mask[i][None, :]
+        drop = None if drop_scale is None else drop_scale[i].double()
+        zi = z[i].double().requires_grad_(train)
+        with torch.set_grad_enabled(train):
+            y = _update64(case, p, zi, valid, drop)
+            out["y"][i] = y.detach()
+            if train:
+                grads = torch.autograd.grad(y, [zi, *p.values()], dy[i].double())
+                out["z"][i] = grads[0]
+                for key, g in zip(p, grads[1:]):
+                    out[key] += g
+        del y
+    return out if train else out["y"]
 
 
 def work(case):
