@@ -244,6 +244,20 @@ int b200_trimul_forward_ex(const void* z, const void* w_left, const void* w_left
                            void* cuda_stream);
 
 /*
+ * b200_trimul_forward_ex for every N >= 1. Nothing is padded: z, y, the masks and drop_scale are dense with N columns,
+ * only the intermediates in the workspace have their columns N rounded up to a multiple of 8 apart. Workspace:
+ * b200_trimul_workspace_bytes of N rounded up to a multiple of 8. A workspace this call leaves behind is read by
+ * b200_trimul_backward_any with the same N.
+ */
+int b200_trimul_forward_any(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
+                            const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,
+                            const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
+                            const void* const* bias_opt, const uint8_t* token_mask, const uint8_t* pair_mask,
+                            const void* drop_scale, void* y, void* workspace, size_t workspace_bytes, int B, int N,
+                            int d_pair, int d_hidden, int direction, float eps_in, float eps_out, int residual,
+                            void* cuda_stream);
+
+/*
  * Weight packing of the bidirectional module (shapes as in b200_trimul_forward_ex): two blocks of
  * b200_trimul_packed_bytes() each. `packed_out` feeds stage 1 of the outgoing half and stage 3, `packed_in` stage 1
  * of the incoming half; stage 3 also reads the second half of w_out from `packed_in`.
@@ -322,6 +336,19 @@ int b200_trimul_backward(const void* dy, const void* z, const void* w_left, cons
                          float* d_ln_in_w, float* d_ln_in_b, float* d_ln_out_w, float* d_ln_out_b, void* workspace,
                          size_t workspace_bytes, int B, int N, int d_pair, int d_hidden, int direction, float eps_in,
                          float eps_out, int residual, void* cuda_stream);
+
+/*
+ * b200_trimul_backward for every N >= 1, after b200_trimul_forward_any. Workspace: b200_trimul_backward_workspace_bytes of
+ * N rounded up to a multiple of 8.
+ */
+int b200_trimul_backward_any(const void* dy, const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
+                             const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,
+                             const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
+                             const void* const* bias_opt, const uint8_t* token_mask, const uint8_t* pair_mask,
+                             const void* drop_scale, const void* forward_workspace, void* dz, void* const* dw,
+                             float* d_ln_in_w, float* d_ln_in_b, float* d_ln_out_w, float* d_ln_out_b, void* workspace,
+                             size_t workspace_bytes, int B, int N, int d_pair, int d_hidden, int direction, float eps_in,
+                             float eps_out, int residual, void* cuda_stream);
 
 /*
  * Pair Transition, the operator on the other side of the triangle update in every block

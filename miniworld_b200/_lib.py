@@ -130,6 +130,10 @@ SIGNATURES = {
     "b200_trimul_read_status": (c_int, [c_void_p, c_void_p, POINTER(c_int)]),
 }
 
+# the same arguments, every N
+SIGNATURES["b200_trimul_forward_any"] = SIGNATURES["b200_trimul_forward_ex"]
+SIGNATURES["b200_trimul_backward_any"] = SIGNATURES["b200_trimul_backward"]
+
 _lib = None
 
 

@@ -208,6 +208,7 @@ struct BwdEpilogueParams {
   int tiles_per_row;   // ceil(N / 128)
   int num_tiles;       // B * N * tiles_per_row
   int n;               // N
+  int ld;              // columns per row of ext_stats and ln_part (N rounded up to a multiple of 8)
   const float* consts;      // [2][128]: d_out = W_out beta_out + bias_out, d_gate = W_gate beta_in + bias_gate
   const float* grad_scale;  // [2]: c, 1 / c
   const uint16_t* drop_scale;  // [B][N][128] bf16 or null
@@ -216,8 +217,8 @@ struct BwdEpilogueParams {
   float* part_m;       // [grid][2][128][128]: per-CTA partial sums of dproj^T t_hat and dgate^T x_hat
   float* part_s;       // [grid][2][128]: per-CTA column sums of dproj and dgate
   // the two-launch form for an output LayerNorm over 256 channels (MODE 1: first 128 channels, MODE 2: the others)
-  const float2* ext_stats;  // [B*N][N]: mean and rstd of the stored t over all 256 channels
-  float2* ln_part;          // [B*N][N]: MODE 1 writes its sums of d t_hat and d t_hat * t_hat; MODE 2 adds its own and
+  const float2* ext_stats;  // [B*N][ld]: mean and rstd of the stored t over all 256 channels
+  float2* ln_part;          // [B*N][ld]: MODE 1 writes its sums of d t_hat and d t_hat * t_hat; MODE 2 adds its own and
                             // writes back the two means over 256 channels
   const uint16_t* p_part;   // [B*N][N][128] fp16, MODE 2: the first launch's part of the output projection
   int* status;
@@ -341,7 +342,7 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
       rstd_out = normalise_tile<false, false>(t_s, xchg, pos, part, p.eps_out);
     } else {
       float2 st = make_float2(0.f, 0.f);
-      if (j0 + pos < p.n) st = p.ext_stats[static_cast<size_t>(row) * p.n + j0 + pos];
+      if (j0 + pos < p.n) st = p.ext_stats[static_cast<size_t>(row) * p.ld + j0 + pos];
       rstd_out = st.y;
       const float nmr = -st.x * st.y;
 #pragma unroll 8
@@ -534,7 +535,7 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
       const bool inside = j0 + pos < p.n;
       float2 other = make_float2(0.f, 0.f);  // MODE 2: the first launch's sums (read before the barrier below)
       if constexpr (MODE == 2) {
-        if (inside) other = p.ln_part[static_cast<size_t>(row) * p.n + j0 + pos];
+        if (inside) other = p.ln_part[static_cast<size_t>(row) * p.ld + j0 + pos];
       }
       float s1 = 0.f, s2 = 0.f;
       float th[kBwdCh];                 // this thread's t_hat values and its d t_hat, both kept for the second pass
@@ -558,10 +559,10 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
       float m1, m2;
       sum_partials(xchg, pos, m1, m2);
       if constexpr (MODE == 1) {
-        if (part == 0 && inside) p.ln_part[static_cast<size_t>(row) * p.n + j0 + pos] = make_float2(m1, m2);
+        if (part == 0 && inside) p.ln_part[static_cast<size_t>(row) * p.ld + j0 + pos] = make_float2(m1, m2);
       } else if constexpr (MODE == 2) {
         m1 = (m1 + other.x) * (1.0f / 256.0f), m2 = (m2 + other.y) * (1.0f / 256.0f);
-        if (part == 0 && inside) p.ln_part[static_cast<size_t>(row) * p.n + j0 + pos] = make_float2(m1, m2);
+        if (part == 0 && inside) p.ln_part[static_cast<size_t>(row) * p.ld + j0 + pos] = make_float2(m1, m2);
       } else {
         m1 *= 1.0f / 128.0f, m2 *= 1.0f / 128.0f;
       }

@@ -310,14 +310,23 @@ static int set_smem(K kernel, int bytes, int device) {
 
 static bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
-static int check_bn(int B, int N) {
-  if (B < 1 || N < 8) return B200_TRIMUL_E_SHAPE;
-  if (N % 8 != 0) return B200_TRIMUL_E_UNSUPPORTED;
+// `any_n`: the call came through an entry point that takes every N; the others take multiples of 8 (their tensors are
+// dense, and a tensor map's strides are multiples of 16 bytes).
+static int check_bn(int B, int N, bool any_n = false) {
+  if (B < 1 || N < (any_n ? 1 : 8)) return B200_TRIMUL_E_SHAPE;
+  if (!any_n && N % 8 != 0) return B200_TRIMUL_E_UNSUPPORTED;
   if (static_cast<long long>(B) * N > 0x7FFFFFFFll / 128) return B200_TRIMUL_E_SHAPE;
   return B200_TRIMUL_OK;
 }
 
 static size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
+
+// Columns from one channel of a pair row to the next in the row-plane intermediates (left, right, tri and their
+// gradients): N rounded up to the 16 bytes a tensor map's strides need. The maps' extents stay N: loads read zeros past
+// it and stores are clipped there, so the columns N .. pitch-1 are never written or used and no input is padded.
+// (N = 203, one sample: copying z, mask and output to and from 208 columns was 43 us of kernels beside the 37 us of the
+// three stages.)
+static int plane_pitch(int N) { return (N + 7) / 8 * 8; }
 
 static size_t plane_tensor_bytes(int B, int rows, int N) {
   return round_up(static_cast<size_t>(B) * rows * kC * N * 2, 1024);
@@ -535,13 +544,13 @@ enum PrologueMode { kLocal, kGatherRight, kChannels };
 static int prologue_impl(const void* z, const void* packed, const uint8_t* token_mask, const uint8_t* pair_mask,
                          void* const* left_dst, int n_left, void* const* right_dst, int n_right, PrologueMode mode,
                          int B, int N, int row_begin, int rows, float eps_in, int has_bias, int* status,
-                         void* cuda_stream, int d_pair = kC) {
+                         void* cuda_stream, int d_pair = kC, bool any_n = false) {
   if (d_pair != kC && d_pair != 64) return B200_TRIMUL_E_UNSUPPORTED;
   if (!z || !packed || !left_dst || !right_dst || !status) return B200_TRIMUL_E_NULL;
   if (n_left < 1 || n_left > kMaxDst || n_right < 1 || n_right > kMaxDst) return B200_TRIMUL_E_SHAPE;
   if (mode != kLocal && B != 1) return B200_TRIMUL_E_SHAPE;
   if (mode == kChannels && (n_left != n_right || kC % n_left != 0 || (kC / n_left) % 8 != 0)) return B200_TRIMUL_E_SHAPE;
-  int rc = check_bn(B, N);
+  int rc = check_bn(B, N, any_n);
   if (rc != B200_TRIMUL_OK) return rc;
   if (rows < 1 || row_begin < 0 || row_begin + rows > N) return B200_TRIMUL_E_SHAPE;
   if (!aligned(z, 16) || !aligned(packed, 1024)) return B200_TRIMUL_E_ALIGN;
@@ -563,7 +572,8 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
     // outputs, row-plane: [rows][channels][N columns]
     const uint64_t n64 = static_cast<uint64_t>(N);
     const uint64_t ch = mode == kChannels ? static_cast<uint64_t>(kC / n_left) : static_cast<uint64_t>(kC);
-    const uint64_t strides[2] = {n64 * 2ull, n64 * ch * 2ull};
+    const uint64_t ld = static_cast<uint64_t>(plane_pitch(N));
+    const uint64_t strides[2] = {ld * 2ull, ld * ch * 2ull};
     const uint32_t box[3] = {64, static_cast<uint32_t>(ch), 1};
     const uint64_t dims_local[3] = {n64, ch, static_cast<uint64_t>(B) * rows};
     const uint64_t dims_all[3] = {n64, ch, n64};
@@ -676,12 +686,12 @@ constexpr int kDirMixed = 3;
 
 static int contract_impl(const void* left, const void* right, void* tri, void* const* owner_dst, int n_owners, int slot,
                          int channels, int B, int N, int row_begin, int rows, int k_rows, int direction, int* status,
-                         void* cuda_stream, int row_channels = 0) {
+                         void* cuda_stream, int row_channels = 0, bool any_n = false) {
   if (!left || !right || !status) return B200_TRIMUL_E_NULL;
   if (n_owners == 0 && !tri) return B200_TRIMUL_E_NULL;
   if (n_owners < 0 || n_owners > kMaxOwners || (n_owners > 0 && !owner_dst)) return B200_TRIMUL_E_SHAPE;
   if (channels < 8 || channels > kC || channels % 8 != 0) return B200_TRIMUL_E_SHAPE;
-  int rc = check_bn(B, N);
+  int rc = check_bn(B, N, any_n);
   if (rc != B200_TRIMUL_OK) return rc;
   if (rows < 1 || row_begin < 0 || row_begin + rows > N) return B200_TRIMUL_E_SHAPE;
   if (k_rows < 1 || k_rows > N) return B200_TRIMUL_E_SHAPE;
@@ -701,9 +711,10 @@ static int contract_impl(const void* left, const void* right, void* tri, void* c
   const bool use_pair = rows >= 256 && (pair_rows - rows) * 4 <= rows;
   const int bn = use_pair ? ((N + 255) / 256 * 256 <= (N + 127) / 128 * 128 ? 256 : 128) : choose_bn(N);
   const uint64_t n64 = static_cast<uint64_t>(N);
+  const uint64_t ld = static_cast<uint64_t>(plane_pitch(N));
   const uint64_t ch64 = static_cast<uint64_t>(channels);
-  const uint64_t row_stride = static_cast<uint64_t>(row_channels > 0 ? row_channels : channels) * n64 * 2;  // bytes between pair rows
-  const uint64_t h_stride = n64 * 2;
+  const uint64_t row_stride = static_cast<uint64_t>(row_channels > 0 ? row_channels : channels) * ld * 2;  // bytes between pair rows
+  const uint64_t h_stride = ld * 2;
   const uint64_t left_rows = a_mn ? static_cast<uint64_t>(k_rows) : static_cast<uint64_t>(rows);
   const uint64_t right_rows = b_mn ? static_cast<uint64_t>(k_rows) : n64;
 
@@ -785,23 +796,28 @@ int b200_trimul_contract(const void* left, const void* right, void* tri, int B, 
   return contract_impl(left, right, tri, nullptr, 0, 0, kC, B, N, row_begin, rows, N, direction, status, cuda_stream);
 }
 
-int b200_trimul_contract_backward(const void* dtri, const void* left, const void* right, void* dleft, void* dright, int B,
-                                  int N, int direction, int* status, void* cuda_stream) {
+static int contract_backward_impl(const void* dtri, const void* left, const void* right, void* dleft, void* dright, int B,
+                                  int N, int direction, int* status, void* cuda_stream, bool any_n) {
   if (!dtri || !left || !right || !dleft || !dright) return B200_TRIMUL_E_NULL;
   int rc;
   if (direction == B200_TRIMUL_OUTGOING) {
     // t_ij = sum_k l_ik r_jk:  dl_ik = sum_j dt_ij r_jk (mixed),  dr_jk = sum_i dt_ij l_ik (the incoming form)
-    rc = contract_impl(dtri, right, dleft, nullptr, 0, 0, kC, B, N, 0, N, N, kDirMixed, status, cuda_stream);
+    rc = contract_impl(dtri, right, dleft, nullptr, 0, 0, kC, B, N, 0, N, N, kDirMixed, status, cuda_stream, 0, any_n);
     if (rc != B200_TRIMUL_OK) return rc;
-    return contract_impl(dtri, left, dright, nullptr, 0, 0, kC, B, N, 0, N, N, B200_TRIMUL_INCOMING, status, cuda_stream);
+    return contract_impl(dtri, left, dright, nullptr, 0, 0, kC, B, N, 0, N, N, B200_TRIMUL_INCOMING, status, cuda_stream, 0, any_n);
   }
   if (direction == B200_TRIMUL_INCOMING) {
     // t_ij = sum_k l_ki r_kj:  dl_ki = sum_j r_kj dt_ij (the outgoing form),  dr_kj = sum_i l_ki dt_ij (mixed)
-    rc = contract_impl(right, dtri, dleft, nullptr, 0, 0, kC, B, N, 0, N, N, B200_TRIMUL_OUTGOING, status, cuda_stream);
+    rc = contract_impl(right, dtri, dleft, nullptr, 0, 0, kC, B, N, 0, N, N, B200_TRIMUL_OUTGOING, status, cuda_stream, 0, any_n);
     if (rc != B200_TRIMUL_OK) return rc;
-    return contract_impl(left, dtri, dright, nullptr, 0, 0, kC, B, N, 0, N, N, kDirMixed, status, cuda_stream);
+    return contract_impl(left, dtri, dright, nullptr, 0, 0, kC, B, N, 0, N, N, kDirMixed, status, cuda_stream, 0, any_n);
   }
   return B200_TRIMUL_E_SHAPE;
+}
+
+int b200_trimul_contract_backward(const void* dtri, const void* left, const void* right, void* dleft, void* dright, int B,
+                                  int N, int direction, int* status, void* cuda_stream) {
+  return contract_backward_impl(dtri, left, right, dleft, dright, B, N, direction, status, cuda_stream, false);
 }
 
 int b200_trimul_contract_partial(const void* left, const void* right, void* tri_partial, int B, int N, int k_rows,
@@ -870,11 +886,12 @@ int b200_trimul_reduce_partials(void* tri, const void* const* partials, int n_sr
 // `groups` = 1: tri is [B*rows][128][N]. groups = P (B = 1): tri is [P][rows][128/P][N], channel group g of every row
 // in slab g (what the channel-sharded contraction of GPU g stored there).
 static int epilogue_impl(const void* tri, const void* z, const void* packed, void* y, int B, int N, int rows, int groups,
-                         float eps_in, float eps_out, int residual, int* status, void* cuda_stream, int d_pair = kC) {
+                         float eps_in, float eps_out, int residual, int* status, void* cuda_stream, int d_pair = kC,
+                         bool any_n = false) {
   if (!tri || !z || !packed || !y || !status) return B200_TRIMUL_E_NULL;
   if (d_pair != kC && d_pair != 64) return B200_TRIMUL_E_UNSUPPORTED;
   if (groups < 1 || groups > 8 || kC % groups != 0 || (groups > 1 && B != 1)) return B200_TRIMUL_E_SHAPE;
-  int rc = check_bn(B, N);
+  int rc = check_bn(B, N, any_n);
   if (rc != B200_TRIMUL_OK) return rc;
   if (rows < 1 || rows > N) return B200_TRIMUL_E_SHAPE;
   if (!aligned(tri, 16) || !aligned(z, 16) || !aligned(y, 16) || !aligned(packed, 1024)) return B200_TRIMUL_E_ALIGN;
@@ -888,7 +905,8 @@ static int epilogue_impl(const void* tri, const void* z, const void* packed, voi
   {
     const uint64_t cg = static_cast<uint64_t>(kC / groups);
     const uint64_t dims[4] = {n64, cg, static_cast<uint64_t>(groups), nrows};
-    const uint64_t strides[3] = {n64 * 2, nrows * cg * n64 * 2, cg * n64 * 2};
+    const uint64_t ld = static_cast<uint64_t>(plane_pitch(N));
+    const uint64_t strides[3] = {ld * 2, nrows * cg * ld * 2, cg * ld * 2};
     const uint32_t box[4] = {64, static_cast<uint32_t>(cg), static_cast<uint32_t>(groups), 1};
     rc = make_map(&map_t, tri, 4, dims, strides, box);
     if (rc != B200_TRIMUL_OK) return rc;
@@ -966,13 +984,13 @@ static int launch_epilogue_wide(const CUtensorMap& mt0, const CUtensorMap& mt1, 
 
 extern "C" {
 
-int b200_trimul_epilogue_wide(const void* tri, const void* tri_in, const void* z, const void* packed,
+static int epilogue_wide_impl(const void* tri, const void* tri_in, const void* z, const void* packed,
                               const void* packed_in, const void* drop_scale, void* y, int B, int N, int rows,
-                              float eps_in, float eps_out, int residual, int* status, void* cuda_stream) {
+                              float eps_in, float eps_out, int residual, int* status, void* cuda_stream, bool any_n) {
   if (!tri || !z || !packed || !y || !status) return B200_TRIMUL_E_NULL;
   const bool bidir = tri_in != nullptr;
   if (bidir && !packed_in) return B200_TRIMUL_E_NULL;
-  int rc = check_bn(B, N);
+  int rc = check_bn(B, N, any_n);
   if (rc != B200_TRIMUL_OK) return rc;
   if (rows < 1 || rows > N) return B200_TRIMUL_E_SHAPE;
   if (!aligned(tri, 16) || !aligned(z, 16) || !aligned(y, 16) || !aligned(packed, 1024)) return B200_TRIMUL_E_ALIGN;
@@ -986,7 +1004,8 @@ int b200_trimul_epilogue_wide(const void* tri, const void* tri_in, const void* z
   CUtensorMap map_t0, map_t1, map_z, map_y, map_w0, map_w1;
   {
     const uint64_t dims[3] = {n64, static_cast<uint64_t>(kC), nrows};
-    const uint64_t strides[2] = {n64 * 2, static_cast<uint64_t>(kC) * n64 * 2};
+    const uint64_t ld = static_cast<uint64_t>(plane_pitch(N));
+    const uint64_t strides[2] = {ld * 2, static_cast<uint64_t>(kC) * ld * 2};
     const uint32_t box[3] = {64, 64, 1};  // one chunk half: 64 positions of 64 channels
     rc = make_map(&map_t0, tri, 3, dims, strides, box);
     if (rc != B200_TRIMUL_OK) return rc;
@@ -1032,21 +1051,30 @@ int b200_trimul_epilogue_wide(const void* tri, const void* tri_in, const void* z
   return launch_epilogue_wide<2, false>(map_t0, map_t1, map_z, map_y, map_w0, map_w1, p, info, stream);
 }
 
-int b200_trimul_forward_ex(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
-                           const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,
+int b200_trimul_epilogue_wide(const void* tri, const void* tri_in, const void* z, const void* packed,
+                              const void* packed_in, const void* drop_scale, void* y, int B, int N, int rows,
+                              float eps_in, float eps_out, int residual, int* status, void* cuda_stream) {
+  return epilogue_wide_impl(tri, tri_in, z, packed, packed_in, drop_scale, y, B, N, rows, eps_in, eps_out, residual, status,
+                            cuda_stream, false);
+}
+
+static int forward_impl(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
+                        const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,
                            const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
                            const void* const* bias_opt, const uint8_t* token_mask, const uint8_t* pair_mask,
                            const void* drop_scale, void* y, void* workspace, size_t workspace_bytes, int B, int N,
                            int d_pair, int d_hidden, int direction, float eps_in, float eps_out, int residual,
-                           void* cuda_stream) {
+                           void* cuda_stream, bool any_n) {
   if (!z || !y || !workspace) return B200_TRIMUL_E_NULL;
   size_t need = 0;
-  int rc = b200_trimul_workspace_bytes(B, N, d_pair, d_hidden, direction, &need);
+  if (any_n && (N < 1 || N > 0x7FFFFFFF / 128)) return B200_TRIMUL_E_SHAPE;
+  const int ld = any_n ? plane_pitch(N) : N;  // the workspace is the one of N rounded up to a multiple of 8
+  int rc = b200_trimul_workspace_bytes(B, ld, d_pair, d_hidden, direction, &need);
   if (rc != B200_TRIMUL_OK) return rc;
   if (workspace_bytes < need) return B200_TRIMUL_E_WORKSPACE;
   if (!aligned(workspace, 1024)) return B200_TRIMUL_E_ALIGN;
   size_t off[5];
-  rc = b200_trimul_workspace_layout(B, N, off);
+  rc = b200_trimul_workspace_layout(B, ld, off);
   if (rc != B200_TRIMUL_OK) return rc;
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   int* status = reinterpret_cast<int*>(ws + off[0]);
@@ -1059,6 +1087,15 @@ int b200_trimul_forward_ex(const void* z, const void* w_left, const void* w_left
   int has_bias = 0;
   if (bias_opt != nullptr)
     for (int i = 0; i < 4; ++i) has_bias |= bias_opt[i] != nullptr;
+  auto prologue = [&](const void* pk) {
+    void* l[1] = {left};
+    void* r[1] = {right};
+    return prologue_impl(z, pk, token_mask, pair_mask, l, 1, r, 1, kLocal, B, N, 0, N, eps_in, has_bias, status, cuda_stream,
+                         d_pair, any_n);
+  };
+  auto contract = [&](void* dst, int dir) {
+    return contract_impl(left, right, dst, nullptr, 0, 0, kC, B, N, 0, N, N, dir, status, cuda_stream, 0, any_n);
+  };
   if (d_pair == 64) {
     // Narrow pair stacks: 64 input channels, 128 contracted channels in one [rows, 128, N] tensor. The parameter
     // shapes are to_left / to_left_gate / to_right / to_right_gate [128, 64], ln_out [128], to_out [64, 128],
@@ -1066,66 +1103,85 @@ int b200_trimul_forward_ex(const void* z, const void* w_left, const void* w_left
     if (drop_scale != nullptr) return B200_TRIMUL_E_UNSUPPORTED;
     if (!w_left || !w_left_gate || !w_right || !w_right_gate || !w_gate || !w_out) return B200_TRIMUL_E_NULL;
     const void* w[6] = {w_left, w_left_gate, w_right, w_right_gate, w_out, w_gate};
-    const int ld[6] = {64, 64, 64, 64, kC, 64};
+    const int w_ld[6] = {64, 64, 64, 64, kC, 64};
     const float* bias[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     if (bias_opt != nullptr) {
       for (int i = 0; i < 4; ++i) bias[i] = static_cast<const float*>(bias_opt[i]);
       bias[5] = static_cast<const float*>(bias_opt[4]);
       bias[4] = static_cast<const float*>(bias_opt[5]);
     }
-    rc = pack_impl(w, ld, weight_dtype, ln_in_w, ln_in_b, ln_out_w, ln_out_b, bias, packed, cuda_stream, 64);
+    rc = pack_impl(w, w_ld, weight_dtype, ln_in_w, ln_in_b, ln_out_w, ln_out_b, bias, packed, cuda_stream, 64);
     if (rc != B200_TRIMUL_OK) return rc;
-    void* l[1] = {left};
-    void* r[1] = {right};
-    rc = prologue_impl(z, packed, token_mask, pair_mask, l, 1, r, 1, kLocal, B, N, 0, N, eps_in, has_bias, status,
-                       cuda_stream, 64);
+    rc = prologue(packed);
     if (rc != B200_TRIMUL_OK) return rc;
     if (direction == B200_TRIMUL_BIDIRECTIONAL) {
-      const size_t half = static_cast<size_t>(64) * N * 2;  // bytes from channel 0 to channel 64 of a pair row
-      rc = contract_impl(left, right, tri, nullptr, 0, 0, 64, B, N, 0, N, N, B200_TRIMUL_OUTGOING, status, cuda_stream, kC);
+      const size_t half = static_cast<size_t>(64) * ld * 2;  // bytes from channel 0 to channel 64 of a pair row
+      rc = contract_impl(left, right, tri, nullptr, 0, 0, 64, B, N, 0, N, N, B200_TRIMUL_OUTGOING, status, cuda_stream, kC,
+                         any_n);
       if (rc != B200_TRIMUL_OK) return rc;
       rc = contract_impl(static_cast<uint8_t*>(left) + half, static_cast<uint8_t*>(right) + half,
                          static_cast<uint8_t*>(tri) + half, nullptr, 0, 0, 64, B, N, 0, N, N, B200_TRIMUL_INCOMING, status,
-                         cuda_stream, kC);
+                         cuda_stream, kC, any_n);
     } else {
-      rc = b200_trimul_contract(left, right, tri, B, N, 0, N, direction, status, cuda_stream);
+      rc = contract(tri, direction);
     }
     if (rc != B200_TRIMUL_OK) return rc;
-    return epilogue_impl(tri, z, packed, y, B, N, N, 1, eps_in, eps_out, residual, status, cuda_stream, 64);
+    return epilogue_impl(tri, z, packed, y, B, N, N, 1, eps_in, eps_out, residual, status, cuda_stream, 64, any_n);
   }
   if (direction == B200_TRIMUL_BIDIRECTIONAL) {
     // workspace tail: second tri tensor, then the second packed block
-    const size_t plane = plane_tensor_bytes(B, N, N);
+    const size_t plane = plane_tensor_bytes(B, ld, ld);
     void* tri_in = ws + off[4] + plane;
     void* packed_in = ws + off[4] + 2 * plane;
     rc = b200_trimul_pack_weights_bidir(w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w,
                                         ln_in_b, ln_out_w, ln_out_b, bias_opt, packed, packed_in, cuda_stream);
     if (rc != B200_TRIMUL_OK) return rc;
-    rc = b200_trimul_prologue(z, packed, token_mask, pair_mask, left, right, B, N, 0, N, eps_in, has_bias, status,
-                              cuda_stream);
+    rc = prologue(packed);
     if (rc != B200_TRIMUL_OK) return rc;
-    rc = b200_trimul_contract(left, right, tri, B, N, 0, N, B200_TRIMUL_OUTGOING, status, cuda_stream);
+    rc = contract(tri, B200_TRIMUL_OUTGOING);
     if (rc != B200_TRIMUL_OK) return rc;
-    rc = b200_trimul_prologue(z, packed_in, token_mask, pair_mask, left, right, B, N, 0, N, eps_in, has_bias, status,
-                              cuda_stream);
+    rc = prologue(packed_in);
     if (rc != B200_TRIMUL_OK) return rc;
-    rc = b200_trimul_contract(left, right, tri_in, B, N, 0, N, B200_TRIMUL_INCOMING, status, cuda_stream);
+    rc = contract(tri_in, B200_TRIMUL_INCOMING);
     if (rc != B200_TRIMUL_OK) return rc;
-    return b200_trimul_epilogue_wide(tri, tri_in, z, packed, packed_in, drop_scale, y, B, N, N, eps_in, eps_out, residual,
-                                     status, cuda_stream);
+    return epilogue_wide_impl(tri, tri_in, z, packed, packed_in, drop_scale, y, B, N, N, eps_in, eps_out, residual,
+                                     status, cuda_stream, any_n);
   }
   rc = b200_trimul_pack_weights(w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w,
                                 ln_in_b, ln_out_w, ln_out_b, bias_opt, packed, cuda_stream);
   if (rc != B200_TRIMUL_OK) return rc;
-  rc = b200_trimul_prologue(z, packed, token_mask, pair_mask, left, right, B, N, 0, N, eps_in, has_bias, status,
-                            cuda_stream);
+  rc = prologue(packed);
   if (rc != B200_TRIMUL_OK) return rc;
-  rc = b200_trimul_contract(left, right, tri, B, N, 0, N, direction, status, cuda_stream);
+  rc = contract(tri, direction);
   if (rc != B200_TRIMUL_OK) return rc;
   if (drop_scale != nullptr)
-    return b200_trimul_epilogue_wide(tri, nullptr, z, packed, nullptr, drop_scale, y, B, N, N, eps_in, eps_out, residual,
-                                     status, cuda_stream);
-  return b200_trimul_epilogue(tri, z, packed, y, B, N, N, eps_in, eps_out, residual, status, cuda_stream);
+    return epilogue_wide_impl(tri, nullptr, z, packed, nullptr, drop_scale, y, B, N, N, eps_in, eps_out, residual,
+                                     status, cuda_stream, any_n);
+  return epilogue_impl(tri, z, packed, y, B, N, N, 1, eps_in, eps_out, residual, status, cuda_stream, kC, any_n);
+}
+
+int b200_trimul_forward_ex(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
+                           const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,
+                           const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
+                           const void* const* bias_opt, const uint8_t* token_mask, const uint8_t* pair_mask,
+                           const void* drop_scale, void* y, void* workspace, size_t workspace_bytes, int B, int N,
+                           int d_pair, int d_hidden, int direction, float eps_in, float eps_out, int residual,
+                           void* cuda_stream) {
+  return forward_impl(z, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
+                      ln_out_b, bias_opt, token_mask, pair_mask, drop_scale, y, workspace, workspace_bytes, B, N, d_pair,
+                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, false);
+}
+
+int b200_trimul_forward_any(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
+                           const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,
+                           const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
+                           const void* const* bias_opt, const uint8_t* token_mask, const uint8_t* pair_mask,
+                           const void* drop_scale, void* y, void* workspace, size_t workspace_bytes, int B, int N,
+                           int d_pair, int d_hidden, int direction, float eps_in, float eps_out, int residual,
+                           void* cuda_stream) {
+  return forward_impl(z, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
+                      ln_out_b, bias_opt, token_mask, pair_mask, drop_scale, y, workspace, workspace_bytes, B, N, d_pair,
+                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, true);
 }
 
 int b200_trimul_forward(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,

@@ -34,6 +34,11 @@ def _require_cuda(t: torch.Tensor, name: str) -> None:
         raise RuntimeError(f"{name} must be a CUDA tensor: this path has no CPU implementation")
 
 
+def aligned16(t: torch.Tensor) -> torch.Tensor:
+    """``t``, or a copy of it when its storage does not start on the 16 bytes that the kernels' copies need."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def aligned_empty(nbytes: int, device: torch.device, align: int = 1024) -> torch.Tensor:
     """uint8 buffer of ``nbytes`` whose data pointer is ``align``-byte aligned."""
     raw = torch.empty(nbytes + align, dtype=torch.uint8, device=device)
@@ -459,6 +464,18 @@ def trimul_forward(
     ``check=True`` synchronises and raises if a device-side wait gave up. ``weights`` is an already validated
     :class:`_Weights` of the same parameters (it only holds pointers: the values are packed on the GPU in every call).
     """
+    return _forward(z, params, mask, outgoing, eps_in, eps_out, pair_mask, residual, biases, workspace, out, check, weights,
+                    drop_scale, any_n=False)
+
+
+def _pitch(N: int) -> int:
+    """Columns between consecutive channels of a pair row in the intermediates: N rounded up to a multiple of 8."""
+    return (N + 7) // 8 * 8
+
+
+def _forward(z, params, mask, outgoing, eps_in, eps_out, pair_mask, residual, biases, workspace, out, check, weights,
+             drop_scale, any_n):
+    """:func:`trimul_forward`; ``any_n`` takes every N (``b200_trimul_forward_any``) instead of multiples of 8."""
     B, N = _check_z(z, widths=(D, 64))
     if z.shape[1] != N:
         raise RuntimeError(f"pair tensor must be square in its token dims, got {tuple(z.shape)}")
@@ -475,7 +492,7 @@ def trimul_forward(
         if drop_scale.numel() != B * N * D or drop_scale.shape[-1] != D or drop_scale.shape[0] != B:  # d_pair = 128 here
             raise RuntimeError(f"drop_scale must be [B, 1, N, {D}] = ({B}, 1, {N}, {D}), got {tuple(drop_scale.shape)}")
         ds = drop_scale.detach().to(torch.bfloat16).contiguous()
-    need = workspace_bytes(B, N, outgoing, C)
+    need = workspace_bytes(B, _pitch(N) if any_n else N, outgoing, C)
     if workspace is None:
         workspace = aligned_empty(need, dev)
     elif workspace.numel() * workspace.element_size() < need:
@@ -489,7 +506,8 @@ def trimul_forward(
     if pm is not None and tuple(pm.shape) != (B, N, N):
         raise RuntimeError(f"pair mask must be [B, N, N], got {tuple(pm.shape)}")
     with torch.cuda.device(dev):
-        rc = _lib.load().b200_trimul_forward_ex(
+        lib = _lib.load()
+        rc = (lib.b200_trimul_forward_any if any_n else lib.b200_trimul_forward_ex)(
             _ptr(z),
             *[_ptr(t) for t in w.weights],
             w.dtype_code,
@@ -548,6 +566,13 @@ def trimul_backward(
     Returns ``(dz bf16, the input's shape, grads)`` with ``grads`` a dict of fp32 tensors of the parameters' shapes under the
     parameter keys.
     """
+    return _backward(dy, z, params, forward_workspace, mask, outgoing, eps_in, eps_out, pair_mask, residual, biases, drop_scale,
+                     workspace, check, any_n=False)
+
+
+def _backward(dy, z, params, forward_workspace, mask, outgoing, eps_in, eps_out, pair_mask, residual, biases, drop_scale,
+              workspace, check, any_n):
+    """:func:`trimul_backward`; ``any_n`` takes every N (``b200_trimul_backward_any``, after the same kind of forward)."""
     B, N = _check_z(z, widths=(D, 64))
     C = int(z.shape[3])
     if z.shape[1] != N:
@@ -568,12 +593,12 @@ def trimul_backward(
         if drop_scale.numel() != B * N * D or drop_scale.shape[-1] != D or drop_scale.shape[0] != B:
             raise RuntimeError(f"drop_scale must be [B, 1, N, {D}], got {tuple(drop_scale.shape)}")
         ds = drop_scale.detach().to(device=dev, dtype=torch.bfloat16).contiguous()
-    need = backward_workspace_bytes(B, N, outgoing)
+    need = backward_workspace_bytes(B, _pitch(N) if any_n else N, outgoing)
     if workspace is None:
         workspace = aligned_empty(need, dev)
     elif workspace.numel() * workspace.element_size() < need:
         raise RuntimeError(f"workspace too small: {workspace.numel() * workspace.element_size()} < {need}")
-    if forward_workspace.numel() * forward_workspace.element_size() < workspace_bytes(B, N, outgoing, C):
+    if forward_workspace.numel() * forward_workspace.element_size() < workspace_bytes(B, _pitch(N) if any_n else N, outgoing, C):
         raise RuntimeError("forward_workspace is smaller than the forward's workspace for this shape")
     tm = as_mask_u8(mask, dev)
     pm = as_mask_u8(pair_mask, dev)
@@ -584,7 +609,8 @@ def trimul_backward(
     dln = [torch.empty(n, dtype=torch.float32, device=dev) for n in (C, C, wide, wide)]
     dw_arr = (c_void_p * 6)(*[t.data_ptr() for t in dws])
     with torch.cuda.device(dev):
-        rc = _lib.load().b200_trimul_backward(
+        lib = _lib.load()
+        rc = (lib.b200_trimul_backward_any if any_n else lib.b200_trimul_backward)(
             _ptr(dy), _ptr(z), *[_ptr(t) for t in w.weights], w.dtype_code, *[_ptr(t) for t in w.lns], w.bias_array,
             _ptr(tm), _ptr(pm), _ptr(ds), _ptr(forward_workspace), _ptr(dz), dw_arr, *[_ptr(t) for t in dln],
             _ptr(workspace), workspace.numel() * workspace.element_size(), B, N, C, w.d_hidden, _direction(outgoing), float(eps_in),

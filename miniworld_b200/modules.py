@@ -241,76 +241,53 @@ class TriangleMultiplication(nn.Module):
             z = z.to(torch.bfloat16)
         z = z.contiguous()
         B, N = int(z.shape[0]), int(z.shape[1])
-        pad = (-N) % 8
+        ragged = N % 8 != 0
         scale = None
         if self.training and self.p_drop > 0.0:
             scale = self._make_drop_row_scale(z, self.p_drop).to(device=z.device, dtype=torch.bfloat16)
-            if pad:
-                sp = scale.new_zeros(B, 1, N + pad, self.d_pair)
-                sp[:, :, :N] = scale
-                scale = sp
-        if pad:
-            # pad with masked tokens: masked rows/columns of left/right are zero, so the crop is exact
-            zp = z.new_zeros(B, N + pad, N + pad, self.d_pair)
-            zp[:, :N, :N] = z
-            tm = torch.ones(B, N, dtype=torch.bool, device=z.device) if token_mask is None else token_mask.to(z.device) != 0
-            tmp = torch.zeros(B, N + pad, dtype=torch.bool, device=z.device)
-            tmp[:, :N] = tm
-            pmp = None
+        if ragged:
+            # any length runs as it is; masks and scale may be given in a form that broadcasts to the batch
+            z = F_.aligned16(z)
+            if token_mask is not None:
+                token_mask = torch.broadcast_to(token_mask.to(z.device), (B, N))
             if pair_mask is not None:
-                pmp = torch.zeros(B, N + pad, N + pad, dtype=torch.bool, device=z.device)
-                pmp[:, :N, :N] = pair_mask.to(z.device) != 0
-            z, token_mask, pair_mask = zp, tmp, pmp
-        Np = N + pad
+                pair_mask = torch.broadcast_to(pair_mask.to(z.device), (B, N, N))
+            if scale is not None:
+                scale = F_.aligned16(torch.broadcast_to(scale, (B, 1, N, self.d_pair)).contiguous())
         with torch.no_grad():
-            y = F_.trimul_forward(
-                z,
-                self._params(),
-                token_mask,
-                outgoing=self._direction(),
-                eps_in=float(self.ln_pair.eps),
-                eps_out=float(self.ln_out.eps),
-                pair_mask=pair_mask,
-                residual=self.residual,
-                biases=self._biases,
-                workspace=self._get_workspace(B, Np, z.device),
-                check=self.check_status,
-                weights=self._weights(z.device),
-                drop_scale=scale,
+            y = F_._forward(
+                z, self._params(), token_mask, self._direction(), float(self.ln_pair.eps), float(self.ln_out.eps), pair_mask,
+                self.residual, self._biases, self._get_workspace(B, F_._pitch(N) if ragged else N, z.device), None,
+                self.check_status, self._weights(z.device), scale, ragged,
             )
-        if pad:
-            y = y[:, :N, :N].contiguous()
         return y if in_dtype == torch.bfloat16 else y.to(in_dtype)
 
     def _run_train(self, pair: torch.Tensor, token_mask, pair_mask) -> torch.Tensor:
         """Differentiable forward (:mod:`miniworld_b200.training`): the stage tensors of this call are kept for the
-        backward in a workspace of their own; padding, cropping and dtype casts are ordinary differentiable ops."""
-        from .training import trimul_train
+        backward in a workspace of their own; dtype casts are ordinary differentiable ops."""
+        from .training import _trimul_train
 
         in_dtype = pair.dtype
         z = pair if pair.dtype == torch.bfloat16 else pair.to(torch.bfloat16)
         z = z.contiguous()
         B, N = int(z.shape[0]), int(z.shape[1])
-        pad = (-N) % 8
+        ragged = N % 8 != 0
         scale = None
         if self.training and self.p_drop > 0.0:
-            scale = self._make_drop_row_scale(z, self.p_drop).to(device=z.device, dtype=torch.bfloat16)
-            if pad:
-                scale = nn.functional.pad(scale, (0, 0, 0, pad))
-            scale = scale.contiguous()
-        if pad:
-            z = nn.functional.pad(z, (0, 0, 0, pad, 0, pad))
-            tm = torch.ones(B, N, dtype=torch.bool, device=z.device) if token_mask is None else token_mask.to(z.device) != 0
-            token_mask = nn.functional.pad(tm, (0, pad))
+            scale = self._make_drop_row_scale(z, self.p_drop).to(device=z.device, dtype=torch.bfloat16).contiguous()
+        if ragged:
+            # any length runs as it is. What the backward reads is this call's own (a caller may change the pair tensor or
+            # the masks in place between the two passes of such a length)
+            if z is pair:
+                z = z.clone()
+            if token_mask is not None:
+                token_mask = token_mask.to(z.device) != 0
             if pair_mask is not None:
-                pair_mask = nn.functional.pad(pair_mask.to(z.device) != 0, (0, pad, 0, pad))
-        y = trimul_train(
-            z, self._params(), token_mask, outgoing=self._direction(), eps_in=float(self.ln_pair.eps),
-            eps_out=float(self.ln_out.eps), pair_mask=pair_mask, residual=self.residual, biases=self._biases,
-            drop_scale=scale, check=self.check_status,
-        )
-        if pad:
-            y = y[:, :N, :N]
+                pair_mask = pair_mask.to(z.device) != 0
+            if scale is not None:
+                scale = F_.aligned16(scale)
+        y = _trimul_train(z, self._params(), token_mask, self._direction(), float(self.ln_pair.eps), float(self.ln_out.eps),
+                          pair_mask, self.residual, self._biases, scale, self.check_status, ragged)
         return y if in_dtype == torch.bfloat16 else y.to(in_dtype)
 
     def forward(self, pair: torch.Tensor, mask: Optional[torch.Tensor] = None) -> torch.Tensor:

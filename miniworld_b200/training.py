@@ -29,18 +29,18 @@ _PARAM_KEYS = (
 
 class TriMulFunction(torch.autograd.Function):
     """``y = TriMulFunction.apply(z, token_mask, pair_mask, drop_scale, cfg, *params)``; ``cfg`` is a dict with
-    ``outgoing``, ``eps_in``, ``eps_out``, ``residual``, ``biases``, ``check``; ``params`` in ``_PARAM_KEYS`` order."""
+    ``outgoing``, ``eps_in``, ``eps_out``, ``residual``, ``biases``, ``check``, ``any_n``; ``params`` in ``_PARAM_KEYS``
+    order."""
 
     @staticmethod
     def forward(ctx, z, token_mask, pair_mask, drop_scale, cfg, *params):
         B, N = int(z.shape[0]), int(z.shape[1])
         p = {k: v.detach() for k, v in zip(_PARAM_KEYS, params)}
-        ws = F_.aligned_empty(F_.workspace_bytes(B, N, cfg["outgoing"], int(z.shape[3])), z.device)  # kept until the backward
-        y = F_.trimul_forward(
-            z.detach(), p, token_mask, outgoing=cfg["outgoing"], eps_in=cfg["eps_in"], eps_out=cfg["eps_out"],
-            pair_mask=pair_mask, residual=cfg["residual"], biases=cfg["biases"], workspace=ws, check=cfg["check"],
-            drop_scale=drop_scale,
-        )
+        any_n = cfg["any_n"]
+        ws = F_.aligned_empty(F_.workspace_bytes(B, F_._pitch(N) if any_n else N, cfg["outgoing"], int(z.shape[3])),
+                              z.device)  # kept until the backward
+        y = F_._forward(z.detach(), p, token_mask, cfg["outgoing"], cfg["eps_in"], cfg["eps_out"], pair_mask, cfg["residual"],
+                        cfg["biases"], ws, None, cfg["check"], None, drop_scale, any_n)
         ctx.save_for_backward(z, *params)
         ctx.ws, ctx.cfg = ws, cfg
         ctx.token_mask, ctx.pair_mask, ctx.drop_scale = token_mask, pair_mask, drop_scale
@@ -55,11 +55,12 @@ class TriMulFunction(torch.autograd.Function):
             raise RuntimeError("the forward's stage tensors were released by the first backward of this call "
                                "(a second backward through the same forward is not supported)")
         B, N = int(z.shape[0]), int(z.shape[1])
-        dz, grads = F_.trimul_backward(
-            dy.to(torch.bfloat16), z.detach(), {k: v.detach() for k, v in zip(_PARAM_KEYS, params)}, ctx.ws, ctx.token_mask,
-            outgoing=cfg["outgoing"], eps_in=cfg["eps_in"], eps_out=cfg["eps_out"], pair_mask=ctx.pair_mask,
-            residual=cfg["residual"], biases=cfg["biases"], drop_scale=ctx.drop_scale, check=cfg["check"],
-        )
+        dy = dy.to(torch.bfloat16)
+        if cfg["any_n"]:
+            dy = F_.aligned16(dy.contiguous())  # (a gradient that is a slice of a larger tensor)
+        dz, grads = F_._backward(dy, z.detach(), {k: v.detach() for k, v in zip(_PARAM_KEYS, params)}, ctx.ws, ctx.token_mask,
+                                 cfg["outgoing"], cfg["eps_in"], cfg["eps_out"], ctx.pair_mask, cfg["residual"],
+                                 cfg["biases"], ctx.drop_scale, None, cfg["check"], cfg["any_n"])
         ctx.ws = None
         out = [dz.to(z.dtype) if ctx.needs_input_grad[0] else None, None, None, None, None]
         for i, (k, prm) in enumerate(zip(_PARAM_KEYS, params)):
@@ -74,8 +75,14 @@ def trimul_train(z: torch.Tensor, params: dict, token_mask: Optional[torch.Tenso
                  check: bool = False) -> torch.Tensor:
     """Differentiable forward: ``z`` [B, N, N, 128] bf16 (N a multiple of 8) and the ten parameters may require grad;
     ``outgoing=None`` is the bidirectional module (parameters of its wider shapes)."""
+    return _trimul_train(z, params, token_mask, outgoing, eps_in, eps_out, pair_mask, residual, biases, drop_scale, check,
+                         any_n=False)
+
+
+def _trimul_train(z, params, token_mask, outgoing, eps_in, eps_out, pair_mask, residual, biases, drop_scale, check, any_n):
+    """:func:`trimul_train`; ``any_n`` takes every N."""
     cfg = {"outgoing": None if outgoing is None else bool(outgoing), "eps_in": float(eps_in), "eps_out": float(eps_out), "residual": bool(residual),
-           "biases": biases, "check": bool(check)}
+           "biases": biases, "check": bool(check), "any_n": bool(any_n)}
     return TriMulFunction.apply(z, token_mask, pair_mask, drop_scale, cfg, *[params[k] for k in _PARAM_KEYS])
 
 

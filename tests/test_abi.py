@@ -96,3 +96,15 @@ def test_backward_entry_points_validate_before_any_cuda_call(lib):
                                   1, 384, 128, 128, 1, 1e-5, 1e-5, 1, None)
     assert rc == -1
     assert lib.b200_trimul_contract_backward(None, None, None, None, None, 1, 384, 1, None, None) == -1
+
+
+def test_any_length_entry_points_validate_before_any_cuda_call(lib):
+    import ctypes as ct
+
+    buf = ct.create_string_buffer(4096)
+    a = (ct.addressof(buf) + 1023) // 1024 * 1024  # never read: every call below is refused on its sizes
+    head, tail = [a] * 7 + [0] + [a] * 4 + [None, None, None, None, a, a], [128, 128, 1, 1e-5, 1e-5, 1, None]
+    assert lib.b200_trimul_forward_any(*([None] * 7), 0, *([None] * 4), None, None, None, None, None, None, 0, 1, 203, *tail) == -1
+    for n, code in ((0, -2), (-3, -2), (2**31 - 1, -2), (203, -5)):
+        assert lib.b200_trimul_forward_any(*head, 8, 1, n, *tail) == code, n
+    assert lib.b200_trimul_forward_ex(*head, 8, 1, 203, *tail) == -3
