@@ -1177,42 +1177,58 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
 }
 
 // ------------------------------------------------------------------------------------------------ small kernels
-// Largest |dy| (bf16) as the bits of a non-negative float: `amax_bits` must be zero before the launch.
-__global__ void __launch_bounds__(256) bwd_amax_kernel(const uint4* dy, size_t n_chunks, unsigned int* amax_bits) {
+// Largest |dy| (bf16) over the blocks `block` of `blocks` of a launch, and from it the scale of the gradient tiles:
+// scale[0] = c = the power of two that brings max |dy| into [8, 16), scale[1] = 1 / c (c = 1 for a zero gradient). `words`
+// (zeroed before the launch): [0] the maximum as the bits of a non-negative float, [1] blocks that have arrived; the last
+// one to arrive forms the scale, so no launch of its own is needed for it.
+__device__ __forceinline__ void amax_and_scale(const uint4* dy, size_t n_chunks, int block, int blocks, unsigned int* words,
+                                               float* scale) {
   // |x| of a bf16 pair compares like the unsigned integer of its bits with the sign cleared, so the maximum is taken on
-  // the packed halves; four loads per thread in flight
+  // the packed halves; eight loads per thread in flight
+  constexpr int kFlight = 8;
   uint32_t mx = 0u;
   auto fold = [&](const uint4& v) {
     const uint32_t w[4] = {v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu, v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu};
 #pragma unroll
     for (int t = 0; t < 4; ++t) mx = __vmaxu2(mx, w[t]);
   };
-  const size_t step = static_cast<size_t>(gridDim.x) * blockDim.x;
-  size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
-  for (; i + 3 * step < n_chunks; i += 4 * step) {
-    const uint4 v0 = __ldg(dy + i), v1 = __ldg(dy + i + step), v2 = __ldg(dy + i + 2 * step), v3 = __ldg(dy + i + 3 * step);
-    fold(v0), fold(v1), fold(v2), fold(v3);
+  const size_t step = static_cast<size_t>(blocks) * blockDim.x;
+  for (size_t i = block * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n_chunks; i += kFlight * step) {
+    uint4 v[kFlight];
+#pragma unroll
+    for (int u = 0; u < kFlight; ++u) v[u] = i + u * step < n_chunks ? __ldg(dy + i + u * step) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int u = 0; u < kFlight; ++u) fold(v[u]);
   }
-  for (; i < n_chunks; i += step) fold(__ldg(dy + i));
   const uint32_t top = (mx >> 16) > (mx & 0xFFFFu) ? (mx >> 16) : (mx & 0xFFFFu);
-  float m = __uint_as_float(top << 16);  // NaN or infinity bits stay above 3e38 and are rejected below
+  float m = __uint_as_float(top << 16);
+  if (!(m <= 3.0e38f)) m = 0.f;  // infinities and NaN do not set the scale
+  __shared__ unsigned int block_max;
+  if (threadIdx.x == 0) block_max = 0u;
+  __syncthreads();
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, off));
-  if ((threadIdx.x & 31) == 0 && m > 0.f && m <= 3.0e38f) atomicMax(amax_bits, __float_as_uint(m));
-}
-// scale[0] = c = the power of two that brings max |dy| into [8, 16), scale[1] = 1 / c (c = 1 for a zero gradient)
-__global__ void bwd_scale_kernel(const unsigned int* amax_bits, float* scale) {
-  const float amax = __uint_as_float(*amax_bits);
-  float c = 1.0f;
-  if (amax > 0.f) {
-    int e = 0;
-    frexpf(amax, &e);           // amax = f * 2^e, f in [0.5, 1)
-    e = 4 - e;                  // amax * 2^(4 - e) in [8, 16)
-    e = e > 100 ? 100 : (e < -100 ? -100 : e);
-    c = ldexpf(1.0f, e);
+  if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(&block_max, __float_as_uint(m));
+  __syncthreads();
+  // one word-sized atomic per block: they all go to one address
+  if (threadIdx.x == 0) {
+    if (block_max != 0u) atomicMax(words, block_max);
+    __threadfence();
   }
-  scale[0] = c;
-  scale[1] = 1.0f / c;
+  if (threadIdx.x == 0 && atomicAdd(words + 1, 1u) == static_cast<unsigned int>(blocks) - 1u) {
+    __threadfence();
+    const float amax = __uint_as_float(atomicMax(words, 0u));
+    float c = 1.0f;
+    if (amax > 0.f) {
+      int e = 0;
+      frexpf(amax, &e);           // amax = f * 2^e, f in [0.5, 1)
+      e = 4 - e;                  // amax * 2^(4 - e) in [8, 16)
+      e = e > 100 ? 100 : (e < -100 ? -100 : e);
+      c = ldexpf(1.0f, e);
+    }
+    scale[0] = c;
+    scale[1] = 1.0f / c;
+  }
 }
 
 // Weights for the backward kernels: all six matrices (PackArgs order: left, left gate, right, right gate, out, gate)
@@ -1220,8 +1236,7 @@ __global__ void bwd_scale_kernel(const unsigned int* amax_bits, float* scale) {
 // d[m][r] = sum_k W[r][k] beta[k] + bias[m][r] (fp32) behind them. One warp per matrix row.
 constexpr size_t kBwdPackedD = 6 * 32768;
 constexpr size_t kBwdPackedBytes = kBwdPackedD + 3072;  // 199680, a multiple of 1024
-__global__ void __launch_bounds__(128) bwd_pack_kernel(const PackArgs a, uint8_t* packed) {
-  const int gw = blockIdx.x * 4 + (threadIdx.x >> 5);  // 0 .. 767
+__device__ __forceinline__ void bwd_pack_row(const PackArgs& a, uint8_t* packed, int gw) {  // gw: 0 .. 767
   const int lane = threadIdx.x & 31;
   const int m = gw >> 7, row = gw & 127;
   const int n_rows = m < 4 ? 128 : a.c;  // a.c = d_pair: matrices 0..3 are [128, c], 4 (out) is [c, 128], 5 (gate) [c, c]
@@ -1261,113 +1276,163 @@ __global__ void __launch_bounds__(128) bwd_pack_kernel(const PackArgs a, uint8_t
     reinterpret_cast<float*>(packed + kBwdPackedD)[m * 128 + row] = d + (a.bias[m] != nullptr ? a.bias[m][row] : 0.f);
 }
 
-// Sum of element e over the partials g, g + 4, g + 8, ... (four loads in flight, fixed order of additions).
-__device__ __forceinline__ float sum_every_fourth(const float* parts, size_t stride, int n_parts, int e, int g) {
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-  int i = g;
-  for (; i + 12 < n_parts; i += 16) {
-    const float a = parts[static_cast<size_t>(i) * stride + e], b = parts[static_cast<size_t>(i + 4) * stride + e];
-    const float c = parts[static_cast<size_t>(i + 8) * stride + e], d = parts[static_cast<size_t>(i + 12) * stride + e];
-    s0 += a, s1 += b, s2 += c, s3 += d;
+
+// One launch before the backward kernels: blocks 0 .. 96 * halves - 1 pack the weights of the halves (eight matrix rows
+// each), the rest find max |dy| and the scale.
+struct BwdSetupArgs {
+  PackArgs w[2];
+  uint8_t* packed[2];
+  int pack_blocks;  // 96 per half
+  const uint4* dy;
+  size_t n_chunks;
+  unsigned int* words;
+  float* scale;
+};
+__global__ void __launch_bounds__(256) bwd_setup_kernel(const __grid_constant__ BwdSetupArgs a) {
+  const int block = blockIdx.x;
+  if (block < a.pack_blocks) {
+    const int h = block >= 96 ? 1 : 0;
+    bwd_pack_row(a.w[h], a.packed[h], (block - h * 96) * 8 + (threadIdx.x >> 5));
+    return;
   }
-  for (; i < n_parts; i += 4) s0 += parts[static_cast<size_t>(i) * stride + e];
-  return (s0 + s1) + (s2 + s3);
+  amax_and_scale(a.dy, a.n_chunks, block - a.pack_blocks, gridDim.x - a.pack_blocks, a.words, a.scale);
 }
 
-// M[e] and S[e] = sums over the CTAs' partials in a fixed order (deterministic). Blocks 0 .. 511 take M (2 x 128 x 128
-// values), blocks 512 .. 515 take S (2 x 128 values).
-__global__ void __launch_bounds__(256) bwd_reduce_kernel(const float* part_m, const float* part_s, int n_parts, float* m_out,
-                                                         float* s_out) {
-  // grid = 512 blocks for M (64 elements each) + 4 for S; a block's four groups of 64 threads take every fourth partial
-  // and are combined in a fixed order
-  __shared__ float comb[4][64];
-  const bool is_s = blockIdx.x >= 512;
-  const float* parts = is_s ? part_s : part_m;
-  const size_t stride = is_s ? 2 * 128 : 2 * 128 * 128;
-  const int el = threadIdx.x & 63, g = threadIdx.x >> 6;
-  const int e = (is_s ? blockIdx.x - 512 : blockIdx.x) * 64 + el;
-  comb[g][el] = sum_every_fourth(parts, stride, n_parts, e, g);
-  __syncthreads();
-  if (g == 0) (is_s ? s_out : m_out)[e] = (comb[0][el] + comb[1][el]) + (comb[2][el] + comb[3][el]);
-}
-
-// Parameter gradients from the reduced sums M[m] = dOut_m^T x_hat (times c) and S[m] = column sums of dOut_m (times c):
+// Parameter gradients from the per-CTA partial sums M[m] = dOut_m^T x_hat (times c) and S[m] = column sums of dOut_m
+// (times c) that the launches of the epilogue's and the prologue's backward left:
 //   dW_m[r][k] = (M[m][r][k] gamma[k] + S[m][r] beta[k]) / c
 //   dgamma[k]  = sum_m sum_r W_m[r][k] M[m][r][k] / c,   dbeta[k] = sum_m sum_r W_m[r][k] S[m][r] / c
 // over the matrices that read that LayerNorm (the output one: matrix 4; the input one: the other five).
-// One call covers one set of six 128 x 128 matrices ("half": the unidirectional module has one, the bidirectional module
-// two, whose matrices are row or column blocks of the module's wider parameters, hence the leading dimensions).
-// Grid (6 matrices, 8 blocks of 16 rows), thread = column k; the LayerNorm sums leave as partials [6][8][2][128] that
-// bwd_finalize_ln_kernel adds in a fixed order.
-struct BwdFinalArgs {
-  PackArgs w;           // raw weights (this half's blocks, with their leading dimensions) and LayerNorm parameters
-  const float* m_all;   // [6][128][128]
-  const float* s_all;   // [6][128]
-  const float* scale;   // [2]
-  float* dw[6];         // fp32 gradient blocks
-  int dw_ld[6];         // their leading dimensions
-  float* ln_part;       // [6][8][2][128]
-  unsigned mask;        // bit m set: matrix m is present in this half
+// One set of six 128 x 128 matrices ("half"): the unidirectional module has one, the bidirectional module two, whose
+// matrices are row or column blocks of the module's wider parameters, hence the leading dimensions.
+// Grid (128 rows, 6 matrices, halves); a block of 512 threads adds one row of the partials, 16 groups of CTAs by 32
+// four-column pieces, every load of a thread in flight at once, and combines the groups in a fixed order: the sums, the
+// parameter gradients and the rows of the LayerNorm sums leave in one pass over the partials. The earlier form (a
+// reduction after every launch that produced partials, then a kernel for the gradients on 6 x 8 blocks, and one block for
+// the LayerNorm sums) was three to six launches of 5.2 us plus 10 and 5 us.
+constexpr int kFinGroups = 16;
+constexpr int kFinFlight = 10;  // 16 * 10 = 160 = the largest number of CTAs
+struct BwdFinalHalf {
+  PackArgs w;              // raw weights (this half's blocks, with their leading dimensions) and LayerNorm parameters
+  const float* part_m[6];  // per matrix: [n_parts][2][128][128] partials, at this matrix's [128][128] of CTA 0
+  const float* part_s[6];  // per matrix: [n_parts][2][128]
+  float* dw[6];            // fp32 gradient blocks
+  int dw_ld[6];            // their leading dimensions
+  float* ln_rows;          // [6][128][2][128]: this matrix row's terms of dgamma and dbeta
+  unsigned mask;           // bit m set: matrix m is present in this half
 };
-__global__ void __launch_bounds__(128) bwd_finalize_kernel(const BwdFinalArgs a) {
-  const int k = threadIdx.x, m = blockIdx.x, rb = blockIdx.y;
-  if (((a.mask >> m) & 1u) == 0u) return;
-  const int n_rows = m < 4 ? 128 : a.w.c, n_cols = m == 4 ? 128 : a.w.c;  // a.w.c = d_pair
-  float* part0 = a.ln_part + ((m * 8 + rb) * 2 + 0) * 128 + k;
-  float* part1 = a.ln_part + ((m * 8 + rb) * 2 + 1) * 128 + k;
-  if (k >= n_cols || rb * 16 >= n_rows) {
-    *part0 = 0.f, *part1 = 0.f;
-    return;
+struct BwdFinalArgs {
+  BwdFinalHalf half[2];
+  int n_parts;
+  const float* scale;  // [2]
+};
+// rows [n_parts] of 128 floats, `stride` floats apart, summed into `out` (512 threads; comb is float[16][128])
+__device__ __forceinline__ float4 sum_partial_rows(const float* parts, size_t stride, int n_parts, float4* comb) {
+  const int piece = threadIdx.x & 31, g = threadIdx.x >> 5;
+  float4 v[kFinFlight];
+#pragma unroll
+  for (int u = 0; u < kFinFlight; ++u) {
+    const int i = g + u * kFinGroups;
+    v[u] = i < n_parts ? __ldcg(reinterpret_cast<const float4*>(parts + static_cast<size_t>(i) * stride) + piece)
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  const float cinv = a.scale[1];
-  const float gamma = (m == 4 ? a.w.ln_out_w : a.w.ln_in_w)[k];
-  const float beta = (m == 4 ? a.w.ln_out_b : a.w.ln_in_b)[k];
-  float ag = 0.f, ab = 0.f;
-#pragma unroll 4
-  for (int r = rb * 16; r < rb * 16 + 16; ++r) {
-    const size_t wi = static_cast<size_t>(r) * a.w.ld[m] + k;
-    const float w = a.w.f32_weights ? static_cast<const float*>(a.w.w[m])[wi]
-                                    : __uint_as_float(static_cast<uint32_t>(static_cast<const uint16_t*>(a.w.w[m])[wi]) << 16);
-    const float mv = a.m_all[(m * 128 + r) * 128 + k] * cinv;
-    const float sv = a.s_all[m * 128 + r] * cinv;
-    a.dw[m][static_cast<size_t>(r) * a.dw_ld[m] + k] = fmaf(mv, gamma, sv * beta);
-    ag = fmaf(w, mv, ag);
-    ab = fmaf(w, sv, ab);
+  float4 s = v[0];
+#pragma unroll
+  for (int u = 1; u < kFinFlight; ++u) s.x += v[u].x, s.y += v[u].y, s.z += v[u].z, s.w += v[u].w;
+  comb[g * 32 + piece] = s;
+  __syncthreads();
+  float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (g == 0) {
+#pragma unroll
+    for (int q = 0; q < kFinGroups; ++q) {
+      const float4 x = comb[q * 32 + piece];
+      t.x += x.x, t.y += x.y, t.z += x.z, t.w += x.w;
+    }
   }
-  *part0 = ag;
-  *part1 = ab;
+  return t;  // warp 0: columns 4 * piece .. + 3
 }
+// the sum over the CTAs of one float, `stride` floats apart, by one warp (every lane returns it)
+__device__ __forceinline__ float sum_partial_scalar(const float* part, size_t stride, int n_parts) {
+  float s = 0.f;
+  for (int i = threadIdx.x & 31; i < n_parts; i += 32) s += __ldcg(part + static_cast<size_t>(i) * stride);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, off);
+  return s;
+}
+__global__ void __launch_bounds__(512) bwd_finalize_kernel(const __grid_constant__ BwdFinalArgs args) {
+  __shared__ float4 comb[kFinGroups * 32];
+  const BwdFinalHalf& a = args.half[blockIdx.z];
+  const int r = blockIdx.x, m = blockIdx.y;
+  const int n_rows = m < 4 ? 128 : a.w.c, n_cols = m == 4 ? 128 : a.w.c;  // a.w.c = d_pair
+  if (((a.mask >> m) & 1u) == 0u || r >= n_rows) return;
+  const float4 mv4 = sum_partial_rows(a.part_m[m] + r * 128, 2 * 128 * 128, args.n_parts, comb);
+  const int k0 = (threadIdx.x & 31) * 4;
+  if (threadIdx.x >= 32) return;
+  const float sum_s = sum_partial_scalar(a.part_s[m] + r, 2 * 128, args.n_parts);
+  if (k0 >= n_cols) return;
+  const float cinv = args.scale[1];
+  const float4 gamma = *reinterpret_cast<const float4*>((m == 4 ? a.w.ln_out_w : a.w.ln_in_w) + k0);
+  const float4 beta = *reinterpret_cast<const float4*>((m == 4 ? a.w.ln_out_b : a.w.ln_in_b) + k0);
+  const size_t wi = static_cast<size_t>(r) * a.w.ld[m] + k0;
+  float4 w;
+  if (a.w.f32_weights) {
+    w = *reinterpret_cast<const float4*>(static_cast<const float*>(a.w.w[m]) + wi);
+  } else {
+    const uint2 v = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(a.w.w[m]) + wi);
+    w = make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
+  }
+  const float sv = sum_s * cinv;
+  const float4 mv = make_float4(mv4.x * cinv, mv4.y * cinv, mv4.z * cinv, mv4.w * cinv);
+  float* dw = a.dw[m] + static_cast<size_t>(r) * a.dw_ld[m] + k0;
+  dw[0] = fmaf(mv.x, gamma.x, sv * beta.x), dw[1] = fmaf(mv.y, gamma.y, sv * beta.y);
+  dw[2] = fmaf(mv.z, gamma.z, sv * beta.z), dw[3] = fmaf(mv.w, gamma.w, sv * beta.w);
+  float4* ln = reinterpret_cast<float4*>(a.ln_rows + (static_cast<size_t>(m) * 128 + r) * 256 + k0);
+  ln[0] = make_float4(w.x * mv.x, w.y * mv.y, w.z * mv.z, w.w * mv.w);
+  ln[32] = make_float4(w.x * sv, w.y * sv, w.z * sv, w.w * sv);
+}
+// Adds the rows of the LayerNorm sums in a fixed order. Grid (2: dgamma or dbeta, 1 + halves: the input LayerNorm, then the
+// output LayerNorm's 128 channels of each half); 1024 threads: 32 four-column pieces by 32 groups of rows.
 struct BwdLnArgs {
-  const float* ln_part[2];  // per half
+  const float* ln_rows[2];  // per half
   unsigned mask[2];
   int halves;
-  float* d_ln_in_w;   // [128]
-  float* d_ln_in_b;
-  float* d_ln_out_w;  // [128 * halves]: half h at + 128 h
-  float* d_ln_out_b;
-  int c;              // d_pair
+  float* d_in[2];   // dgamma, dbeta of the input LayerNorm [c]
+  float* d_out[2];  // of the output LayerNorm [128 * halves]: half h at + 128 h
+  int c;            // d_pair
 };
-__global__ void __launch_bounds__(128) bwd_finalize_ln_kernel(const BwdLnArgs a) {
-  const int k = threadIdx.x;
-  float g_in = 0.f, b_in = 0.f;
-  for (int h = 0; h < a.halves; ++h) {
-    float g_out = 0.f, b_out = 0.f;
-    for (int m = 0; m < 6; ++m) {
-      if (((a.mask[h] >> m) & 1u) == 0u) continue;
-      float ag = 0.f, ab = 0.f;
-      for (int rb = 0; rb < 8; ++rb) {
-        ag += a.ln_part[h][((m * 8 + rb) * 2 + 0) * 128 + k];
-        ab += a.ln_part[h][((m * 8 + rb) * 2 + 1) * 128 + k];
+__global__ void __launch_bounds__(1024) bwd_finalize_ln_kernel(const BwdLnArgs a) {
+  __shared__ float4 comb[32 * 32];
+  const int piece = threadIdx.x & 31, g = threadIdx.x >> 5, vec = blockIdx.x;
+  const bool input = blockIdx.y == 0;
+  const int n_cols = input ? a.c : 128;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (piece * 4 < n_cols) {
+    for (int h = input ? 0 : static_cast<int>(blockIdx.y) - 1; h < (input ? a.halves : static_cast<int>(blockIdx.y)); ++h) {
+#pragma unroll
+      for (int m = 0; m < 6; ++m) {
+        const int n_rows = m < 4 ? 128 : a.c;
+        if ((m == 4) == input || ((a.mask[h] >> m) & 1u) == 0u) continue;
+        const float4* src = reinterpret_cast<const float4*>(a.ln_rows[h] + m * 128 * 256 + vec * 128) + piece;
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          v[u] = g + u * 32 < n_rows ? __ldcg(src + static_cast<size_t>(g + u * 32) * 64) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s.x += v[u].x, s.y += v[u].y, s.z += v[u].z, s.w += v[u].w;
       }
-      if (m == 4) g_out += ag, b_out += ab;
-      else g_in += ag, b_in += ab;
     }
-    a.d_ln_out_w[h * 128 + k] = g_out;
-    a.d_ln_out_b[h * 128 + k] = b_out;
   }
-  if (k < a.c) {  // the input LayerNorm has d_pair channels
-    a.d_ln_in_w[k] = g_in;
-    a.d_ln_in_b[k] = b_in;
+  comb[g * 32 + piece] = s;
+  __syncthreads();
+  if (g == 0 && piece * 4 < n_cols) {
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      const float4 x = comb[q * 32 + piece];
+      t.x += x.x, t.y += x.y, t.z += x.z, t.w += x.w;
+    }
+    float* dst = (input ? a.d_in[vec] : a.d_out[vec] + 128 * (static_cast<int>(blockIdx.y) - 1)) + piece * 4;
+    dst[0] = t.x, dst[1] = t.y, dst[2] = t.z, dst[3] = t.w;
   }
 }
 

@@ -478,8 +478,8 @@ __device__ __forceinline__ float tr_load_w(const void* w, size_t i, int f32) {
   return f32 ? static_cast<const float*>(w)[i]
              : __uint_as_float(static_cast<uint32_t>(static_cast<const uint16_t*>(w)[i]) << 16);
 }
-__global__ void __launch_bounds__(128) tr_bwd_pack_kernel(const TrBwdPackArgs a, uint8_t* packed) {
-  const int gw = blockIdx.x * 4 + (threadIdx.x >> 5);  // 0 .. 1535: rows of Wa (0-511), Wb (512-1023), then Ws rows by 4
+// gw: 0 .. 1535: rows of Wa (0-511), Wb (512-1023), then Ws rows by 4
+__device__ __forceinline__ void tr_bwd_pack_row(const TrBwdPackArgs& a, uint8_t* packed, int gw) {
   const int lane = threadIdx.x & 31;
   if (gw < 1024) {
     const int m = gw >> 9, row = gw & 511;
@@ -512,71 +512,99 @@ __global__ void __launch_bounds__(128) tr_bwd_pack_kernel(const TrBwdPackArgs a,
   }
 }
 
-// m_out[e] (3 x 128 x 128 values: blocks 0 .. 767) and s_out[e] (2 x 512 values: blocks 768 .. 783) = sums over the CTAs'
-// partials; a block covers 64 elements, its four groups of 64 threads take every fourth partial and are combined in a
-// fixed order.
-__global__ void __launch_bounds__(256) tr_bwd_reduce_kernel(const float* part_m, const float* part_s, int n_parts, float* m_out,
-                                                            float* s_out) {
-  __shared__ float comb[4][64];
-  const bool is_s = blockIdx.x >= 768;
-  const float* parts = is_s ? part_s : part_m;
-  const size_t stride = is_s ? 2 * 512 : 3 * 128 * 128;
-  const int el = threadIdx.x & 63, g = threadIdx.x >> 6;
-  const int e = (is_s ? blockIdx.x - 768 : blockIdx.x) * 64 + el;
-  comb[g][el] = sum_every_fourth(parts, stride, n_parts, e, g);
-  __syncthreads();
-  if (g == 0) (is_s ? s_out : m_out)[e] = (comb[0][el] + comb[1][el]) + (comb[2][el] + comb[3][el]);
+// One launch before the backward kernels: the first kTrBwdPackBlocks blocks pack the weights (eight rows each), the rest
+// find max |dy| and the scale.
+constexpr int kTrBwdPackBlocks = 1536 / 8;
+struct TrBwdSetupArgs {
+  TrBwdPackArgs w;
+  uint8_t* packed;
+  const uint4* dy;
+  size_t n_chunks;
+  unsigned int* words;
+  float* scale;
+};
+__global__ void __launch_bounds__(256) tr_bwd_setup_kernel(const __grid_constant__ TrBwdSetupArgs a) {
+  if (blockIdx.x < kTrBwdPackBlocks) {
+    tr_bwd_pack_row(a.w, a.packed, blockIdx.x * 8 + (threadIdx.x >> 5));
+    return;
+  }
+  amax_and_scale(a.dy, a.n_chunks, blockIdx.x - kTrBwdPackBlocks, gridDim.x - kTrBwdPackBlocks, a.words, a.scale);
 }
 
-// Parameter gradients of the Transition from the reduced sums of all four blocks:
-//   m_all [4][3][128][128] (Ma_j, Mb_j: [hidden][k]; dWs_j: [c][hidden]), s_all [4][2][4][128] (column sums per quarter)
+// Parameter gradients of the Transition from the per-CTA partials of the four launches j:
+//   part_m [4][n_parts][3][128][128] (Ma_j, Mb_j: [hidden][k]; dWs_j: [c][hidden]), part_s [4][n_parts][2][4][128]
+//   (column sums, held by quarter 0)
 //   dWa[j*128+r][k] = (Ma_j[r][k] gamma[k] + sa_j[r] beta[k]) / c, dWb likewise, dWs[c][j*128+h] = dWs_j[c][h] / c
 //   dgamma[k] = sum_j sum_r (Wa Ma + Wb Mb) / c,  dbeta[k] = sum_j sum_r (Wa sa + Wb sb) / c
-// Grid (4 blocks j, 8 row groups of 16), thread = column; LayerNorm partials [4][8][2][128] added by tr_bwd_final_ln_kernel.
+// Grid (128 rows, 3 matrices, 4 blocks j), one row of the partials per block as in bwd_finalize_kernel; the rows of the
+// LayerNorm sums [1024][2][128] are added by tr_bwd_final_ln_kernel. (A reduction per launch and a gradient kernel on
+// 4 x 8 blocks were 4 x 5.9 + 22.4 us.)
 struct TrBwdFinalArgs {
   TrBwdPackArgs w;
-  const float* m_all;
-  const float* s_all;
+  const float* part_m;
+  const float* part_s;
+  int n_parts;
   const float* scale;
-  float* d_wa;    // [512][128]
-  float* d_wb;    // [512][128]
-  float* d_ws;    // [128][512]
-  float* ln_part; // [4][8][2][128]
-  float* d_ln_w;  // [128]
-  float* d_ln_b;
+  float* d_wa;     // [512][128]
+  float* d_wb;     // [512][128]
+  float* d_ws;     // [128][512]
+  float* ln_rows;  // [2][512][2][128]
+  float* d_ln[2];  // dgamma, dbeta [128]
 };
-__global__ void __launch_bounds__(128) tr_bwd_final_kernel(const TrBwdFinalArgs a) {
-  const int k = threadIdx.x, j = blockIdx.x, rb = blockIdx.y;
+__global__ void __launch_bounds__(512) tr_bwd_final_kernel(const __grid_constant__ TrBwdFinalArgs a) {
+  __shared__ float4 comb[kFinGroups * 32];
+  const int r = blockIdx.x, m = blockIdx.y, j = blockIdx.z;
+  const float* parts = a.part_m + (static_cast<size_t>(j) * a.n_parts * 3 + m) * 128 * 128 + r * 128;
+  const float4 mv4 = sum_partial_rows(parts, 3 * 128 * 128, a.n_parts, comb);
+  if (threadIdx.x >= 32) return;
+  const int k0 = (threadIdx.x & 31) * 4;
   const float cinv = a.scale[1];
-  const float gamma = a.w.ln_w[k], beta = a.w.ln_b[k];
-  float ag = 0.f, ab = 0.f;
-  for (int r = rb * 16; r < rb * 16 + 16; ++r) {
-    const float* sq = a.s_all + static_cast<size_t>(j) * 2 * 512;
-    const float sa = (sq[r] + sq[128 + r] + sq[256 + r] + sq[384 + r]) * cinv;
-    const float sb = (sq[512 + r] + sq[512 + 128 + r] + sq[512 + 256 + r] + sq[512 + 384 + r]) * cinv;
-    const float ma = a.m_all[((static_cast<size_t>(j) * 3 + 0) * 128 + r) * 128 + k] * cinv;
-    const float mb = a.m_all[((static_cast<size_t>(j) * 3 + 1) * 128 + r) * 128 + k] * cinv;
-    const size_t wi = static_cast<size_t>(j * 128 + r) * 128 + k;
-    const float wa = tr_load_w(a.w.w_a, wi, a.w.f32_weights), wb = tr_load_w(a.w.w_b, wi, a.w.f32_weights);
-    a.d_wa[wi] = fmaf(ma, gamma, sa * beta);
-    a.d_wb[wi] = fmaf(mb, gamma, sb * beta);
-    ag = fmaf(wa, ma, fmaf(wb, mb, ag));
-    ab = fmaf(wa, sa, fmaf(wb, sb, ab));
-    // dWs: row c = r (of this row group), column block j, column h = k
-    a.d_ws[static_cast<size_t>(r) * 512 + j * 128 + k] = a.m_all[((static_cast<size_t>(j) * 3 + 2) * 128 + r) * 128 + k] * cinv;
+  const float mv[4] = {mv4.x * cinv, mv4.y * cinv, mv4.z * cinv, mv4.w * cinv};
+  if (m == 2) {
+    float* dst = a.d_ws + static_cast<size_t>(r) * 512 + j * 128 + k0;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) dst[t] = mv[t];
+    return;
   }
-  a.ln_part[((j * 8 + rb) * 2 + 0) * 128 + k] = ag;
-  a.ln_part[((j * 8 + rb) * 2 + 1) * 128 + k] = ab;
+  const float sv =
+      cinv * sum_partial_scalar(a.part_s + (static_cast<size_t>(j) * a.n_parts * 2 + m) * 512 + r, 2 * 512, a.n_parts);
+  const size_t wi = static_cast<size_t>(j * 128 + r) * 128 + k0;
+  float* dst = (m == 0 ? a.d_wa : a.d_wb) + wi;
+  float* ln = a.ln_rows + (static_cast<size_t>(m) * 512 + j * 128 + r) * 256 + k0;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const float w = tr_load_w(m == 0 ? a.w.w_a : a.w.w_b, wi + t, a.w.f32_weights);
+    dst[t] = fmaf(mv[t], a.w.ln_w[k0 + t], sv * a.w.ln_b[k0 + t]);
+    ln[t] = w * mv[t];
+    ln[128 + t] = w * sv;
+  }
 }
-__global__ void __launch_bounds__(128) tr_bwd_final_ln_kernel(const TrBwdFinalArgs a) {
-  const int k = threadIdx.x;
-  float g = 0.f, b = 0.f;
-  for (int i = 0; i < 32; ++i) {
-    g += a.ln_part[(i * 2 + 0) * 128 + k];
-    b += a.ln_part[(i * 2 + 1) * 128 + k];
+// grid 2 (dgamma, dbeta), 1024 threads: 32 four-column pieces by 32 groups of rows, fixed order
+__global__ void __launch_bounds__(1024) tr_bwd_final_ln_kernel(const TrBwdFinalArgs a) {
+  __shared__ float4 comb[32 * 32];
+  const int piece = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const float4* src = reinterpret_cast<const float4*>(a.ln_rows + blockIdx.x * 128) + piece;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < 32; i += 8) {
+    float4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = __ldcg(src + static_cast<size_t>(g + (i + u) * 32) * 64);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s.x += v[u].x, s.y += v[u].y, s.z += v[u].z, s.w += v[u].w;
   }
-  a.d_ln_w[k] = g;
-  a.d_ln_b[k] = b;
+  comb[g * 32 + piece] = s;
+  __syncthreads();
+  if (g == 0) {
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      const float4 x = comb[q * 32 + piece];
+      t.x += x.x, t.y += x.y, t.z += x.z, t.w += x.w;
+    }
+    float* dst = a.d_ln[blockIdx.x] + piece * 4;
+    dst[0] = t.x, dst[1] = t.y, dst[2] = t.z, dst[3] = t.w;
+  }
 }
 
 }  // namespace trimul
