@@ -220,6 +220,7 @@ struct BwdEpilogueParams {
   const float2* ext_stats;  // [B*N][ld]: mean and rstd of the stored t over all 256 channels
   float2* ln_part;          // [B*N][ld]: MODE 1 writes its sums of d t_hat and d t_hat * t_hat; MODE 2 adds its own and
                             // writes back the two means over 256 channels
+  float* rstd;              // [B*N][ld], not MODE 1: 1 / standard deviation of the input LayerNorm (x_hat leaves through map_xh)
   const uint16_t* p_part;   // [B*N][N][128] fp16, MODE 2: the first launch's part of the output projection
   int* status;
 };
@@ -240,7 +241,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_z,
                     const __grid_constant__ CUtensorMap map_dy, const __grid_constant__ CUtensorMap map_wo,
                     const __grid_constant__ CUtensorMap map_wg, const __grid_constant__ CUtensorMap map_dt,
-                    const __grid_constant__ CUtensorMap map_dx, const BwdEpilogueParams p) {
+                    const __grid_constant__ CUtensorMap map_dx, const __grid_constant__ CUtensorMap map_xh,
+                    const BwdEpilogueParams p) {
   // C = d_pair: the channels of z, dy, dproj, dgate and the rows of both weight matrices (128, or 64 for the narrow pair
   // stacks; MODE 0 only). The contracted width (channels of t) is 128 in both cases.
   static_assert(C == 128 || (C == 64 && MODE == 0), "d_pair is 128, or 64 with one output tensor");
@@ -360,7 +362,10 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
       for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(dy_s + kh * 16384, &map_dy, dy_full, kh * 64, j0, row);
       dy_pending = it;
     }
-    normalise_tile<true, true, C>(z_s, xchg + kBwdXchgHalf, pos, part, p.eps_in);  // (the other exchange buffer)
+    const float rstd_in = normalise_tile<true, true, C>(z_s, xchg + kBwdXchgHalf, pos, part, p.eps_in);  // (other buffer)
+    if constexpr (MODE != 1) {
+      if (part == 0 && j0 + pos < p.n) p.rstd[static_cast<size_t>(row) * p.ld + j0 + pos] = rstd_in;
+    }
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -382,6 +387,12 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
                   umma_desc_kmajor(wg_s + (ks >> 2) * kWHalf) + kb, idesc_g, ks != 0 ? 1u : 0u);
       }
       umma_commit(mma_bar);
+      if constexpr (MODE != 1) {
+        // x_hat for the prologue's backward, read from the z buffer before phase 5 writes over it
+#pragma unroll
+        for (int kh = 0; kh < kZHalves; ++kh) tma_store_3d(&map_xh, z_s + kh * 16384, kh * 64, j0, row);
+        bulk_commit();
+      }
     }
     // per-thread global operands of phase 3 (MODE 2: the first launch's part of the projection; the dropout scale),
     // requested before the waits
@@ -457,6 +468,9 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
           st_chunk(dg_s + zaddr, 0u, 0u, 0u, 0u);
         }
       }
+    }
+    if constexpr (MODE != 1) {
+      if (threadIdx.x == 0) bulk_wait_read<0>();  // the store of x_hat
     }
     tc_fence_before();
     fence_proxy_async_smem();
@@ -759,26 +773,38 @@ struct BwdPrologueParams {
   int tiles_per_row;
   int num_tiles;
   int n;
+  int ld;                     // columns per row of rstd
   const float* consts;        // [2][128]: d_value = W beta_in + bias, d_gate likewise (this side's two matrices)
   const float* grad_scale;    // [2]: c, 1 / c
   const uint8_t* token_mask;  // [B][N] or null
   const uint8_t* pair_mask;   // [B][N][N] or null
-  const uint16_t* dx_in;      // [B*N][N][128] fp16: c * d loss / d x_hat gathered so far (read)
-  const uint16_t* dy;         // LAST only: upstream gradient [B*N][N][128] bf16 (the residual path), or null
-  float eps_in;
+  const uint16_t* dx_in;      // [B*N][N][C] fp16: c * d loss / d x_hat gathered so far (read)
+  const uint16_t* dy;         // LAST only: upstream gradient [B*N][N][C] bf16 (the residual path), or null
+  const float* rstd;          // LAST only: [B*N][ld] 1 / standard deviation of the input LayerNorm
   float* part_m;              // [grid][2][128][128]: partial dvalue^T x_hat, dgate^T x_hat
   float* part_s;              // [grid][2][128]
   int* status;
 };
 
-// Prologue backward for one side (left or right). Inputs: z [B*N][N][128] bf16, dO = the contraction's gradient for
-// this side [B*N][128][N] fp16 (times c / 16). It recomputes value / gate, forms dvalue = dO sig m, dgate = dO value
-// sig (1 - sig) m, adds dvalue W_v' + dgate W_g' to the running d x_hat, and accumulates the two weight gradients.
-// !LAST: the running d x_hat (fp16, times c) is written back through map_out. LAST: the input LayerNorm's backward
-// and the residual finish d loss / d z (bf16, unscaled) through map_out.
+// Prologue backward for one side (left or right). Inputs: x_hat [B*N][N][C] fp16 and rstd (both left by the epilogue's
+// backward, which normalises z anyway), dO = the contraction's gradient for this side [B*N][128][N] fp16 (times c / 16).
+// It recomputes value / gate, forms dvalue = dO sig m, dgate = dO value sig (1 - sig) m, adds dvalue W_v' + dgate W_g' to
+// the running d x_hat, and accumulates the two weight gradients. !LAST: the running d x_hat (fp16, times c) is written
+// back through map_out. LAST: the input LayerNorm's backward and the residual finish d loss / d z (bf16, unscaled).
+//
+// 16 arithmetic warps (four threads per channel or position, as in the epilogue's backward) and one warp whose first lane
+// issues every copy and MMA. The arithmetic warps never wait for one another but once per tile (LAST): they arrive at
+// named barriers the issuing warp waits at, and wait for its MMAs on mbarriers. Per tile:
+//   arithmetic: wait value / gate -> dvalue, dgate tiles -> arrive A -> (requests for the running sums) -> wait gradients
+//               -> d x_hat out of tensor memory -> arrive B -> LayerNorm backward, output tile -> arrive C
+//   issuing:    A: gradient GEMMs, next x_hat copy; their end: next dO copy; B: value / gate GEMMs of the NEXT tile, which
+//               run under the arithmetic that finishes this one; C: output store, and the word that its buffer was read.
+// What bounds it: the chain wait -> arithmetic -> gradient GEMMs (32 MMAs) -> read of one tile per SM; shared memory holds
+// two weight matrices and four tiles.
+constexpr int kBwdProThreads = kBwdThreads + 32;
 template <bool LAST, int C = 128>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_do,
+__global__ void __launch_bounds__(kBwdProThreads, 1)
+bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_do,
                     const __grid_constant__ CUtensorMap map_wv, const __grid_constant__ CUtensorMap map_wg,
                     const __grid_constant__ CUtensorMap map_out, const BwdPrologueParams p) {
   // C = d_pair: the channels of z, d x_hat, dz and the columns of both weight matrices (128, or 64 for the narrow pair
@@ -787,6 +813,7 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   constexpr int kZCh = C / kBwdParts;   // z-side channels per thread
   constexpr int kZChunks = kZCh / 8;
   constexpr int kZHalves = C / 64;      // 64-channel halves of a [pos][C] tile = k halves of a [128][C] weight matrix
+  constexpr int kBarA = 2, kBarB = 3, kBarC = 4;  // named barriers of the arithmetic warps and the issuing warp
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -795,23 +822,23 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   const uint32_t xchg = smem_base + 6 * kBwdTile;
   const uint32_t const_s = xchg + kBwdXchg;
   const uint32_t bar_base = const_s + 1024;
-  const uint32_t w_full = bar_base, z_full = bar_base + 8, mma_bar = bar_base + 16, do_full = bar_base + 24;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 6 * kBwdTile + kBwdXchg + 1024 + 32);
+  const uint32_t w_full = bar_base, x_full = bar_base + 8, do_full = bar_base + 16;
+  const uint32_t fwd_done = bar_base + 24, grad_done = bar_base + 32, out_free = bar_base + 40;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 6 * kBwdTile + kBwdXchg + 1024 + 48);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q = warp & 3, part = warp >> 2;
-  const int pos = q * 32 + lane;
-  const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
 
   if (threadIdx.x == 0) {
     mbar_init(w_full, 1);
-    mbar_init(z_full, 1);   // a tile's z and dO copies are issued and awaited at different times
+    mbar_init(x_full, 1);
     mbar_init(do_full, 1);
-    mbar_init(mma_bar, 2);  // two issuing threads commit to it in every GEMM round
+    mbar_init(fwd_done, 1);
+    mbar_init(grad_done, 1);
+    mbar_init(out_free, 1);
     *abort_flag = 0;
     fence_mbar_init();
-    prefetch_tmap(&map_z);
+    prefetch_tmap(&map_x);
     prefetch_tmap(&map_do);
     prefetch_tmap(&map_out);
   }
@@ -823,287 +850,313 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const float gc_inv = p.grad_scale[1];
-  const float c_value = p.consts[pos], c_gate_half = 0.5f * p.consts[128 + pos];  // this thread's channel
 
-  if (threadIdx.x == 0) {
-    mbar_arrive_expect_tx(w_full, 2 * kZHalves * 16384);
-#pragma unroll
-    for (int kh = 0; kh < kZHalves; ++kh) {
-      tma_load_2d(wv_s + kh * 16384, &map_wv, w_full, kh * 64, 0);
-      tma_load_2d(wg_s + kh * 16384, &map_wg, w_full, kh * 64, 0);
-    }
-  }
-  // Phases 2-3 work on the transposed projections (TMEM lanes = contracted channels, columns = positions): a thread
-  // owns channel `pos` (its lane) and the position quarter `part`, so its constants and its column sums are scalars
-  // and dO, stored [channel][position], is read in 16-byte runs of positions.
-  float acc_sv = 0.f, acc_sg = 0.f;
-  // validity of a tile's positions, one bit each: [2][4] words (tile parity, 32 positions per word). The mask bytes of
-  // the NEXT tile are requested by the first four warps before a GEMM wait and turned into the words after it, so that
-  // their latency is off the path.
-  uint32_t* valid_words = reinterpret_cast<uint32_t*>(smem + 6 * kBwdTile + kBwdXchg + 1024 + 64);
-  auto mask_bytes = [&](int tile_i, bool& in_range, uint32_t& m_i, uint32_t& m_j, uint32_t& m_p) {
-    const int row_i = tile_i / p.tiles_per_row;
-    const int j_i = (tile_i - row_i * p.tiles_per_row) * 128 + pos;
-    const int b = row_i / p.n;
-    const int i = row_i - b * p.n;
-    in_range = j_i < p.n;
-    m_i = 1u, m_j = 1u, m_p = 1u;
-    if (in_range) {
-      if (p.token_mask != nullptr) {
-        m_i = p.token_mask[static_cast<size_t>(b) * p.n + i];
-        m_j = p.token_mask[static_cast<size_t>(b) * p.n + j_i];
-      }
-      if (p.pair_mask != nullptr) m_p = p.pair_mask[(static_cast<size_t>(b) * p.n + i) * p.n + j_i];
-    }
-  };
-  auto publish_valid = [&](int it_i, bool in_range, uint32_t m_i, uint32_t m_j, uint32_t m_p) {
-    const uint32_t word = __ballot_sync(0xFFFFFFFFu, in_range && m_i != 0u && m_j != 0u && m_p != 0u);
-    if (lane == 0) valid_words[(it_i & 1) * 4 + q] = word;
-  };
-
-  // Buffer roles (z, dO, dvalue, dgate) of tile `it`, one nibble each, period 4: the next tile's z and dO are copied
-  // into this tile's dO buffer (free after phase 3) and dgate buffer (free after the gradient GEMMs) while this tile
-  // finishes; its dvalue scratch is this tile's z buffer and its dgate scratch this tile's dvalue buffer, which holds
+  // Buffer roles (x_hat, dO, dvalue, dgate) of tile `it`, one nibble each, period 4: the next tile's x_hat and dO are
+  // copied into this tile's dO buffer (free once dvalue / dgate are formed) and dgate buffer (free after the gradient
+  // GEMMs); its dvalue scratch is this tile's x_hat buffer and its dgate scratch this tile's dvalue buffer, which holds
   // the output until the store has read it.
   auto role = [&](int it_i, int r) {
     const uint32_t rr = static_cast<uint32_t>(0x1302012320313210ull >> (16 * (it_i & 3))) & 0xFFFFu;
     return tiles_s + ((rr >> (4 * r)) & 0xFu) * kBwdTile;
   };
-  auto issue_z = [&](int tile_i, int it_i) {
-    const int row_i = tile_i / p.tiles_per_row;
-    const int j_i = (tile_i - row_i * p.tiles_per_row) * 128;
-    const uint32_t z_i = role(it_i, 0);
-    mbar_arrive_expect_tx(z_full, kZHalves * 16384);
+  // (thread_wait: a thread that gives up sets the abort word and carries on; every later wait of the CTA returns within
+  // one poll, so that all warps walk through the same barriers to the end)
+  if (warp == kBwdThreads / 32) {
+    // ------------------------------------------------------------ copies and MMAs
+    auto issue_x = [&](int tile_i, int it_i) {
+      const int row_i = tile_i / p.tiles_per_row;
+      const int j_i = (tile_i - row_i * p.tiles_per_row) * 128;
+      mbar_arrive_expect_tx(x_full, kZHalves * 16384);
 #pragma unroll
-    for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(z_i + kh * 16384, &map_z, z_full, kh * 64, j_i, row_i);
-  };
-  auto issue_do = [&](int tile_i, int it_i) {
-    const int row_i = tile_i / p.tiles_per_row;
-    const int j_i = (tile_i - row_i * p.tiles_per_row) * 128;
-    const uint32_t do_i = role(it_i, 1);
-    mbar_arrive_expect_tx(do_full, kBwdTile);
+      for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(role(it_i, 0) + kh * 16384, &map_x, x_full, kh * 64, j_i, row_i);
+    };
+    auto issue_do = [&](int tile_i, int it_i) {
+      const int row_i = tile_i / p.tiles_per_row;
+      const int j_i = (tile_i - row_i * p.tiles_per_row) * 128;
+      mbar_arrive_expect_tx(do_full, kBwdTile);
 #pragma unroll
-    for (int kh = 0; kh < 2; ++kh) tma_load_3d(do_i + kh * 16384, &map_do, do_full, j_i + kh * 64, 0, row_i);
-  };
-  // The single-thread jobs of a tile sit on three different warps so that they do not queue behind one another: the MMA
-  // issue (threads 0 and 32), the TMA loads of the next tile (thread 96) and the TMA store with its bulk group (thread 64).
-  const bool load_thread = threadIdx.x == 96, store_thread = threadIdx.x == 64;
-  // tile -> (row, column block) without a division per tile
-  const int step_rows = static_cast<int>(gridDim.x) / p.tiles_per_row;
-  const int step_cols = static_cast<int>(gridDim.x) - step_rows * p.tiles_per_row;
-  int row = static_cast<int>(blockIdx.x) / p.tiles_per_row;
-  int jt = static_cast<int>(blockIdx.x) - row * p.tiles_per_row;
-  bool ok = true;
-  int it = 0;
-  int z_pending = -1, do_pending = -1;  // load thread: iteration whose copy is in flight, or -1
-  if (load_thread && static_cast<int>(blockIdx.x) < p.num_tiles) {
-    issue_z(blockIdx.x, 0);
-    issue_do(blockIdx.x, 0);
-    z_pending = 0, do_pending = 0;
-  }
-  if (part == 0 && static_cast<int>(blockIdx.x) < p.num_tiles) {
-    bool in0;
-    uint32_t a0, b0, c0;
-    mask_bytes(blockIdx.x, in0, a0, b0, c0);
-    publish_valid(0, in0, a0, b0, c0);
-  }
-  for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
-    if (it != 0) {
-      row += step_rows, jt += step_cols;
-      if (jt >= p.tiles_per_row) jt -= p.tiles_per_row, ++row;
-    }
-    const int j0 = jt * 128;
-    const uint32_t z_s = role(it, 0), do_s = role(it, 1), dv_s = role(it, 2), dg_s = role(it, 3);
-    const int j = j0 + pos;
-    if (it == 0) ok &= thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
-    ok &= thread_wait(z_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
-    if (load_thread) z_pending = -1;
-    // ---- phase 1: x_hat in place
-    const float rstd_in = normalise_tile<true, true, C>(z_s, xchg, pos, part, p.eps_in);
-    // this tile's dgate scratch held the previous tile's output: its store must have read it before phase 3 (the
-    // barrier that closes phase 1 orders this wait before every thread's phase 3)
-    if (store_thread) bulk_wait_read<0>();
-    fence_proxy_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    // ---- phase 2: value^T = Wv' x_hat^T (columns 0-127), gate^T = Wg' x_hat^T (128-255): lanes = contracted channels
-    // (the GEMMs of a round are issued by two threads, one per accumulator group: one thread's issue rate does not
-    // keep the tensor pipe busy)
-    if (threadIdx.x == 0 || threadIdx.x == 32) {
-      const int m = threadIdx.x >> 5;
+      for (int kh = 0; kh < 2; ++kh) tma_load_3d(role(it_i, 1) + kh * 16384, &map_do, do_full, j_i + kh * 64, 0, row_i);
+    };
+    // value^T = Wv' x_hat^T (columns 0-127), gate^T = Wg' x_hat^T (128-255): lanes = contracted channels
+    auto issue_fwd = [&](int it_i) {
+      thread_wait(x_full, it_i & 1, abort_flag, p.status, kDevTimeoutMma);
       tc_fence_after();
       constexpr uint32_t idesc = umma_idesc(128, 128, false, false, kFmtF16, kFmtF16);
-#pragma unroll
-      for (int ks = 0; ks < C / 16; ++ks) {
-        const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
-        umma_bf16(tmem_base + m * 128, umma_desc_kmajor((m == 0 ? wv_s : wg_s) + (ks >> 2) * 16384) + kb,
-                  umma_desc_kmajor(z_s + (ks >> 2) * 16384) + kb, idesc, ks != 0 ? 1u : 0u);
-      }
-      umma_commit(mma_bar);
-    }
-    bool nx_in = false;
-    uint32_t nx_i = 1u, nx_j = 1u, nx_p = 1u;
-    const bool has_next = tile + static_cast<int>(gridDim.x) < p.num_tiles;
-    if (part == 0 && has_next) mask_bytes(tile + gridDim.x, nx_in, nx_i, nx_j, nx_p);
-    ok &= thread_wait(mma_bar, 0, abort_flag, p.status, kDevTimeoutEpilogue);
-    tc_fence_after();
-    if (part == 0 && has_next) publish_valid(it + 1, nx_in, nx_i, nx_j, nx_p);
-    ok &= thread_wait(do_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
-    if (load_thread) do_pending = -1;
-    // ---- phase 3: dvalue, dgate for this thread's channel and 32 positions, stored [channel][position]
-    {
-      const uint32_t vbits = valid_words[(it & 1) * 4 + part];
-      uint32_t vv[32], vg[32];
-      tmem_ld32(tmem_base + lane_sel + part * 32, vv);
-      tmem_ld32(tmem_base + lane_sel + 128 + part * 32, vg);
-      uint4 dov[4];
-#pragma unroll
-      for (int k4 = 0; k4 < 4; ++k4) dov[k4] = ld_chunk(do_s + tile_chunk(pos, part * 4 + k4));
-      tmem_ld_wait();
-#pragma unroll
-      for (int k4 = 0; k4 < 4; ++k4) {
-        const uint32_t dw[4] = {dov[k4].x, dov[k4].y, dov[k4].z, dov[k4].w};
-        uint32_t ov[4], og[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          float2 d_o = f16x2_to_float2(dw[t]);
-          const int e0 = k4 * 8 + 2 * t;
-          if (vbits != 0xFFFFFFFFu) {
-            d_o.x = ((vbits >> e0) & 1u) ? d_o.x : 0.f;
-            d_o.y = ((vbits >> (e0 + 1)) & 1u) ? d_o.y : 0.f;
-          }
-          float dv2[2], dg2[2];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const float val = __uint_as_float(vv[e0 + u]) + c_value;
-            const float th = tanh_approx(fmaf(__uint_as_float(vg[e0 + u]), 0.5f, c_gate_half));
-            const float sg = fmaf(th, 0.5f, 0.5f);
-            const float sg16 = fmaf(th, 8.0f, 8.0f);  // the contraction's outputs are stored times 2^-4
-            dv2[u] = (u == 0 ? d_o.x : d_o.y) * sg16;
-            dg2[u] = dv2[u] * fmaf(-val, sg, val);
-            acc_sv += dv2[u];
-            acc_sg += dg2[u];
-          }
-          ov[t] = pack_f16x2_sat(make_float2(dv2[0], dv2[1]));
-          og[t] = pack_f16x2_sat(make_float2(dg2[0], dg2[1]));
-        }
-        const uint32_t addr = tile_chunk(pos, part * 4 + k4);
-        st_chunk(dv_s + addr, ov[0], ov[1], ov[2], ov[3]);
-        st_chunk(dg_s + addr, og[0], og[1], og[2], og[3]);
-      }
-    }
-    tc_fence_before();
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (load_thread && tile + static_cast<int>(gridDim.x) < p.num_tiles) {
-      issue_z(tile + gridDim.x, it + 1);  // into this tile's dO buffer, read for the last time in phase 3
-      z_pending = it + 1;
-    }
-    // ---- phase 4: d x_hat = dvalue Wv' + dgate Wg' (columns 0-127, lanes = positions); Mv += dvalue^T x_hat (256-383),
-    // Mg += dgate^T x_hat (384-511). dvalue / dgate are [channel][position] tiles: MN-major as the A operand of the
-    // first pair of GEMMs (M = positions), K-major as that of the second (M = channels, K = positions).
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      constexpr uint32_t idesc_d = umma_idesc(128, C, true, true, kFmtF16, kFmtF16);
+      const uint32_t x_s = role(it_i, 0);
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          umma_bf16(tmem_base, umma_desc_mnmajor((m == 0 ? dv_s : dg_s) + ks * 2048, 16384),
-                    umma_desc_mnmajor((m == 0 ? wv_s : wg_s) + ks * 2048, 16384), idesc_d, (m | ks) != 0 ? 1u : 0u);
-        }
-      }
-      umma_commit(mma_bar);
-    } else if (threadIdx.x == 32) {
-      tc_fence_after();
-      constexpr uint32_t idesc_m = umma_idesc(128, C, false, true, kFmtF16, kFmtF16);
-      const uint32_t accum = it != 0 ? 1u : 0u;
-#pragma unroll
-      for (int m = 0; m < 2; ++m) {
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
+        for (int ks = 0; ks < C / 16; ++ks) {
           const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
-          umma_bf16(tmem_base + 256 + m * 128, umma_desc_kmajor((m == 0 ? dv_s : dg_s) + (ks >> 2) * 16384) + kb,
-                    umma_desc_mnmajor(z_s + ks * 2048, 16384), idesc_m, (ks != 0 ? 1u : 0u) | accum);
+          umma_bf16(tmem_base + m * 128, umma_desc_kmajor((m == 0 ? wv_s : wg_s) + (ks >> 2) * 16384) + kb,
+                    umma_desc_kmajor(x_s + (ks >> 2) * 16384) + kb, idesc, ks != 0 ? 1u : 0u);
         }
       }
-      umma_commit(mma_bar);
-    }
-    // the running d x_hat of this thread's channels: requested now, used after the GEMM round
-    const bool inside = j < p.n;
-    uint4 dx_prev[kZChunks];
+      umma_commit(fwd_done);
+    };
+    if (lane == 0) {
+      mbar_arrive_expect_tx(w_full, 2 * kZHalves * 16384);
 #pragma unroll
-    for (int ch = 0; ch < kZChunks; ++ch) dx_prev[ch] = make_uint4(0u, 0u, 0u, 0u);
-    if (inside) {
-      const uint4* src = reinterpret_cast<const uint4*>(p.dx_in + (static_cast<size_t>(row) * p.n + j) * C + part * kZCh);
-      ldg_chunks(src, true, dx_prev);  // the workspace is 1024-byte aligned
-    }
-    uint4 dy_res[LAST ? kZChunks : 2];  // LAST: the residual branch's share of dz, requested at the same time
-    if constexpr (LAST) {
-#pragma unroll
-      for (int ch = 0; ch < kZChunks; ++ch) dy_res[ch] = make_uint4(0u, 0u, 0u, 0u);
-      if (p.dy != nullptr && inside) {
-        const uint4* dyp = reinterpret_cast<const uint4*>(p.dy + (static_cast<size_t>(row) * p.n + j) * C + part * kZCh);
-        ldg_chunks(dyp, (reinterpret_cast<uintptr_t>(p.dy) & 31u) == 0, dy_res);
+      for (int kh = 0; kh < kZHalves; ++kh) {
+        tma_load_2d(wv_s + kh * 16384, &map_wv, w_full, kh * 64, 0);
+        tma_load_2d(wg_s + kh * 16384, &map_wg, w_full, kh * 64, 0);
       }
+      issue_x(blockIdx.x, 0);
+      issue_do(blockIdx.x, 0);
+      thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
+      issue_fwd(0);
     }
-    ok &= thread_wait(mma_bar, 1, abort_flag, p.status, kDevTimeoutEpilogue);
-    tc_fence_after();
-    if (load_thread && tile + static_cast<int>(gridDim.x) < p.num_tiles) {
-      issue_do(tile + gridDim.x, it + 1);  // into this tile's dgate buffer, free once the gradient GEMMs are done
-      do_pending = it + 1;
+    int it = 0;
+    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
+      const int next = tile + static_cast<int>(gridDim.x);
+      const bool has_next = next < p.num_tiles;
+      const uint32_t x_s = role(it, 0), dv_s = role(it, 2), dg_s = role(it, 3);
+      named_bar_sync(kBarA, kBwdProThreads);  // dvalue and dgate are written, value / gate and dO are read
+      if (lane == 0) {
+        // d x_hat = dvalue Wv' + dgate Wg' (columns 0-127, lanes = positions); Mv += dvalue^T x_hat (256-383), Mg +=
+        // dgate^T x_hat (384-511). dvalue / dgate are [channel][position] tiles: MN-major as the A operand of the first
+        // pair of GEMMs (M = positions), K-major as that of the second (M = channels, K = positions).
+        tc_fence_after();
+        constexpr uint32_t idesc_d = umma_idesc(128, C, true, true, kFmtF16, kFmtF16);
+        constexpr uint32_t idesc_m = umma_idesc(128, C, false, true, kFmtF16, kFmtF16);
+        const uint32_t accum = it != 0 ? 1u : 0u;
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks)
+            umma_bf16(tmem_base, umma_desc_mnmajor((m == 0 ? dv_s : dg_s) + ks * 2048, 16384),
+                      umma_desc_mnmajor((m == 0 ? wv_s : wg_s) + ks * 2048, 16384), idesc_d, (m | ks) != 0 ? 1u : 0u);
+        }
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) {
+            const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
+            umma_bf16(tmem_base + 256 + m * 128, umma_desc_kmajor((m == 0 ? dv_s : dg_s) + (ks >> 2) * 16384) + kb,
+                      umma_desc_mnmajor(x_s + ks * 2048, 16384), idesc_m, (ks != 0 ? 1u : 0u) | accum);
+          }
+        }
+        umma_commit(grad_done);
+        thread_wait(do_full, it & 1, abort_flag, p.status, kDevTimeoutMma);  // (long since complete: the arithmetic read it)
+        if (has_next) {
+          issue_x(next, it + 1);
+          thread_wait(grad_done, it & 1, abort_flag, p.status, kDevTimeoutMma);
+          issue_do(next, it + 1);
+        }
+      }
+      __syncwarp();
+      named_bar_sync(kBarB, kBwdProThreads);  // d x_hat has left tensor memory
+      if (lane == 0 && has_next) issue_fwd(it + 1);
+      __syncwarp();
+      named_bar_sync(kBarC, kBwdProThreads);  // the output tile is written
+      if (lane == 0) {
+        const int row = tile / p.tiles_per_row;
+        const int j0 = (tile - row * p.tiles_per_row) * 128;
+#pragma unroll
+        for (int kh = 0; kh < kZHalves; ++kh) tma_store_3d(&map_out, dv_s + kh * 16384, kh * 64, j0, row);
+        bulk_commit();
+        bulk_wait_read<0>();
+        mbar_arrive(out_free);
+      }
+      __syncwarp();
     }
-    // ---- phase 5: add the running d x_hat; !LAST: write it back, LAST: LayerNorm backward + residual -> dz
+    if (lane == 0) {
+      // Every copy has been waited for above unless the CTA is giving up; then those in flight must land before it exits
+      // (the last iteration issued none, so the phases to look at are the last tile's).
+      if (*abort_flag != 0) {
+        const uint32_t last = static_cast<uint32_t>((it - 1) & 1);
+        const long long t0 = clock64();
+        while (!mbar_try_wait(w_full, 0) || !mbar_try_wait(x_full, last) || !mbar_try_wait(do_full, last)) {
+          if (clock64() - t0 > kWaitLimitCycles) {
+            atomicCAS(p.status, 0, kDevTimeoutDrain);
+            break;
+          }
+        }
+      }
+      bulk_wait<0>();
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------ arithmetic
+    const int q = warp & 3, part = warp >> 2;
+    const int pos = q * 32 + lane;
+    const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
+    const float gc_inv = p.grad_scale[1];
+    const float c_value = p.consts[pos], c_gate_half = 0.5f * p.consts[128 + pos];  // this thread's channel
+    // dvalue / dgate are formed on the transposed projections (TMEM lanes = contracted channels, columns = positions): a
+    // thread owns channel `pos` (its lane) and the position quarter `part`, so its constants and its column sums are
+    // scalars and dO, stored [channel][position], is read in 16-byte runs of positions.
+    float acc_sv = 0.f, acc_sg = 0.f;
+    // validity of the 32 positions of this warp's quarter, one bit each. The mask bytes of the NEXT tile are requested
+    // before a GEMM wait and turned into the word after it, so that their latency is off the path.
+    auto mask_bytes = [&](int row_i, int j_i, uint32_t& m_i, uint32_t& m_j, uint32_t& m_p) {
+      const int b = row_i / p.n;
+      const int i = row_i - b * p.n;
+      const int j = j_i + part * 32 + lane;
+      m_i = 1u, m_j = j < p.n ? 1u : 0u, m_p = 1u;
+      if (j < p.n) {
+        if (p.token_mask != nullptr) {
+          m_i = p.token_mask[static_cast<size_t>(b) * p.n + i];
+          m_j = p.token_mask[static_cast<size_t>(b) * p.n + j];
+        }
+        if (p.pair_mask != nullptr) m_p = p.pair_mask[(static_cast<size_t>(b) * p.n + i) * p.n + j];
+      }
+    };
+    // tile -> (row, column block) without a division per tile
+    const int step_rows = static_cast<int>(gridDim.x) / p.tiles_per_row;
+    const int step_cols = static_cast<int>(gridDim.x) - step_rows * p.tiles_per_row;
+    int row = static_cast<int>(blockIdx.x) / p.tiles_per_row;
+    int jt = static_cast<int>(blockIdx.x) - row * p.tiles_per_row;
+    uint32_t vbits;
     {
-      float tot[kZCh];
-      float s1 = 0.f, s2 = 0.f;
+      uint32_t m_i, m_j, m_p;
+      mask_bytes(row, jt * 128, m_i, m_j, m_p);
+      vbits = __ballot_sync(0xFFFFFFFFu, m_i != 0u && m_j != 0u && m_p != 0u);
+    }
+    int it = 0;
+    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
+      const int j0 = jt * 128;
+      const uint32_t x_s = role(it, 0), do_s = role(it, 1), dv_s = role(it, 2), dg_s = role(it, 3);
+      const int j = j0 + pos;
+      const bool inside = j < p.n;
+      const size_t cell = (static_cast<size_t>(row) * p.n + j) * C + part * kZCh;  // (read only when inside)
+      const size_t rcell = static_cast<size_t>(row) * p.ld + j;
+      thread_wait(fwd_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
+      __syncwarp();
+      tc_fence_after();
+      thread_wait(do_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+      __syncwarp();
+      // ---- dvalue, dgate for this thread's channel and 32 positions, stored [channel][position]
+      {
+        uint32_t dg_p[16];  // (the dgate buffer still holds the previous tile's output while its store reads it)
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t vv[16], vg[16];
+          tmem_ld16(tmem_base + lane_sel + part * 32 + hf * 16, vv);
+          tmem_ld16(tmem_base + lane_sel + 128 + part * 32 + hf * 16, vg);
+          uint4 dov[2];
+#pragma unroll
+          for (int k4 = 0; k4 < 2; ++k4) dov[k4] = ld_chunk(do_s + tile_chunk(pos, part * 4 + hf * 2 + k4));
+          tmem_ld_wait();
+#pragma unroll
+          for (int k4 = 0; k4 < 2; ++k4) {
+            const uint32_t dw[4] = {dov[k4].x, dov[k4].y, dov[k4].z, dov[k4].w};
+            uint32_t ov[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              float2 d_o = f16x2_to_float2(dw[t]);
+              const int e0 = k4 * 8 + 2 * t;
+              if (vbits != 0xFFFFFFFFu) {
+                d_o.x = ((vbits >> (hf * 16 + e0)) & 1u) ? d_o.x : 0.f;
+                d_o.y = ((vbits >> (hf * 16 + e0 + 1)) & 1u) ? d_o.y : 0.f;
+              }
+              float dv2[2], dg2[2];
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+                const float val = __uint_as_float(vv[e0 + u]) + c_value;
+                const float th = tanh_approx(fmaf(__uint_as_float(vg[e0 + u]), 0.5f, c_gate_half));
+                const float sg = fmaf(th, 0.5f, 0.5f);
+                const float sg16 = fmaf(th, 8.0f, 8.0f);  // the contraction's outputs are stored times 2^-4
+                dv2[u] = (u == 0 ? d_o.x : d_o.y) * sg16;
+                dg2[u] = dv2[u] * fmaf(-val, sg, val);
+                acc_sv += dv2[u];
+                acc_sg += dg2[u];
+              }
+              ov[t] = pack_f16x2_sat(make_float2(dv2[0], dv2[1]));
+              dg_p[hf * 8 + k4 * 4 + t] = pack_f16x2_sat(make_float2(dg2[0], dg2[1]));
+            }
+            st_chunk(dv_s + tile_chunk(pos, part * 4 + hf * 2 + k4), ov[0], ov[1], ov[2], ov[3]);
+          }
+        }
+        if (it != 0) thread_wait(out_free, (it - 1) & 1, abort_flag, p.status, kDevTimeoutStats);
+#pragma unroll
+        for (int k4 = 0; k4 < 4; ++k4)
+          st_chunk(dg_s + tile_chunk(pos, part * 4 + k4), dg_p[k4 * 4], dg_p[k4 * 4 + 1], dg_p[k4 * 4 + 2], dg_p[k4 * 4 + 3]);
+      }
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      named_bar_arrive(kBarA, kBwdProThreads);
+      // the running d x_hat of this thread's channels, LAST: the residual branch's share of dz and rstd, and the next
+      // tile's mask bytes: requested now, used after the GEMM round
+      uint4 dx_prev[kZChunks];
+      uint4 dy_res[LAST ? kZChunks : 2];
+      float rstd_in = 0.f;
+#pragma unroll
+      for (int ch = 0; ch < kZChunks; ++ch) dx_prev[ch] = make_uint4(0u, 0u, 0u, 0u);
+      if (inside) ldg_chunks(reinterpret_cast<const uint4*>(p.dx_in + cell), true, dx_prev);  // (workspace: 1024-byte aligned)
+      if constexpr (LAST) {
+#pragma unroll
+        for (int ch = 0; ch < kZChunks; ++ch) dy_res[ch] = make_uint4(0u, 0u, 0u, 0u);
+        if (inside) {
+          if (p.dy != nullptr)
+            ldg_chunks(reinterpret_cast<const uint4*>(p.dy + cell), (reinterpret_cast<uintptr_t>(p.dy) & 31u) == 0, dy_res);
+          rstd_in = __ldg(p.rstd + rcell);
+        }
+      }
+      const bool has_next = tile + static_cast<int>(gridDim.x) < p.num_tiles;
+      row += step_rows, jt += step_cols;
+      if (jt >= p.tiles_per_row) jt -= p.tiles_per_row, ++row;
+      uint32_t m_i = 0u, m_j = 0u, m_p = 0u;
+      if (has_next) mask_bytes(row, jt * 128, m_i, m_j, m_p);
+      thread_wait(grad_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
+      __syncwarp();
+      tc_fence_after();
+      vbits = __ballot_sync(0xFFFFFFFFu, m_i != 0u && m_j != 0u && m_p != 0u);
+      // ---- add the running d x_hat; !LAST: write it back, LAST: LayerNorm backward + residual -> dz
       uint32_t vt[kZChunks][8];
 #pragma unroll
       for (int ch = 0; ch < kZChunks; ++ch) tmem_ld8(tmem_base + lane_sel + part * kZCh + ch * 8, vt[ch]);
       tmem_ld_wait();
+      tc_fence_before();
+      if constexpr (!LAST) {
+        __syncwarp();
+        named_bar_arrive(kBarB, kBwdProThreads);
 #pragma unroll
-      for (int ch = 0; ch < kZChunks; ++ch) {
-        const uint32_t(&v)[8] = vt[ch];
-        const uint4 in = dx_prev[ch];
-        uint4 xh = make_uint4(0u, 0u, 0u, 0u);
-        if constexpr (LAST) xh = ld_chunk(z_s + tile_chunk(pos, part * kZChunks + ch));
-        const uint32_t iw[4] = {in.x, in.y, in.z, in.w};
-        const uint32_t xw[4] = {xh.x, xh.y, xh.z, xh.w};
+        for (int ch = 0; ch < kZChunks; ++ch) {
+          const uint32_t iw[4] = {dx_prev[ch].x, dx_prev[ch].y, dx_prev[ch].z, dx_prev[ch].w};
+          uint32_t o[4];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const float2 a = f16x2_to_float2(iw[t]);
-          const float t0 = __uint_as_float(v[2 * t]) + a.x, t1 = __uint_as_float(v[2 * t + 1]) + a.y;
-          tot[ch * 8 + 2 * t] = t0;
-          tot[ch * 8 + 2 * t + 1] = t1;
-          if constexpr (LAST) {
+          for (int t = 0; t < 4; ++t) {
+            const float2 a = f16x2_to_float2(iw[t]);
+            o[t] = pack_f16x2_sat(
+                make_float2(__uint_as_float(vt[ch][2 * t]) + a.x, __uint_as_float(vt[ch][2 * t + 1]) + a.y));
+          }
+          st_chunk(dv_s + tile_chunk(pos, part * kZChunks + ch), o[0], o[1], o[2], o[3]);
+        }
+      } else {
+        float tot[kZCh];
+        uint4 xh[kZChunks];
+        float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+        for (int ch = 0; ch < kZChunks; ++ch) {
+          // x_hat is read for the last time before barrier B: the next tile's dvalue is written over it
+          xh[ch] = ld_chunk(x_s + tile_chunk(pos, part * kZChunks + ch));
+          const uint32_t iw[4] = {dx_prev[ch].x, dx_prev[ch].y, dx_prev[ch].z, dx_prev[ch].w};
+          const uint32_t xw[4] = {xh[ch].x, xh[ch].y, xh[ch].z, xh[ch].w};
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const float2 a = f16x2_to_float2(iw[t]);
             const float2 x = f16x2_to_float2(xw[t]);
+            const float t0 = __uint_as_float(vt[ch][2 * t]) + a.x, t1 = __uint_as_float(vt[ch][2 * t + 1]) + a.y;
+            tot[ch * 8 + 2 * t] = t0;
+            tot[ch * 8 + 2 * t + 1] = t1;
             s1 += t0 + t1;
             s2 = fmaf(t0, x.x, fmaf(t1, x.y, s2));
           }
         }
-      }
-      if constexpr (!LAST) {
-#pragma unroll
-        for (int ch = 0; ch < kZChunks; ++ch)
-          st_chunk(dv_s + tile_chunk(pos, part * kZChunks + ch), pack_f16x2_sat(make_float2(tot[ch * 8], tot[ch * 8 + 1])),
-                   pack_f16x2_sat(make_float2(tot[ch * 8 + 2], tot[ch * 8 + 3])),
-                   pack_f16x2_sat(make_float2(tot[ch * 8 + 4], tot[ch * 8 + 5])),
-                   pack_f16x2_sat(make_float2(tot[ch * 8 + 6], tot[ch * 8 + 7])));
-      } else {
-        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + kBwdXchgHalf + (part * 128 + pos) * 8), "f"(s1), "f"(s2)
-                     : "memory");
-        named_bar_sync(1, kBwdThreads);
+        // (written again only after barrier A of the next tile, which every thread arrives at after its reads below)
+        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + (part * 128 + pos) * 8), "f"(s1), "f"(s2) : "memory");
+        __syncwarp();
+        named_bar_sync(kBarB, kBwdProThreads);
         float m1, m2;
-        sum_partials(xchg + kBwdXchgHalf, pos, m1, m2);
+        sum_partials(xchg, pos, m1, m2);
         m1 *= 1.0f / C, m2 *= 1.0f / C;
         const float rs = rstd_in * gc_inv;
 #pragma unroll
         for (int ch = 0; ch < kZChunks; ++ch) {
-          const uint4 xh = ld_chunk(z_s + tile_chunk(pos, part * kZChunks + ch));
-          const uint4 dyv = dy_res[ch];
-          const uint32_t xw[4] = {xh.x, xh.y, xh.z, xh.w};
-          const uint32_t dw[4] = {dyv.x, dyv.y, dyv.z, dyv.w};
+          const uint32_t xw[4] = {xh[ch].x, xh[ch].y, xh[ch].z, xh[ch].w};
+          const uint32_t dw[4] = {dy_res[ch].x, dy_res[ch].y, dy_res[ch].z, dy_res[ch].w};
           uint32_t o[4];
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
@@ -1115,33 +1168,11 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
           st_chunk(dv_s + tile_chunk(pos, part * kZChunks + ch), o[0], o[1], o[2], o[3]);
         }
       }
+      fence_proxy_async_smem();
+      __syncwarp();
+      named_bar_arrive(kBarC, kBwdProThreads);
     }
-    tc_fence_before();
-    fence_proxy_async_smem();
-    ok = __syncthreads_and(ok ? 1 : 0) != 0;  // a thread that gave up takes the whole CTA out here
-    if (!ok) break;
-    if (store_thread) {
-#pragma unroll
-      for (int kh = 0; kh < kZHalves; ++kh) tma_store_3d(&map_out, dv_s + kh * 16384, kh * 64, j0, row);
-      bulk_commit();
-    }
-  }
-  if (store_thread) bulk_wait<0>();
-  if (load_thread) {
-    if (!ok) {  // a wait gave up: copies in flight must land before the CTA exits
-      const long long t0 = clock64();
-      while (!mbar_try_wait(w_full, 0) || (z_pending >= 0 && !mbar_try_wait(z_full, z_pending & 1)) ||
-             (do_pending >= 0 && !mbar_try_wait(do_full, do_pending & 1))) {
-        if (clock64() - t0 > kWaitLimitCycles) {
-          atomicCAS(p.status, 0, kDevTimeoutDrain);
-          break;
-        }
-      }
-    }
-  }
-  __syncthreads();
-  if (ok && it > 0) {
-    tc_fence_after();
+    // ---- per-CTA partials of the weight gradients (every GEMM has been waited for) and of the column sums
     float* pm = p.part_m + static_cast<size_t>(blockIdx.x) * 2 * 128 * 128;
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
@@ -1155,13 +1186,13 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
         dst[1] = make_float4(__uint_as_float(v[4]), __uint_as_float(v[5]), __uint_as_float(v[6]), __uint_as_float(v[7]));
       }
     }
-  }
-  {  // column sums: the four position quarters of a channel, fixed order
-    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + (part * 128 + pos) * 8), "f"(acc_sv), "f"(acc_sg) : "memory");
-    __syncthreads();
+    // column sums: the four position quarters of a channel, fixed order
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + kBwdXchgHalf + (part * 128 + pos) * 8), "f"(acc_sv), "f"(acc_sg)
+                 : "memory");
+    named_bar_sync(1, kBwdThreads);
     if (threadIdx.x < 128) {
       float a, b;
-      sum_partials(xchg, threadIdx.x, a, b);
+      sum_partials(xchg + kBwdXchgHalf, threadIdx.x, a, b);
       float* ps = p.part_s + static_cast<size_t>(blockIdx.x) * 2 * 128;
       ps[threadIdx.x] = a;
       ps[128 + threadIdx.x] = b;

@@ -125,6 +125,10 @@ __device__ __forceinline__ void tc_fence_after() {
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
+// The arriving side of a barrier other threads of the `nthreads` wait at (orders this thread's earlier memory accesses).
+__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
 
 // Barrier over `nthreads` threads that also ANDs a predicate across them, so that a group of warps
 // takes the same give-up decision and never splits around a later barrier.
