@@ -204,6 +204,15 @@ __device__ __forceinline__ void flush_colsums(const float (&a0)[NCH], const floa
   __syncthreads();
 }
 
+// Eight columns (8 * chunk ..) of row `row` of a CTA's partial weight gradient. The matrix lies in memory as [32 groups of
+// four columns][128 rows] float4, so that a warp, whose lanes hold consecutive rows, stores 512 contiguous bytes (row by
+// row its 32 lanes would hit 32 different lines with every store: 12 us per launch for the two matrices of 148 CTAs).
+__device__ __forceinline__ void store_partial(float* m, int row, int chunk, const uint32_t (&v)[8]) {
+  float4* dst = reinterpret_cast<float4*>(m) + chunk * 2 * 128 + row;
+  dst[0] = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
+  dst[128] = make_float4(__uint_as_float(v[4]), __uint_as_float(v[5]), __uint_as_float(v[6]), __uint_as_float(v[7]));
+}
+
 struct BwdEpilogueParams {
   int tiles_per_row;   // ceil(N / 128)
   int num_tiles;       // B * N * tiles_per_row
@@ -214,7 +223,7 @@ struct BwdEpilogueParams {
   const uint16_t* drop_scale;  // [B][N][128] bf16 or null
   float eps_in;
   float eps_out;       // scaled by 2^-8: tri is stored times 2^-4
-  float* part_m;       // [grid][2][128][128]: per-CTA partial sums of dproj^T t_hat and dgate^T x_hat
+  float* part_m;       // [grid][2] matrices as store_partial lays them out: per-CTA partial sums of dproj^T t_hat and dgate^T x_hat
   float* part_s;       // [grid][2][128]: per-CTA column sums of dproj and dgate
   // the two-launch form for an output LayerNorm over 256 channels (MODE 1: first 128 channels, MODE 2: the others)
   const float2* ext_stats;  // [B*N][ld]: mean and rstd of the stored t over all 256 channels
@@ -644,9 +653,7 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
         uint32_t v[8];
         tmem_ld8(tmem_base + lane_sel + 256 + m * 128 + part * kBwdCh + ch * 8, v);
         tmem_ld_wait();
-        float4* dst = reinterpret_cast<float4*>(pm + (m * 128 + pos) * 128 + part * kBwdCh + ch * 8);
-        dst[0] = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
-        dst[1] = make_float4(__uint_as_float(v[4]), __uint_as_float(v[5]), __uint_as_float(v[6]), __uint_as_float(v[7]));
+        store_partial(pm + m * 128 * 128, pos, part * kBwdChunks + ch, v);
       }
     }
   }
@@ -781,7 +788,7 @@ struct BwdPrologueParams {
   const uint16_t* dx_in;      // [B*N][N][C] fp16: c * d loss / d x_hat gathered so far (read)
   const uint16_t* dy;         // LAST only: upstream gradient [B*N][N][C] bf16 (the residual path), or null
   const float* rstd;          // LAST only: [B*N][ld] 1 / standard deviation of the input LayerNorm
-  float* part_m;              // [grid][2][128][128]: partial dvalue^T x_hat, dgate^T x_hat
+  float* part_m;              // [grid][2] matrices (store_partial): partial dvalue^T x_hat, dgate^T x_hat
   float* part_s;              // [grid][2][128]
   int* status;
 };
@@ -1181,9 +1188,7 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         uint32_t v[8];
         tmem_ld8(tmem_base + lane_sel + 256 + m * 128 + part * kBwdCh + ch * 8, v);
         tmem_ld_wait();
-        float4* dst = reinterpret_cast<float4*>(pm + (m * 128 + pos) * 128 + part * kBwdCh + ch * 8);
-        dst[0] = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
-        dst[1] = make_float4(__uint_as_float(v[4]), __uint_as_float(v[5]), __uint_as_float(v[6]), __uint_as_float(v[7]));
+        store_partial(pm + m * 128 * 128, pos, part * kBwdChunks + ch, v);
       }
     }
     // column sums: the four position quarters of a channel, fixed order
@@ -1336,20 +1341,20 @@ __global__ void __launch_bounds__(256) bwd_setup_kernel(const __grid_constant__ 
 // over the matrices that read that LayerNorm (the output one: matrix 4; the input one: the other five).
 // One set of six 128 x 128 matrices ("half"): the unidirectional module has one, the bidirectional module two, whose
 // matrices are row or column blocks of the module's wider parameters, hence the leading dimensions.
-// Grid (128 rows, 6 matrices, halves); a block of 512 threads adds one row of the partials, 16 groups of CTAs by 32
-// four-column pieces, every load of a thread in flight at once, and combines the groups in a fixed order: the sums, the
-// parameter gradients and the rows of the LayerNorm sums leave in one pass over the partials. The earlier form (a
-// reduction after every launch that produced partials, then a kernel for the gradients on 6 x 8 blocks, and one block for
-// the LayerNorm sums) was three to six launches of 5.2 us plus 10 and 5 us.
+// Grid (128: group of four columns and quarter of the rows, 6 matrices, halves); a block of 512 threads adds 32 rows x 4
+// columns of the partials, one group of CTAs per warp, every load of a thread in flight at once, and combines the groups
+// in a fixed order: the sums, the parameter gradients and this block's share of the LayerNorm sums leave in one pass over
+// the partials. The earlier form (a reduction after every launch that produced partials, then a kernel for the gradients on
+// 6 x 8 blocks, and one block for the LayerNorm sums) was three to six launches of 5.2 us plus 10 and 5 us.
 constexpr int kFinGroups = 16;
 constexpr int kFinFlight = 10;  // 16 * 10 = 160 = the largest number of CTAs
 struct BwdFinalHalf {
   PackArgs w;              // raw weights (this half's blocks, with their leading dimensions) and LayerNorm parameters
-  const float* part_m[6];  // per matrix: [n_parts][2][128][128] partials, at this matrix's [128][128] of CTA 0
+  const float* part_m[6];  // per matrix: partials [n_parts][2] matrices, at this matrix of CTA 0
   const float* part_s[6];  // per matrix: [n_parts][2][128]
   float* dw[6];            // fp32 gradient blocks
   int dw_ld[6];            // their leading dimensions
-  float* ln_rows;          // [6][128][2][128]: this matrix row's terms of dgamma and dbeta
+  float* ln_rows;          // [6][4][2][128]: the terms of dgamma and dbeta from 32 matrix rows each
   unsigned mask;           // bit m set: matrix m is present in this half
 };
 struct BwdFinalArgs {
@@ -1357,72 +1362,86 @@ struct BwdFinalArgs {
   int n_parts;
   const float* scale;  // [2]
 };
-// rows [n_parts] of 128 floats, `stride` floats apart, summed into `out` (512 threads; comb is float[16][128])
-__device__ __forceinline__ float4 sum_partial_rows(const float* parts, size_t stride, int n_parts, float4* comb) {
-  const int piece = threadIdx.x & 31, g = threadIdx.x >> 5;
+// Sums over the CTAs, for the block's 32 rows (lanes): four columns of the matrix (`m` points at CTA 0's, matrices
+// `m_stride` floats apart) and the column sum belonging to the row (`col_sum` likewise, or null). Valid in warp 0.
+__device__ __forceinline__ void sum_partials_of_rows(const float* m, size_t m_stride, const float* col_sum, size_t s_stride,
+                                                     int n_parts, int group, int row0, float4& mv, float& sv) {
+  __shared__ float4 comb[kFinGroups * 32];
+  __shared__ float comb_s[kFinGroups * 32];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   float4 v[kFinFlight];
+  float c[kFinFlight];
 #pragma unroll
   for (int u = 0; u < kFinFlight; ++u) {
-    const int i = g + u * kFinGroups;
-    v[u] = i < n_parts ? __ldcg(reinterpret_cast<const float4*>(parts + static_cast<size_t>(i) * stride) + piece)
-                       : make_float4(0.f, 0.f, 0.f, 0.f);
+    const size_t i = g + u * kFinGroups;
+    const bool there = g + u * kFinGroups < n_parts;
+    v[u] = there ? __ldcg(reinterpret_cast<const float4*>(m + i * m_stride) + group * 128 + row0 + lane)
+                 : make_float4(0.f, 0.f, 0.f, 0.f);
+    c[u] = there && col_sum != nullptr ? __ldcg(col_sum + i * s_stride + row0 + lane) : 0.f;
   }
   float4 s = v[0];
+  float t = c[0];
 #pragma unroll
-  for (int u = 1; u < kFinFlight; ++u) s.x += v[u].x, s.y += v[u].y, s.z += v[u].z, s.w += v[u].w;
-  comb[g * 32 + piece] = s;
+  for (int u = 1; u < kFinFlight; ++u) s.x += v[u].x, s.y += v[u].y, s.z += v[u].z, s.w += v[u].w, t += c[u];
+  comb[g * 32 + lane] = s;
+  comb_s[g * 32 + lane] = t;
   __syncthreads();
-  float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+  mv = make_float4(0.f, 0.f, 0.f, 0.f);
+  sv = 0.f;
   if (g == 0) {
 #pragma unroll
     for (int q = 0; q < kFinGroups; ++q) {
-      const float4 x = comb[q * 32 + piece];
-      t.x += x.x, t.y += x.y, t.z += x.z, t.w += x.w;
+      const float4 x = comb[q * 32 + lane];
+      mv.x += x.x, mv.y += x.y, mv.z += x.z, mv.w += x.w;
+      sv += comb_s[q * 32 + lane];
     }
   }
-  return t;  // warp 0: columns 4 * piece .. + 3
 }
-// the sum over the CTAs of one float, `stride` floats apart, by one warp (every lane returns it)
-__device__ __forceinline__ float sum_partial_scalar(const float* part, size_t stride, int n_parts) {
-  float s = 0.f;
-  for (int i = threadIdx.x & 31; i < n_parts; i += 32) s += __ldcg(part + static_cast<size_t>(i) * stride);
+// the sum of a value over the 32 lanes (rows) of a warp
+__device__ __forceinline__ float sum_lanes(float x) {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, off);
-  return s;
+  for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xFFFFFFFFu, x, off);
+  return x;
+}
+// warp 0: one row per lane; w, mv: four columns of the weights and of M / c, sv: S / c. Lane 0 writes the block's terms.
+__device__ __forceinline__ void store_ln_terms(float* dst, const float (&w)[4], const float (&mv)[4], float sv) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const float a = sum_lanes(w[t] * mv[t]), b = sum_lanes(w[t] * sv);
+    if (lane == 0) dst[t] = a, dst[128 + t] = b;
+  }
 }
 __global__ void __launch_bounds__(512) bwd_finalize_kernel(const __grid_constant__ BwdFinalArgs args) {
-  __shared__ float4 comb[kFinGroups * 32];
   const BwdFinalHalf& a = args.half[blockIdx.z];
-  const int r = blockIdx.x, m = blockIdx.y;
-  const int n_rows = m < 4 ? 128 : a.w.c, n_cols = m == 4 ? 128 : a.w.c;  // a.w.c = d_pair
-  if (((a.mask >> m) & 1u) == 0u || r >= n_rows) return;
-  const float4 mv4 = sum_partial_rows(a.part_m[m] + r * 128, 2 * 128 * 128, args.n_parts, comb);
-  const int k0 = (threadIdx.x & 31) * 4;
+  const int group = blockIdx.x >> 2, q = blockIdx.x & 3, m = blockIdx.y;
+  const int n_rows = m < 4 ? 128 : a.w.c, n_cols = m == 4 ? 128 : a.w.c;  // a.w.c = d_pair: 128 or 64
+  if (((a.mask >> m) & 1u) == 0u || q * 32 >= n_rows || group * 4 >= n_cols) return;
+  float4 m4;
+  float s1;
+  sum_partials_of_rows(a.part_m[m], 2 * 128 * 128, a.part_s[m], 2 * 128, args.n_parts, group, q * 32, m4, s1);
   if (threadIdx.x >= 32) return;
-  const float sum_s = sum_partial_scalar(a.part_s[m] + r, 2 * 128, args.n_parts);
-  if (k0 >= n_cols) return;
+  const int r = q * 32 + threadIdx.x, k0 = group * 4;
   const float cinv = args.scale[1];
+  const float sv = s1 * cinv, mv[4] = {m4.x * cinv, m4.y * cinv, m4.z * cinv, m4.w * cinv};
   const float4 gamma = *reinterpret_cast<const float4*>((m == 4 ? a.w.ln_out_w : a.w.ln_in_w) + k0);
   const float4 beta = *reinterpret_cast<const float4*>((m == 4 ? a.w.ln_out_b : a.w.ln_in_b) + k0);
   const size_t wi = static_cast<size_t>(r) * a.w.ld[m] + k0;
-  float4 w;
+  float w[4];
   if (a.w.f32_weights) {
-    w = *reinterpret_cast<const float4*>(static_cast<const float*>(a.w.w[m]) + wi);
+    const float4 v = *reinterpret_cast<const float4*>(static_cast<const float*>(a.w.w[m]) + wi);
+    w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
   } else {
     const uint2 v = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(a.w.w[m]) + wi);
-    w = make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
+    w[0] = bf16_lo(v.x), w[1] = bf16_hi(v.x), w[2] = bf16_lo(v.y), w[3] = bf16_hi(v.y);
   }
-  const float sv = sum_s * cinv;
-  const float4 mv = make_float4(mv4.x * cinv, mv4.y * cinv, mv4.z * cinv, mv4.w * cinv);
   float* dw = a.dw[m] + static_cast<size_t>(r) * a.dw_ld[m] + k0;
-  dw[0] = fmaf(mv.x, gamma.x, sv * beta.x), dw[1] = fmaf(mv.y, gamma.y, sv * beta.y);
-  dw[2] = fmaf(mv.z, gamma.z, sv * beta.z), dw[3] = fmaf(mv.w, gamma.w, sv * beta.w);
-  float4* ln = reinterpret_cast<float4*>(a.ln_rows + (static_cast<size_t>(m) * 128 + r) * 256 + k0);
-  ln[0] = make_float4(w.x * mv.x, w.y * mv.y, w.z * mv.z, w.w * mv.w);
-  ln[32] = make_float4(w.x * sv, w.y * sv, w.z * sv, w.w * sv);
+  dw[0] = fmaf(mv[0], gamma.x, sv * beta.x), dw[1] = fmaf(mv[1], gamma.y, sv * beta.y);
+  dw[2] = fmaf(mv[2], gamma.z, sv * beta.z), dw[3] = fmaf(mv[3], gamma.w, sv * beta.w);
+  store_ln_terms(a.ln_rows + (m * 4 + q) * 256 + k0, w, mv, sv);
 }
-// Adds the rows of the LayerNorm sums in a fixed order. Grid (2: dgamma or dbeta, 1 + halves: the input LayerNorm, then the
-// output LayerNorm's 128 channels of each half); 1024 threads: 32 four-column pieces by 32 groups of rows.
+// Adds the LayerNorm terms in a fixed order. Grid 1 + halves: the input LayerNorm, then the output LayerNorm's 128 channels
+// of each half; thread = gamma or beta and channel.
 struct BwdLnArgs {
   const float* ln_rows[2];  // per half
   unsigned mask[2];
@@ -1431,40 +1450,21 @@ struct BwdLnArgs {
   float* d_out[2];  // of the output LayerNorm [128 * halves]: half h at + 128 h
   int c;            // d_pair
 };
-__global__ void __launch_bounds__(1024) bwd_finalize_ln_kernel(const BwdLnArgs a) {
-  __shared__ float4 comb[32 * 32];
-  const int piece = threadIdx.x & 31, g = threadIdx.x >> 5, vec = blockIdx.x;
-  const bool input = blockIdx.y == 0;
-  const int n_cols = input ? a.c : 128;
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (piece * 4 < n_cols) {
-    for (int h = input ? 0 : static_cast<int>(blockIdx.y) - 1; h < (input ? a.halves : static_cast<int>(blockIdx.y)); ++h) {
+__global__ void __launch_bounds__(256) bwd_finalize_ln_kernel(const BwdLnArgs a) {
+  const int vec = threadIdx.x >> 7, k = threadIdx.x & 127;
+  const bool input = blockIdx.x == 0;
+  if (input && k >= a.c) return;
+  float s = 0.f;
+  for (int h = input ? 0 : static_cast<int>(blockIdx.x) - 1; h < (input ? a.halves : static_cast<int>(blockIdx.x)); ++h) {
 #pragma unroll
-      for (int m = 0; m < 6; ++m) {
-        const int n_rows = m < 4 ? 128 : a.c;
-        if ((m == 4) == input || ((a.mask[h] >> m) & 1u) == 0u) continue;
-        const float4* src = reinterpret_cast<const float4*>(a.ln_rows[h] + m * 128 * 256 + vec * 128) + piece;
-        float4 v[4];
+    for (int m = 0; m < 6; ++m) {
+      if ((m == 4) == input || ((a.mask[h] >> m) & 1u) == 0u) continue;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          v[u] = g + u * 32 < n_rows ? __ldcg(src + static_cast<size_t>(g + u * 32) * 64) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) s.x += v[u].x, s.y += v[u].y, s.z += v[u].z, s.w += v[u].w;
-      }
+      for (int q = 0; q < 4; ++q)
+        if (m < 4 || q * 32 < a.c) s += __ldcg(a.ln_rows[h] + (m * 4 + q) * 256 + threadIdx.x);
     }
   }
-  comb[g * 32 + piece] = s;
-  __syncthreads();
-  if (g == 0 && piece * 4 < n_cols) {
-    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < 32; ++q) {
-      const float4 x = comb[q * 32 + piece];
-      t.x += x.x, t.y += x.y, t.z += x.z, t.w += x.w;
-    }
-    float* dst = (input ? a.d_in[vec] : a.d_out[vec] + 128 * (static_cast<int>(blockIdx.y) - 1)) + piece * 4;
-    dst[0] = t.x, dst[1] = t.y, dst[2] = t.z, dst[3] = t.w;
-  }
+  (input ? a.d_in[vec] : a.d_out[vec] + 128 * (static_cast<int>(blockIdx.x) - 1))[k] = s;
 }
 
 }  // namespace trimul

@@ -27,7 +27,7 @@ struct BwdTransitionParams {
   const uint16_t* dx_in;  // [positions][128] fp16: c * d loss / d x_hat gathered by the earlier launches (not FIRST)
   float eps;
   int residual;
-  float* part_m;          // [grid][3][128][128]: Ma_j, Mb_j, dWs_j partials
+  float* part_m;          // [grid][3] matrices (store_partial): Ma_j, Mb_j, dWs_j partials
   float* part_s;          // [grid][2][4][128]: column sums of da and db per position quarter
   int* status;
 };
@@ -428,9 +428,7 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         uint32_t v[8];
         tmem_ld8(tmem_base + lane_sel + 128 + m * 128 + part * kBwdCh + ch * 8, v);
         tmem_ld_wait();
-        float4* dst = reinterpret_cast<float4*>(pm + (m * 128 + pos) * 128 + part * kBwdCh + ch * 8);
-        dst[0] = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
-        dst[1] = make_float4(__uint_as_float(v[4]), __uint_as_float(v[5]), __uint_as_float(v[6]), __uint_as_float(v[7]));
+        store_partial(pm + m * 128 * 128, pos, part * kBwdChunks + ch, v);
       }
     }
   }
@@ -536,9 +534,9 @@ __global__ void __launch_bounds__(256) tr_bwd_setup_kernel(const __grid_constant
 //   (column sums, held by quarter 0)
 //   dWa[j*128+r][k] = (Ma_j[r][k] gamma[k] + sa_j[r] beta[k]) / c, dWb likewise, dWs[c][j*128+h] = dWs_j[c][h] / c
 //   dgamma[k] = sum_j sum_r (Wa Ma + Wb Mb) / c,  dbeta[k] = sum_j sum_r (Wa sa + Wb sb) / c
-// Grid (128 rows, 3 matrices, 4 blocks j), one row of the partials per block as in bwd_finalize_kernel; the rows of the
-// LayerNorm sums [1024][2][128] are added by tr_bwd_final_ln_kernel. (A reduction per launch and a gradient kernel on
-// 4 x 8 blocks were 4 x 5.9 + 22.4 us.)
+// Grid (128: group of four columns and quarter of the rows, 3 matrices, 4 blocks j), as bwd_finalize_kernel; the LayerNorm
+// terms [2][4][4][2][128] are added by tr_bwd_final_ln_kernel. (A reduction per launch and a gradient kernel on 4 x 8 blocks
+// were 4 x 5.9 + 22.4 us.)
 struct TrBwdFinalArgs {
   TrBwdPackArgs w;
   const float* part_m;
@@ -548,63 +546,41 @@ struct TrBwdFinalArgs {
   float* d_wa;     // [512][128]
   float* d_wb;     // [512][128]
   float* d_ws;     // [128][512]
-  float* ln_rows;  // [2][512][2][128]
+  float* ln_rows;  // [2][4][4][2][128]
   float* d_ln[2];  // dgamma, dbeta [128]
 };
 __global__ void __launch_bounds__(512) tr_bwd_final_kernel(const __grid_constant__ TrBwdFinalArgs a) {
-  __shared__ float4 comb[kFinGroups * 32];
-  const int r = blockIdx.x, m = blockIdx.y, j = blockIdx.z;
-  const float* parts = a.part_m + (static_cast<size_t>(j) * a.n_parts * 3 + m) * 128 * 128 + r * 128;
-  const float4 mv4 = sum_partial_rows(parts, 3 * 128 * 128, a.n_parts, comb);
+  const int group = blockIdx.x >> 2, q = blockIdx.x & 3, m = blockIdx.y, j = blockIdx.z;
+  const float* parts = a.part_m + (static_cast<size_t>(j) * a.n_parts * 3 + m) * 128 * 128;
+  const float* sums = m == 2 ? nullptr : a.part_s + (static_cast<size_t>(j) * a.n_parts * 2 + m) * 512;
+  float4 m4;
+  float s1;
+  sum_partials_of_rows(parts, 3 * 128 * 128, sums, 2 * 512, a.n_parts, group, q * 32, m4, s1);
   if (threadIdx.x >= 32) return;
-  const int k0 = (threadIdx.x & 31) * 4;
+  const int r = q * 32 + threadIdx.x, k0 = group * 4;
   const float cinv = a.scale[1];
-  const float mv[4] = {mv4.x * cinv, mv4.y * cinv, mv4.z * cinv, mv4.w * cinv};
+  const float sv = s1 * cinv, mv[4] = {m4.x * cinv, m4.y * cinv, m4.z * cinv, m4.w * cinv};
   if (m == 2) {
     float* dst = a.d_ws + static_cast<size_t>(r) * 512 + j * 128 + k0;
 #pragma unroll
     for (int t = 0; t < 4; ++t) dst[t] = mv[t];
     return;
   }
-  const float sv =
-      cinv * sum_partial_scalar(a.part_s + (static_cast<size_t>(j) * a.n_parts * 2 + m) * 512 + r, 2 * 512, a.n_parts);
   const size_t wi = static_cast<size_t>(j * 128 + r) * 128 + k0;
   float* dst = (m == 0 ? a.d_wa : a.d_wb) + wi;
-  float* ln = a.ln_rows + (static_cast<size_t>(m) * 512 + j * 128 + r) * 256 + k0;
+  float w[4];
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
-    const float w = tr_load_w(m == 0 ? a.w.w_a : a.w.w_b, wi + t, a.w.f32_weights);
+    w[t] = tr_load_w(m == 0 ? a.w.w_a : a.w.w_b, wi + t, a.w.f32_weights);
     dst[t] = fmaf(mv[t], a.w.ln_w[k0 + t], sv * a.w.ln_b[k0 + t]);
-    ln[t] = w * mv[t];
-    ln[128 + t] = w * sv;
   }
+  store_ln_terms(a.ln_rows + ((m * 4 + j) * 4 + q) * 256 + k0, w, mv, sv);
 }
-// grid 2 (dgamma, dbeta), 1024 threads: 32 four-column pieces by 32 groups of rows, fixed order
-__global__ void __launch_bounds__(1024) tr_bwd_final_ln_kernel(const TrBwdFinalArgs a) {
-  __shared__ float4 comb[32 * 32];
-  const int piece = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const float4* src = reinterpret_cast<const float4*>(a.ln_rows + blockIdx.x * 128) + piece;
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+__global__ void __launch_bounds__(256) tr_bwd_final_ln_kernel(const TrBwdFinalArgs a) {
+  float s = 0.f;
 #pragma unroll
-  for (int i = 0; i < 32; i += 8) {
-    float4 v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = __ldcg(src + static_cast<size_t>(g + (i + u) * 32) * 64);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) s.x += v[u].x, s.y += v[u].y, s.z += v[u].z, s.w += v[u].w;
-  }
-  comb[g * 32 + piece] = s;
-  __syncthreads();
-  if (g == 0) {
-    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < 32; ++q) {
-      const float4 x = comb[q * 32 + piece];
-      t.x += x.x, t.y += x.y, t.z += x.z, t.w += x.w;
-    }
-    float* dst = a.d_ln[blockIdx.x] + piece * 4;
-    dst[0] = t.x, dst[1] = t.y, dst[2] = t.z, dst[3] = t.w;
-  }
+  for (int i = 0; i < 32; ++i) s += __ldcg(a.ln_rows + i * 256 + threadIdx.x);
+  a.d_ln[threadIdx.x >> 7][threadIdx.x & 127] = s;
 }
 
 }  // namespace trimul
