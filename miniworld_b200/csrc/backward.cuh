@@ -681,49 +681,64 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
   }
 }
 
-// Mean and rstd of the stored t over the 256 channels of two tensors [rows][128][N] (fp16), one thread per row and
-// group of eight columns: stats[row][j] = {mean, rsqrt(var + eps)} (eps already scaled like the stored t). Eight
-// channels' loads are in flight per thread.
+// Mean and rstd of the stored t over the 256 channels of two tensors [rows][128][N] (fp16): stats[row][j] = {mean,
+// rsqrt(var + eps)} (eps already scaled like the stored t). A block takes 32 groups of eight columns, a warp 32 of the 256
+// channels of all of them (16-byte loads, 512 bytes per warp and channel, eight in flight); the eight warps' partial means
+// and squared deviations are merged through shared memory. (One thread per group over all 256 channels left the chip idle
+// at small N: 8192 threads at N = 256, 29 us for 34 MB.)
+constexpr int kLnStatsGroups = 32;
 __global__ void __launch_bounds__(256) bwd_ln_stats_kernel(const uint4* t0, const uint4* t1, int n, long long groups, float eps,
                                                            float2* stats) {
-  const long long g = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  if (g >= groups) return;
+  constexpr int kPerWarp = 32;  // channels
+  __shared__ float2 part[8][8][kLnStatsGroups];  // [warp][column][group]: mean, sum of squared deviations
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const long long g = blockIdx.x * static_cast<long long>(kLnStatsGroups) + lane;
   const int per_row = n / 8;
   const long long row = g / per_row;
   const int jc = static_cast<int>(g - row * per_row);
   float pv[8], s1[8], s2[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) pv[e] = 0.f, s1[e] = 0.f, s2[e] = 0.f;
-  for (int c0 = 0; c0 < 256; c0 += 8) {
-    const uint4* src = (c0 < 128 ? t0 : t1) + (row * 128 + (c0 & 127)) * per_row + jc;
-    uint4 v[8];
+  if (g < groups) {
+    const int c_first = (wp & 3) * kPerWarp;
+    const uint4* src = (wp < 4 ? t0 : t1) + (row * 128 + c_first) * per_row + jc;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = __ldg(src + static_cast<long long>(k) * per_row);
+    for (int c0 = 0; c0 < kPerWarp; c0 += 8) {
+      uint4 v[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const uint32_t w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+      for (int k = 0; k < 8; ++k) v[k] = __ldg(src + static_cast<long long>(c0 + k) * per_row);
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float2 x = f16x2_to_float2(w[t]);
-        if (c0 == 0 && k == 0) pv[2 * t] = x.x, pv[2 * t + 1] = x.y;
-        const float d0 = x.x - pv[2 * t], d1 = x.y - pv[2 * t + 1];
-        s1[2 * t] += d0, s1[2 * t + 1] += d1;
-        s2[2 * t] = fmaf(d0, d0, s2[2 * t]), s2[2 * t + 1] = fmaf(d1, d1, s2[2 * t + 1]);
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const float2 x = f16x2_to_float2(w[t]);
+          if (c0 == 0 && k == 0) pv[2 * t] = x.x, pv[2 * t + 1] = x.y;
+          const float d0 = x.x - pv[2 * t], d1 = x.y - pv[2 * t + 1];
+          s1[2 * t] += d0, s1[2 * t + 1] += d1;
+          s2[2 * t] = fmaf(d0, d0, s2[2 * t]), s2[2 * t + 1] = fmaf(d1, d1, s2[2 * t + 1]);
+        }
       }
     }
   }
-  float4* dst = reinterpret_cast<float4*>(stats + row * n + jc * 8);  // 64-byte aligned: n is a multiple of 8
 #pragma unroll
-  for (int e = 0; e < 8; e += 2) {
-    float m[2], r[2];
+  for (int e = 0; e < 8; ++e)
+    part[wp][e][lane] = make_float2(pv[e] + s1[e] * (1.0f / kPerWarp), fmaxf(s2[e] - s1[e] * s1[e] * (1.0f / kPerWarp), 0.f));
+  __syncthreads();
+  if (g >= groups) return;
+  // this thread: column `wp` of group `lane`; equal-sized partials: mean of means, M2 = sum M2_k + n_k sum (mean_k - mean)^2
+  float2 p[8];
+  float mean = 0.f, m2 = 0.f;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      m[u] = pv[e + u] + s1[e + u] * (1.0f / 256.0f);
-      const float var = fmaxf(s2[e + u] - s1[e + u] * s1[e + u] * (1.0f / 256.0f), 0.f) * (1.0f / 256.0f);
-      r[u] = rsqrtf(var + eps);
-    }
-    dst[e >> 1] = make_float4(m[0], r[0], m[1], r[1]);
+  for (int k = 0; k < 8; ++k) {
+    p[k] = part[k][wp][lane];
+    mean += p[k].x;
+    m2 += p[k].y;
   }
+  mean *= 0.125f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) m2 = fmaf(static_cast<float>(kPerWarp) * (p[k].x - mean), p[k].x - mean, m2);
+  stats[row * n + jc * 8 + wp] = make_float2(mean, rsqrtf(m2 * (1.0f / 256.0f) + eps));
 }
 
 // Finishes the first tensor's gradient of the 256-channel LayerNorm backward, in place over the raw d t_hat the MODE 1
