@@ -156,6 +156,23 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_native = None
+
+
+def native():
+    """The native host side of the module calls (``csrc/host.cpp``); raise if it has not been built."""
+    global _native
+    if _native is None:
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise RuntimeError(
+                "miniworld_b200/_native.so is missing or does not load: build it with `python -m miniworld_b200.build`"
+            ) from e
+        _native = module
+    return _native
+
+
 def strerror(code: int) -> str:
     return load().b200_trimul_strerror(int(code)).decode()
 

@@ -1,4 +1,5 @@
-"""Build recipe for the C-ABI shared library (one ``nvcc`` call, sm_100a only, in-tree output)."""
+"""Build recipe of the two in-tree libraries: the kernels behind the C ABI (one ``nvcc`` call, sm_100a only) and the native
+host side of the module calls (``csrc/host.cpp``, one ``g++`` call against PyTorch's headers, linked to the first)."""
 
 from __future__ import annotations
 
@@ -11,6 +12,9 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_NAME = "libb200_trimul.so"
 LIB_PATH = PKG_DIR / LIB_NAME
+NATIVE_PATH = PKG_DIR / "_native.so"
+HOST_SOURCE = CSRC / "host.cpp"
+HEADER = PKG_DIR.parent / "include" / "b200_trimul.h"
 
 NVCC_FLAGS = [
     "-gencode",
@@ -25,7 +29,7 @@ NVCC_FLAGS = [
 
 
 def _sources() -> list[Path]:
-    return sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.inc")) + [PKG_DIR.parent / "include" / "b200_trimul.h"]
+    return sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.inc")) + [HEADER]
 
 
 def is_stale() -> bool:
@@ -35,6 +39,13 @@ def is_stale() -> bool:
     return any(src.stat().st_mtime > built for src in _sources())
 
 
+def native_is_stale() -> bool:
+    if not NATIVE_PATH.exists():
+        return True
+    built = NATIVE_PATH.stat().st_mtime
+    return any(src.stat().st_mtime > built for src in (HOST_SOURCE, HEADER))
+
+
 def find_nvcc() -> str:
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
@@ -42,21 +53,45 @@ def find_nvcc() -> str:
     return nvcc
 
 
-def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile ``csrc/trimul_abi.cu`` into ``libb200_trimul.so`` beside the package (no GPU needed)."""
-    if not force and not is_stale():
-        return LIB_PATH
-    cmd = [find_nvcc(), *NVCC_FLAGS]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    tmp = LIB_PATH.with_suffix(".so.tmp")
-    cmd += ["-o", str(tmp), str(CSRC / "trimul_abi.cu")]
+def _run(cmd: list[str]) -> subprocess.CompletedProcess:
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + proc.stdout + proc.stderr)
-    os.replace(tmp, LIB_PATH)
-    if verbose:
-        print(proc.stderr)
+        raise RuntimeError(f"{cmd[0]} failed:\n" + proc.stdout + proc.stderr)
+    return proc
+
+
+def build_native(force: bool = False) -> Path:
+    """Compile ``csrc/host.cpp`` into ``_native.so`` beside the package (needs the kernels' library to link to)."""
+    if not force and not native_is_stale():
+        return NATIVE_PATH
+    import sysconfig
+
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(find_nvcc()).resolve().parent.parent
+    tmp = NATIVE_PATH.with_suffix(".so.tmp")
+    _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native", "-DTORCH_API_INCLUDE_EXTENSION_H",
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{root}/include",
+          f"-I{root}/include/torch/csrc/api/include", f"-I{cuda}/include", f"-I{sysconfig.get_paths()['include']}",
+          str(HOST_SOURCE), "-o", str(tmp), f"-L{root}/lib", "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda",
+          f"-L{PKG_DIR}", f"-l:{LIB_NAME}", "-Wl,-rpath,$ORIGIN"])
+    os.replace(tmp, NATIVE_PATH)
+    return NATIVE_PATH
+
+
+def build(force: bool = False, verbose: bool = False) -> Path:
+    """Compile ``csrc/trimul_abi.cu`` into ``libb200_trimul.so`` beside the package (no GPU needed), then ``_native.so``."""
+    if force or is_stale():
+        cmd = [find_nvcc(), *NVCC_FLAGS]
+        if verbose:
+            cmd += ["-Xptxas", "-v"]
+        tmp = LIB_PATH.with_suffix(".so.tmp")
+        proc = _run(cmd + ["-o", str(tmp), str(CSRC / "trimul_abi.cu")])
+        os.replace(tmp, LIB_PATH)
+        if verbose:
+            print(proc.stderr)
+    build_native(force)
     return LIB_PATH
 
 

@@ -28,6 +28,7 @@ from typing import Optional
 import torch
 from torch import nn
 
+from . import _lib
 from . import functional as F_
 
 D_SUPPORTED = 128
@@ -69,6 +70,20 @@ def from_openfold_state_dict(sd: dict) -> dict:
     return out
 
 
+def _registered(module: nn.Module, names) -> Optional[list]:
+    """The registered parameters ``"child.name"`` of ``names``, or None if one of them is not there under that name (a child
+    was wrapped or re-parametrised; attribute access then says what it is). Attribute access costs about 1 us per tensor."""
+    children = module._modules
+    try:
+        out = [children[child]._parameters[name] for child, name in names]
+    except (KeyError, AttributeError):
+        return None
+    for t in out:
+        if t is None:
+            return None
+    return out
+
+
 class Fp32LayerNorm(nn.LayerNorm):
     """LayerNorm parameter holder whose affine parameters are pinned to fp32: ``module.to(torch.bfloat16)`` moves them
     between devices but never changes (or rounds) their values, like the reference's fp32-pinned LayerNorm
@@ -83,6 +98,12 @@ class Fp32LayerNorm(nn.LayerNorm):
             return out
 
         return super()._apply(pinned, recurse)
+
+
+_TRI_NAMES = [tuple(k.split(".")) for k in (
+    "ln_pair.weight", "ln_pair.bias", "to_left.weight", "to_left_gate.weight", "to_right.weight", "to_right_gate.weight",
+    "ln_out.weight", "ln_out.bias", "to_gate.weight", "to_out.weight")]
+_TRANSITION_NAMES = [tuple(k.split(".")) for k in F_.TRANSITION_KEYS]
 
 
 class TriangleMultiplication(nn.Module):
@@ -222,6 +243,10 @@ class TriangleMultiplication(nn.Module):
         train = torch.is_grad_enabled() and (
             pair.requires_grad or (self.training and any(q.requires_grad for q in self.parameters()))
         )
+        if not train and self._biases is None and not self.check_status and not (self.training and self.p_drop > 0.0):
+            y = self._run_native(pair, token_mask, pair_mask)
+            if y is not None:
+                return y
         if train and not self._backward_supported():
             if pair.requires_grad:
                 raise NotImplementedError(
@@ -262,10 +287,26 @@ class TriangleMultiplication(nn.Module):
             )
         return y if in_dtype == torch.bfloat16 else y.to(in_dtype)
 
+    def _run_native(self, pair, token_mask, pair_mask) -> Optional[torch.Tensor]:
+        """The forward without a graph as one native call, or None for a call that needs converting or refusing."""
+        from .training import ordinary
+
+        params = _registered(self, _TRI_NAMES) if ordinary(pair) and pair.dim() == 4 else None
+        if params is None:
+            return None
+        got = _lib.native().trimul_forward(
+            pair, params, token_mask, pair_mask, self._workspace, self.d_pair, F_._direction(self._direction()),
+            self.ln_pair.eps, self.ln_out.eps, self.residual, pair.shape[1] % 8 != 0,
+        )
+        if got is None:
+            return None
+        y, self._workspace = got
+        return y
+
     def _run_train(self, pair: torch.Tensor, token_mask, pair_mask) -> torch.Tensor:
         """Differentiable forward (:mod:`miniworld_b200.training`): the stage tensors of this call are kept for the
         backward in a workspace of their own; dtype casts are ordinary differentiable ops."""
-        from .training import _trimul_train
+        from .training import _PARAM_KEYS, _trimul_train
 
         in_dtype = pair.dtype
         z = pair if pair.dtype == torch.bfloat16 else pair.to(torch.bfloat16)
@@ -286,7 +327,9 @@ class TriangleMultiplication(nn.Module):
                 pair_mask = pair_mask.to(z.device) != 0
             if scale is not None:
                 scale = F_.aligned16(scale)
-        y = _trimul_train(z, self._params(), token_mask, self._direction(), float(self.ln_pair.eps), float(self.ln_out.eps),
+        plain = _registered(self, _TRI_NAMES)
+        params = self._params() if plain is None else dict(zip(_PARAM_KEYS, plain))
+        y = _trimul_train(z, params, token_mask, self._direction(), float(self.ln_pair.eps), float(self.ln_out.eps),
                           pair_mask, self.residual, self._biases, scale, self.check_status, ragged)
         return y if in_dtype == torch.bfloat16 else y.to(in_dtype)
 
@@ -374,18 +417,20 @@ class Transition(nn.Module):
         return 0 if self._scratch is None else F_.read_status(self._scratch[1])
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        from .training import ordinary, transition_train
+
         if not x.is_cuda:
             raise RuntimeError("input must be a CUDA tensor: this module has no CPU implementation")
         if x.shape[-1] != self.d:
             raise RuntimeError(f"input must be [..., {self.d}], got {tuple(x.shape)}")
         in_dtype = x.dtype
+        plain = _registered(self, _TRANSITION_NAMES)
+        params = dict(zip(F_.TRANSITION_KEYS, plain)) if plain is not None else {
+            "ln_in.weight": self.ln_in.weight, "ln_in.bias": self.ln_in.bias, "expand_a.weight": self.expand_a.weight,
+            "expand_b.weight": self.expand_b.weight, "squeeze.weight": self.squeeze.weight}
         # the differentiable path is taken when the input requires grad, or in training mode when a parameter does
         if torch.is_grad_enabled() and (x.requires_grad or (self.training and any(q.requires_grad for q in self.parameters()))):
-            from .training import transition_train
-
             xb = (x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)).contiguous()
-            params = {"ln_in.weight": self.ln_in.weight, "ln_in.bias": self.ln_in.bias, "expand_a.weight": self.expand_a.weight,
-                      "expand_b.weight": self.expand_b.weight, "squeeze.weight": self.squeeze.weight}
             y = transition_train(xb, params, eps=float(self.ln_in.eps), residual=self.residual, check=self.check_status)
             return y if in_dtype == torch.bfloat16 else y.to(in_dtype)
         xb = x.detach()
@@ -396,8 +441,10 @@ class Transition(nn.Module):
             self._scratch = (F_.aligned_empty(F_.transition_packed_bytes(), xb.device),
                              torch.zeros(16, dtype=torch.int32, device=xb.device))
         packed, status = self._scratch
-        params = {"ln_in.weight": self.ln_in.weight, "ln_in.bias": self.ln_in.bias, "expand_a.weight": self.expand_a.weight,
-                  "expand_b.weight": self.expand_b.weight, "squeeze.weight": self.squeeze.weight}
+        if plain is not None and not self.check_status and in_dtype == torch.bfloat16 and ordinary(x):
+            y = _lib.native().transition_forward(xb, plain, packed, status, self.ln_in.eps, self.residual)
+            if y is not None:
+                return y
         with torch.no_grad():
             F_.transition_pack_weights(params, packed)  # packed in every call: a captured graph replays current weights
             y = F_.transition_forward(xb, packed, status, eps=float(self.ln_in.eps), residual=self.residual)

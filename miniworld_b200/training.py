@@ -18,9 +18,21 @@ from typing import Optional
 
 import torch
 
+from . import _lib
 from . import functional as F_
 
 D = F_.D
+
+
+def ordinary(t: torch.Tensor) -> bool:
+    """A call on ``t`` can take the native path: a CUDA tensor of the base class, no transform or trace that has to see the
+    autograd function below."""
+    return (
+        type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda
+        and not torch._C._are_functorch_transforms_active() and torch._C._get_tracing_state() is None
+    )
+
+
 _PARAM_KEYS = (
     "ln_pair.weight", "ln_pair.bias", "to_left.weight", "to_left_gate.weight", "to_right.weight", "to_right_gate.weight",
     "ln_out.weight", "ln_out.bias", "to_gate.weight", "to_out.weight",
@@ -28,7 +40,7 @@ _PARAM_KEYS = (
 
 
 class TriMulFunction(torch.autograd.Function):
-    """``y = TriMulFunction.apply(z, token_mask, pair_mask, drop_scale, cfg, *params)``; ``cfg`` is a dict with
+    """(General form of the node in ``csrc/host.cpp``, for the calls that one does not take.) ``y = TriMulFunction.apply(z, token_mask, pair_mask, drop_scale, cfg, *params)``; ``cfg`` is a dict with
     ``outgoing``, ``eps_in``, ``eps_out``, ``residual``, ``biases``, ``check``, ``any_n``; ``params`` in ``_PARAM_KEYS``
     order."""
 
@@ -81,6 +93,11 @@ def trimul_train(z: torch.Tensor, params: dict, token_mask: Optional[torch.Tenso
 
 def _trimul_train(z, params, token_mask, outgoing, eps_in, eps_out, pair_mask, residual, biases, drop_scale, check, any_n):
     """:func:`trimul_train`; ``any_n`` takes every N."""
+    if biases is None and not check and ordinary(z):
+        y = _lib.native().trimul_train(z, [params[k] for k in _PARAM_KEYS], token_mask, pair_mask, drop_scale, z.shape[-1],
+                                       F_._direction(outgoing), eps_in, eps_out, bool(residual), any_n)
+        if y is not None:
+            return y
     cfg = {"outgoing": None if outgoing is None else bool(outgoing), "eps_in": float(eps_in), "eps_out": float(eps_out), "residual": bool(residual),
            "biases": biases, "check": bool(check), "any_n": bool(any_n)}
     return TriMulFunction.apply(z, token_mask, pair_mask, drop_scale, cfg, *[params[k] for k in _PARAM_KEYS])
@@ -123,5 +140,9 @@ class TransitionFunction(torch.autograd.Function):
 
 def transition_train(x: torch.Tensor, params: dict, *, eps: float = 1e-5, residual: bool = True, check: bool = False):
     """Differentiable pair Transition: ``x`` [..., 128] bf16 contiguous and the five parameters may require grad."""
+    if not check and ordinary(x):
+        y = _lib.native().transition_train(x, [params[k] for k in _TRANSITION_KEYS], eps, bool(residual))
+        if y is not None:
+            return y
     cfg = {"eps": float(eps), "residual": bool(residual), "check": bool(check)}
     return TransitionFunction.apply(x, cfg, *[params[k] for k in _TRANSITION_KEYS])
