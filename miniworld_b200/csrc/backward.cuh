@@ -800,8 +800,7 @@ struct BwdPrologueParams {
   const float* grad_scale;    // [2]: c, 1 / c
   const uint8_t* token_mask;  // [B][N] or null
   const uint8_t* pair_mask;   // [B][N][N] or null
-  const uint16_t* dx_in;      // [B*N][N][C] fp16: c * d loss / d x_hat gathered so far (read)
-  const uint16_t* dy;         // LAST only: upstream gradient [B*N][N][C] bf16 (the residual path), or null
+  const void* dy;             // LAST only: non-null if the residual path's dy (map_dy) is added
   const float* rstd;          // LAST only: [B*N][ld] 1 / standard deviation of the input LayerNorm
   float* part_m;              // [grid][2] matrices (store_partial): partial dvalue^T x_hat, dgate^T x_hat
   float* part_s;              // [grid][2][128]
@@ -814,20 +813,25 @@ struct BwdPrologueParams {
 // the running d x_hat, and accumulates the two weight gradients. !LAST: the running d x_hat (fp16, times c) is written
 // back through map_out. LAST: the input LayerNorm's backward and the residual finish d loss / d z (bf16, unscaled).
 //
-// 16 arithmetic warps (four threads per channel or position, as in the epilogue's backward) and one warp whose first lane
-// issues every copy and MMA. The arithmetic warps never wait for one another but once per tile (LAST): they arrive at
-// named barriers the issuing warp waits at, and wait for its MMAs on mbarriers. Per tile:
-//   arithmetic: wait value / gate -> dvalue, dgate tiles -> arrive A -> (requests for the running sums) -> wait gradients
-//               -> d x_hat out of tensor memory -> arrive B -> LayerNorm backward, output tile -> arrive C
-//   issuing:    A: gradient GEMMs, next x_hat copy; their end: next dO copy; B: value / gate GEMMs of the NEXT tile, which
-//               run under the arithmetic that finishes this one; C: output store, and the word that its buffer was read.
-// What bounds it: the chain wait -> arithmetic -> gradient GEMMs (32 MMAs) -> read of one tile per SM; shared memory holds
-// two weight matrices and four tiles.
-constexpr int kBwdProThreads = kBwdThreads + 32;
+// The running d x_hat (c * d loss / d x_hat gathered so far, fp16) comes through map_dx, LAST: dy (bf16) through map_dy.
+// 16 arithmetic warps (four threads per channel or position, as in the epilogue's backward), a warp that issues the MMAs and
+// one that issues the copies. The arithmetic warps never wait for one another but once per tile (LAST): they arrive at
+// named barriers the issuing warps wait at, and wait for MMAs and copies on mbarriers. Per tile:
+//   arithmetic: wait value / gate -> dvalue, dgate tiles -> arrive A -> wait d x_hat -> out of tensor memory -> arrive B
+//               -> running sum added, LAST: LayerNorm backward and residual -> output tile -> arrive C
+//   MMAs:       A: d x_hat GEMMs, weight-gradient GEMMs; B: value / gate GEMMs of the NEXT tile, behind them in the pipe
+//   copies:     A: next x_hat; weight gradients done: dy (LAST) and next dO; C: output store, next running sum
+// Every global operand comes through TMA: read by the threads, 32 bytes per lane, the running sum alone held the load path
+// for 2.8 k of the 8.8 k cycles of a tile (with dy 4-5 k).
+// What bounds it: the chain value / gate GEMMs -> arithmetic -> gradient GEMMs -> read of one tile per SM; shared memory
+// holds two weight matrices and five tiles and has no room for a second tile in flight.
+constexpr int kBwdProThreads = kBwdThreads + 64;
+constexpr int kBwdProSmemBytes = 7 * kBwdTile + 512 /* barriers */ + 1024;
 template <bool LAST, int C = 128>
 __global__ void __launch_bounds__(kBwdProThreads, 1)
 bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_do,
                     const __grid_constant__ CUtensorMap map_wv, const __grid_constant__ CUtensorMap map_wg,
+                    const __grid_constant__ CUtensorMap map_dx, const __grid_constant__ CUtensorMap map_dy,
                     const __grid_constant__ CUtensorMap map_out, const BwdPrologueParams p) {
   // C = d_pair: the channels of z, d x_hat, dz and the columns of both weight matrices (128, or 64 for the narrow pair
   // stacks). The contracted width (channels of dO, rows of the weight matrices) is 128 in both cases.
@@ -835,33 +839,30 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   constexpr int kZCh = C / kBwdParts;   // z-side channels per thread
   constexpr int kZChunks = kZCh / 8;
   constexpr int kZHalves = C / 64;      // 64-channel halves of a [pos][C] tile = k halves of a [128][C] weight matrix
-  constexpr int kBarA = 2, kBarB = 3, kBarC = 4;  // named barriers of the arithmetic warps and the issuing warp
+  // named barriers of the arithmetic warps and the issuing warps
+  constexpr int kBarA = 2, kBarB = 3, kBarC = 4, kCountA = kBwdThreads + 64, kCountB = kBwdThreads + 32;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t wv_s = smem_base, wg_s = smem_base + kBwdTile;
   const uint32_t tiles_s = smem_base + 2 * kBwdTile;  // four tile buffers whose roles rotate from tile to tile
-  const uint32_t xchg = smem_base + 6 * kBwdTile;
-  const uint32_t const_s = xchg + kBwdXchg;
-  const uint32_t bar_base = const_s + 1024;
-  const uint32_t w_full = bar_base, x_full = bar_base + 8, do_full = bar_base + 16;
-  const uint32_t fwd_done = bar_base + 24, grad_done = bar_base + 32, out_free = bar_base + 40;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 6 * kBwdTile + kBwdXchg + 1024 + 48);
+  const uint32_t dx_s = smem_base + 6 * kBwdTile;     // the running d x_hat, later the exchange of partial sums
+  const uint32_t bar_base = smem_base + 7 * kBwdTile;
+  const uint32_t w_full = bar_base, x_full = bar_base + 8, do_full = bar_base + 16, dx_full = bar_base + 24;
+  const uint32_t dy_full = bar_base + 32, fwd_done = bar_base + 40, dx_done = bar_base + 48, grad_done = bar_base + 56;
+  const uint32_t out_free = bar_base + 64;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 7 * kBwdTile + 72);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    mbar_init(w_full, 1);
-    mbar_init(x_full, 1);
-    mbar_init(do_full, 1);
-    mbar_init(fwd_done, 1);
-    mbar_init(grad_done, 1);
-    mbar_init(out_free, 1);
+    for (uint32_t b = w_full; b <= out_free; b += 8) mbar_init(b, 1);
     *abort_flag = 0;
     fence_mbar_init();
     prefetch_tmap(&map_x);
     prefetch_tmap(&map_do);
+    prefetch_tmap(&map_dx);
     prefetch_tmap(&map_out);
   }
   if (warp == 0) {
@@ -875,8 +876,8 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 
   // Buffer roles (x_hat, dO, dvalue, dgate) of tile `it`, one nibble each, period 4: the next tile's x_hat and dO are
   // copied into this tile's dO buffer (free once dvalue / dgate are formed) and dgate buffer (free after the gradient
-  // GEMMs); its dvalue scratch is this tile's x_hat buffer and its dgate scratch this tile's dvalue buffer, which holds
-  // the output until the store has read it.
+  // GEMMs); its dvalue scratch is this tile's x_hat buffer and its dgate scratch this tile's dvalue buffer, which receives
+  // dy (LAST) after the gradient GEMMs and then, in place, the output, and is free once the store has read it.
   auto role = [&](int it_i, int r) {
     const uint32_t rr = static_cast<uint32_t>(0x1302012320313210ull >> (16 * (it_i & 3))) & 0xFFFFu;
     return tiles_s + ((rr >> (4 * r)) & 0xFu) * kBwdTile;
@@ -884,21 +885,7 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   // (thread_wait: a thread that gives up sets the abort word and carries on; every later wait of the CTA returns within
   // one poll, so that all warps walk through the same barriers to the end)
   if (warp == kBwdThreads / 32) {
-    // ------------------------------------------------------------ copies and MMAs
-    auto issue_x = [&](int tile_i, int it_i) {
-      const int row_i = tile_i / p.tiles_per_row;
-      const int j_i = (tile_i - row_i * p.tiles_per_row) * 128;
-      mbar_arrive_expect_tx(x_full, kZHalves * 16384);
-#pragma unroll
-      for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(role(it_i, 0) + kh * 16384, &map_x, x_full, kh * 64, j_i, row_i);
-    };
-    auto issue_do = [&](int tile_i, int it_i) {
-      const int row_i = tile_i / p.tiles_per_row;
-      const int j_i = (tile_i - row_i * p.tiles_per_row) * 128;
-      mbar_arrive_expect_tx(do_full, kBwdTile);
-#pragma unroll
-      for (int kh = 0; kh < 2; ++kh) tma_load_3d(role(it_i, 1) + kh * 16384, &map_do, do_full, j_i + kh * 64, 0, row_i);
-    };
+    // ------------------------------------------------------------ MMAs
     // value^T = Wv' x_hat^T (columns 0-127), gate^T = Wg' x_hat^T (128-255): lanes = contracted channels
     auto issue_fwd = [&](int it_i) {
       thread_wait(x_full, it_i & 1, abort_flag, p.status, kDevTimeoutMma);
@@ -917,23 +904,14 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       umma_commit(fwd_done);
     };
     if (lane == 0) {
-      mbar_arrive_expect_tx(w_full, 2 * kZHalves * 16384);
-#pragma unroll
-      for (int kh = 0; kh < kZHalves; ++kh) {
-        tma_load_2d(wv_s + kh * 16384, &map_wv, w_full, kh * 64, 0);
-        tma_load_2d(wg_s + kh * 16384, &map_wg, w_full, kh * 64, 0);
-      }
-      issue_x(blockIdx.x, 0);
-      issue_do(blockIdx.x, 0);
       thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
       issue_fwd(0);
     }
+    __syncwarp();
     int it = 0;
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
-      const int next = tile + static_cast<int>(gridDim.x);
-      const bool has_next = next < p.num_tiles;
       const uint32_t x_s = role(it, 0), dv_s = role(it, 2), dg_s = role(it, 3);
-      named_bar_sync(kBarA, kBwdProThreads);  // dvalue and dgate are written, value / gate and dO are read
+      named_bar_sync(kBarA, kCountA);  // dvalue and dgate are written, value / gate are read
       if (lane == 0) {
         // d x_hat = dvalue Wv' + dgate Wg' (columns 0-127, lanes = positions); Mv += dvalue^T x_hat (256-383), Mg +=
         // dgate^T x_hat (384-511). dvalue / dgate are [channel][position] tiles: MN-major as the A operand of the first
@@ -949,6 +927,7 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             umma_bf16(tmem_base, umma_desc_mnmajor((m == 0 ? dv_s : dg_s) + ks * 2048, 16384),
                       umma_desc_mnmajor((m == 0 ? wv_s : wg_s) + ks * 2048, 16384), idesc_d, (m | ks) != 0 ? 1u : 0u);
         }
+        umma_commit(dx_done);
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
 #pragma unroll
@@ -959,36 +938,93 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
           }
         }
         umma_commit(grad_done);
-        thread_wait(do_full, it & 1, abort_flag, p.status, kDevTimeoutMma);  // (long since complete: the arithmetic read it)
-        if (has_next) {
-          issue_x(next, it + 1);
-          thread_wait(grad_done, it & 1, abort_flag, p.status, kDevTimeoutMma);
-          issue_do(next, it + 1);
-        }
       }
       __syncwarp();
-      named_bar_sync(kBarB, kBwdProThreads);  // d x_hat has left tensor memory
-      if (lane == 0 && has_next) issue_fwd(it + 1);
+      named_bar_sync(kBarB, kCountB);  // d x_hat has left tensor memory
+      if (lane == 0 && tile + static_cast<int>(gridDim.x) < p.num_tiles) issue_fwd(it + 1);
       __syncwarp();
-      named_bar_sync(kBarC, kBwdProThreads);  // the output tile is written
+    }
+  } else if (warp == kBwdThreads / 32 + 1) {
+    // ------------------------------------------------------------ copies
+    auto issue_x = [&](int tile_i, int it_i) {
+      const int row_i = tile_i / p.tiles_per_row;
+      const int j_i = (tile_i - row_i * p.tiles_per_row) * 128;
+      mbar_arrive_expect_tx(x_full, kZHalves * 16384);
+#pragma unroll
+      for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(role(it_i, 0) + kh * 16384, &map_x, x_full, kh * 64, j_i, row_i);
+    };
+    auto issue_do = [&](int tile_i, int it_i) {
+      const int row_i = tile_i / p.tiles_per_row;
+      const int j_i = (tile_i - row_i * p.tiles_per_row) * 128;
+      mbar_arrive_expect_tx(do_full, kBwdTile);
+#pragma unroll
+      for (int kh = 0; kh < 2; ++kh) tma_load_3d(role(it_i, 1) + kh * 16384, &map_do, do_full, j_i + kh * 64, 0, row_i);
+    };
+    auto issue_dx = [&](int tile_i) {
+      const int row_i = tile_i / p.tiles_per_row;
+      const int j_i = (tile_i - row_i * p.tiles_per_row) * 128;
+      mbar_arrive_expect_tx(dx_full, kZHalves * 16384);
+#pragma unroll
+      for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(dx_s + kh * 16384, &map_dx, dx_full, kh * 64, j_i, row_i);
+    };
+    if (lane == 0) {
+      mbar_arrive_expect_tx(w_full, 2 * kZHalves * 16384);
+#pragma unroll
+      for (int kh = 0; kh < kZHalves; ++kh) {
+        tma_load_2d(wv_s + kh * 16384, &map_wv, w_full, kh * 64, 0);
+        tma_load_2d(wg_s + kh * 16384, &map_wg, w_full, kh * 64, 0);
+      }
+      issue_x(blockIdx.x, 0);
+      issue_do(blockIdx.x, 0);
+      issue_dx(blockIdx.x);
+    }
+    __syncwarp();
+    int it = 0;
+    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
+      const int next = tile + static_cast<int>(gridDim.x);
+      const bool has_next = next < p.num_tiles;
+      const int row = tile / p.tiles_per_row;
+      const int j0 = (tile - row * p.tiles_per_row) * 128;
+      const uint32_t dv_s = role(it, 2);
+      named_bar_sync(kBarA, kCountA);  // dO is read
       if (lane == 0) {
-        const int row = tile / p.tiles_per_row;
-        const int j0 = (tile - row * p.tiles_per_row) * 128;
+        if constexpr (LAST) {
+          if (p.dy != nullptr) {
+#pragma unroll
+            for (int kh = 0; kh < kZHalves; ++kh) tma_prefetch_3d(&map_dy, kh * 64, j0, row);
+          }
+        }
+        if (has_next) issue_x(next, it + 1);
+        thread_wait(grad_done, it & 1, abort_flag, p.status, kDevTimeoutProducer);
+        if constexpr (LAST) {
+          if (p.dy != nullptr) {
+            mbar_arrive_expect_tx(dy_full, kZHalves * 16384);
+#pragma unroll
+            for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(dv_s + kh * 16384, &map_dy, dy_full, kh * 64, j0, row);
+          }
+        }
+        if (has_next) issue_do(next, it + 1);
+      }
+      __syncwarp();
+      named_bar_sync(kBarC, kCountB);  // the output tile is written, the running sum is read
+      if (lane == 0) {
 #pragma unroll
         for (int kh = 0; kh < kZHalves; ++kh) tma_store_3d(&map_out, dv_s + kh * 16384, kh * 64, j0, row);
         bulk_commit();
+        if (has_next) issue_dx(next);
         bulk_wait_read<0>();
         mbar_arrive(out_free);
       }
       __syncwarp();
     }
     if (lane == 0) {
-      // Every copy has been waited for above unless the CTA is giving up; then those in flight must land before it exits
-      // (the last iteration issued none, so the phases to look at are the last tile's).
+      // Every copy has been waited for by its readers unless the CTA is giving up; then those in flight must land before
+      // it exits (the last copies of every kind were the last tile's).
       if (*abort_flag != 0) {
         const uint32_t last = static_cast<uint32_t>((it - 1) & 1);
         const long long t0 = clock64();
-        while (!mbar_try_wait(w_full, 0) || !mbar_try_wait(x_full, last) || !mbar_try_wait(do_full, last)) {
+        while (!mbar_try_wait(w_full, 0) || !mbar_try_wait(x_full, last) || !mbar_try_wait(do_full, last) ||
+               !mbar_try_wait(dx_full, last) || (LAST && p.dy != nullptr && !mbar_try_wait(dy_full, last))) {
           if (clock64() - t0 > kWaitLimitCycles) {
             atomicCAS(p.status, 0, kDevTimeoutDrain);
             break;
@@ -1037,12 +1073,12 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
     int it = 0;
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
-      const int j0 = jt * 128;
+      const int j = jt * 128 + pos;
       const uint32_t x_s = role(it, 0), do_s = role(it, 1), dv_s = role(it, 2), dg_s = role(it, 3);
-      const int j = j0 + pos;
-      const bool inside = j < p.n;
-      const size_t cell = (static_cast<size_t>(row) * p.n + j) * C + part * kZCh;  // (read only when inside)
-      const size_t rcell = static_cast<size_t>(row) * p.ld + j;
+      float rstd_in = 0.f;
+      if constexpr (LAST) {
+        if (j < p.n) rstd_in = __ldg(p.rstd + static_cast<size_t>(row) * p.ld + j);
+      }
       thread_wait(fwd_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
       __syncwarp();
       tc_fence_after();
@@ -1098,63 +1134,57 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       tc_fence_before();
       fence_proxy_async_smem();
       __syncwarp();
-      named_bar_arrive(kBarA, kBwdProThreads);
-      // the running d x_hat of this thread's channels, LAST: the residual branch's share of dz and rstd, and the next
-      // tile's mask bytes: requested now, used after the GEMM round
-      uint4 dx_prev[kZChunks];
-      uint4 dy_res[LAST ? kZChunks : 2];
-      float rstd_in = 0.f;
-#pragma unroll
-      for (int ch = 0; ch < kZChunks; ++ch) dx_prev[ch] = make_uint4(0u, 0u, 0u, 0u);
-      if (inside) ldg_chunks(reinterpret_cast<const uint4*>(p.dx_in + cell), true, dx_prev);  // (workspace: 1024-byte aligned)
-      if constexpr (LAST) {
-#pragma unroll
-        for (int ch = 0; ch < kZChunks; ++ch) dy_res[ch] = make_uint4(0u, 0u, 0u, 0u);
-        if (inside) {
-          if (p.dy != nullptr)
-            ldg_chunks(reinterpret_cast<const uint4*>(p.dy + cell), (reinterpret_cast<uintptr_t>(p.dy) & 31u) == 0, dy_res);
-          rstd_in = __ldg(p.rstd + rcell);
-        }
-      }
+      named_bar_arrive(kBarA, kCountA);
+      // the next tile's mask bytes: requested now, used after the GEMM round
       const bool has_next = tile + static_cast<int>(gridDim.x) < p.num_tiles;
       row += step_rows, jt += step_cols;
       if (jt >= p.tiles_per_row) jt -= p.tiles_per_row, ++row;
       uint32_t m_i = 0u, m_j = 0u, m_p = 0u;
       if (has_next) mask_bytes(row, jt * 128, m_i, m_j, m_p);
-      thread_wait(grad_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
+      thread_wait(dx_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
       __syncwarp();
       tc_fence_after();
-      vbits = __ballot_sync(0xFFFFFFFFu, m_i != 0u && m_j != 0u && m_p != 0u);
-      // ---- add the running d x_hat; !LAST: write it back, LAST: LayerNorm backward + residual -> dz
       uint32_t vt[kZChunks][8];
 #pragma unroll
       for (int ch = 0; ch < kZChunks; ++ch) tmem_ld8(tmem_base + lane_sel + part * kZCh + ch * 8, vt[ch]);
+      uint4 xh[LAST ? kZChunks : 1];
+      if constexpr (LAST) {
+        // x_hat is read for the last time before barrier B: the next tile's dvalue is written over it
+#pragma unroll
+        for (int ch = 0; ch < kZChunks; ++ch) xh[ch] = ld_chunk(x_s + tile_chunk(pos, part * kZChunks + ch));
+      }
       tmem_ld_wait();
       tc_fence_before();
+      __syncwarp();
+      named_bar_arrive(kBarB, kCountB);
+      vbits = __ballot_sync(0xFFFFFFFFu, m_i != 0u && m_j != 0u && m_p != 0u);
+      // ---- add the running d x_hat; !LAST: write it back, LAST: LayerNorm backward + residual -> dz
+      thread_wait(dx_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+      __syncwarp();
       if constexpr (!LAST) {
-        __syncwarp();
-        named_bar_arrive(kBarB, kBwdProThreads);
+        uint32_t o[kZChunks][4];
 #pragma unroll
         for (int ch = 0; ch < kZChunks; ++ch) {
-          const uint32_t iw[4] = {dx_prev[ch].x, dx_prev[ch].y, dx_prev[ch].z, dx_prev[ch].w};
-          uint32_t o[4];
+          const uint4 in = ld_chunk(dx_s + tile_chunk(pos, part * kZChunks + ch));
+          const uint32_t iw[4] = {in.x, in.y, in.z, in.w};
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
             const float2 a = f16x2_to_float2(iw[t]);
-            o[t] = pack_f16x2_sat(
+            o[ch][t] = pack_f16x2_sat(
                 make_float2(__uint_as_float(vt[ch][2 * t]) + a.x, __uint_as_float(vt[ch][2 * t + 1]) + a.y));
           }
-          st_chunk(dv_s + tile_chunk(pos, part * kZChunks + ch), o[0], o[1], o[2], o[3]);
         }
+        thread_wait(grad_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);  // the GEMMs read the dvalue buffer
+#pragma unroll
+        for (int ch = 0; ch < kZChunks; ++ch)
+          st_chunk(dv_s + tile_chunk(pos, part * kZChunks + ch), o[ch][0], o[ch][1], o[ch][2], o[ch][3]);
       } else {
         float tot[kZCh];
-        uint4 xh[kZChunks];
         float s1 = 0.f, s2 = 0.f;
 #pragma unroll
         for (int ch = 0; ch < kZChunks; ++ch) {
-          // x_hat is read for the last time before barrier B: the next tile's dvalue is written over it
-          xh[ch] = ld_chunk(x_s + tile_chunk(pos, part * kZChunks + ch));
-          const uint32_t iw[4] = {dx_prev[ch].x, dx_prev[ch].y, dx_prev[ch].z, dx_prev[ch].w};
+          const uint4 in = ld_chunk(dx_s + tile_chunk(pos, part * kZChunks + ch));
+          const uint32_t iw[4] = {in.x, in.y, in.z, in.w};
           const uint32_t xw[4] = {xh[ch].x, xh[ch].y, xh[ch].z, xh[ch].w};
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
@@ -1167,18 +1197,28 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             s2 = fmaf(t0, x.x, fmaf(t1, x.y, s2));
           }
         }
-        // (written again only after barrier A of the next tile, which every thread arrives at after its reads below)
-        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + (part * 128 + pos) * 8), "f"(s1), "f"(s2) : "memory");
-        __syncwarp();
-        named_bar_sync(kBarB, kBwdProThreads);
-        float m1, m2;
-        sum_partials(xchg, pos, m1, m2);
+        // the partial sums go where this thread's part of the running sum was
+        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dx_s + tile_chunk(pos, part * kZChunks)), "f"(s1), "f"(s2) : "memory");
+        named_bar_sync(1, kBwdThreads);
+        float m1 = 0.f, m2 = 0.f;
+#pragma unroll
+        for (int k = 0; k < kBwdParts; ++k) {
+          float a, b;
+          asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(dx_s + tile_chunk(pos, k * kZChunks)));
+          m1 += a, m2 += b;
+        }
         m1 *= 1.0f / C, m2 *= 1.0f / C;
         const float rs = rstd_in * gc_inv;
+        // dy arrives where the output goes; without it (no residual) that buffer is free once the GEMMs have read it
+        if (p.dy != nullptr) thread_wait(dy_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+        else thread_wait(grad_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
 #pragma unroll
         for (int ch = 0; ch < kZChunks; ++ch) {
+          const uint32_t addr = dv_s + tile_chunk(pos, part * kZChunks + ch);
+          uint4 dyv = make_uint4(0u, 0u, 0u, 0u);
+          if (p.dy != nullptr) dyv = ld_chunk(addr);
           const uint32_t xw[4] = {xh[ch].x, xh[ch].y, xh[ch].z, xh[ch].w};
-          const uint32_t dw[4] = {dy_res[ch].x, dy_res[ch].y, dy_res[ch].z, dy_res[ch].w};
+          const uint32_t dw[4] = {dyv.x, dyv.y, dyv.z, dyv.w};
           uint32_t o[4];
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
@@ -1187,14 +1227,17 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             o[t] = pack_bf16x2(fmaf(rs, tot[ch * 8 + 2 * t] - m1 - x.x * m2, r.x),
                                fmaf(rs, tot[ch * 8 + 2 * t + 1] - m1 - x.y * m2, r.y));
           }
-          st_chunk(dv_s + tile_chunk(pos, part * kZChunks + ch), o[0], o[1], o[2], o[3]);
+          st_chunk(addr, o[0], o[1], o[2], o[3]);
         }
       }
       fence_proxy_async_smem();
       __syncwarp();
-      named_bar_arrive(kBarC, kBwdProThreads);
+      named_bar_arrive(kBarC, kCountB);
     }
-    // ---- per-CTA partials of the weight gradients (every GEMM has been waited for) and of the column sums
+    // ---- per-CTA partials of the weight gradients and of the column sums
+    thread_wait(grad_done, (it - 1) & 1, abort_flag, p.status, kDevTimeoutEpilogue);
+    __syncwarp();
+    tc_fence_after();
     float* pm = p.part_m + static_cast<size_t>(blockIdx.x) * 2 * 128 * 128;
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
@@ -1206,13 +1249,13 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         store_partial(pm + m * 128 * 128, pos, part * kBwdChunks + ch, v);
       }
     }
-    // column sums: the four position quarters of a channel, fixed order
-    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + kBwdXchgHalf + (part * 128 + pos) * 8), "f"(acc_sv), "f"(acc_sg)
-                 : "memory");
+    // column sums: the four position quarters of a channel, fixed order (through the running sum's buffer, read by all)
+    named_bar_sync(1, kBwdThreads);
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dx_s + (part * 128 + pos) * 8), "f"(acc_sv), "f"(acc_sg) : "memory");
     named_bar_sync(1, kBwdThreads);
     if (threadIdx.x < 128) {
       float a, b;
-      sum_partials(xchg + kBwdXchgHalf, threadIdx.x, a, b);
+      sum_partials(dx_s, threadIdx.x, a, b);
       float* ps = p.part_s + static_cast<size_t>(blockIdx.x) * 2 * 128;
       ps[threadIdx.x] = a;
       ps[128 + threadIdx.x] = b;
