@@ -977,7 +977,7 @@ static int launch_epilogue_wide(const CUtensorMap& mt0, const CUtensorMap& mt1, 
   int rc = set_smem(kernel, kWideSmemBytes, info.device);
   if (rc != B200_TRIMUL_OK) return rc;
   const int grid = p.num_tiles < info.sms ? p.num_tiles : info.sms;
-  kernel<<<grid, kEpilogueThreads, kWideSmemBytes, stream>>>(mt0, mt1, mz, my, mw0, mw1, p);
+  kernel<<<grid, kWideThreads, kWideSmemBytes, stream>>>(mt0, mt1, mz, my, mw0, mw1, p);
   TRIMUL_CUDA(cudaGetLastError());
   return B200_TRIMUL_OK;
 }
