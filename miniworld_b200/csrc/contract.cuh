@@ -120,6 +120,8 @@ contract_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     tmem_alloc(smem_u32(tmem_slot), kTmemCols);
     tmem_relinquish();
   }
+  grid_dependency_wait();
+  grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

@@ -80,6 +80,8 @@ contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
     tmem_relinquish_pair();
   }
+  grid_dependency_wait();
+  grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // barriers of both CTAs are initialised before any signal crosses

@@ -102,6 +102,8 @@ epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant
     prefetch_tmap(&map_wo);
     prefetch_tmap(&map_wg);
   }
+  grid_dependency_wait();
+  grid_dependents_launch();
   if (threadIdx.x >= 64 && threadIdx.x < 64 + C / 2) {
     // constants regrouped per channel pair so that one 16-byte load feeds a packed fp32x2 FMA
     const int cp = threadIdx.x - 64;

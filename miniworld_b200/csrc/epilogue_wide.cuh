@@ -109,6 +109,8 @@ epilogue_wide_kernel(const __grid_constant__ CUtensorMap map_t0, const __grid_co
     prefetch_tmap(&map_w0);
     prefetch_tmap(&map_w1);
   }
+  grid_dependency_wait();
+  grid_dependents_launch();
   if (threadIdx.x >= 64 && threadIdx.x < 128) {
     // constants regrouped per channel pair so that one 16-byte load feeds a packed fp32x2 FMA
     const int cp = threadIdx.x - 64;

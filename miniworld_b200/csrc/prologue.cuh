@@ -150,6 +150,8 @@ prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant
     tmem_alloc_pair(smem_u32(tmem_slot), 512);
     tmem_relinquish_pair();
   }
+  grid_dependency_wait();
+  grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // barriers of both CTAs are initialised before any signal crosses

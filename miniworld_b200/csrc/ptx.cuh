@@ -112,6 +112,13 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   return __all_sync(0xFFFFFFFFu, got) != 0;
 }
 
+// ------------------------------------------------------------------ dependent launches
+// Waits until the kernel before this one on the stream has completed and its writes are visible (returns at once if the
+// launch does not overlap it). Every thread calls it before it touches global memory.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel's blocks may be placed as this one's leave their SMs (they wait as above before they touch memory).
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------------ fences
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

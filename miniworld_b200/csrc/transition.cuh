@@ -123,6 +123,8 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     tmem_alloc_pair(smem_u32(tmem_slot), 512);
     tmem_relinquish_pair();
   }
+  grid_dependency_wait();
+  grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // barriers of both CTAs are initialised before any signal crosses
@@ -482,6 +484,7 @@ __device__ __forceinline__ float load_weight(const void* w, size_t idx, int f32)
 }
 
 __global__ void __launch_bounds__(256) transition_pack_kernel(const TransitionPackArgs a, uint8_t* packed) {
+  grid_dependents_launch();
   const int i = blockIdx.x * 256 + threadIdx.x;  // 0 .. 196607
   __half* ab = reinterpret_cast<__half*>(packed);
   __half* ws = reinterpret_cast<__half*>(packed + kTrPackedAbBytes);
