@@ -292,6 +292,8 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
     prefetch_tmap(&map_dt);
     prefetch_tmap(&map_dx);
   }
+  grid_dependency_wait();
+  grid_dependents_launch();
   if (threadIdx.x < 256) const_ptr[threadIdx.x] = p.consts[threadIdx.x];
   if (warp == 0) {
     tmem_alloc(smem_u32(tmem_slot), 512);
@@ -689,6 +691,8 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
 constexpr int kLnStatsGroups = 32;
 __global__ void __launch_bounds__(256) bwd_ln_stats_kernel(const uint4* t0, const uint4* t1, int n, long long groups, float eps,
                                                            float2* stats) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   constexpr int kPerWarp = 32;  // channels
   __shared__ float2 part[8][8][kLnStatsGroups];  // [warp][column][group]: mean, sum of squared deviations
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -747,6 +751,8 @@ __global__ void __launch_bounds__(256) bwd_ln_stats_kernel(const uint4* t0, cons
 constexpr int kLnFinishChannels = 16;
 __global__ void __launch_bounds__(256) bwd_ln_finish_kernel(uint4* dt, const uint4* t, const float2* stats, const float2* means,
                                                             int n, long long threads) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   const long long g = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (g >= threads) return;
   const int per_row = n / 8;
@@ -869,6 +875,8 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
   }
+  grid_dependency_wait();
+  grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1383,6 +1391,7 @@ struct BwdSetupArgs {
   float* scale;
 };
 __global__ void __launch_bounds__(256) bwd_setup_kernel(const __grid_constant__ BwdSetupArgs a) {
+  grid_dependents_launch();
   const int block = blockIdx.x;
   if (block < a.pack_blocks) {
     const int h = block >= 96 ? 1 : 0;
@@ -1471,6 +1480,8 @@ __device__ __forceinline__ void store_ln_terms(float* dst, const float (&w)[4], 
   }
 }
 __global__ void __launch_bounds__(512) bwd_finalize_kernel(const __grid_constant__ BwdFinalArgs args) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   const BwdFinalHalf& a = args.half[blockIdx.z];
   const int group = blockIdx.x >> 2, q = blockIdx.x & 3, m = blockIdx.y;
   const int n_rows = m < 4 ? 128 : a.w.c, n_cols = m == 4 ? 128 : a.w.c;  // a.w.c = d_pair: 128 or 64
@@ -1509,6 +1520,8 @@ struct BwdLnArgs {
   int c;            // d_pair
 };
 __global__ void __launch_bounds__(256) bwd_finalize_ln_kernel(const BwdLnArgs a) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   const int vec = threadIdx.x >> 7, k = threadIdx.x & 127;
   const bool input = blockIdx.x == 0;
   if (input && k >= a.c) return;

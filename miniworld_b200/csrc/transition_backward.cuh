@@ -67,6 +67,8 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     prefetch_tmap(&map_dy);
     prefetch_tmap(&map_out);
   }
+  grid_dependency_wait();
+  grid_dependents_launch();
   if (threadIdx.x < 256) const_ptr[threadIdx.x] = p.consts[(threadIdx.x >> 7) * 512 + p.block * 128 + (threadIdx.x & 127)];
   if (warp == 0) {
     tmem_alloc(smem_u32(tmem_slot), 512);
@@ -522,6 +524,7 @@ struct TrBwdSetupArgs {
   float* scale;
 };
 __global__ void __launch_bounds__(256) tr_bwd_setup_kernel(const __grid_constant__ TrBwdSetupArgs a) {
+  grid_dependents_launch();
   if (blockIdx.x < kTrBwdPackBlocks) {
     tr_bwd_pack_row(a.w, a.packed, blockIdx.x * 8 + (threadIdx.x >> 5));
     return;
@@ -550,6 +553,8 @@ struct TrBwdFinalArgs {
   float* d_ln[2];  // dgamma, dbeta [128]
 };
 __global__ void __launch_bounds__(512) tr_bwd_final_kernel(const __grid_constant__ TrBwdFinalArgs a) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   const int group = blockIdx.x >> 2, q = blockIdx.x & 3, m = blockIdx.y, j = blockIdx.z;
   const float* parts = a.part_m + (static_cast<size_t>(j) * a.n_parts * 3 + m) * 128 * 128;
   const float* sums = m == 2 ? nullptr : a.part_s + (static_cast<size_t>(j) * a.n_parts * 2 + m) * 512;
@@ -577,6 +582,8 @@ __global__ void __launch_bounds__(512) tr_bwd_final_kernel(const __grid_constant
   store_ln_terms(a.ln_rows + ((m * 4 + j) * 4 + q) * 256 + k0, w, mv, sv);
 }
 __global__ void __launch_bounds__(256) tr_bwd_final_ln_kernel(const TrBwdFinalArgs a) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   float s = 0.f;
 #pragma unroll
   for (int i = 0; i < 32; ++i) s += __ldcg(a.ln_rows + i * 256 + threadIdx.x);

@@ -323,9 +323,9 @@ static int set_smem(K kernel, int bytes, int device) {
 // takes the set-up (barriers, tensor memory, cluster start) and part of the tail off every boundary: with the status clear
 // folded into the packing, the forward goes 28.5 -> 21.9 us at N = 64, 47 -> 40.5 us at N = 203, 97 -> 89 us at N = 384.
 template <typename... P, typename... A>
-static cudaError_t launch_overlapped(void (*kernel)(P...), int grid, int threads, int smem, cudaStream_t stream, const A&... args) {
+static cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t stream, const A&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
