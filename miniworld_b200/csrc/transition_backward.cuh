@@ -3,15 +3,20 @@
 // One launch per block of 128 hidden units (four launches): the weight gradients of a block (expand_a, expand_b and
 // squeeze: three 128 x 128 accumulators) stay in tensor memory over all position tiles of a CTA, which leaves one
 // 128-column working region; the running d x_hat is carried between the launches in HBM (fp16, in place) and the last
-// launch finishes the LayerNorm backward and the residual. Structure as in backward.cuh: one CTA per SM, 512 threads
-// (four per position, 32 hidden units or channels each), tiles of 128 positions, phases separated by CTA-wide barriers,
-// one thread issuing TMA copies and MMAs. Per tile and block j:
-//   x_hat = LN(x) and dy * c as fp16 tiles (c: the power-of-two gradient scale of backward.cuh)
-//   dh = dy Ws_j      -> registers        a = x_hat Wa_j'^T + ca -> registers        b = x_hat Wb_j'^T + cb
-//   da = dh b silu'(a),  db = dh silu(a),  h = silu(a) b     (one scratch tile, used three times in turn)
-//   d x_hat (+)= da Wa_j' + db Wb_j'        Ma_j += da^T x_hat     Mb_j += db^T x_hat     dWs_j += dy^T h
-// Wa' = Wa gamma, Wb' = Wb gamma (fp16), ca = Wa beta, cb = Wb beta; the column sums of da and db (the beta terms of
-// the weight gradients) are read back from the scratch tile by a thread per hidden unit and kept in a register.
+// launch finishes the LayerNorm backward and the residual. The first launch normalises x and scales dy and leaves both as
+// fp16 tensors (and 1 / sigma) for the others. Per tile of 128 positions and block j, everything transposed like the
+// prologue's backward (tensor-memory lanes = hidden units, columns = positions: a thread owns one unit and 32 positions, so
+// its constants and column sums are scalars and the tiles are written in 16-byte runs):
+//   dh^T = Ws_j^T dy^T -> registers    a^T = Wa_j' x_hat^T + ca -> registers    b^T = Wb_j' x_hat^T + cb
+//   da = dh b silu'(a),  db = dh silu(a)  (tiles S1, S2)      h = silu(a) b  (registers, then S1)
+//   d x_hat (+)= da Wa_j' + db Wb_j'   Ma_j += da x_hat   Mb_j += db x_hat   (one round)      dWs_j += dy^T h^T
+// Wa' = Wa gamma, Wb' = Wb gamma (fp16), ca = Wa beta, cb = Wb beta; dy carries the power-of-two scale c of backward.cuh.
+//
+// 16 arithmetic warps, a warp that issues the MMAs and one that issues the copies, joined as in bwd_prologue_kernel. The
+// next tile's inputs land while this one finishes: dy in S2 and x_hat in its own buffer as soon as the first gradient round
+// is done. What bounds it: the chain of one tile per SM, five GEMM rounds with the working region's read between them (three
+// weight matrices and four tiles fill shared memory, the accumulators three quarters of tensor memory). The form before it
+// (positions on the lanes, six rounds between eleven CTA-wide barriers, LayerNorm in every launch) took 21 k cycles per tile.
 #pragma once
 
 #include "backward.cuh"
@@ -25,402 +30,413 @@ struct BwdTransitionParams {
   const float* consts;    // [2][512]: ca, cb
   const float* grad_scale;
   const uint16_t* dx_in;  // [positions][128] fp16: c * d loss / d x_hat gathered by the earlier launches (not FIRST)
+  float* rstd;            // [positions]: written by FIRST, read by LAST
   float eps;
   int residual;
   float* part_m;          // [grid][3] matrices (store_partial): Ma_j, Mb_j, dWs_j partials
-  float* part_s;          // [grid][2][4][128]: column sums of da and db per position quarter
+  float* part_s;          // [grid][2][512]: column sums of da and db in the first 128 entries
   int* status;
 };
 
-constexpr int kTrBwdSmemBytes = 6 * kBwdTile + kBwdXchg + 1024 + 256 + 1024;
+constexpr int kTrBwdThreads = kBwdThreads + 64;
+constexpr int kTrBwdSmemBytes = 7 * kBwdTile + 512 /* barriers */ + 1024;
 
+// map_x, map_dy: FIRST the module's x and dy (bf16), else x_hat and c * dy (fp16), which FIRST stores through map_xh, map_dyc.
 template <bool FIRST, bool LAST>
-__global__ void __launch_bounds__(kBwdThreads, 1)
+__global__ void __launch_bounds__(kTrBwdThreads, 1)
 bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_dy,
                       const __grid_constant__ CUtensorMap map_wa, const __grid_constant__ CUtensorMap map_wb,
-                      const __grid_constant__ CUtensorMap map_ws, const __grid_constant__ CUtensorMap map_out,
+                      const __grid_constant__ CUtensorMap map_ws, const __grid_constant__ CUtensorMap map_xh,
+                      const __grid_constant__ CUtensorMap map_dyc, const __grid_constant__ CUtensorMap map_out,
                       const BwdTransitionParams p) {
+  // named barriers: inputs converted (FIRST), dh read, a read, da / db written, h written and d x_hat read, output written
+  constexpr int kBarN = 2, kBarR1 = 3, kBarR2 = 4, kBarA = 5, kBarH = 6, kBarC = 7;
+  constexpr int kOne = kBwdThreads + 32, kTwo = kBwdThreads + 64;  // with one or both issuing warps
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t wa_s = smem_base, wb_s = wa_s + kBwdTile, ws_s = wb_s + kBwdTile;
-  const uint32_t x_s = ws_s + kBwdTile, y_s = x_s + kBwdTile, s_s = y_s + kBwdTile;  // x_hat, dy * c, scratch
-  const uint32_t xchg = smem_base + 6 * kBwdTile;
-  const uint32_t bar_base = xchg + kBwdXchg + 1024;
-  const uint32_t w_full = bar_base, in_full = bar_base + 8, mma_bar = bar_base + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 6 * kBwdTile + kBwdXchg + 1024 + 32);
+  const uint32_t wa_s = smem_base, wb_s = wa_s + kBwdTile, ws_s = wb_s + kBwdTile, x_s = ws_s + kBwdTile;
+  const uint32_t ring_s = x_s + kBwdTile;  // three buffers in the roles dy, S1, S2, which rotate from tile to tile
+  const uint32_t bar_base = smem_base + 7 * kBwdTile;
+  const uint32_t w_full = bar_base, x_full = bar_base + 8, y_full = bar_base + 16, dh_done = bar_base + 24;
+  const uint32_t a_done = bar_base + 32, b_done = bar_base + 40, ra_done = bar_base + 48, h_done = bar_base + 56;
+  const uint32_t out_free = bar_base + 64;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 7 * kBwdTile + 72);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* const_ptr = reinterpret_cast<float*>(smem + 6 * kBwdTile + kBwdXchg);  // ca_j[128], cb_j[128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q = warp & 3, part = warp >> 2;
-  const int pos = q * 32 + lane;
-  const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
 
   if (threadIdx.x == 0) {
-    mbar_init(w_full, 1);
-    mbar_init(in_full, 1);
-    mbar_init(mma_bar, 1);
+    for (uint32_t b = w_full; b <= out_free; b += 8) mbar_init(b, 1);
     *abort_flag = 0;
     fence_mbar_init();
     prefetch_tmap(&map_x);
     prefetch_tmap(&map_dy);
     prefetch_tmap(&map_out);
   }
-  grid_dependency_wait();
-  grid_dependents_launch();
-  if (threadIdx.x < 256) const_ptr[threadIdx.x] = p.consts[(threadIdx.x >> 7) * 512 + p.block * 128 + (threadIdx.x & 127)];
   if (warp == 0) {
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
   }
+  grid_dependency_wait();
+  grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const float gc = p.grad_scale[0], gc_inv = p.grad_scale[1];
 
-  if (threadIdx.x == 0) {
-    mbar_arrive_expect_tx(w_full, 3 * kBwdTile);
+  // role 0 = dy, 1 = S1 (da, then h, then the output), 2 = S2 (db): the next tile's dy comes into S2, its S1 is this tile's
+  // dy buffer and its S2 this tile's S1, whose output has been stored by then
+  auto ring = [&](int it_i, int r) { return ring_s + static_cast<uint32_t>((r + 2 * it_i) % 3) * kBwdTile; };
+  // (thread_wait: a thread that gives up sets the abort word and carries on; every later wait of the CTA returns within
+  // one poll, so that all warps walk through the same barriers to the end)
+  if (warp == kBwdThreads / 32) {
+    // ------------------------------------------------------------ MMAs
+    if (lane == 0) thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
+    __syncwarp();
+    constexpr uint32_t idesc_kk = umma_idesc(128, 128, false, false, kFmtF16, kFmtF16);
+    constexpr uint32_t idesc_mk = umma_idesc(128, 128, true, false, kFmtF16, kFmtF16);
+    constexpr uint32_t idesc_km = umma_idesc(128, 128, false, true, kFmtF16, kFmtF16);
+    constexpr uint32_t idesc_mm = umma_idesc(128, 128, true, true, kFmtF16, kFmtF16);
+    auto kmaj = [](uint32_t tile, int ks) {
+      return umma_desc_kmajor(tile + (ks >> 2) * 16384) + static_cast<uint64_t>((ks & 3) * 2);
+    };
+    auto mnmaj = [](uint32_t tile, int ks) { return umma_desc_mnmajor(tile + ks * 2048, 16384); };
+    int it = 0;
+    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
+      const uint32_t y_s = ring(it, 0), s1_s = ring(it, 1), s2_s = ring(it, 2);
+      const uint32_t accum = it != 0 ? 1u : 0u;
+      if constexpr (FIRST) named_bar_sync(kBarN, kTwo);
+      if (lane == 0) {
+        // dh^T: A = Ws_j [c][hid] read MN-major, B = dy [pos][c]
+        if constexpr (!FIRST) thread_wait(y_full, it & 1, abort_flag, p.status, kDevTimeoutMma);
+        tc_fence_after();
 #pragma unroll
-    for (int kh = 0; kh < 2; ++kh) {
-      tma_load_2d(wa_s + kh * 16384, &map_wa, w_full, kh * 64, p.block * 128);  // Wa' rows of block j, [128 hid][128 k]
-      tma_load_2d(wb_s + kh * 16384, &map_wb, w_full, kh * 64, p.block * 128);
-      tma_load_2d(ws_s + kh * 16384, &map_ws, w_full, p.block * 128 + kh * 64, 0);  // Ws columns of block j, [128 c][128 hid]
-    }
-  }
-  // column sums of da and db: this thread's 16-byte chunk (eight hidden units) of four position rows of the scratch tile
-  const int sum_chunk = threadIdx.x & 15, sum_rows = (threadIdx.x >> 4) * 4;
-  float sa_acc[8], sb_acc[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) sa_acc[c] = 0.f, sb_acc[c] = 0.f;
-
-  bool ok = true;
-  int it = 0;
-  bool loads_pending = false;
-  uint32_t mma_phase = 0;
-  auto mma_wait = [&]() {
-    // per thread, no CTA-wide barrier: a thread that gives up carries on and the CTA leaves at the tile's last barrier
-    const bool got = thread_wait(mma_bar, mma_phase, abort_flag, p.status, kDevTimeoutEpilogue);
-    mma_phase ^= 1u;
-    return got;
-  };
-  // adds this thread's share of the scratch tile's column sums
-  auto column_sum = [&](float (&acc)[8]) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const uint4 a = ld_chunk(s_s + tile_chunk(sum_rows + r, sum_chunk));
-      const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float2 x = f16x2_to_float2(aw[t]);
-        acc[2 * t] += x.x, acc[2 * t + 1] += x.y;
+        for (int ks = 0; ks < 8; ++ks) umma_bf16(tmem_base, mnmaj(ws_s, ks), kmaj(y_s, ks), idesc_mk, ks != 0 ? 1u : 0u);
+        umma_commit(dh_done);
       }
-    }
-  };
-  auto issue_inputs = [&](int p0_i) {  // thread 0
-    mbar_arrive_expect_tx(in_full, 2 * kBwdTile);
+      __syncwarp();
+      named_bar_sync(kBarR1, kOne);
+      if (lane == 0) {
+        if constexpr (!FIRST) thread_wait(x_full, it & 1, abort_flag, p.status, kDevTimeoutMma);
+        tc_fence_after();
 #pragma unroll
-    for (int kh = 0; kh < 2; ++kh) {
-      tma_load_2d(y_s + kh * 16384, &map_dy, in_full, kh * 64, p0_i);
-      tma_load_2d(x_s + kh * 16384, &map_x, in_full, kh * 64, p0_i);
-    }
-    loads_pending = true;
-  };
-  for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
-    const int p0 = tile * 128;
-    if (threadIdx.x == 0) {
-      if (!loads_pending) issue_inputs(p0);  // (not LAST: requested while the previous tile finished)
-    }
-    if (it == 0) ok &= thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
-    ok &= thread_wait(in_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
-    loads_pending = false;  // (only thread 0's copy is read)
-    // ---- dy * c as fp16 in place (x_hat follows while the first GEMM runs)
-#pragma unroll
-    for (int ch = 0; ch < kBwdChunks; ++ch) {
-      const uint32_t addr = y_s + tile_chunk(pos, part * kBwdChunks + ch);
-      const uint4 v = ld_chunk(addr);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-      uint32_t o[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float2 d = bf16x2_to_float2(w[t]);
-        o[t] = pack_f16x2_sat(make_float2(d.x * gc, d.y * gc));
+        for (int ks = 0; ks < 8; ++ks) umma_bf16(tmem_base, kmaj(wa_s, ks), kmaj(x_s, ks), idesc_kk, ks != 0 ? 1u : 0u);
+        umma_commit(a_done);
       }
-      st_chunk(addr, o[0], o[1], o[2], o[3]);
-    }
-    // the previous tile's store has read the scratch tile (rewritten after the third GEMM round; the barrier below
-    // orders this wait before every thread's writes)
-    if (threadIdx.x == 0) bulk_wait_read<0>();
-    fence_proxy_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    // ---- dh = dy Ws_j (A: dy K-major over c; B: Ws_j [c rows][hid] read MN-major) -> working columns 0-127
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      constexpr uint32_t idesc = umma_idesc(128, 128, false, true, kFmtF16, kFmtF16);
+      __syncwarp();
+      named_bar_sync(kBarR2, kOne);
+      if (lane == 0) {
+        tc_fence_after();
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks)
-        umma_bf16(tmem_base, umma_desc_kmajor(y_s + (ks >> 2) * 16384) + static_cast<uint64_t>((ks & 3) * 2),
-                  umma_desc_mnmajor(ws_s + ks * 2048, 16384), idesc, ks != 0 ? 1u : 0u);
-      umma_commit(mma_bar);
-    }
-    // ---- x_hat in place, in the shadow of the dh GEMM (which reads dy and Ws only)
-    const float rstd_in = normalise_tile<true, true, 128>(x_s, xchg, pos, part, p.eps);
-    fence_proxy_async_smem();
-    ok &= mma_wait();
-    tc_fence_after();
-    float dh[kBwdCh];
-#pragma unroll
-    for (int ch = 0; ch < kBwdChunks; ++ch) {
-      uint32_t v[8];
-      tmem_ld8(tmem_base + lane_sel + part * kBwdCh + ch * 8, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int e = 0; e < 8; ++e) dh[ch * 8 + e] = __uint_as_float(v[e]);
-    }
-    tc_fence_before();
-    __syncthreads();
-    // ---- a = x_hat Wa_j'^T
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      constexpr uint32_t idesc = umma_idesc(128, 128, false, false, kFmtF16, kFmtF16);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
-        umma_bf16(tmem_base, umma_desc_kmajor(x_s + (ks >> 2) * 16384) + kb, umma_desc_kmajor(wa_s + (ks >> 2) * 16384) + kb,
-                  idesc, ks != 0 ? 1u : 0u);
+        for (int ks = 0; ks < 8; ++ks) umma_bf16(tmem_base, kmaj(wb_s, ks), kmaj(x_s, ks), idesc_kk, ks != 0 ? 1u : 0u);
+        umma_commit(b_done);
       }
-      umma_commit(mma_bar);
-    }
-    ok &= mma_wait();
-    tc_fence_after();
-    float av[kBwdCh];
+      __syncwarp();
+      named_bar_sync(kBarA, kOne);
+      if (lane == 0) {
+        // d x_hat (columns 0-127, lanes = positions), Ma (128-255), Mb (256-383; lanes = hidden units)
+        tc_fence_after();
 #pragma unroll
-    for (int ch = 0; ch < kBwdChunks; ++ch) {
-      uint32_t v[8];
-      tmem_ld8(tmem_base + lane_sel + part * kBwdCh + ch * 8, v);
-      tmem_ld_wait();
-      {
-        const float4* cp = reinterpret_cast<const float4*>(const_ptr + part * kBwdCh + ch * 8);
-        const float4 c0 = cp[0], c1 = cp[1];
-        const float cc[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int e = 0; e < 8; ++e) av[ch * 8 + e] = __uint_as_float(v[e]) + cc[e];
+          for (int ks = 0; ks < 8; ++ks)
+            umma_bf16(tmem_base, mnmaj(m == 0 ? s1_s : s2_s, ks), mnmaj(m == 0 ? wa_s : wb_s, ks), idesc_mm, (m | ks) != 0 ? 1u : 0u);
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks)
+            umma_bf16(tmem_base + 128 + m * 128, kmaj(m == 0 ? s1_s : s2_s, ks), mnmaj(x_s, ks), idesc_km,
+                      (ks != 0 ? 1u : 0u) | accum);
+        umma_commit(ra_done);
       }
-    }
-    tc_fence_before();
-    __syncthreads();
-    // ---- b = x_hat Wb_j'^T; then da -> scratch tile, db and h kept packed in registers
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      constexpr uint32_t idesc = umma_idesc(128, 128, false, false, kFmtF16, kFmtF16);
+      __syncwarp();
+      named_bar_sync(kBarH, kOne);
+      if (lane == 0) {
+        // dWs (384-511, lanes = channels c, columns = hidden units): A = dy read MN-major, B = h [hid][pos]
+        tc_fence_after();
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
-        umma_bf16(tmem_base, umma_desc_kmajor(x_s + (ks >> 2) * 16384) + kb, umma_desc_kmajor(wb_s + (ks >> 2) * 16384) + kb,
-                  idesc, ks != 0 ? 1u : 0u);
+        for (int ks = 0; ks < 8; ++ks)
+          umma_bf16(tmem_base + 384, mnmaj(y_s, ks), kmaj(s1_s, ks), idesc_mk, (ks != 0 ? 1u : 0u) | accum);
+        umma_commit(h_done);
       }
-      umma_commit(mma_bar);
+      __syncwarp();
     }
-    ok &= mma_wait();
-    tc_fence_after();
-    uint32_t db_p[kBwdCh / 2], h_p[kBwdCh / 2];
+  } else if (warp == kBwdThreads / 32 + 1) {
+    // ------------------------------------------------------------ copies
+    auto issue_y = [&](int tile_i, int it_i) {
+      mbar_arrive_expect_tx(y_full, kBwdTile);
 #pragma unroll
-    for (int ch = 0; ch < kBwdChunks; ++ch) {
-      uint32_t v[8];
-      tmem_ld8(tmem_base + lane_sel + part * kBwdCh + ch * 8, v);
-      tmem_ld_wait();
-      uint32_t da_p[4];
-      const float4* cbp = reinterpret_cast<const float4*>(const_ptr + 128 + part * kBwdCh + ch * 8);
-      const float4 cb0 = cbp[0], cb1 = cbp[1];
-      const float cbv[8] = {cb0.x, cb0.y, cb0.z, cb0.w, cb1.x, cb1.y, cb1.z, cb1.w};
+      for (int kh = 0; kh < 2; ++kh) tma_load_2d(ring(it_i, 0) + kh * 16384, &map_dy, y_full, kh * 64, tile_i * 128);
+    };
+    auto issue_x = [&](int tile_i) {
+      mbar_arrive_expect_tx(x_full, kBwdTile);
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        float dav[2], dbv[2], hv[2];
+      for (int kh = 0; kh < 2; ++kh) tma_load_2d(x_s + kh * 16384, &map_x, x_full, kh * 64, tile_i * 128);
+    };
+    if (lane == 0) {
+      mbar_arrive_expect_tx(w_full, 3 * kBwdTile);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i = ch * 8 + t * 2 + e;
-          const float b = __uint_as_float(v[t * 2 + e]) + cbv[t * 2 + e];
-          const float a = av[i];
-          const float sg = sigmoid_fast(a);
-          const float silu = a * sg;
-          const float dsilu = sg * fmaf(a, 1.0f - sg, 1.0f);
-          dav[e] = dh[i] * b * dsilu;
-          dbv[e] = dh[i] * silu;
-          hv[e] = silu * b;
+      for (int kh = 0; kh < 2; ++kh) {
+        tma_load_2d(ws_s + kh * 16384, &map_ws, w_full, p.block * 128 + kh * 64, 0);  // Ws columns of block j, [128 c][128 hid]
+        tma_load_2d(wa_s + kh * 16384, &map_wa, w_full, kh * 64, p.block * 128);      // Wa' rows of block j, [128 hid][128 k]
+        tma_load_2d(wb_s + kh * 16384, &map_wb, w_full, kh * 64, p.block * 128);
+      }
+      issue_y(blockIdx.x, 0);
+      issue_x(blockIdx.x);
+    }
+    __syncwarp();
+    int it = 0;
+    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
+      const int next = tile + static_cast<int>(gridDim.x);
+      const bool has_next = next < p.num_tiles;
+      if constexpr (FIRST) {
+        named_bar_sync(kBarN, kTwo);
+        if (lane == 0) {
+#pragma unroll
+          for (int kh = 0; kh < 2; ++kh) {
+            tma_store_2d(&map_xh, x_s + kh * 16384, kh * 64, tile * 128);
+            tma_store_2d(&map_dyc, ring(it, 0) + kh * 16384, kh * 64, tile * 128);
+          }
+          bulk_commit();
         }
-        da_p[t] = pack_f16x2_sat(make_float2(dav[0], dav[1]));
-        db_p[ch * 4 + t] = pack_f16x2_sat(make_float2(dbv[0], dbv[1]));
-        h_p[ch * 4 + t] = pack_f16x2_sat(make_float2(hv[0], hv[1]));
+        __syncwarp();
       }
-      st_chunk(s_s + tile_chunk(pos, part * kBwdChunks + ch), da_p[0], da_p[1], da_p[2], da_p[3]);
-    }
-    tc_fence_before();
-    fence_proxy_async_smem();
-    __syncthreads();
-    // ---- d x_hat = da Wa_j' (working columns), Ma += da^T x_hat (columns 128-255)
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      constexpr uint32_t idesc_d = umma_idesc(128, 128, false, true, kFmtF16, kFmtF16);
-      constexpr uint32_t idesc_m = umma_idesc(128, 128, true, true, kFmtF16, kFmtF16);
-      const uint32_t accum = it != 0 ? 1u : 0u;
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks)
-        umma_bf16(tmem_base, umma_desc_kmajor(s_s + (ks >> 2) * 16384) + static_cast<uint64_t>((ks & 3) * 2),
-                  umma_desc_mnmajor(wa_s + ks * 2048, 16384), idesc_d, ks != 0 ? 1u : 0u);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks)
-        umma_bf16(tmem_base + 128, umma_desc_mnmajor(s_s + ks * 2048, 16384), umma_desc_mnmajor(x_s + ks * 2048, 16384),
-                  idesc_m, (ks != 0 ? 1u : 0u) | accum);
-      umma_commit(mma_bar);
-    }
-    column_sum(sa_acc);  // reads the tile the MMAs read
-    ok &= mma_wait();
-    named_bar_sync(1, kBwdThreads);  // every thread's column-sum reads come before the tile is rewritten
-    // ---- db -> scratch; d x_hat += db Wb_j', Mb += db^T x_hat (columns 256-383)
-#pragma unroll
-    for (int ch = 0; ch < kBwdChunks; ++ch)
-      st_chunk(s_s + tile_chunk(pos, part * kBwdChunks + ch), db_p[ch * 4], db_p[ch * 4 + 1], db_p[ch * 4 + 2], db_p[ch * 4 + 3]);
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      constexpr uint32_t idesc_d = umma_idesc(128, 128, false, true, kFmtF16, kFmtF16);
-      constexpr uint32_t idesc_m = umma_idesc(128, 128, true, true, kFmtF16, kFmtF16);
-      const uint32_t accum = it != 0 ? 1u : 0u;
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks)
-        umma_bf16(tmem_base, umma_desc_kmajor(s_s + (ks >> 2) * 16384) + static_cast<uint64_t>((ks & 3) * 2),
-                  umma_desc_mnmajor(wb_s + ks * 2048, 16384), idesc_d, 1u);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks)
-        umma_bf16(tmem_base + 256, umma_desc_mnmajor(s_s + ks * 2048, 16384), umma_desc_mnmajor(x_s + ks * 2048, 16384),
-                  idesc_m, (ks != 0 ? 1u : 0u) | accum);
-      umma_commit(mma_bar);
-    }
-    column_sum(sb_acc);
-    ok &= mma_wait();
-    named_bar_sync(1, kBwdThreads);
-    // ---- h -> scratch; dWs_j += dy^T h (columns 384-511; lanes = channels c, columns = hidden units)
-#pragma unroll
-    for (int ch = 0; ch < kBwdChunks; ++ch)
-      st_chunk(s_s + tile_chunk(pos, part * kBwdChunks + ch), h_p[ch * 4], h_p[ch * 4 + 1], h_p[ch * 4 + 2], h_p[ch * 4 + 3]);
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      constexpr uint32_t idesc_m = umma_idesc(128, 128, true, true, kFmtF16, kFmtF16);
-      const uint32_t accum = it != 0 ? 1u : 0u;
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks)
-        umma_bf16(tmem_base + 384, umma_desc_mnmajor(y_s + ks * 2048, 16384), umma_desc_mnmajor(s_s + ks * 2048, 16384),
-                  idesc_m, (ks != 0 ? 1u : 0u) | accum);
-      umma_commit(mma_bar);
-    }
-    // the earlier launches' running d x_hat for this thread: requested now, used after the GEMM round
-    const long long gp = static_cast<long long>(p0) + pos;
-    const bool inside = gp < p.positions;
-    uint4 dx_prev[kBwdChunks];
-#pragma unroll
-    for (int ch = 0; ch < kBwdChunks; ++ch) dx_prev[ch] = make_uint4(0u, 0u, 0u, 0u);
-    if constexpr (!FIRST) {
-      if (inside) {
-        const uint4* src = reinterpret_cast<const uint4*>(p.dx_in + gp * 128 + part * kBwdCh);
-        ldg_chunks(src, true, dx_prev);  // the workspace is 1024-byte aligned
+      if (lane == 0 && has_next) {
+        thread_wait(ra_done, it & 1, abort_flag, p.status, kDevTimeoutProducer);
+        issue_y(next, it + 1);  // into S2
+        if constexpr (FIRST) bulk_wait_read<0>();
+        if constexpr (!LAST) issue_x(next);
       }
-    }
-    ok &= mma_wait();
-    tc_fence_after();
-    if constexpr (!LAST) {
-      // x_hat and dy * c have been read for the last time: the next tile's inputs land while this one finishes
-      if (threadIdx.x == 0 && tile + static_cast<int>(gridDim.x) < p.num_tiles) issue_inputs((tile + gridDim.x) * 128);
-    }
-    // ---- the running d x_hat: add the earlier launches' sum; LAST: LayerNorm backward + residual -> dx (bf16)
-    {
-      float tot[kBwdCh];
-      float s1 = 0.f, s2 = 0.f;
+      __syncwarp();
+      named_bar_sync(kBarC, kOne);
+      if (lane == 0) {
 #pragma unroll
-      for (int ch = 0; ch < kBwdChunks; ++ch) {
+        for (int kh = 0; kh < 2; ++kh) tma_store_2d(&map_out, ring(it, 1) + kh * 16384, kh * 64, tile * 128);
+        bulk_commit();
+        if constexpr (LAST) {
+          if (has_next) issue_x(next);  // (the x_hat buffer was the exchange of partial sums until here)
+        }
+        bulk_wait_read<0>();
+        mbar_arrive(out_free);
+      }
+      __syncwarp();
+    }
+    if (lane == 0) {
+      // Every copy has been waited for by its readers unless the CTA is giving up; then those in flight must land before
+      // it exits (the last copies of every kind were the last tile's).
+      if (*abort_flag != 0) {
+        const uint32_t last = static_cast<uint32_t>((it - 1) & 1);
+        const long long t0 = clock64();
+        while (!mbar_try_wait(w_full, 0) || !mbar_try_wait(x_full, last) || !mbar_try_wait(y_full, last)) {
+          if (clock64() - t0 > kWaitLimitCycles) {
+            atomicCAS(p.status, 0, kDevTimeoutDrain);
+            break;
+          }
+        }
+      }
+      bulk_wait<0>();
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------ arithmetic
+    const int q = warp & 3, part = warp >> 2;
+    const int pos = q * 32 + lane;  // this thread's hidden unit (first part of a tile) or position (second part)
+    const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
+    const float gc = p.grad_scale[0], gc_inv = p.grad_scale[1];
+    const float ca = p.consts[p.block * 128 + pos], cb = p.consts[512 + p.block * 128 + pos];
+    float acc_a = 0.f, acc_b = 0.f;  // column sums of da and db over this thread's positions
+    int it = 0;
+    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
+      const uint32_t y_s = ring(it, 0), s1_s = ring(it, 1), s2_s = ring(it, 2);
+      const long long gp = static_cast<long long>(tile) * 128 + pos;
+      const bool inside = gp < p.positions;
+      float rstd_in = 0.f;
+      if constexpr (FIRST) {
+        // ---- dy * c and x_hat as fp16 in place
+        thread_wait(y_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+#pragma unroll
+        for (int ch = 0; ch < kBwdChunks; ++ch) {
+          const uint32_t addr = y_s + tile_chunk(pos, part * kBwdChunks + ch);
+          const uint4 v = ld_chunk(addr);
+          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+          uint32_t o[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const float2 d = bf16x2_to_float2(w[t]);
+            o[t] = pack_f16x2_sat(make_float2(d.x * gc, d.y * gc));
+          }
+          st_chunk(addr, o[0], o[1], o[2], o[3]);
+        }
+        thread_wait(x_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+        // (the exchange of the statistics uses S1, the previous tile's dy buffer, once its store has read it)
+        if (it != 0) thread_wait(out_free, (it - 1) & 1, abort_flag, p.status, kDevTimeoutStats);
+        rstd_in = normalise_tile<true, true, 128>(x_s, s1_s, pos, part, p.eps);
+        if (part == 0 && inside) p.rstd[gp] = rstd_in;
+        fence_proxy_async_smem();
+        __syncwarp();
+        named_bar_arrive(kBarN, kTwo);
+      } else if constexpr (LAST) {
+        if (inside) rstd_in = __ldg(p.rstd + gp);
+        // (this thread reads dy and x_hat later; their barriers are waited for here, before they can enter another phase)
+        thread_wait(y_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+      }
+      // ---- dh, a into registers (this thread's hidden unit, 32 positions)
+      uint32_t dh[32], av[32];
+      thread_wait(dh_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
+      __syncwarp();
+      tc_fence_after();
+      tmem_ld32(tmem_base + lane_sel + part * 32, dh);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      named_bar_arrive(kBarR1, kOne);
+      if constexpr (LAST) thread_wait(x_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+      thread_wait(a_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
+      __syncwarp();
+      tc_fence_after();
+      tmem_ld32(tmem_base + lane_sel + part * 32, av);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      named_bar_arrive(kBarR2, kOne);
+      // S2 held the previous tile's output
+      if (it != 0) thread_wait(out_free, (it - 1) & 1, abort_flag, p.status, kDevTimeoutStats);
+      thread_wait(b_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
+      __syncwarp();
+      tc_fence_after();
+      // ---- da -> S1, db -> S2 ([hidden unit][position]), h packed in registers
+      uint32_t h_p[16];
+#pragma unroll
+      for (int k4 = 0; k4 < 4; ++k4) {
         uint32_t v[8];
-        tmem_ld8(tmem_base + lane_sel + part * kBwdCh + ch * 8, v);
-        const uint4 in = dx_prev[ch];
-        uint4 xh = make_uint4(0u, 0u, 0u, 0u);
-        if constexpr (LAST) xh = ld_chunk(x_s + tile_chunk(pos, part * kBwdChunks + ch));
+        tmem_ld8(tmem_base + lane_sel + part * 32 + k4 * 8, v);
         tmem_ld_wait();
-        const uint32_t iw[4] = {in.x, in.y, in.z, in.w};
-        const uint32_t xw[4] = {xh.x, xh.y, xh.z, xh.w};
+        uint32_t da_p[4], db_p[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-          const float2 a = f16x2_to_float2(iw[t]);
-          const float t0 = __uint_as_float(v[2 * t]) + a.x, t1 = __uint_as_float(v[2 * t + 1]) + a.y;
-          tot[ch * 8 + 2 * t] = t0;
-          tot[ch * 8 + 2 * t + 1] = t1;
-          if constexpr (LAST) {
+          float dav[2], dbv[2], hv[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int i = k4 * 8 + t * 2 + e;
+            const float b = __uint_as_float(v[t * 2 + e]) + cb;
+            const float a = __uint_as_float(av[i]) + ca;
+            const float d = __uint_as_float(dh[i]);
+            const float sg = sigmoid_fast(a);
+            const float silu = a * sg;
+            const float dsilu = sg * fmaf(a, 1.0f - sg, 1.0f);
+            dav[e] = d * b * dsilu;
+            dbv[e] = d * silu;
+            hv[e] = silu * b;
+          }
+          da_p[t] = pack_f16x2_sat(make_float2(dav[0], dav[1]));
+          db_p[t] = pack_f16x2_sat(make_float2(dbv[0], dbv[1]));
+          h_p[k4 * 4 + t] = pack_f16x2_sat(make_float2(hv[0], hv[1]));
+          // the column sums are those of the fp16 tiles the GEMMs read
+          const float2 ra = f16x2_to_float2(da_p[t]), rb = f16x2_to_float2(db_p[t]);
+          acc_a += ra.x + ra.y;
+          acc_b += rb.x + rb.y;
+        }
+        const uint32_t off = tile_chunk(pos, part * 4 + k4);
+        st_chunk(s1_s + off, da_p[0], da_p[1], da_p[2], da_p[3]);
+        st_chunk(s2_s + off, db_p[0], db_p[1], db_p[2], db_p[3]);
+      }
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      named_bar_arrive(kBarA, kOne);
+      // the earlier launches' running d x_hat for this thread's position: requested now, used after the GEMM round
+      uint4 dx_prev[kBwdChunks];
+#pragma unroll
+      for (int ch = 0; ch < kBwdChunks; ++ch) dx_prev[ch] = make_uint4(0u, 0u, 0u, 0u);
+      if constexpr (!FIRST) {
+        if (inside) ldg_chunks(reinterpret_cast<const uint4*>(p.dx_in + gp * 128 + part * kBwdCh), true, dx_prev);
+      }
+      thread_wait(ra_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
+      __syncwarp();
+      tc_fence_after();
+      // ---- h -> S1; d x_hat of this thread's position out of tensor memory
+#pragma unroll
+      for (int k4 = 0; k4 < 4; ++k4)
+        st_chunk(s1_s + tile_chunk(pos, part * 4 + k4), h_p[k4 * 4], h_p[k4 * 4 + 1], h_p[k4 * 4 + 2], h_p[k4 * 4 + 3]);
+      uint32_t vt[kBwdChunks][8];
+#pragma unroll
+      for (int ch = 0; ch < kBwdChunks; ++ch) tmem_ld8(tmem_base + lane_sel + part * kBwdCh + ch * 8, vt[ch]);
+      tmem_ld_wait();
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      named_bar_arrive(kBarH, kOne);
+      // ---- the running d x_hat; LAST: LayerNorm backward + residual -> dx (bf16). The output goes into S1 after dWs.
+      uint32_t o[kBwdChunks][4];
+      if constexpr (!LAST) {
+#pragma unroll
+        for (int ch = 0; ch < kBwdChunks; ++ch) {
+          const uint32_t iw[4] = {dx_prev[ch].x, dx_prev[ch].y, dx_prev[ch].z, dx_prev[ch].w};
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const float2 a = f16x2_to_float2(iw[t]);
+            o[ch][t] = pack_f16x2_sat(
+                make_float2(__uint_as_float(vt[ch][2 * t]) + a.x, __uint_as_float(vt[ch][2 * t + 1]) + a.y));
+          }
+        }
+      } else {
+        float tot[kBwdCh];
+        uint4 xh[kBwdChunks];
+        float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+        for (int ch = 0; ch < kBwdChunks; ++ch) {
+          xh[ch] = ld_chunk(x_s + tile_chunk(pos, part * kBwdChunks + ch));
+          const uint32_t iw[4] = {dx_prev[ch].x, dx_prev[ch].y, dx_prev[ch].z, dx_prev[ch].w};
+          const uint32_t xw[4] = {xh[ch].x, xh[ch].y, xh[ch].z, xh[ch].w};
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const float2 a = f16x2_to_float2(iw[t]);
             const float2 x = f16x2_to_float2(xw[t]);
+            const float t0 = __uint_as_float(vt[ch][2 * t]) + a.x, t1 = __uint_as_float(vt[ch][2 * t + 1]) + a.y;
+            tot[ch * 8 + 2 * t] = t0;
+            tot[ch * 8 + 2 * t + 1] = t1;
             s1 += t0 + t1;
             s2 = fmaf(t0, x.x, fmaf(t1, x.y, s2));
           }
         }
-      }
-      if constexpr (!LAST) {
-#pragma unroll
-        for (int ch = 0; ch < kBwdChunks; ++ch)
-          st_chunk(s_s + tile_chunk(pos, part * kBwdChunks + ch), pack_f16x2_sat(make_float2(tot[ch * 8], tot[ch * 8 + 1])),
-                   pack_f16x2_sat(make_float2(tot[ch * 8 + 2], tot[ch * 8 + 3])),
-                   pack_f16x2_sat(make_float2(tot[ch * 8 + 4], tot[ch * 8 + 5])),
-                   pack_f16x2_sat(make_float2(tot[ch * 8 + 6], tot[ch * 8 + 7])));
-      } else {
-        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + kBwdXchgHalf + (part * 128 + pos) * 8), "f"(s1), "f"(s2)
-                     : "memory");
+        // the partial sums go where this thread's x_hat was (the GEMMs that read it are complete)
+        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(x_s + tile_chunk(pos, part * kBwdChunks)), "f"(s1), "f"(s2) : "memory");
         named_bar_sync(1, kBwdThreads);
-        float m1, m2;
-        sum_partials(xchg + kBwdXchgHalf, pos, m1, m2);
+        float m1 = 0.f, m2 = 0.f;
+#pragma unroll
+        for (int k = 0; k < kBwdParts; ++k) {
+          float a, b;
+          asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(x_s + tile_chunk(pos, k * kBwdChunks)));
+          m1 += a, m2 += b;
+        }
         m1 *= 1.0f / 128.0f, m2 *= 1.0f / 128.0f;
         const float rs = rstd_in * gc_inv;
         const float res = p.residual ? gc_inv : 0.f;  // the dy tile holds dy * c
 #pragma unroll
         for (int ch = 0; ch < kBwdChunks; ++ch) {
-          const uint4 xh = ld_chunk(x_s + tile_chunk(pos, part * kBwdChunks + ch));
           const uint4 dyv = ld_chunk(y_s + tile_chunk(pos, part * kBwdChunks + ch));
-          const uint32_t xw[4] = {xh.x, xh.y, xh.z, xh.w};
+          const uint32_t xw[4] = {xh[ch].x, xh[ch].y, xh[ch].z, xh[ch].w};
           const uint32_t dw[4] = {dyv.x, dyv.y, dyv.z, dyv.w};
-          uint32_t o[4];
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
             const float2 x = f16x2_to_float2(xw[t]);
             const float2 r = f16x2_to_float2(dw[t]);
-            o[t] = pack_bf16x2(fmaf(rs, tot[ch * 8 + 2 * t] - m1 - x.x * m2, r.x * res),
-                               fmaf(rs, tot[ch * 8 + 2 * t + 1] - m1 - x.y * m2, r.y * res));
+            o[ch][t] = pack_bf16x2(fmaf(rs, tot[ch * 8 + 2 * t] - m1 - x.x * m2, r.x * res),
+                                   fmaf(rs, tot[ch * 8 + 2 * t + 1] - m1 - x.y * m2, r.y * res));
           }
-          st_chunk(s_s + tile_chunk(pos, part * kBwdChunks + ch), o[0], o[1], o[2], o[3]);
         }
       }
-    }
-    tc_fence_before();
-    fence_proxy_async_smem();
-    ok = __syncthreads_and(ok ? 1 : 0) != 0;  // a thread that gave up takes the whole CTA out here
-    if (!ok) break;
-    if (threadIdx.x == 0) {
+      thread_wait(h_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
+      __syncwarp();
 #pragma unroll
-      for (int kh = 0; kh < 2; ++kh) tma_store_2d(&map_out, s_s + kh * 16384, kh * 64, p0);
-      bulk_commit();
+      for (int ch = 0; ch < kBwdChunks; ++ch)
+        st_chunk(s1_s + tile_chunk(pos, part * kBwdChunks + ch), o[ch][0], o[ch][1], o[ch][2], o[ch][3]);
+      fence_proxy_async_smem();
+      __syncwarp();
+      named_bar_arrive(kBarC, kOne);
     }
-  }
-  if (threadIdx.x == 0) {
-    if (loads_pending || !ok) {
-      const long long t0 = clock64();
-      while (!mbar_try_wait(w_full, 0) || (loads_pending && !mbar_try_wait(in_full, it & 1))) {
-        if (clock64() - t0 > kWaitLimitCycles) {
-          atomicCAS(p.status, 0, kDevTimeoutDrain);
-          break;
-        }
-      }
-    }
-    bulk_wait<0>();
-  }
-  __syncthreads();
-  if (ok && it > 0) {
+    // ---- per-CTA partials of the weight gradients (every GEMM has been waited for) and of the column sums
     tc_fence_after();
     float* pm = p.part_m + static_cast<size_t>(blockIdx.x) * 3 * 128 * 128;
 #pragma unroll
@@ -433,24 +449,17 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         store_partial(pm + m * 128 * 128, pos, part * kBwdChunks + ch, v);
       }
     }
-  }
-  {  // the 32 row groups of a hidden unit, fixed order (every tile region is free by now); the sums go to quarter 0
-    float* sc = reinterpret_cast<float*>(smem);  // [32 row groups][2][128]
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      sc[((threadIdx.x >> 4) * 2 + 0) * 128 + sum_chunk * 8 + c] = sa_acc[c];
-      sc[((threadIdx.x >> 4) * 2 + 1) * 128 + sum_chunk * 8 + c] = sb_acc[c];
+    // the four position quarters of a hidden unit, fixed order (through the x_hat buffer, read by all)
+    named_bar_sync(1, kBwdThreads);
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(x_s + (part * 128 + pos) * 8), "f"(acc_a), "f"(acc_b) : "memory");
+    named_bar_sync(1, kBwdThreads);
+    if (threadIdx.x < 128) {
+      float a, b;
+      sum_partials(x_s, threadIdx.x, a, b);
+      float* ps = p.part_s + static_cast<size_t>(blockIdx.x) * 2 * 512;
+      ps[threadIdx.x] = a;
+      ps[512 + threadIdx.x] = b;
     }
-    __syncthreads();
-    float* ps = p.part_s + static_cast<size_t>(blockIdx.x) * 2 * 512;
-    float sum = 0.f;
-    if (threadIdx.x < 256)
-      for (int g = 0; g < 32; ++g) sum += sc[g * 256 + threadIdx.x];
-    __syncthreads();
-    // [vector][quarter][hidden unit]: threads 0-255 hold (vector, unit); quarters 1-3 are zero
-    if (threadIdx.x < 256) ps[(threadIdx.x >> 7) * 512 + (threadIdx.x & 127)] = sum;
-    else ps[((threadIdx.x - 256) >> 7) * 512 + 128 + (threadIdx.x & 127)] = 0.f;
-    ps[(threadIdx.x >> 8) * 512 + 256 + (threadIdx.x & 255)] = 0.f;
   }
   tc_fence_before();
   __syncthreads();
@@ -533,8 +542,8 @@ __global__ void __launch_bounds__(256) tr_bwd_setup_kernel(const __grid_constant
 }
 
 // Parameter gradients of the Transition from the per-CTA partials of the four launches j:
-//   part_m [4][n_parts][3][128][128] (Ma_j, Mb_j: [hidden][k]; dWs_j: [c][hidden]), part_s [4][n_parts][2][4][128]
-//   (column sums, held by quarter 0)
+//   part_m [4][n_parts][3] matrices (Ma_j, Mb_j: [hidden][k]; dWs_j: [c][hidden]), part_s [4][n_parts][2][512]
+//   (column sums in the first 128 entries)
 //   dWa[j*128+r][k] = (Ma_j[r][k] gamma[k] + sa_j[r] beta[k]) / c, dWb likewise, dWs[c][j*128+h] = dWs_j[c][h] / c
 //   dgamma[k] = sum_j sum_r (Wa Ma + Wb Mb) / c,  dbeta[k] = sum_j sum_r (Wa sa + Wb sb) / c
 // Grid (128: group of four columns and quarter of the rows, 3 matrices, 4 blocks j), as bwd_finalize_kernel; the LayerNorm
