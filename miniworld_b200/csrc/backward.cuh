@@ -1052,7 +1052,10 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     // dvalue / dgate are formed on the transposed projections (TMEM lanes = contracted channels, columns = positions): a
     // thread owns channel `pos` (its lane) and the position quarter `part`, so its constants and its column sums are
     // scalars and dO, stored [channel][position], is read in 16-byte runs of positions.
-    float acc_sv = 0.f, acc_sg = 0.f;
+    float2 acc_v2 = make_float2(0.f, 0.f), acc_g2 = make_float2(0.f, 0.f);  // over the even and the odd positions
+    const float2 c_value2 = make_float2(c_value, c_value), c_gate_half2 = make_float2(c_gate_half, c_gate_half);
+    const float2 half2 = make_float2(0.5f, 0.5f), eight2 = make_float2(8.f, 8.f);
+    auto pair_of = [](uint32_t lo, uint32_t hi) { return make_float2(__uint_as_float(lo), __uint_as_float(hi)); };
     // validity of the 32 positions of this warp's quarter, one bit each. The mask bytes of the NEXT tile are requested
     // before a GEMM wait and turned into the word after it, so that their latency is off the path.
     auto mask_bytes = [&](int row_i, int j_i, uint32_t& m_i, uint32_t& m_j, uint32_t& m_p) {
@@ -1116,20 +1119,18 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 d_o.x = ((vbits >> (hf * 16 + e0)) & 1u) ? d_o.x : 0.f;
                 d_o.y = ((vbits >> (hf * 16 + e0 + 1)) & 1u) ? d_o.y : 0.f;
               }
-              float dv2[2], dg2[2];
-#pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                const float val = __uint_as_float(vv[e0 + u]) + c_value;
-                const float th = tanh_approx(fmaf(__uint_as_float(vg[e0 + u]), 0.5f, c_gate_half));
-                const float sg = fmaf(th, 0.5f, 0.5f);
-                const float sg16 = fmaf(th, 8.0f, 8.0f);  // the contraction's outputs are stored times 2^-4
-                dv2[u] = (u == 0 ? d_o.x : d_o.y) * sg16;
-                dg2[u] = dv2[u] * fmaf(-val, sg, val);
-                acc_sv += dv2[u];
-                acc_sg += dg2[u];
-              }
-              ov[t] = pack_f16x2_sat(make_float2(dv2[0], dv2[1]));
-              dg_p[hf * 8 + k4 * 4 + t] = pack_f16x2_sat(make_float2(dg2[0], dg2[1]));
+              // (packed fp32 pairs: this pass is bound by its instruction count)
+              const float2 val = __fadd2_rn(pair_of(vv[e0], vv[e0 + 1]), c_value2);
+              const float2 gh = __ffma2_rn(pair_of(vg[e0], vg[e0 + 1]), half2, c_gate_half2);
+              const float2 th = make_float2(tanh_approx(gh.x), tanh_approx(gh.y));
+              const float2 sg = __ffma2_rn(th, half2, half2);
+              // the contraction's outputs are stored times 2^-4: 16 sg = 8 tanh + 8
+              const float2 dv = __fmul2_rn(d_o, __ffma2_rn(th, eight2, eight2));
+              const float2 dg = __fmul2_rn(dv, __ffma2_rn(make_float2(-val.x, -val.y), sg, val));
+              acc_v2 = __fadd2_rn(acc_v2, dv);
+              acc_g2 = __fadd2_rn(acc_g2, dg);
+              ov[t] = pack_f16x2_sat(dv);
+              dg_p[hf * 8 + k4 * 4 + t] = pack_f16x2_sat(dg);
             }
             st_chunk(dv_s + tile_chunk(pos, part * 4 + hf * 2 + k4), ov[0], ov[1], ov[2], ov[3]);
           }
@@ -1259,7 +1260,8 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
     // column sums: the four position quarters of a channel, fixed order (through the running sum's buffer, read by all)
     named_bar_sync(1, kBwdThreads);
-    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dx_s + (part * 128 + pos) * 8), "f"(acc_sv), "f"(acc_sg) : "memory");
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dx_s + (part * 128 + pos) * 8), "f"(acc_v2.x + acc_v2.y),
+                 "f"(acc_g2.x + acc_g2.y) : "memory");
     named_bar_sync(1, kBwdThreads);
     if (threadIdx.x < 128) {
       float a, b;

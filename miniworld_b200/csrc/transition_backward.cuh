@@ -245,7 +245,11 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
     const float gc = p.grad_scale[0], gc_inv = p.grad_scale[1];
     const float ca = p.consts[p.block * 128 + pos], cb = p.consts[512 + p.block * 128 + pos];
-    float acc_a = 0.f, acc_b = 0.f;  // column sums of da and db over this thread's positions
+    // column sums of da and db over this thread's even and odd positions
+    float2 acc_a2 = make_float2(0.f, 0.f), acc_b2 = make_float2(0.f, 0.f);
+    const float2 ca2 = make_float2(ca, ca), cb2 = make_float2(cb, cb), half2 = make_float2(0.5f, 0.5f);
+    const float2 one = make_float2(1.f, 1.f), minus1 = make_float2(-1.f, -1.f);
+    auto pair_of = [](uint32_t lo, uint32_t hi) { return make_float2(__uint_as_float(lo), __uint_as_float(hi)); };
     int it = 0;
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
       const uint32_t y_s = ring(it, 0), s1_s = ring(it, 1), s2_s = ring(it, 2);
@@ -306,36 +310,33 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       __syncwarp();
       tc_fence_after();
       // ---- da -> S1, db -> S2 ([hidden unit][position]), h packed in registers
+      // (packed fp32 pairs: the pass is bound by its instruction count)
       uint32_t h_p[16];
+      uint32_t v[2][8];
+      tmem_ld8(tmem_base + lane_sel + part * 32, v[0]);
 #pragma unroll
       for (int k4 = 0; k4 < 4; ++k4) {
-        uint32_t v[8];
-        tmem_ld8(tmem_base + lane_sel + part * 32 + k4 * 8, v);
         tmem_ld_wait();
+        if (k4 < 3) tmem_ld8(tmem_base + lane_sel + part * 32 + (k4 + 1) * 8, v[(k4 + 1) & 1]);
         uint32_t da_p[4], db_p[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-          float dav[2], dbv[2], hv[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int i = k4 * 8 + t * 2 + e;
-            const float b = __uint_as_float(v[t * 2 + e]) + cb;
-            const float a = __uint_as_float(av[i]) + ca;
-            const float d = __uint_as_float(dh[i]);
-            const float sg = sigmoid_fast(a);
-            const float silu = a * sg;
-            const float dsilu = sg * fmaf(a, 1.0f - sg, 1.0f);
-            dav[e] = d * b * dsilu;
-            dbv[e] = d * silu;
-            hv[e] = silu * b;
-          }
-          da_p[t] = pack_f16x2_sat(make_float2(dav[0], dav[1]));
-          db_p[t] = pack_f16x2_sat(make_float2(dbv[0], dbv[1]));
-          h_p[k4 * 4 + t] = pack_f16x2_sat(make_float2(hv[0], hv[1]));
-          // the column sums are those of the fp16 tiles the GEMMs read
-          const float2 ra = f16x2_to_float2(da_p[t]), rb = f16x2_to_float2(db_p[t]);
-          acc_a += ra.x + ra.y;
-          acc_b += rb.x + rb.y;
+          const int i = k4 * 8 + t * 2;
+          const float2 b2 = __fadd2_rn(pair_of(v[k4 & 1][t * 2], v[k4 & 1][t * 2 + 1]), cb2);
+          const float2 a2 = __fadd2_rn(pair_of(av[i], av[i + 1]), ca2);
+          const float2 d2 = pair_of(dh[i], dh[i + 1]);
+          const float2 ah = __fmul2_rn(a2, half2);
+          const float2 sg = __ffma2_rn(make_float2(tanh_approx(ah.x), tanh_approx(ah.y)), half2, half2);
+          const float2 silu = __fmul2_rn(a2, sg);
+          // silu' = sg (1 + a (1 - sg)) = sg + silu (1 - sg)
+          const float2 dsilu = __ffma2_rn(silu, __ffma2_rn(sg, minus1, one), sg);
+          const float2 da = __fmul2_rn(__fmul2_rn(d2, b2), dsilu);
+          const float2 db = __fmul2_rn(d2, silu);
+          acc_a2 = __fadd2_rn(acc_a2, da);
+          acc_b2 = __fadd2_rn(acc_b2, db);
+          da_p[t] = pack_f16x2_sat(da);
+          db_p[t] = pack_f16x2_sat(db);
+          h_p[k4 * 4 + t] = pack_f16x2_sat(__fmul2_rn(silu, b2));
         }
         const uint32_t off = tile_chunk(pos, part * 4 + k4);
         st_chunk(s1_s + off, da_p[0], da_p[1], da_p[2], da_p[3]);
@@ -451,7 +452,8 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     }
     // the four position quarters of a hidden unit, fixed order (through the x_hat buffer, read by all)
     named_bar_sync(1, kBwdThreads);
-    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(x_s + (part * 128 + pos) * 8), "f"(acc_a), "f"(acc_b) : "memory");
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(x_s + (part * 128 + pos) * 8), "f"(acc_a2.x + acc_a2.y),
+                 "f"(acc_b2.x + acc_b2.y) : "memory");
     named_bar_sync(1, kBwdThreads);
     if (threadIdx.x < 128) {
       float a, b;
