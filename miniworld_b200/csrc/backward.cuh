@@ -219,6 +219,7 @@ struct BwdEpilogueParams {
   int n;               // N
   int ld;              // columns per row of ext_stats and ln_part (N rounded up to a multiple of 8)
   const float* consts;      // [2][128]: d_out = W_out beta_out + bias_out, d_gate = W_gate beta_in + bias_gate
+  const float* row_sums;    // [128]: row sums of Wo'
   const float* grad_scale;  // [2]: c, 1 / c
   const uint16_t* drop_scale;  // [B][N][128] bf16 or null
   float eps_in;
@@ -230,7 +231,6 @@ struct BwdEpilogueParams {
   float2* ln_part;          // [B*N][ld]: MODE 1 writes its sums of d t_hat and d t_hat * t_hat; MODE 2 adds its own and
                             // writes back the two means over 256 channels
   float* rstd;              // [B*N][ld], not MODE 1: 1 / standard deviation of the input LayerNorm (x_hat leaves through map_xh)
-  const uint16_t* p_part;   // [B*N][N][128] fp16, MODE 2: the first launch's part of the output projection
   int* status;
 };
 
@@ -245,13 +245,27 @@ struct BwdEpilogueParams {
 //   MODE 2 (second tensor): proj = part + t_hat_2 Wo_2'^T + d_2; dproj, dgate; d t_hat_2, dxg, Mo_2, Mg; the
 //                           LayerNorm backward of its own 128 channels with the sums over all 256 (means -> ln_part);
 //                           `bwd_ln_finish_kernel` then finishes the first tensor's gradient.
+//
+// 16 arithmetic warps, a warp that issues the MMAs and one that issues the copies (joined as in bwd_prologue_kernel). Per tile
+//   arithmetic: t and z normalised in place (statistics by shuffles inside a warp) -> N -> wait P / G -> dproj, dgate tiles
+//               and the sums of the LayerNorm backward -> A -> column sums, per-position coefficients -> wait d t_hat
+//               (transposed: lanes = channels), d x_hat -> wait weight gradients -> output tiles -> C
+//   MMAs:       N: P, G;  A: d t_hat^T and d x_hat, then Mo and Mg
+//   copies:     N: x_hat out, next tile into L2; weight gradients done: next t, z; C: output stores, then next dy
+// The two sums the LayerNorm backward needs per position come from dproj, before the gradient GEMMs: sum_c d t_hat =
+// dproj . rowsum(Wo'), sum_c d t_hat t_hat = dproj . P. d t_hat is computed transposed because t is stored [channel][pos]: a
+// thread then owns one channel and reads and writes t in 16-byte runs (2-byte accesses to 32 channels of one position, two
+// exchanges of statistics and eight CTA-wide barriers made 17 k cycles per tile). What bounds it: the chain of one tile per
+// SM; two weight matrices and four tiles, all live during the gradient GEMMs, leave no room for a second tile.
+constexpr int kBwdEpiThreads = kBwdThreads + 64;
+constexpr int kBwdEpiSmemBytes = 6 * kBwdTile + 8192 /* exchange, constants */ + 512 /* barriers */ + 1024;
 template <int MODE, int C = 128>
-__global__ void __launch_bounds__(kBwdThreads, 1)
+__global__ void __launch_bounds__(kBwdEpiThreads, 1)
 bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_z,
                     const __grid_constant__ CUtensorMap map_dy, const __grid_constant__ CUtensorMap map_wo,
                     const __grid_constant__ CUtensorMap map_wg, const __grid_constant__ CUtensorMap map_dt,
                     const __grid_constant__ CUtensorMap map_dx, const __grid_constant__ CUtensorMap map_xh,
-                    const BwdEpilogueParams p) {
+                    const __grid_constant__ CUtensorMap map_pp, const BwdEpilogueParams p) {
   // C = d_pair: the channels of z, dy, dproj, dgate and the rows of both weight matrices (128, or 64 for the narrow pair
   // stacks; MODE 0 only). The contracted width (channels of t) is 128 in both cases.
   static_assert(C == 128 || (C == 64 && MODE == 0), "d_pair is 128, or 64 with one output tensor");
@@ -259,31 +273,26 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
   constexpr int kZChunks = kZCh / 8;
   constexpr int kZHalves = C / 64;      // 64-channel halves of a [pos][C] tile
   constexpr uint32_t kWHalf = C * 128;  // bytes of one 64-wide k half of a weight matrix with C rows
+  constexpr int kBarN = 2, kBarA = 3, kBarS = 4, kBarC = 5, kOne = kBwdThreads + 32, kTwo = kBwdThreads + 64;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t wo_s = smem_base, wg_s = smem_base + kBwdTile;
   const uint32_t tiles_s = smem_base + 2 * kBwdTile;  // four tile buffers whose roles rotate from tile to tile
-  const uint32_t xchg = smem_base + 6 * kBwdTile;
-  const uint32_t const_s = xchg + kBwdXchg;
-  const uint32_t bar_base = const_s + 1024;
-  const uint32_t w_full = bar_base, tz_full = bar_base + 8, mma_bar = bar_base + 16, dy_full = bar_base + 24;
-  const uint32_t sums_done = bar_base + 48;  // every thread arrives once it has read the gradient tiles for the column sums
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 6 * kBwdTile + kBwdXchg + 1024 + 32);
+  const uint32_t xchg = smem_base + 6 * kBwdTile;     // float2 [kBwdParts][128]: partial sums of the LayerNorm backward
+  const uint32_t coef_s = xchg + kBwdXchgHalf;        // float [3][128]: d t = a d t_hat + b + c t_hat
+  const uint32_t rstd_s = coef_s + 1536;              // float [128]: 1 / sigma of the output LayerNorm
+  float* const_ptr = reinterpret_cast<float*>(smem + 6 * kBwdTile + kBwdXchgHalf + 2048);  // d_out, d_gate, rowsum(Wo') [3][128]
+  const uint32_t bar_base = smem_base + 6 * kBwdTile + 8192;
+  const uint32_t w_full = bar_base, t_full = bar_base + 8, z_full = bar_base + 16, dy_full = bar_base + 24;
+  const uint32_t pp_full = bar_base + 32, fwd_done = bar_base + 40, d_done = bar_base + 48, grad_done = bar_base + 56;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 6 * kBwdTile + 8192 + 64);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* const_ptr = reinterpret_cast<float*>(smem + 6 * kBwdTile + kBwdXchg);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q = warp & 3, part = warp >> 2;
-  const int pos = q * 32 + lane;
-  const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
 
   if (threadIdx.x == 0) {
-    mbar_init(w_full, 1);
-    mbar_init(tz_full, 1);
-    mbar_init(dy_full, 1);
-    mbar_init(mma_bar, 1);
-    mbar_init(sums_done, kBwdThreads);
+    for (uint32_t b = w_full; b <= grad_done; b += 8) mbar_init(b, 1);
     *abort_flag = 0;
     fence_mbar_init();
     prefetch_tmap(&map_t);
@@ -292,360 +301,540 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
     prefetch_tmap(&map_dt);
     prefetch_tmap(&map_dx);
   }
-  grid_dependency_wait();
-  grid_dependents_launch();
-  if (threadIdx.x < 256) const_ptr[threadIdx.x] = p.consts[threadIdx.x];
   if (warp == 0) {
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
   }
+  grid_dependency_wait();
+  grid_dependents_launch();
+  if (threadIdx.x < 256) const_ptr[threadIdx.x] = p.consts[threadIdx.x];
+  else if (threadIdx.x < 384) const_ptr[threadIdx.x] = p.row_sums[threadIdx.x - 256];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const float gc = p.grad_scale[0];
 
-  if (threadIdx.x == 0) {
-    // Wo' [C, 128] as two k halves, Wg' [C, C] as C / 64 k halves
-    mbar_arrive_expect_tx(w_full, (2 + kZHalves) * kWHalf);
+  // Buffer roles of tile `it`: t, z, dy, dgate = buffers (0, 1, 2, 3) for even it and (2, 3, 0, 1) for odd it. The outputs of
+  // a tile are written over its t and z buffers and stored from there; its dy and dgate buffers are free once the gradient
+  // GEMMs are done, and receive the next tile's t and z while this tile finishes. The next tile's dy (MODE 2: and the first
+  // launch's part of the projection, where dgate will be) goes into this tile's t (z) buffer once the store has read it.
+  auto t_buf = [&](int it_i) { return tiles_s + static_cast<uint32_t>((it_i & 1) * 2) * kBwdTile; };
+  auto y_buf = [&](int it_i) { return tiles_s + static_cast<uint32_t>(((it_i & 1) ^ 1) * 2) * kBwdTile; };
+  // (thread_wait: a thread that gives up sets the abort word and carries on; every later wait of the CTA returns within
+  // one poll, so that all warps walk through the same barriers to the end)
+  if (warp == kBwdThreads / 32) {
+    // ------------------------------------------------------------ MMAs
+    if (lane == 0) thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
+    __syncwarp();
+    int it = 0;
+    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
+      const uint32_t t_s = t_buf(it), z_s = t_s + kBwdTile, dy_s = y_buf(it), dg_s = dy_s + kBwdTile;
+      named_bar_sync(kBarN, kTwo);
+      if (lane == 0) {
+        // P = t_hat Wo'^T (columns 0-127), G = x_hat Wg'^T (columns 128-255); lanes = positions
+        tc_fence_after();
+        constexpr uint32_t idesc_p = umma_idesc(128, C, true, false, kFmtF16, kFmtF16);
+        constexpr uint32_t idesc_g = umma_idesc(128, C, false, false, kFmtF16, kFmtF16);
 #pragma unroll
-    for (int kh = 0; kh < 2; ++kh) tma_load_2d(wo_s + kh * kWHalf, &map_wo, w_full, kh * 64, 0);
-#pragma unroll
-    for (int kh = 0; kh < kZHalves; ++kh) tma_load_2d(wg_s + kh * kWHalf, &map_wg, w_full, kh * 64, 0);
-  }
-  // Column sums of dproj and dgate (the bias / beta terms of the weight gradients): gathered from the fp16 tiles while
-  // the gradient GEMMs run, this thread taking the 16-byte chunk `sum_chunk` (eight channels) of four position rows.
-  const int sum_chunk = threadIdx.x & 15, sum_rows = (threadIdx.x >> 4) * 4;
-  float acc_so[8], acc_sg[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) acc_so[c] = 0.f, acc_sg[c] = 0.f;
-
-  // Buffer roles of tile `it`: t, z, dy, dgate = buffers (0, 1, 2, 3) for even it and (2, 3, 0, 1) for odd it. The
-  // outputs of a tile are written over its t and z buffers and stored from there; its dy and dgate buffers are free
-  // once the gradient GEMMs are done, and receive the next tile's t and z while this tile finishes. The next tile's dy
-  // goes into this tile's t buffer as soon as the store has read it.
-  auto issue_tz = [&](int tile_i, int it_i) {
-    const int row_i = tile_i / p.tiles_per_row;
-    const int j_i = (tile_i - row_i * p.tiles_per_row) * 128;
-    const uint32_t t_i = tiles_s + ((it_i & 1) * 2) * kBwdTile, z_i = t_i + kBwdTile;
-    mbar_arrive_expect_tx(tz_full, kBwdTile + kZHalves * 16384);
-#pragma unroll
-    for (int kh = 0; kh < 2; ++kh) tma_load_3d(t_i + kh * 16384, &map_t, tz_full, j_i + kh * 64, 0, row_i);
-#pragma unroll
-    for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(z_i + kh * 16384, &map_z, tz_full, kh * 64, j_i, row_i);
-  };
-  bool ok = true;
-  int it = 0;
-  int tz_pending = -1, dy_pending = -1;  // thread 0: iteration whose copies are in flight, or -1
-  if (threadIdx.x == 0 && static_cast<int>(blockIdx.x) < p.num_tiles) {
-    issue_tz(blockIdx.x, 0);
-    tz_pending = 0;
-  }
-  for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
-    const int row = tile / p.tiles_per_row;
-    const int j0 = (tile - row * p.tiles_per_row) * 128;
-    const uint32_t t_s = tiles_s + ((it & 1) * 2) * kBwdTile, z_s = t_s + kBwdTile;
-    const uint32_t dy_s = tiles_s + (((it & 1) ^ 1) * 2) * kBwdTile, dg_s = dy_s + kBwdTile;
-    if (it == 0) ok &= thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
-    ok &= thread_wait(tz_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
-    if (threadIdx.x == 0) tz_pending = -1;
-    // ---- phase 1: normalise t (rows = channels) and z (rows = positions) in place
-    float rstd_out;
-    if constexpr (MODE == 0) {
-      rstd_out = normalise_tile<false, false>(t_s, xchg, pos, part, p.eps_out);
-    } else {
-      float2 st = make_float2(0.f, 0.f);
-      if (j0 + pos < p.n) st = p.ext_stats[static_cast<size_t>(row) * p.ld + j0 + pos];
-      rstd_out = st.y;
-      const float nmr = -st.x * st.y;
-#pragma unroll 8
-      for (int cc = 0; cc < kBwdCh; ++cc) {
-        const uint32_t addr = t_s + tile_off(part * kBwdCh + cc, pos);
-        st_f16_sat(addr, fmaf(ld_f16(addr), st.y, nmr));
-      }
-    }
-    if (threadIdx.x == 0) {
-      // this tile's dy and dgate buffers held the previous tile's outputs: their store (issued a normalisation pass
-      // ago) must have read them before the dy copy lands there
-      bulk_wait_read<0>();
-      mbar_arrive_expect_tx(dy_full, kZHalves * 16384);
-#pragma unroll
-      for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(dy_s + kh * 16384, &map_dy, dy_full, kh * 64, j0, row);
-      dy_pending = it;
-    }
-    const float rstd_in = normalise_tile<true, true, C>(z_s, xchg + kBwdXchgHalf, pos, part, p.eps_in);  // (other buffer)
-    if constexpr (MODE != 1) {
-      if (part == 0 && j0 + pos < p.n) p.rstd[static_cast<size_t>(row) * p.ld + j0 + pos] = rstd_in;
-    }
-    fence_proxy_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    // ---- phase 2: P = t_hat Wo'^T (columns 0-127), G = x_hat Wg'^T (columns 128-255)
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      constexpr uint32_t idesc_p = umma_idesc(128, C, true, false, kFmtF16, kFmtF16);
-      constexpr uint32_t idesc_g = umma_idesc(128, C, false, false, kFmtF16, kFmtF16);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
-        umma_bf16(tmem_base, umma_desc_mnmajor(t_s + ks * 2048, 16384), umma_desc_kmajor(wo_s + (ks >> 2) * kWHalf) + kb,
-                  idesc_p, ks != 0 ? 1u : 0u);
-      }
-#pragma unroll
-      for (int ks = 0; ks < C / 16; ++ks) {
-        const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
-        umma_bf16(tmem_base + 128, umma_desc_kmajor(z_s + (ks >> 2) * 16384) + kb,
-                  umma_desc_kmajor(wg_s + (ks >> 2) * kWHalf) + kb, idesc_g, ks != 0 ? 1u : 0u);
-      }
-      umma_commit(mma_bar);
-      if constexpr (MODE != 1) {
-        // x_hat for the prologue's backward, read from the z buffer before phase 5 writes over it
-#pragma unroll
-        for (int kh = 0; kh < kZHalves; ++kh) tma_store_3d(&map_xh, z_s + kh * 16384, kh * 64, j0, row);
-        bulk_commit();
-      }
-    }
-    // per-thread global operands of phase 3 (MODE 2: the first launch's part of the projection; the dropout scale),
-    // requested before the waits
-    const int j = j0 + pos;
-    uint4 ppv[kZChunks], scv[kZChunks];
-#pragma unroll
-    for (int ch = 0; ch < kZChunks; ++ch) {
-      ppv[ch] = make_uint4(0u, 0u, 0u, 0u);
-      scv[ch] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);  // bf16 ones
-    }
-    if constexpr (MODE == 2) {
-      if (j < p.n)
-        ldg_chunks(reinterpret_cast<const uint4*>(p.p_part + (static_cast<size_t>(row) * p.n + j) * C + part * kZCh), true,
-                   ppv);  // the workspace is 1024-byte aligned
-    }
-    if (p.drop_scale != nullptr && j < p.n) {
-      const int b = row / p.n;
-      ldg_chunks(reinterpret_cast<const uint4*>(p.drop_scale + (static_cast<size_t>(b) * p.n + j) * C + part * kZCh),
-                 (reinterpret_cast<uintptr_t>(p.drop_scale) & 31u) == 0, scv);
-    }
-    ok &= thread_wait(mma_bar, 0, abort_flag, p.status, kDevTimeoutEpilogue);
-    ok &= thread_wait(dy_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
-    if (threadIdx.x == 0) dy_pending = -1;
-    tc_fence_after();
-    // ---- phase 3: dproj = c du gate, dgate = c du proj gate (1 - gate); du = dy (* dropout scale)
-    {
-      uint32_t vp[kZChunks][8], vg[kZChunks][8];
-#pragma unroll
-      for (int ch = 0; ch < kZChunks; ++ch) {
-        tmem_ld8(tmem_base + lane_sel + part * kZCh + ch * 8, vp[ch]);
-        tmem_ld8(tmem_base + lane_sel + 128 + part * kZCh + ch * 8, vg[ch]);
-      }
-      tmem_ld_wait();
-#pragma unroll
-      for (int ch = 0; ch < kZChunks; ++ch) {
-        const uint32_t addr = tile_chunk(pos, part * kZChunks + ch);
-        const uint4 dyv = ld_chunk(dy_s + addr);
-        float co[8], cg[8];  // the eight channels' constants (the same addresses for the whole warp)
-        {
-          const float4* cp = reinterpret_cast<const float4*>(const_ptr + part * kZCh + ch * 8);
-          const float4 a0 = cp[0], a1 = cp[1], b0 = cp[32], b1 = cp[33];
-          co[0] = a0.x, co[1] = a0.y, co[2] = a0.z, co[3] = a0.w, co[4] = a1.x, co[5] = a1.y, co[6] = a1.z, co[7] = a1.w;
-          cg[0] = b0.x, cg[1] = b0.y, cg[2] = b0.z, cg[3] = b0.w, cg[4] = b1.x, cg[5] = b1.y, cg[6] = b1.z, cg[7] = b1.w;
-        }
-        const uint32_t pw[4] = {ppv[ch].x, ppv[ch].y, ppv[ch].z, ppv[ch].w};
-        const uint32_t dw[4] = {dyv.x, dyv.y, dyv.z, dyv.w};
-        const uint32_t sw[4] = {scv[ch].x, scv[ch].y, scv[ch].z, scv[ch].w};
-        uint32_t op[4], og[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const float2 d2 = bf16x2_to_float2(dw[t]);
-          const float2 s2 = bf16x2_to_float2(sw[t]);
-          const float2 p2 = f16x2_to_float2(pw[t]);
-          float dpv[2], dgv[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float proj = __uint_as_float(vp[ch][t * 2 + e]) + co[t * 2 + e] + (e == 0 ? p2.x : p2.y);
-            const float gate = sigmoid_fast(__uint_as_float(vg[ch][t * 2 + e]) + cg[t * 2 + e]);
-            const float du = (e == 0 ? d2.x * s2.x : d2.y * s2.y) * gc;
-            dpv[e] = du * gate;
-            dgv[e] = MODE == 1 ? proj : dpv[e] * fmaf(-proj, gate, proj);  // MODE 1 hands its part of proj on
-          }
-          op[t] = pack_f16x2_sat(make_float2(dpv[0], dpv[1]));
-          og[t] = pack_f16x2_sat(make_float2(dgv[0], dgv[1]));
-        }
-        st_chunk(dy_s + addr, op[0], op[1], op[2], op[3]);
-        // MODE 1: the part of proj leaves through the z buffer (x_hat is only needed by the G GEMM, which is done)
-        st_chunk((MODE == 1 ? z_s : dg_s) + addr, og[0], og[1], og[2], og[3]);
-        if constexpr (C == 64) {
-          // the weight-gradient GEMMs read these tiles as 128-row operands: rows 64-127 (the second 64-channel block) are zero
-          const uint32_t zaddr = tile_chunk(pos, 8 + part * kZChunks + ch);
-          st_chunk(dy_s + zaddr, 0u, 0u, 0u, 0u);
-          st_chunk(dg_s + zaddr, 0u, 0u, 0u, 0u);
-        }
-      }
-    }
-    if constexpr (MODE != 1) {
-      if (threadIdx.x == 0) bulk_wait_read<0>();  // the store of x_hat
-    }
-    tc_fence_before();
-    fence_proxy_async_smem();
-    __syncthreads();
-    // ---- phase 4: dt_hat = dproj Wo' (0-127), dxg = dgate Wg' (128-255); Mo += dproj^T t_hat (256-383),
-    //      Mg += dgate^T x_hat (384-511)
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      constexpr uint32_t idesc_d = umma_idesc(128, 128, false, true, kFmtF16, kFmtF16);   // d t_hat: N = 128
-      constexpr uint32_t idesc_dx = umma_idesc(128, C, false, true, kFmtF16, kFmtF16);    // d x_hat: N = C
-      constexpr uint32_t idesc_mo = umma_idesc(128, 128, true, false, kFmtF16, kFmtF16);
-      constexpr uint32_t idesc_mg = umma_idesc(128, C, true, true, kFmtF16, kFmtF16);
-      const uint32_t accum = it != 0 ? 1u : 0u;
-#pragma unroll
-      for (int ks = 0; ks < C / 16; ++ks) {  // K = the C channels of dproj; Wo' read MN-major: its k halves are the N blocks
-        const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
-        umma_bf16(tmem_base, umma_desc_kmajor(dy_s + (ks >> 2) * 16384) + kb, umma_desc_mnmajor(wo_s + ks * 2048, kWHalf),
-                  idesc_d, ks != 0 ? 1u : 0u);
-      }
-      if constexpr (MODE != 1) {
+        for (int ks = 0; ks < 8; ++ks)
+          umma_bf16(tmem_base, umma_desc_mnmajor(t_s + ks * 2048, 16384),
+                    umma_desc_kmajor(wo_s + (ks >> 2) * kWHalf) + static_cast<uint64_t>((ks & 3) * 2), idesc_p, ks != 0 ? 1u : 0u);
 #pragma unroll
         for (int ks = 0; ks < C / 16; ++ks) {
           const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
-          umma_bf16(tmem_base + 128, umma_desc_kmajor(dg_s + (ks >> 2) * 16384) + kb,
-                    umma_desc_mnmajor(wg_s + ks * 2048, kWHalf), idesc_dx, ks != 0 ? 1u : 0u);
+          umma_bf16(tmem_base + 128, umma_desc_kmajor(z_s + (ks >> 2) * 16384) + kb,
+                    umma_desc_kmajor(wg_s + (ks >> 2) * kWHalf) + kb, idesc_g, ks != 0 ? 1u : 0u);
         }
+        umma_commit(fwd_done);
       }
+      __syncwarp();
+      named_bar_sync(kBarA, kTwo);
+      if (lane == 0) {
+        // d t_hat^T = Wo'^T dproj^T (0-127, lanes = channels of t, columns = positions), d x_hat = dgate Wg' (128-255, lanes
+        // = positions); Mo += dproj^T t_hat (256-383), Mg += dgate^T x_hat (384-511)
+        tc_fence_after();
+        constexpr uint32_t idesc_d = umma_idesc(128, 128, true, false, kFmtF16, kFmtF16);
+        constexpr uint32_t idesc_dx = umma_idesc(128, C, false, true, kFmtF16, kFmtF16);
+        constexpr uint32_t idesc_mo = umma_idesc(128, 128, true, false, kFmtF16, kFmtF16);
+        constexpr uint32_t idesc_mg = umma_idesc(128, C, true, true, kFmtF16, kFmtF16);
+        const uint32_t accum = it != 0 ? 1u : 0u;
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
-        umma_bf16(tmem_base + 256, umma_desc_mnmajor(dy_s + ks * 2048, 16384),
-                  umma_desc_kmajor(t_s + (ks >> 2) * 16384) + kb, idesc_mo, (ks != 0 ? 1u : 0u) | accum);
-      }
-      if constexpr (MODE != 1) {
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          umma_bf16(tmem_base + 384, umma_desc_mnmajor(dg_s + ks * 2048, 16384), umma_desc_mnmajor(z_s + ks * 2048, 16384),
-                    idesc_mg, (ks != 0 ? 1u : 0u) | accum);
-        }
-      }
-      umma_commit(mma_bar);
-    }
-    if (sum_chunk < C / 8) {  // column sums of the two fp16 tiles the GEMMs are reading
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const uint32_t addr = tile_chunk(sum_rows + r, sum_chunk);
-        const uint4 a = ld_chunk(dy_s + addr);
-        const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const float2 x = f16x2_to_float2(aw[t]);
-          acc_so[2 * t] += x.x, acc_so[2 * t + 1] += x.y;
+        for (int ks = 0; ks < C / 16; ++ks) {  // K = the C channels of dproj; Wo' [C][128] read MN-major (its k halves are M blocks)
+          const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
+          umma_bf16(tmem_base, umma_desc_mnmajor(wo_s + ks * 2048, kWHalf), umma_desc_kmajor(dy_s + (ks >> 2) * 16384) + kb,
+                    idesc_d, ks != 0 ? 1u : 0u);
         }
         if constexpr (MODE != 1) {
-          const uint4 b = ld_chunk(dg_s + addr);
-          const uint32_t bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const float2 x = f16x2_to_float2(bw[t]);
-            acc_sg[2 * t] += x.x, acc_sg[2 * t + 1] += x.y;
+          for (int ks = 0; ks < C / 16; ++ks) {
+            const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
+            umma_bf16(tmem_base + 128, umma_desc_kmajor(dg_s + (ks >> 2) * 16384) + kb,
+                      umma_desc_mnmajor(wg_s + ks * 2048, kWHalf), idesc_dx, ks != 0 ? 1u : 0u);
+          }
+        }
+        umma_commit(d_done);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+          const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
+          umma_bf16(tmem_base + 256, umma_desc_mnmajor(dy_s + ks * 2048, 16384),
+                    umma_desc_kmajor(t_s + (ks >> 2) * 16384) + kb, idesc_mo, (ks != 0 ? 1u : 0u) | accum);
+        }
+        if constexpr (MODE != 1) {
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks)
+            umma_bf16(tmem_base + 384, umma_desc_mnmajor(dg_s + ks * 2048, 16384), umma_desc_mnmajor(z_s + ks * 2048, 16384),
+                      idesc_mg, (ks != 0 ? 1u : 0u) | accum);
+        }
+        umma_commit(grad_done);
+      }
+      __syncwarp();
+    }
+  } else if (warp == kBwdThreads / 32 + 1) {
+    // ------------------------------------------------------------ copies
+    auto place = [&](int tile_i, int& row_i, int& j_i) {
+      row_i = tile_i / p.tiles_per_row;
+      j_i = (tile_i - row_i * p.tiles_per_row) * 128;
+    };
+    auto issue_tz = [&](int tile_i, int it_i) {
+      int row_i, j_i;
+      place(tile_i, row_i, j_i);
+      const uint32_t t_i = t_buf(it_i), z_i = t_i + kBwdTile;
+      mbar_arrive_expect_tx(t_full, kBwdTile);
+#pragma unroll
+      for (int kh = 0; kh < 2; ++kh) tma_load_3d(t_i + kh * 16384, &map_t, t_full, j_i + kh * 64, 0, row_i);
+      mbar_arrive_expect_tx(z_full, kZHalves * 16384);
+#pragma unroll
+      for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(z_i + kh * 16384, &map_z, z_full, kh * 64, j_i, row_i);
+    };
+    auto issue_dy = [&](int tile_i, int it_i) {
+      int row_i, j_i;
+      place(tile_i, row_i, j_i);
+      const uint32_t y_i = y_buf(it_i);
+      mbar_arrive_expect_tx(dy_full, kZHalves * 16384);
+#pragma unroll
+      for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(y_i + kh * 16384, &map_dy, dy_full, kh * 64, j_i, row_i);
+      if constexpr (MODE == 2) {
+        mbar_arrive_expect_tx(pp_full, kBwdTile);
+#pragma unroll
+        for (int kh = 0; kh < 2; ++kh) tma_load_3d(y_i + kBwdTile + kh * 16384, &map_pp, pp_full, kh * 64, j_i, row_i);
+      }
+    };
+    if (lane == 0) {
+      // Wo' [C, 128] as two k halves, Wg' [C, C] as C / 64 k halves
+      mbar_arrive_expect_tx(w_full, (2 + kZHalves) * kWHalf);
+#pragma unroll
+      for (int kh = 0; kh < 2; ++kh) tma_load_2d(wo_s + kh * kWHalf, &map_wo, w_full, kh * 64, 0);
+#pragma unroll
+      for (int kh = 0; kh < kZHalves; ++kh) tma_load_2d(wg_s + kh * kWHalf, &map_wg, w_full, kh * 64, 0);
+      issue_tz(blockIdx.x, 0);
+      issue_dy(blockIdx.x, 0);
+    }
+    __syncwarp();
+    int it = 0;
+    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
+      const int next = tile + static_cast<int>(gridDim.x);
+      const bool has_next = next < p.num_tiles;
+      int row, j0;
+      place(tile, row, j0);
+      const uint32_t t_s = t_buf(it), z_s = t_s + kBwdTile;
+      named_bar_sync(kBarN, kTwo);
+      if (lane == 0) {
+        if constexpr (MODE != 1) {  // x_hat for the prologue's backward
+#pragma unroll
+          for (int kh = 0; kh < kZHalves; ++kh) tma_store_3d(&map_xh, z_s + kh * 16384, kh * 64, j0, row);
+          bulk_commit();
+        }
+        if (has_next) {
+          int row_n, j_n;
+          place(next, row_n, j_n);
+#pragma unroll
+          for (int kh = 0; kh < 2; ++kh)
+            if (j_n + kh * 64 < p.n) tma_prefetch_3d(&map_t, j_n + kh * 64, 0, row_n);
+#pragma unroll
+          for (int kh = 0; kh < kZHalves; ++kh) tma_prefetch_3d(&map_z, kh * 64, j_n, row_n);
+        }
+        if constexpr (MODE != 1) bulk_wait_read<0>();  // (the z buffer is written again after barrier A)
+      }
+      __syncwarp();
+      named_bar_sync(kBarA, kTwo);
+      named_bar_sync(kBarS, kOne);  // the column sums have been read off the dproj and dgate tiles
+      if (lane == 0 && has_next) {
+        thread_wait(grad_done, it & 1, abort_flag, p.status, kDevTimeoutProducer);
+        issue_tz(next, it + 1);  // into this tile's dy and dgate buffers
+      }
+      __syncwarp();
+      named_bar_sync(kBarC, kOne);
+      if (lane == 0) {
+#pragma unroll
+        for (int kh = 0; kh < 2; ++kh)
+          if (j0 + kh * 64 < p.n) tma_store_3d(&map_dt, t_s + kh * 16384, j0 + kh * 64, 0, row);
+#pragma unroll
+        for (int kh = 0; kh < kZHalves; ++kh) tma_store_3d(&map_dx, z_s + kh * 16384, kh * 64, j0, row);
+        bulk_commit();
+        bulk_wait_read<0>();
+        if (has_next) issue_dy(next, it + 1);  // into this tile's t (and z) buffer
+      }
+      __syncwarp();
+    }
+    if (lane == 0) {
+      // Every copy has been waited for by its readers unless the CTA is giving up; then those in flight must land before
+      // it exits (the last copies of every kind were the last tile's).
+      if (*abort_flag != 0) {
+        const uint32_t last = static_cast<uint32_t>((it - 1) & 1);
+        const long long t0 = clock64();
+        while (!mbar_try_wait(w_full, 0) || !mbar_try_wait(t_full, last) || !mbar_try_wait(z_full, last) ||
+               !mbar_try_wait(dy_full, last) || (MODE == 2 && !mbar_try_wait(pp_full, last))) {
+          if (clock64() - t0 > kWaitLimitCycles) {
+            atomicCAS(p.status, 0, kDevTimeoutDrain);
+            break;
           }
         }
       }
+      bulk_wait<0>();
     }
-    mbar_arrive(sums_done);
-    ok &= thread_wait(mma_bar, 1, abort_flag, p.status, kDevTimeoutEpilogue);
-    tc_fence_after();
-    if (threadIdx.x == 0 && tile + static_cast<int>(gridDim.x) < p.num_tiles) {
-      // into this tile's dy and dgate buffers: the GEMMs have finished with them, and so must every thread's column sums
-      ok &= thread_wait(sums_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
-      issue_tz(tile + gridDim.x, it + 1);
-      tz_pending = it + 1;
-    }
-    // ---- phase 5: LayerNorm backward of the output normalisation, in place over t_hat; dxg over x_hat
-    {
-      const bool inside = j0 + pos < p.n;
-      float2 other = make_float2(0.f, 0.f);  // MODE 2: the first launch's sums (read before the barrier below)
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------ arithmetic
+    const int q = warp & 3, part = warp >> 2;
+    const int pos = q * 32 + lane;
+    const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
+    const float gc = p.grad_scale[0];
+    auto pair_of = [](uint32_t lo, uint32_t hi) { return make_float2(__uint_as_float(lo), __uint_as_float(hi)); };
+    // Column sums of dproj and dgate (the bias / beta terms of the weight gradients): gathered from the fp16 tiles while
+    // the gradient GEMMs run, this thread taking the 16-byte chunk `sum_chunk` (eight channels) of four position rows.
+    const int sum_chunk = threadIdx.x & 15, sum_rows = (threadIdx.x >> 4) * 4;
+    float acc_so[8], acc_sg[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc_so[c] = 0.f, acc_sg[c] = 0.f;
+    int it = 0;
+    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
+      const int row = tile / p.tiles_per_row;
+      const int j0 = (tile - row * p.tiles_per_row) * 128;
+      const int j = j0 + pos;
+      const uint32_t t_s = t_buf(it), z_s = t_s + kBwdTile, dy_s = y_buf(it), dg_s = dy_s + kBwdTile;
+      // ---- t normalised in place: a warp takes eight positions (one 16-byte chunk column), a lane four of the 128 channels
+      thread_wait(t_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+      __syncwarp();
+      {
+        const uint32_t col = t_s + static_cast<uint32_t>(warp >> 3) * 16384;
+        uint32_t addr[4];
+        float2 v[4][4];  // [channel][position pair]
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int c = k * 32 + lane;
+          addr[k] = col + c * 128 + (((warp & 7) ^ (c & 7)) << 4);
+          const uint4 x = ld_chunk(addr[k]);
+          v[k][0] = f16x2_to_float2(x.x), v[k][1] = f16x2_to_float2(x.y);
+          v[k][2] = f16x2_to_float2(x.z), v[k][3] = f16x2_to_float2(x.w);
+        }
+        // sums over the 32 lanes of eight values: three halving exchanges, then two plain ones; the lane ends with the sum
+        // of position `mine` of the eight
+        auto reduce8 = [&](const float2 (&s)[4]) {
+          const bool u16 = (lane & 16) != 0, u8 = (lane & 8) != 0, u4 = (lane & 4) != 0;
+          float2 k0 = u16 ? s[2] : s[0], k1 = u16 ? s[3] : s[1];
+          const float2 g0 = u16 ? s[0] : s[2], g1 = u16 ? s[1] : s[3];
+          k0.x += __shfl_xor_sync(0xFFFFFFFFu, g0.x, 16), k0.y += __shfl_xor_sync(0xFFFFFFFFu, g0.y, 16);
+          k1.x += __shfl_xor_sync(0xFFFFFFFFu, g1.x, 16), k1.y += __shfl_xor_sync(0xFFFFFFFFu, g1.y, 16);
+          float2 m = u8 ? k1 : k0;
+          const float2 h = u8 ? k0 : k1;
+          m.x += __shfl_xor_sync(0xFFFFFFFFu, h.x, 8), m.y += __shfl_xor_sync(0xFFFFFFFFu, h.y, 8);
+          float r = u4 ? m.y : m.x;
+          r += __shfl_xor_sync(0xFFFFFFFFu, u4 ? m.x : m.y, 4);
+          r += __shfl_xor_sync(0xFFFFFFFFu, r, 2);
+          r += __shfl_xor_sync(0xFFFFFFFFu, r, 1);
+          return r;
+        };
+        const int mine = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+        auto owner = [](int e) { return ((e >> 2) & 1) * 16 + ((e >> 1) & 1) * 8 + (e & 1) * 4; };
+        float2 nmean[4], rstd[4];
+        float my_rstd = 0.f;
+        if constexpr (MODE == 0) {
+          float2 s[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[e] = __fadd2_rn(__fadd2_rn(v[0][e], v[1][e]), __fadd2_rn(v[2][e], v[3][e]));
+          const float mean = reduce8(s) * (1.0f / 128.0f);
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            nmean[e] = make_float2(-__shfl_sync(0xFFFFFFFFu, mean, owner(2 * e)), -__shfl_sync(0xFFFFFFFFu, mean, owner(2 * e + 1)));
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            s[e] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              v[k][e] = __fadd2_rn(v[k][e], nmean[e]);
+              s[e] = __ffma2_rn(v[k][e], v[k][e], s[e]);
+            }
+          }
+          my_rstd = rsqrtf(reduce8(s) * (1.0f / 128.0f) + p.eps_out);
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            rstd[e] = make_float2(__shfl_sync(0xFFFFFFFFu, my_rstd, owner(2 * e)), __shfl_sync(0xFFFFFFFFu, my_rstd, owner(2 * e + 1)));
+        } else {
+          const int j8 = j0 + warp * 8;
+          float2 st = make_float2(0.f, 0.f);  // (positions past the end stay zero)
+          if (j8 + mine < p.n) st = p.ext_stats[static_cast<size_t>(row) * p.ld + j8 + mine];
+          my_rstd = st.y;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            nmean[e] = make_float2(-__shfl_sync(0xFFFFFFFFu, st.x, owner(2 * e)), -__shfl_sync(0xFFFFFFFFu, st.x, owner(2 * e + 1)));
+            rstd[e] = make_float2(__shfl_sync(0xFFFFFFFFu, st.y, owner(2 * e)), __shfl_sync(0xFFFFFFFFu, st.y, owner(2 * e + 1)));
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k][e] = __fadd2_rn(v[k][e], nmean[e]);
+          }
+        }
+        if ((lane & 3) == 0)
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(rstd_s + (warp * 8 + mine) * 4), "f"(my_rstd) : "memory");
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          st_chunk(addr[k], pack_f16x2_sat(__fmul2_rn(v[k][0], rstd[0])), pack_f16x2_sat(__fmul2_rn(v[k][1], rstd[1])),
+                   pack_f16x2_sat(__fmul2_rn(v[k][2], rstd[2])), pack_f16x2_sat(__fmul2_rn(v[k][3], rstd[3])));
+      }
+      // ---- z normalised in place: eight lanes per position, 64 positions per pass
+      thread_wait(z_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+      __syncwarp();
+      {
+        constexpr int kPairs = 4 * kZHalves;  // channel pairs per lane
+        const int sub = threadIdx.x & 7, slot = threadIdx.x >> 3;
+        uint32_t addr[2];
+        float2 v[2][kPairs];
+#pragma unroll
+        for (int pass = 0; pass < 2; ++pass) {
+          const int zp = pass * 64 + slot;
+          addr[pass] = z_s + zp * 128 + ((sub ^ (zp & 7)) << 4);
+#pragma unroll
+          for (int h = 0; h < kZHalves; ++h) {
+            const uint4 x = ld_chunk(addr[pass] + h * 16384);
+            v[pass][4 * h] = bf16x2_to_float2(x.x), v[pass][4 * h + 1] = bf16x2_to_float2(x.y);
+            v[pass][4 * h + 2] = bf16x2_to_float2(x.z), v[pass][4 * h + 3] = bf16x2_to_float2(x.w);
+          }
+        }
+#pragma unroll
+        for (int pass = 0; pass < 2; ++pass) {
+          float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int i = 0; i < kPairs; ++i) s = __fadd2_rn(s, v[pass][i]);
+          float sum = s.x + s.y;
+          sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+          sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
+          sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 4);
+          const float mean = sum * (1.0f / C);
+          float2 qs = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int i = 0; i < kPairs; ++i) {
+            v[pass][i] = __fadd2_rn(v[pass][i], make_float2(-mean, -mean));
+            qs = __ffma2_rn(v[pass][i], v[pass][i], qs);
+          }
+          float ssq = qs.x + qs.y;
+          ssq += __shfl_xor_sync(0xFFFFFFFFu, ssq, 1);
+          ssq += __shfl_xor_sync(0xFFFFFFFFu, ssq, 2);
+          ssq += __shfl_xor_sync(0xFFFFFFFFu, ssq, 4);
+          const float rs = rsqrtf(ssq * (1.0f / C) + p.eps_in);
+          const float2 rs2 = make_float2(rs, rs);
+          if constexpr (MODE != 1) {
+            const int jz = j0 + pass * 64 + slot;
+            if (sub == 0 && jz < p.n) p.rstd[static_cast<size_t>(row) * p.ld + jz] = rs;
+          }
+#pragma unroll
+          for (int h = 0; h < kZHalves; ++h)
+            st_chunk(addr[pass] + h * 16384, pack_f16x2_sat(__fmul2_rn(v[pass][4 * h], rs2)),
+                     pack_f16x2_sat(__fmul2_rn(v[pass][4 * h + 1], rs2)), pack_f16x2_sat(__fmul2_rn(v[pass][4 * h + 2], rs2)),
+                     pack_f16x2_sat(__fmul2_rn(v[pass][4 * h + 3], rs2)));
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      named_bar_arrive(kBarN, kTwo);
+      // the dropout scale of this thread's position, requested before the waits
+      uint4 scv[kZChunks];
+#pragma unroll
+      for (int ch = 0; ch < kZChunks; ++ch) scv[ch] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);  // bf16 ones
+      if (p.drop_scale != nullptr && j < p.n) {
+        const int b = row / p.n;
+        ldg_chunks(reinterpret_cast<const uint4*>(p.drop_scale + (static_cast<size_t>(b) * p.n + j) * C + part * kZCh),
+                   (reinterpret_cast<uintptr_t>(p.drop_scale) & 31u) == 0, scv);
+      }
+      float2 other = make_float2(0.f, 0.f);  // MODE 2: the first launch's sums of this position
       if constexpr (MODE == 2) {
-        if (inside) other = p.ln_part[static_cast<size_t>(row) * p.ld + j0 + pos];
+        if (part == 0 && j < p.n) other = p.ln_part[static_cast<size_t>(row) * p.ld + j];
       }
-      float s1 = 0.f, s2 = 0.f;
-      float th[kBwdCh];                 // this thread's t_hat values and its d t_hat, both kept for the second pass
-      uint32_t dtv[kBwdChunks][8];
-#pragma unroll
-      for (int ch = 0; ch < kBwdChunks; ++ch) tmem_ld8(tmem_base + lane_sel + part * kBwdCh + ch * 8, dtv[ch]);
-#pragma unroll
-      for (int cc = 0; cc < kBwdCh; ++cc) th[cc] = ld_f16(t_s + tile_off(part * kBwdCh + cc, pos));
-      tmem_ld_wait();
-#pragma unroll
-      for (int ch = 0; ch < kBwdChunks; ++ch) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float d = __uint_as_float(dtv[ch][e]);
-          s1 += d;
-          s2 = fmaf(d, th[ch * 8 + e], s2);
-        }
-      }
-      asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + (part * 128 + pos) * 8), "f"(s1), "f"(s2) : "memory");
-      named_bar_sync(1, kBwdThreads);
-      float m1, m2;
-      sum_partials(xchg, pos, m1, m2);
-      if constexpr (MODE == 1) {
-        if (part == 0 && inside) p.ln_part[static_cast<size_t>(row) * p.ld + j0 + pos] = make_float2(m1, m2);
-      } else if constexpr (MODE == 2) {
-        m1 = (m1 + other.x) * (1.0f / 256.0f), m2 = (m2 + other.y) * (1.0f / 256.0f);
-        if (part == 0 && inside) p.ln_part[static_cast<size_t>(row) * p.ld + j0 + pos] = make_float2(m1, m2);
-      } else {
-        m1 *= 1.0f / 128.0f, m2 *= 1.0f / 128.0f;
-      }
-      const float rs = rstd_out * 0.0625f;  // d / d t of the stored t / 16
-#pragma unroll
-      for (int ch = 0; ch < kBwdChunks; ++ch) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const uint32_t addr = t_s + tile_off(part * kBwdCh + ch * 8 + e, pos);
-          if constexpr (MODE == 1) st_f16_sat(addr, __uint_as_float(dtv[ch][e]));  // finished by bwd_ln_finish_kernel
-          else st_f16_sat(addr, rs * (__uint_as_float(dtv[ch][e]) - m1 - th[ch * 8 + e] * m2));
-        }
-      }
-      if constexpr (MODE != 1) {
-        uint32_t xg[kZChunks][8];
-#pragma unroll
-        for (int ch = 0; ch < kZChunks; ++ch) tmem_ld8(tmem_base + lane_sel + 128 + part * kZCh + ch * 8, xg[ch]);
-        tmem_ld_wait();
+      thread_wait(dy_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+      if constexpr (MODE == 2) thread_wait(pp_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+      thread_wait(fwd_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
+      __syncwarp();
+      tc_fence_after();
+      // ---- dproj = c du gate, dgate = c du proj gate (1 - gate); du = dy (* dropout scale). This thread: one position,
+      // kZCh channels; s = sums over them of dproj rowsum(Wo') and dproj P.
+      float2 sum1 = make_float2(0.f, 0.f), sum2 = make_float2(0.f, 0.f);
+      {
+        const float2 half2 = make_float2(0.5f, 0.5f), gc2 = make_float2(gc, gc);
+        uint32_t vp[2][8], vg[2][8];
+        tmem_ld8(tmem_base + lane_sel + part * kZCh, vp[0]);
+        tmem_ld8(tmem_base + lane_sel + 128 + part * kZCh, vg[0]);
 #pragma unroll
         for (int ch = 0; ch < kZChunks; ++ch) {
-          const uint32_t(&x)[8] = xg[ch];
-          st_chunk(z_s + tile_chunk(pos, part * kZChunks + ch),
-                   pack_f16x2_sat(make_float2(__uint_as_float(x[0]), __uint_as_float(x[1]))),
-                   pack_f16x2_sat(make_float2(__uint_as_float(x[2]), __uint_as_float(x[3]))),
-                   pack_f16x2_sat(make_float2(__uint_as_float(x[4]), __uint_as_float(x[5]))),
-                   pack_f16x2_sat(make_float2(__uint_as_float(x[6]), __uint_as_float(x[7]))));
+          tmem_ld_wait();
+          if (ch < kZChunks - 1) {
+            tmem_ld8(tmem_base + lane_sel + part * kZCh + (ch + 1) * 8, vp[(ch + 1) & 1]);
+            tmem_ld8(tmem_base + lane_sel + 128 + part * kZCh + (ch + 1) * 8, vg[(ch + 1) & 1]);
+          }
+          const uint32_t addr = tile_chunk(pos, part * kZChunks + ch);
+          const uint4 dyv = ld_chunk(dy_s + addr);
+          uint4 ppv = make_uint4(0u, 0u, 0u, 0u);
+          if constexpr (MODE == 2) ppv = ld_chunk(dg_s + addr);
+          const uint32_t pw[4] = {ppv.x, ppv.y, ppv.z, ppv.w};
+          const uint32_t dw[4] = {dyv.x, dyv.y, dyv.z, dyv.w};
+          const uint32_t sw[4] = {scv[ch].x, scv[ch].y, scv[ch].z, scv[ch].w};
+          const float2* cp = reinterpret_cast<const float2*>(const_ptr + part * kZCh + ch * 8);
+          uint32_t op[4], og[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const float2 praw = pair_of(vp[ch & 1][2 * t], vp[ch & 1][2 * t + 1]);
+            float2 proj = __fadd2_rn(praw, cp[t]);
+            if constexpr (MODE == 2) proj = __fadd2_rn(proj, f16x2_to_float2(pw[t]));
+            const float2 gh = __fmul2_rn(__fadd2_rn(pair_of(vg[ch & 1][2 * t], vg[ch & 1][2 * t + 1]), cp[64 + t]), half2);
+            const float2 gate = __ffma2_rn(make_float2(tanh_approx(gh.x), tanh_approx(gh.y)), half2, half2);
+            const float2 du = __fmul2_rn(__fmul2_rn(bf16x2_to_float2(dw[t]), bf16x2_to_float2(sw[t])), gc2);
+            const float2 dp = __fmul2_rn(du, gate);
+            op[t] = pack_f16x2_sat(dp);
+            const float2 dpr = f16x2_to_float2(op[t]);  // what the gradient GEMMs read
+            sum1 = __ffma2_rn(dpr, cp[128 + t], sum1);
+            sum2 = __ffma2_rn(dpr, praw, sum2);
+            // MODE 1 hands its part of proj on
+            og[t] = pack_f16x2_sat(MODE == 1 ? proj
+                                             : __fmul2_rn(dp, __ffma2_rn(make_float2(-proj.x, -proj.y), gate, proj)));
+          }
+          st_chunk(dy_s + addr, op[0], op[1], op[2], op[3]);
+          // MODE 1: the part of proj leaves through the z buffer (x_hat is only needed by the G GEMM, which is done)
+          st_chunk((MODE == 1 ? z_s : dg_s) + addr, og[0], og[1], og[2], og[3]);
+          if constexpr (C == 64) {
+            // the weight-gradient GEMMs read these tiles as 128-row operands: rows 64-127 (the second 64-channel block) are zero
+            const uint32_t zaddr = tile_chunk(pos, 8 + part * kZChunks + ch);
+            st_chunk(dy_s + zaddr, 0u, 0u, 0u, 0u);
+            st_chunk(dg_s + zaddr, 0u, 0u, 0u, 0u);
+          }
         }
       }
-    }
-    tc_fence_before();
-    fence_proxy_async_smem();
-    ok = __syncthreads_and(ok ? 1 : 0) != 0;  // a thread that gave up takes the whole CTA out here
-    if (!ok) break;
-    if (threadIdx.x == 0) {
-#pragma unroll
-      for (int kh = 0; kh < 2; ++kh)
-        if (j0 + kh * 64 < p.n) tma_store_3d(&map_dt, t_s + kh * 16384, j0 + kh * 64, 0, row);
-#pragma unroll
-      for (int kh = 0; kh < kZHalves; ++kh) tma_store_3d(&map_dx, z_s + kh * 16384, kh * 64, j0, row);
-      bulk_commit();
-    }
-  }
-  if (threadIdx.x == 0) {
-    if (!ok) {  // a wait gave up: copies in flight must land before the CTA exits
-      const long long t0 = clock64();
-      while (!mbar_try_wait(w_full, 0) || (tz_pending >= 0 && !mbar_try_wait(tz_full, tz_pending & 1)) ||
-             (dy_pending >= 0 && !mbar_try_wait(dy_full, dy_pending & 1))) {
-        if (clock64() - t0 > kWaitLimitCycles) {
-          atomicCAS(p.status, 0, kDevTimeoutDrain);
-          break;
+      asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + (part * 128 + pos) * 8), "f"(sum1.x + sum1.y),
+                   "f"(sum2.x + sum2.y) : "memory");
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      named_bar_sync(kBarA, kTwo);
+      // ---- (under the gradient GEMMs) the position's two means and the coefficients of its LayerNorm backward
+      if (part == 0) {
+        float m1, m2;
+        sum_partials(xchg, pos, m1, m2);
+        if constexpr (MODE == 1) {
+          if (j < p.n) p.ln_part[static_cast<size_t>(row) * p.ld + j] = make_float2(m1, m2);
+        } else {
+          if constexpr (MODE == 2) {
+            m1 = (m1 + other.x) * (1.0f / 256.0f), m2 = (m2 + other.y) * (1.0f / 256.0f);
+            if (j < p.n) p.ln_part[static_cast<size_t>(row) * p.ld + j] = make_float2(m1, m2);
+          } else {
+            m1 *= 1.0f / 128.0f, m2 *= 1.0f / 128.0f;
+          }
+          float rs;
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(rs) : "r"(rstd_s + pos * 4));
+          rs *= 0.0625f;  // d / d t of the stored t / 16
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(coef_s + pos * 4), "f"(rs) : "memory");
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(coef_s + 512 + pos * 4), "f"(-rs * m1) : "memory");
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(coef_s + 1024 + pos * 4), "f"(-rs * m2) : "memory");
         }
       }
+      if (sum_chunk < C / 8) {  // column sums of the two fp16 tiles the GEMMs are reading
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const uint32_t addr = tile_chunk(sum_rows + r, sum_chunk);
+          const uint4 a = ld_chunk(dy_s + addr);
+          const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const float2 x = f16x2_to_float2(aw[t]);
+            acc_so[2 * t] += x.x, acc_so[2 * t + 1] += x.y;
+          }
+          if constexpr (MODE != 1) {
+            const uint4 b = ld_chunk(dg_s + addr);
+            const uint32_t bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              const float2 x = f16x2_to_float2(bw[t]);
+              acc_sg[2 * t] += x.x, acc_sg[2 * t + 1] += x.y;
+            }
+          }
+        }
+      }
+      __syncwarp();
+      named_bar_arrive(kBarS, kOne);
+      if constexpr (MODE != 1) named_bar_sync(1, kBwdThreads);  // the coefficients are there
+      // ---- LayerNorm backward of the output normalisation for this thread's channel and 32 positions; d x_hat of its position
+      thread_wait(d_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
+      __syncwarp();
+      tc_fence_after();
+      uint32_t ot[16];
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t dv[16];
+        tmem_ld16(tmem_base + lane_sel + part * 32 + hf * 16, dv);
+        uint4 th[2];
+        if constexpr (MODE != 1) {
+#pragma unroll
+          for (int k = 0; k < 2; ++k) th[k] = ld_chunk(t_s + tile_chunk(pos, part * 4 + hf * 2 + k));
+        }
+        tmem_ld_wait();
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const uint32_t tw[4] = {th[k].x, th[k].y, th[k].z, th[k].w};
+#pragma unroll
+          for (int t2 = 0; t2 < 2; ++t2) {
+            const uint32_t cpos = static_cast<uint32_t>(part * 32 + hf * 16 + k * 8 + t2 * 4) * 4;
+            float4 ca, cb, cc;  // four positions (the same addresses for the whole warp)
+            if constexpr (MODE != 1) {
+              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(ca.x), "=f"(ca.y), "=f"(ca.z), "=f"(ca.w) : "r"(coef_s + cpos));
+              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(cb.x), "=f"(cb.y), "=f"(cb.z), "=f"(cb.w) : "r"(coef_s + 512 + cpos));
+              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(cc.x), "=f"(cc.y), "=f"(cc.z), "=f"(cc.w) : "r"(coef_s + 1024 + cpos));
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int t = t2 * 2 + u;
+              float2 d = pair_of(dv[k * 8 + 2 * t], dv[k * 8 + 2 * t + 1]);
+              if constexpr (MODE != 1) {
+                const float2 a2 = u == 0 ? make_float2(ca.x, ca.y) : make_float2(ca.z, ca.w);
+                const float2 b2 = u == 0 ? make_float2(cb.x, cb.y) : make_float2(cb.z, cb.w);
+                const float2 c2 = u == 0 ? make_float2(cc.x, cc.y) : make_float2(cc.z, cc.w);
+                d = __ffma2_rn(d, a2, __ffma2_rn(f16x2_to_float2(tw[t]), c2, b2));
+              }
+              ot[hf * 8 + k * 4 + t] = pack_f16x2_sat(d);  // (MODE 1: finished by bwd_ln_finish_kernel)
+            }
+          }
+        }
+      }
+      uint32_t ox[MODE != 1 ? kZChunks * 4 : 1];
+      if constexpr (MODE != 1) {
+#pragma unroll
+        for (int ch = 0; ch < kZChunks; ++ch) {
+          uint32_t x[8];
+          tmem_ld8(tmem_base + lane_sel + 128 + part * kZCh + ch * 8, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int t = 0; t < 4; ++t) ox[ch * 4 + t] = pack_f16x2_sat(pair_of(x[2 * t], x[2 * t + 1]));
+        }
+      }
+      tc_fence_before();
+      thread_wait(grad_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);  // the GEMMs have read t_hat and x_hat
+      __syncwarp();
+#pragma unroll
+      for (int k4 = 0; k4 < 4; ++k4)
+        st_chunk(t_s + tile_chunk(pos, part * 4 + k4), ot[k4 * 4], ot[k4 * 4 + 1], ot[k4 * 4 + 2], ot[k4 * 4 + 3]);
+      if constexpr (MODE != 1) {
+#pragma unroll
+        for (int ch = 0; ch < kZChunks; ++ch)
+          st_chunk(z_s + tile_chunk(pos, part * kZChunks + ch), ox[ch * 4], ox[ch * 4 + 1], ox[ch * 4 + 2], ox[ch * 4 + 3]);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      named_bar_arrive(kBarC, kOne);
     }
-    bulk_wait<0>();
-  }
-  __syncthreads();
-  if (ok && it > 0) {
-    // weight-gradient accumulators: lane = output row of the matrix, this thread's 64 columns
+    // ---- per-CTA partials of the weight gradients (every GEMM has been waited for) and of the column sums
     tc_fence_after();
     float* pm = p.part_m + static_cast<size_t>(blockIdx.x) * 2 * 128 * 128;
 #pragma unroll
@@ -658,21 +847,20 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
         store_partial(pm + m * 128 * 128, pos, part * kBwdChunks + ch, v);
       }
     }
-  }
-  {  // the 32 row groups of a channel, fixed order; every tile region is free by now
-    float* sc = reinterpret_cast<float*>(smem);  // [32 row groups][2][128]
+    {  // the 32 row groups of a channel, fixed order (through the weights' region, which no GEMM reads any more)
+      float* sc = reinterpret_cast<float*>(smem);  // [32 row groups][2][128]
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      sc[((threadIdx.x >> 4) * 2 + 0) * 128 + sum_chunk * 8 + c] = acc_so[c];
-      sc[((threadIdx.x >> 4) * 2 + 1) * 128 + sum_chunk * 8 + c] = acc_sg[c];
+      for (int c = 0; c < 8; ++c) {
+        sc[((threadIdx.x >> 4) * 2 + 0) * 128 + sum_chunk * 8 + c] = acc_so[c];
+        sc[((threadIdx.x >> 4) * 2 + 1) * 128 + sum_chunk * 8 + c] = acc_sg[c];
+      }
+      named_bar_sync(1, kBwdThreads);
+      if (threadIdx.x < 256 && (threadIdx.x & 127) < C) {
+        float sum = 0.f;
+        for (int g = 0; g < 32; ++g) sum += sc[g * 256 + threadIdx.x];
+        p.part_s[static_cast<size_t>(blockIdx.x) * 2 * 128 + threadIdx.x] = sum;
+      }
     }
-    __syncthreads();
-    if (threadIdx.x < 256 && (threadIdx.x & 127) < C) {
-      float sum = 0.f;
-      for (int g = 0; g < 32; ++g) sum += sc[g * 256 + threadIdx.x];
-      p.part_s[static_cast<size_t>(blockIdx.x) * 2 * 128 + threadIdx.x] = sum;
-    }
-    __syncthreads();
   }
   tc_fence_before();
   __syncthreads();
@@ -1339,7 +1527,8 @@ __device__ __forceinline__ void amax_and_scale(const uint4* dy, size_t n_chunks,
 // as dense fp16 [128][128] with the LayerNorm gamma of their input folded in, W'[r][k] = W[r][k] gamma[k], and
 // d[m][r] = sum_k W[r][k] beta[k] + bias[m][r] (fp32) behind them. One warp per matrix row.
 constexpr size_t kBwdPackedD = 6 * 32768;
-constexpr size_t kBwdPackedBytes = kBwdPackedD + 3072;  // 199680, a multiple of 1024
+constexpr size_t kBwdPackedRowSum = kBwdPackedD + 3072;        // float[128]: row sums of W'_out
+constexpr size_t kBwdPackedBytes = kBwdPackedRowSum + 1024;    // 200704, a multiple of 1024
 __device__ __forceinline__ void bwd_pack_row(const PackArgs& a, uint8_t* packed, int gw) {  // gw: 0 .. 767
   const int lane = threadIdx.x & 31;
   const int m = gw >> 7, row = gw & 127;
@@ -1361,11 +1550,13 @@ __device__ __forceinline__ void bwd_pack_row(const PackArgs& a, uint8_t* packed,
   const float4 g = active ? reinterpret_cast<const float4*>(gamma)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float4 b = active ? reinterpret_cast<const float4*>(beta)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float gg[4] = {g.x, g.y, g.z, g.w}, bb[4] = {b.x, b.y, b.z, b.w};
-  float d = 0.f;
+  float d = 0.f, rs = 0.f;
   uint16_t o[4];
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
-    o[t] = __half_as_ushort(__float2half_rn(fminf(fmaxf(w[t] * gg[t], -65504.f), 65504.f)));
+    const __half r = __float2half_rn(fminf(fmaxf(w[t] * gg[t], -65504.f), 65504.f));
+    o[t] = __half_as_ushort(r);
+    rs += __half2float(r);
     d = fmaf(w[t], bb[t], d);
   }
   if (active) {
@@ -1375,7 +1566,11 @@ __device__ __forceinline__ void bwd_pack_row(const PackArgs& a, uint8_t* packed,
     reinterpret_cast<uint2*>(packed + static_cast<size_t>(m) * 32768)[row * (k / 4) + lane] = ov;
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) d += __shfl_xor_sync(0xFFFFFFFFu, d, off);
+  for (int off = 16; off > 0; off >>= 1) {
+    d += __shfl_xor_sync(0xFFFFFFFFu, d, off);
+    rs += __shfl_xor_sync(0xFFFFFFFFu, rs, off);
+  }
+  if (lane == 0 && m == 4) reinterpret_cast<float*>(packed + kBwdPackedRowSum)[row] = rs;
   if (lane == 0)
     reinterpret_cast<float*>(packed + kBwdPackedD)[m * 128 + row] = d + (a.bias[m] != nullptr ? a.bias[m][row] : 0.f);
 }
