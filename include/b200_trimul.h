@@ -315,16 +315,16 @@ int b200_trimul_forward_static(const void* z, const void* w_left, const void* w_
  *                                    order): [128, 128] each, or [256, 128] x 4, [128, 128], [128, 256] for direction 0
  *   d_ln_in_w / _b fp32 [128],  d_ln_out_w / _b fp32 [128] (direction 0: [256])
  * Every output is overwritten, not accumulated into. Biases are constants (no gradient). drop_scale as in the forward.
- * Launches, one direction: weight packing, max |dy| and the power-of-two scale the fp16 gradient tiles carry, the
+ * Launches, one direction: one for weight packing, max |dy| and the power-of-two scale the fp16 gradient tiles carry, the
  * epilogue's backward (one kernel: both LayerNorm-folded GEMMs recomputed, four gradient GEMMs on the tensor cores), the
- * two contraction gradient launches, the prologue's backward once per side, partial-sum reductions, the parameter
- * gradients. Direction 0 (the bidirectional module): the statistics of the 256-channel output LayerNorm, the epilogue's
+ * two contraction gradient launches, the prologue's backward once per side, two for the parameter gradients (the sums over
+ * the CTAs' partials and the LayerNorm terms). Direction 0 (the bidirectional module): the statistics of the 256-channel output LayerNorm, the epilogue's
  * backward once per 128-channel tensor plus a kernel that finishes the first tensor's LayerNorm backward, the forward's
  * prologue once more (left / right of the first half, which the forward overwrote), four contraction gradient launches,
  * the prologue's backward four times (side x half).
  * The result is deterministic (fixed summation order). Workspace: b200_trimul_backward_workspace_bytes, 1024-byte
- * aligned; _layout gives its 17 region offsets + the total (status, packed weights, scale, reduced sums M and S, per-CTA
- * partials of M and S, dtri, dleft, dright, d x_hat, then the bidirectional module's extra regions) for tests.
+ * aligned; _layout gives its 17 region offsets + the total (status, packed weights, scale, LayerNorm terms, x_hat and
+ * 1 / sigma, per-CTA partials of M and S of every launch, dtri, dleft, dright, d x_hat, then the bidirectional module's extra regions) for tests.
  */
 int b200_trimul_backward_workspace_bytes(int B, int N, int direction, size_t* out_bytes);
 int b200_trimul_backward_workspace_layout(int B, int N, int direction, size_t* offsets18);
@@ -378,8 +378,8 @@ int b200_trimul_read_status(const int* status, void* cuda_stream, int* host_stat
  * bf16) and the forward's inputs, writes dx ([positions, 128] bf16, the residual path included when `residual` is
  * non-zero) and, in fp32 and the parameters' shapes, d_expand_a / d_expand_b [512, 128], d_squeeze [128, 512],
  * d_ln_w / d_ln_b [128]. Every output is overwritten. One launch per block of 128 hidden units (four), whose three
- * weight-gradient accumulators stay in tensor memory over all positions; the running d x_hat is carried between the
- * launches in the workspace. Deterministic. Workspace: b200_transition_backward_workspace_bytes, 1024-byte aligned.
+ * weight-gradient accumulators stay in tensor memory over all positions; x_hat, the scaled dy (both left by the first
+ * launch) and the running d x_hat are carried between the launches in the workspace. Deterministic. Workspace: b200_transition_backward_workspace_bytes, 1024-byte aligned.
  */
 int b200_transition_backward_workspace_bytes(long long positions, size_t* out_bytes);
 int b200_transition_backward(const void* dy, const void* x, const void* w_expand_a, const void* w_expand_b,

@@ -1,10 +1,11 @@
 // Backward of the triangle update around the contraction: the epilogue's gradients (output LayerNorm, output
 // projection, output gate) and the prologue's gradients (input LayerNorm, the four gated projections, the mask).
 //
-// Both kernels walk tiles of 128 consecutive columns j of one pair row, one CTA per SM, 512 threads: four threads per
-// position (its TMEM lane), each covering a quarter of the channels. A tile goes through a fixed sequence of phases
-// separated by CTA-wide barriers; one thread issues the TMA copies and the MMAs. Per tile:
-//   1. TMA loads of the tile's inputs; the LayerNorm inputs are normalised in place in shared memory (fp16),
+// Both kernels walk tiles of 128 consecutive columns j of one pair row, one CTA per SM: 16 arithmetic warps (four threads per
+// position or channel, its TMEM lane, each covering a quarter of the other dimension), a warp that issues the MMAs and one
+// that issues the TMA copies. Per tile:
+//   1. the inputs arrive; the epilogue's backward normalises t and z in place (fp16) and leaves x_hat and 1 / sigma for the
+//      prologue's backward,
 //   2. the forward GEMMs are recomputed on the tensor cores (weights with the LayerNorm gamma folded in, fp16),
 //   3. the threads turn the upstream gradient into the gradients of the GEMM outputs (fp16 tiles in shared memory),
 //   4. the tensor cores compute, from those tiles, the gradients with respect to the normalised inputs (the same weight
@@ -13,12 +14,12 @@
 // The four tile buffers of a CTA rotate their roles from tile to tile: the next tile's inputs are copied into the
 // buffers the gradient GEMMs have finished with while the tile completes, and a store is only waited for when its
 // buffer is needed again. Column sums of the dOut tiles (the bias-like terms) are accumulated per thread in
-// registers. At the end every CTA writes its partial M and column sums; small kernels add the partials and form the
-// parameter gradients. Both kernels are templates on the input width C (128, or 64 for the narrow pair stacks); the
+// registers. At the end every CTA writes its partial M and column sums; one pass over the partials of all launches forms
+// the parameter gradients. Both kernels are templates on the input width C (128, or 64 for the narrow pair stacks); the
 // epilogue's backward also has a two-launch form for an output LayerNorm over 256 channels (the bidirectional module).
 //
 // Gradients travel in fp16 tiles, so the upstream gradient is multiplied by a power of two c (read from device
-// memory, chosen from max |dy| by `bwd_amax_kernel` / `bwd_scale_kernel`); every output of these kernels carries that
+// memory, chosen from max |dy| by `amax_and_scale`); every output of these kernels carries that
 // factor, and the final kernels divide it out in fp32.
 #pragma once
 
@@ -34,30 +35,15 @@ constexpr int kBwdThreads = 128 * kBwdParts;
 constexpr int kBwdCh = 128 / kBwdParts;          // channels per thread of a 128-channel tile
 constexpr int kBwdChunks = kBwdCh / 8;           // 16-byte chunks (8 channels) per thread
 constexpr int kBwdTile = 32768;  // one [128][128] 16-bit tile
-constexpr int kBwdXchgHalf = kBwdParts * 128 * 8;  // float2 [kBwdParts][128]
-constexpr int kBwdXchg = 2 * kBwdXchgHalf;         // two exchange buffers, used in turn (see normalise_tile)
-constexpr int kBwdSmemBytes = 6 * kBwdTile + kBwdXchg + 1024 /* constants */ + 256 /* barriers */ + 1024;
+constexpr int kBwdXchg = kBwdParts * 128 * 8;  // float2 [kBwdParts][128]
 
-// swizzled byte offset of element (r, e) in a [128 rows][128 elements] 16-bit tile stored as two halves of 64 elements,
-// each [128 rows][128 bytes] with the 128-byte TMA swizzle
-__device__ __forceinline__ uint32_t tile_off(int r, int e) {
-  return static_cast<uint32_t>((e >> 6) * 16384 + r * 128 + ((((e & 63) >> 3) ^ (r & 7)) << 4) + (e & 7) * 2);
-}
+// [128 rows][128 elements] 16-bit tiles are stored as two halves of 64 elements, each [128 rows][128 bytes] with the 128-byte
+// TMA swizzle:
 // offset of the 16-byte chunk holding elements 8*ch .. 8*ch+7 (ch = 0..15) of row r
 __device__ __forceinline__ uint32_t tile_chunk(int r, int ch) {
   return static_cast<uint32_t>((ch >> 3) * 16384 + r * 128 + (((ch & 7) ^ (r & 7)) << 4));
 }
 
-__device__ __forceinline__ float ld_f16(uint32_t addr) {
-  uint16_t v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-  return __half2float(__ushort_as_half(v));
-}
-__device__ __forceinline__ void st_f16_sat(uint32_t addr, float x) {
-  uint16_t v;
-  asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(v) : "f"(x));
-  asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
-}
 __device__ __forceinline__ uint4 ld_chunk(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
@@ -87,53 +73,30 @@ __device__ __forceinline__ void ldg_chunks(const uint4* p, bool wide, uint4 (&ou
 }
 __device__ __forceinline__ float sigmoid_fast(float x) { return fmaf(tanh_approx(0.5f * x), 0.5f, 0.5f); }
 
-// (see mbar_wait_thread: a thread that gives up carries on and the CTA leaves together at the tile's closing barrier)
+// (see mbar_wait_thread: a thread that gives up sets the abort word and carries on)
 __device__ __forceinline__ bool thread_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
   return mbar_wait_thread(bar, parity, abort_flag, status, code);
 }
-// CTA-wide bounded wait on an mbarrier: one lane per warp polls, the decision is shared by all 256 threads.
-__device__ __forceinline__ bool cta_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  const bool got = mbar_wait_warp(bar, parity, abort_flag, status, code);
-  return named_bar_and(1, kBwdThreads, got);
-}
-
-// Normalise the CT channels of every position of a tile in place (fp16 result), the thread covering CT / kBwdParts of them.
-// ROWS_ARE_POSITIONS: element (pos, c) (a [pos][c] tile, input bf16 or fp16), else element (c, pos) (a [c][pos] tile,
-// fp16). Returns rstd of the thread's position. `xchg` holds float2 [kBwdParts][128]; the caller must not pass the same
-// buffer to two calls (or other uses) without a CTA-wide barrier between them.
-template <bool ROWS_ARE_POSITIONS, bool IN_BF16, int CT = 128>
+// Normalise the 128 channels of every position of a [pos][c] tile in place (bf16 in, fp16 out), the thread covering
+// 128 / kBwdParts of them. Returns rstd of the thread's position. `xchg` holds float2 [kBwdParts][128]; the caller must not
+// use it again without a barrier among the arithmetic threads.
 __device__ __forceinline__ float normalise_tile(uint32_t tile, uint32_t xchg, int pos, int part, float eps) {
-  constexpr int kCh = CT / kBwdParts;  // channels per thread
-  constexpr int kChunks = kCh / 8;
   float pv = 0.f, s1 = 0.f, s2 = 0.f;
-  float xt[ROWS_ARE_POSITIONS ? 1 : kCh];  // the [c][pos] form keeps its values between the two passes
-  if constexpr (ROWS_ARE_POSITIONS) {
 #pragma unroll
-    for (int ch = 0; ch < kChunks; ++ch) {
-      const uint4 v = ld_chunk(tile + tile_chunk(pos, part * kChunks + ch));
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  for (int ch = 0; ch < kBwdChunks; ++ch) {
+    const uint4 v = ld_chunk(tile + tile_chunk(pos, part * kBwdChunks + ch));
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float2 x = IN_BF16 ? bf16x2_to_float2(w[t]) : f16x2_to_float2(w[t]);
-        if (ch == 0 && t == 0) pv = x.x;
-        const float d0 = x.x - pv, d1 = x.y - pv;
-        s1 += d0 + d1;
-        s2 = fmaf(d0, d0, fmaf(d1, d1, s2));
-      }
-    }
-  } else {
-#pragma unroll
-    for (int cc = 0; cc < kCh; ++cc) xt[cc] = ld_f16(tile + tile_off(part * kCh + cc, pos));
-    pv = xt[0];
-#pragma unroll
-    for (int cc = 0; cc < kCh; ++cc) {
-      const float d = xt[cc] - pv;
-      s1 += d;
-      s2 = fmaf(d, d, s2);
+    for (int t = 0; t < 4; ++t) {
+      const float2 x = bf16x2_to_float2(w[t]);
+      if (ch == 0 && t == 0) pv = x.x;
+      const float d0 = x.x - pv, d1 = x.y - pv;
+      s1 += d0 + d1;
+      s2 = fmaf(d0, d0, fmaf(d1, d1, s2));
     }
   }
-  const float mean_h = pv + s1 * (1.0f / kCh);
-  const float m2_h = fmaxf(s2 - s1 * s1 * (1.0f / kCh), 0.f);
+  const float mean_h = pv + s1 * (1.0f / kBwdCh);
+  const float m2_h = fmaxf(s2 - s1 * s1 * (1.0f / kBwdCh), 0.f);
   asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + (part * 128 + pos) * 8), "f"(mean_h), "f"(m2_h) : "memory");
   named_bar_sync(1, kBwdThreads);
   // merge the equal-sized partials of this position: mean of means, M2 = sum M2_k + n_k sum (mean_k - mean)^2
@@ -147,28 +110,23 @@ __device__ __forceinline__ float normalise_tile(uint32_t tile, uint32_t xchg, in
   }
   mean *= 1.0f / kBwdParts;
 #pragma unroll
-  for (int k = 0; k < kBwdParts; ++k) m2 = fmaf(static_cast<float>(kCh) * (mk[k] - mean), mk[k] - mean, m2);
-  const float rstd = rsqrtf(m2 * (1.0f / CT) + eps);
+  for (int k = 0; k < kBwdParts; ++k) m2 = fmaf(static_cast<float>(kBwdCh) * (mk[k] - mean), mk[k] - mean, m2);
+  const float rstd = rsqrtf(m2 * (1.0f / 128.0f) + eps);
   const float nmr = -mean * rstd;
-  if constexpr (ROWS_ARE_POSITIONS) {
 #pragma unroll
-    for (int ch = 0; ch < kChunks; ++ch) {
-      const uint32_t addr = tile + tile_chunk(pos, part * kChunks + ch);
-      const uint4 v = ld_chunk(addr);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-      uint32_t o[4];
+  for (int ch = 0; ch < kBwdChunks; ++ch) {
+    const uint32_t addr = tile + tile_chunk(pos, part * kBwdChunks + ch);
+    const uint4 v = ld_chunk(addr);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t o[4];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float2 x = IN_BF16 ? bf16x2_to_float2(w[t]) : f16x2_to_float2(w[t]);
-        o[t] = pack_f16x2_sat(make_float2(fmaf(x.x, rstd, nmr), fmaf(x.y, rstd, nmr)));
-      }
-      st_chunk(addr, o[0], o[1], o[2], o[3]);
+    for (int t = 0; t < 4; ++t) {
+      const float2 x = bf16x2_to_float2(w[t]);
+      o[t] = pack_f16x2_sat(make_float2(fmaf(x.x, rstd, nmr), fmaf(x.y, rstd, nmr)));
     }
-  } else {
-#pragma unroll
-    for (int cc = 0; cc < kCh; ++cc) st_f16_sat(tile + tile_off(part * kCh + cc, pos), fmaf(xt[cc], rstd, nmr));
+    st_chunk(addr, o[0], o[1], o[2], o[3]);
   }
-  return rstd;  // (no closing barrier: consecutive calls alternate between the two exchange buffers)
+  return rstd;
 }
 
 // Sum of the float2 partials the kBwdParts threads of a position left in `xchg` (fixed order).
@@ -180,28 +138,6 @@ __device__ __forceinline__ void sum_partials(uint32_t xchg, int pos, float& a, f
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(xchg + (k * 128 + pos) * 8));
     a += x, b += y;
   }
-}
-
-// Sum the per-thread column partials of a CTA over its 128 positions: `acc` holds this thread's channels (part
-// `part`) for two vectors; scratch is float[256][129] (a tile region, padded against bank conflicts).
-template <int NCH>
-__device__ __forceinline__ void flush_colsums(const float (&a0)[NCH], const float (&a1)[NCH], uint8_t* scratch, int pos,
-                                              int part, float* out0, float* out1) {
-  float* s = reinterpret_cast<float*>(scratch);
-  // rows: (vector * 128 + channel), columns: position
-#pragma unroll
-  for (int c = 0; c < NCH; ++c) {
-    s[(0 * 128 + part * NCH + c) * 129 + pos] = a0[c];
-    s[(1 * 128 + part * NCH + c) * 129 + pos] = a1[c];
-  }
-  __syncthreads();
-  const int r = threadIdx.x;  // 0..255: vector r / 128, channel r % 128 (channels beyond 4 * NCH do not exist)
-  if (r < 256 && (r & 127) < NCH * kBwdParts) {
-    float sum = 0.f;
-    for (int p = 0; p < 128; ++p) sum += s[r * 129 + p];
-    (r < 128 ? out0 : out1)[r & 127] = sum;
-  }
-  __syncthreads();
 }
 
 // Eight columns (8 * chunk ..) of row `row` of a CTA's partial weight gradient. The matrix lies in memory as [32 groups of
@@ -280,9 +216,9 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
   const uint32_t wo_s = smem_base, wg_s = smem_base + kBwdTile;
   const uint32_t tiles_s = smem_base + 2 * kBwdTile;  // four tile buffers whose roles rotate from tile to tile
   const uint32_t xchg = smem_base + 6 * kBwdTile;     // float2 [kBwdParts][128]: partial sums of the LayerNorm backward
-  const uint32_t coef_s = xchg + kBwdXchgHalf;        // float [3][128]: d t = a d t_hat + b + c t_hat
+  const uint32_t coef_s = xchg + kBwdXchg;        // float [3][128]: d t = a d t_hat + b + c t_hat
   const uint32_t rstd_s = coef_s + 1536;              // float [128]: 1 / sigma of the output LayerNorm
-  float* const_ptr = reinterpret_cast<float*>(smem + 6 * kBwdTile + kBwdXchgHalf + 2048);  // d_out, d_gate, rowsum(Wo') [3][128]
+  float* const_ptr = reinterpret_cast<float*>(smem + 6 * kBwdTile + kBwdXchg + 2048);  // d_out, d_gate, rowsum(Wo') [3][128]
   const uint32_t bar_base = smem_base + 6 * kBwdTile + 8192;
   const uint32_t w_full = bar_base, t_full = bar_base + 8, z_full = bar_base + 16, dy_full = bar_base + 24;
   const uint32_t pp_full = bar_base + 32, fwd_done = bar_base + 40, d_done = bar_base + 48, grad_done = bar_base + 56;

@@ -275,7 +275,7 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         thread_wait(x_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
         // (the exchange of the statistics uses S1, the previous tile's dy buffer, once its store has read it)
         if (it != 0) thread_wait(out_free, (it - 1) & 1, abort_flag, p.status, kDevTimeoutStats);
-        rstd_in = normalise_tile<true, true, 128>(x_s, s1_s, pos, part, p.eps);
+        rstd_in = normalise_tile(x_s, s1_s, pos, part, p.eps);
         if (part == 0 && inside) p.rstd[gp] = rstd_in;
         fence_proxy_async_smem();
         __syncwarp();

@@ -1,0 +1,85 @@
+"""Backward kernels where their tilings and reductions have edges: position counts around one tile and around one tile per
+CTA for the Transition, short rows for the wide LayerNorm statistics, and gradients of zero or with a non-finite value for the
+scale, against float64 torch on the GPU.
+
+Bound: an input gradient is rounded to bf16 (relative 2^-9 / sqrt(3) = 1.1e-3, up to 1.7e-3 by how values lie in their
+binades) after three fp16 roundings (2^-12 each, through products): 2.5 times their sum."""
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+import miniworld_b200 as mw
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+TOL = 5e-3
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm().clamp_min(1e-30))
+
+
+def _transition64(m, x, dy):
+    p = {k: v.detach().double().requires_grad_(True) for k, v in m.named_parameters()}
+    z = x.double().requires_grad_(True)
+    h = F.layer_norm(z, (128,), p["ln_in.weight"], p["ln_in.bias"], 1e-5)
+    y = z + F.linear(F.silu(F.linear(h, p["expand_a.weight"])) * F.linear(h, p["expand_b.weight"]), p["squeeze.weight"])
+    return torch.autograd.grad(y, [z, *p.values()], dy.double())
+
+
+def _module(make, seed):
+    g = torch.Generator().manual_seed(seed)
+    m = make()
+    for p in m.parameters():
+        p.data = torch.randn(p.shape, generator=g) * (p.shape[-1] ** -0.5 if p.dim() == 2 else 0.1) + (p.dim() == 1) * 0.7
+    return m.to(DEV).train(), g
+
+
+@pytest.mark.parametrize("positions", [1, 127, 128, 129, 147 * 128 + 1, 148 * 128, 148 * 128 + 1, 4 * 148 * 128 + 77])
+def test_transition_position_counts(positions):
+    m, g = _module(lambda: mw.Transition(128), positions)
+    x = torch.randn(positions, 128, generator=g).to(torch.bfloat16).to(DEV)
+    dy = (torch.randn(positions, 128, generator=g) * 0.02).to(torch.bfloat16).to(DEV)
+    xr = x.clone().requires_grad_(True)
+    got = torch.autograd.grad(m(xr), [xr, *m.parameters()], dy)
+    for name, a, b in zip(["x", *dict(m.named_parameters())], got, _transition64(m, x, dy)):
+        assert _rel(a, b) <= TOL, (name, _rel(a, b))
+
+
+@pytest.mark.parametrize("B,N", [(1, 8), (3, 8), (1, 24), (1, 136)])
+def test_wide_statistics_of_short_rows(B, N):
+    """The bidirectional module's gradients do not depend on the batch they are computed in (its statistics kernel takes 32
+    column groups per block, across rows and samples)."""
+    m, g = _module(lambda: mw.BidirectionalTriangleMultiplication(128), 7 * N)
+    z = torch.randn(B, N, N, 128, generator=g).to(torch.bfloat16).to(DEV)
+    dy = (torch.randn(B, N, N, 128, generator=g) * 0.02).to(torch.bfloat16).to(DEV)
+    dy[..., 0, 0, 0] = 0.5  # the same largest value, hence the same scale, in every sample
+
+    def grad(a, b):
+        a = a.clone().requires_grad_(True)
+        return torch.autograd.grad(m(a), a, b)[0]
+
+    whole = grad(z, dy)
+    for i in range(B):
+        assert torch.equal(whole[i : i + 1], grad(z[i : i + 1], dy[i : i + 1]))
+
+
+@pytest.mark.parametrize("make,shape", [(lambda: mw.Transition(128), (300, 128)), (lambda: mw.TriangleMultiplication(128), (1, 24, 24, 128))])
+def test_scale_of_special_gradients(make, shape):
+    m, g = _module(make, 5)
+    x = torch.randn(*shape, generator=g).to(torch.bfloat16).to(DEV).requires_grad_(True)
+    dy = (torch.randn(*shape, generator=g) * 0.02).to(torch.bfloat16).to(DEV)
+    for t in torch.autograd.grad(m(x), [x, *m.parameters()], torch.zeros_like(dy)):
+        assert torch.equal(t, torch.zeros_like(t))
+    # a power of two through the whole backward: exactly that power in every gradient
+    a = torch.autograd.grad(m(x), [x, *m.parameters()], dy)
+    b = torch.autograd.grad(m(x), [x, *m.parameters()], dy * 2.0**-20)
+    for u, v in zip(a, b):
+        assert torch.equal(u * 2.0**-20, v)
+    # an infinity does not set the scale: the finite gradients stay finite where it does not reach
+    bad = dy.clone()
+    bad.view(-1, 128)[-1, 3] = float("inf")
+    out = torch.autograd.grad(m(x), x, bad)[0]
+    if len(shape) == 2:  # (the Transition works position by position)
+        assert torch.equal(out[:-1], a[0][:-1])
