@@ -450,14 +450,14 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         store_partial(pm + m * 128 * 128, pos, part * kBwdChunks + ch, v);
       }
     }
-    // the four position quarters of a hidden unit, fixed order (through the x_hat buffer, read by all)
-    named_bar_sync(1, kBwdThreads);
-    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(x_s + (part * 128 + pos) * 8), "f"(acc_a2.x + acc_a2.y),
+    // the four position quarters of a hidden unit, fixed order (through the weights' region: every GEMM that reads it has been
+    // waited for, while the store of x_hat of the last tile may still be reading the x_hat buffer)
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(wa_s + (part * 128 + pos) * 8), "f"(acc_a2.x + acc_a2.y),
                  "f"(acc_b2.x + acc_b2.y) : "memory");
     named_bar_sync(1, kBwdThreads);
     if (threadIdx.x < 128) {
       float a, b;
-      sum_partials(x_s, threadIdx.x, a, b);
+      sum_partials(wa_s, threadIdx.x, a, b);
       float* ps = p.part_s + static_cast<size_t>(blockIdx.x) * 2 * 512;
       ps[threadIdx.x] = a;
       ps[512 + threadIdx.x] = b;

@@ -47,6 +47,25 @@ def test_transition_position_counts(positions):
         assert _rel(a, b) <= TOL, (name, _rel(a, b))
 
 
+@pytest.mark.parametrize("positions", [128, 148 * 128, 2 * 148 * 128])
+def test_transition_last_tile_repeats(positions):
+    """The first launch stores x_hat of a block's last tile (of its only one at up to 148 tiles) for the three launches after it
+    while the block gathers its column sums: the copy must not see them, in any of forty calls."""
+    m, g = _module(lambda: mw.Transition(128), positions)
+    x = torch.randn(positions, 128, generator=g).to(torch.bfloat16).to(DEV)
+    dy = (torch.randn(positions, 128, generator=g) * 0.02).to(torch.bfloat16).to(DEV)
+
+    def grads():
+        xr = x.clone().requires_grad_(True)
+        return torch.autograd.grad(m(xr), [xr, *m.parameters()], dy)
+
+    first = grads()
+    for a, b in zip(first, _transition64(m, x, dy)):
+        assert _rel(a, b) <= TOL
+    for _ in range(39):
+        assert all(torch.equal(a, b) for a, b in zip(first, grads()))
+
+
 @pytest.mark.parametrize("B,N", [(1, 8), (3, 8), (1, 24), (1, 136)])
 def test_wide_statistics_of_short_rows(B, N):
     """The bidirectional module's gradients do not depend on the batch they are computed in (its statistics kernel takes 32
