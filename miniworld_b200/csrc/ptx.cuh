@@ -114,7 +114,11 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
 
 // ------------------------------------------------------------------ dependent launches
 // Waits until the kernel before this one on the stream has completed and its writes are visible (returns at once if the
-// launch does not overlap it). Every thread calls it before it touches global memory.
+// launch does not overlap it). Every thread calls it before it touches global memory. A kernel's life begins before the one
+// before it has ended, so non-coherent loads (ld.global.nc, __ldg: of data that does not change during the kernel's life) must
+// not read what that one may write: a kernel that an entry point launches first reads every operand with plain or .cg loads or
+// through TMA, a later one the operands its direct predecessor writes. Memory written earlier is safe: the predecessor has
+// itself waited before it let this kernel begin.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The next kernel's blocks may be placed as this one's leave their SMs (they wait as above before they touch memory).
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

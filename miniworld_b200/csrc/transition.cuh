@@ -393,7 +393,7 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       const uint4* xp = reinterpret_cast<const uint4*>(p.x + (in_range ? grow : 0) * 128);
       uint4 xr[2][2];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) xr[0][c] = (p.residual && in_range) ? __ldg(xp + c) : make_uint4(0u, 0u, 0u, 0u);
+      for (int c = 0; c < 2; ++c) xr[0][c] = (p.residual && in_range) ? xp[c] : make_uint4(0u, 0u, 0u, 0u);
       {
         const bool got = mbar_wait_warp(d2_full(t & 1), (t >> 1) & 1, abort_flag, p.status, kDevTimeoutEpilogue);
         if (!named_bar_and(1, 128, got)) break;
@@ -406,7 +406,7 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         if (ps < 7) {
 #pragma unroll
           for (int c = 0; c < 2; ++c)
-            xr[(ps + 1) & 1][c] = (p.residual && in_range) ? __ldg(xp + (ps + 1) * 2 + c) : make_uint4(0u, 0u, 0u, 0u);
+            xr[(ps + 1) & 1][c] = (p.residual && in_range) ? xp[(ps + 1) * 2 + c] : make_uint4(0u, 0u, 0u, 0u);
         }
         uint32_t v[16];
         tmem_ld16(t_d2 + ps * 16, v);
