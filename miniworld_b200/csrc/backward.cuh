@@ -44,6 +44,22 @@ __device__ __forceinline__ uint32_t tile_chunk(int r, int ch) {
   return static_cast<uint32_t>((ch >> 3) * 16384 + r * 128 + (((ch & 7) ^ (r & 7)) << 4));
 }
 
+// offset of element e of row r
+__device__ __forceinline__ uint32_t tile_off(int r, int e) {
+  return static_cast<uint32_t>((e >> 6) * 16384 + r * 128 + ((((e & 63) >> 3) ^ (r & 7)) << 4) + (e & 7) * 2);
+}
+
+__device__ __forceinline__ uint32_t ld_word(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void st_word(uint32_t addr, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+__device__ __forceinline__ uint32_t ld_half(uint32_t addr) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+  return v;
+}
 __device__ __forceinline__ uint4 ld_chunk(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
@@ -90,15 +106,15 @@ __device__ __forceinline__ float sigmoid_fast(float x) { return fmaf(tanh_approx
 __device__ __forceinline__ bool thread_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
   return mbar_wait_thread(bar, parity, abort_flag, status, code);
 }
-// Normalise the 128 channels of every position of a [pos][c] tile in place (bf16 in, fp16 out), the thread covering
-// 128 / kBwdParts of them. Returns rstd of the thread's position. `xchg` holds float2 [kBwdParts][128]; the caller must not
-// use it again without a barrier among the arithmetic threads.
-__device__ __forceinline__ float normalise_tile(uint32_t tile, uint32_t xchg, int pos, int part, float eps) {
+// LayerNorm statistics of a position from the kBwdParts threads that hold a part of its channels each. The order of the additions
+// is part of the results (they are repeatable bit for bit): shifted sums over a part's channels in order, then the parts.
+// Mean and sum of squared deviations of 8 * CHUNKS bf16 channels.
+template <int CHUNKS>
+__device__ __forceinline__ float2 partial_statistics(const uint4 (&v)[CHUNKS]) {
   float pv = 0.f, s1 = 0.f, s2 = 0.f;
 #pragma unroll
-  for (int ch = 0; ch < kBwdChunks; ++ch) {
-    const uint4 v = ld_chunk(tile + tile_chunk(pos, part * kBwdChunks + ch));
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  for (int ch = 0; ch < CHUNKS; ++ch) {
+    const uint32_t w[4] = {v[ch].x, v[ch].y, v[ch].z, v[ch].w};
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const float2 x = bf16x2_to_float2(w[t]);
@@ -108,11 +124,13 @@ __device__ __forceinline__ float normalise_tile(uint32_t tile, uint32_t xchg, in
       s2 = fmaf(d0, d0, fmaf(d1, d1, s2));
     }
   }
-  const float mean_h = pv + s1 * (1.0f / kBwdCh);
-  const float m2_h = fmaxf(s2 - s1 * s1 * (1.0f / kBwdCh), 0.f);
-  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + (part * 128 + pos) * 8), "f"(mean_h), "f"(m2_h) : "memory");
-  named_bar_sync(1, kBwdThreads);
-  // merge the equal-sized partials of this position: mean of means, M2 = sum M2_k + n_k sum (mean_k - mean)^2
+  constexpr float kInv = 1.0f / (8 * CHUNKS);
+  return make_float2(pv + s1 * kInv, fmaxf(s2 - s1 * s1 * kInv, 0.f));
+}
+// Mean and 1 / sigma of position `pos` from the equal-sized partials (CH channels each) in `xchg` (float2 [kBwdParts][128]):
+// mean of means, M2 = sum M2_k + n_k sum (mean_k - mean)^2.
+template <int CH>
+__device__ __forceinline__ float2 merge_partials(uint32_t xchg, int pos, float eps) {
   float mk[kBwdParts], qk[kBwdParts];
   float mean = 0.f, m2 = 0.f;
 #pragma unroll
@@ -123,21 +141,31 @@ __device__ __forceinline__ float normalise_tile(uint32_t tile, uint32_t xchg, in
   }
   mean *= 1.0f / kBwdParts;
 #pragma unroll
-  for (int k = 0; k < kBwdParts; ++k) m2 = fmaf(static_cast<float>(kBwdCh) * (mk[k] - mean), mk[k] - mean, m2);
-  const float rstd = rsqrtf(m2 * (1.0f / 128.0f) + eps);
-  const float nmr = -mean * rstd;
+  for (int k = 0; k < kBwdParts; ++k) m2 = fmaf(static_cast<float>(CH) * (mk[k] - mean), mk[k] - mean, m2);
+  return make_float2(mean, rsqrtf(m2 * (1.0f / (CH * kBwdParts)) + eps));
+}
+// Normalise the 128 channels of every position of a [pos][c] tile in place (bf16 in, fp16 out), the thread covering
+// 128 / kBwdParts of them. Returns rstd of the thread's position. `xchg` holds float2 [kBwdParts][128]; the caller must not
+// use it again without a barrier among the arithmetic threads.
+__device__ __forceinline__ float normalise_tile(uint32_t tile, uint32_t xchg, int pos, int part, float eps) {
+  uint4 v[kBwdChunks];
+#pragma unroll
+  for (int ch = 0; ch < kBwdChunks; ++ch) v[ch] = ld_chunk(tile + tile_chunk(pos, part * kBwdChunks + ch));
+  const float2 m = partial_statistics<kBwdChunks>(v);
+  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + (part * 128 + pos) * 8), "f"(m.x), "f"(m.y) : "memory");
+  named_bar_sync(1, kBwdThreads);
+  const float2 st = merge_partials<kBwdCh>(xchg, pos, eps);
+  const float rstd = st.y, nmr = -st.x * st.y;
 #pragma unroll
   for (int ch = 0; ch < kBwdChunks; ++ch) {
-    const uint32_t addr = tile + tile_chunk(pos, part * kBwdChunks + ch);
-    const uint4 v = ld_chunk(addr);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const uint32_t w[4] = {v[ch].x, v[ch].y, v[ch].z, v[ch].w};
     uint32_t o[4];
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const float2 x = bf16x2_to_float2(w[t]);
       o[t] = pack_f16x2_sat(make_float2(fmaf(x.x, rstd, nmr), fmaf(x.y, rstd, nmr)));
     }
-    st_chunk(addr, o[0], o[1], o[2], o[3]);
+    st_chunk(tile + tile_chunk(pos, part * kBwdChunks + ch), o[0], o[1], o[2], o[3]);
   }
   return rstd;
 }
@@ -168,7 +196,6 @@ struct BwdEpilogueParams {
   int n;               // N
   int ld;              // columns per row of ext_stats and ln_part (N rounded up to a multiple of 8)
   const float* consts;      // [2][128]: d_out = W_out beta_out + bias_out, d_gate = W_gate beta_in + bias_gate
-  const float* row_sums;    // [128]: row sums of Wo'
   const float* grad_scale;  // [2]: c, 1 / c
   const uint16_t* drop_scale;  // [B][N][128] bf16 or null
   float eps_in;
@@ -196,18 +223,19 @@ struct BwdEpilogueParams {
 //                           `bwd_ln_finish_kernel` then finishes the first tensor's gradient.
 //
 // 16 arithmetic warps, a warp that issues the MMAs and one that issues the copies (joined as in bwd_prologue_kernel). Per tile
-//   arithmetic: t and z normalised in place (statistics by shuffles inside a warp) -> N -> wait P / G -> dproj, dgate tiles
-//               and the sums of the LayerNorm backward -> A -> column sums, per-position coefficients -> wait d t_hat
-//               (transposed: lanes = channels), d x_hat -> wait weight gradients -> output tiles -> C
-//   MMAs:       N: P, G;  A: d t_hat^T and d x_hat, then Mo and Mg
+//   arithmetic: eight warps normalise t in place, eight z -> N -> wait P / G -> dproj, dgate tiles -> A -> column sums -> S
+//               -> wait d t_hat: the sums of the LayerNorm backward, d t, d x_hat -> wait weight gradients -> output tiles -> C
+//   MMAs:       N: P, G;  A: d t_hat and d x_hat, then Mo and Mg
 //   copies:     N: x_hat out, next tile into L2; weight gradients done: next t, z; C: output stores, then next dy
-// The two sums the LayerNorm backward needs per position come from dproj, before the gradient GEMMs: sum_c d t_hat =
-// dproj . rowsum(Wo'), sum_c d t_hat t_hat = dproj . P. d t_hat is computed transposed because t is stored [channel][pos]: a
-// thread then owns one channel and reads and writes t in 16-byte runs (2-byte accesses to 32 channels of one position, two
-// exchanges of statistics and eight CTA-wide barriers made 17 k cycles per tile). What bounds it: the chain of one tile per
-// SM; two weight matrices and four tiles, all live during the gradient GEMMs, leave no room for a second tile.
+// t is stored [channel][position] while its statistics and sums run over the channels of a position: a thread normalises two
+// neighbouring positions (4-byte accesses, a whole channel row per warp), and after the LayerNorm backward neighbouring lanes
+// swap halves so that the gradient leaves in 4-byte accesses, too. What bounds it: the chain of one tile per SM; two weight
+// matrices and four tiles, all live during the gradient GEMMs, leave no room for a second tile. (The statistics by shuffles, d
+// t_hat transposed and the two sums taken from dproj save 5 us of a step of 360 at N = 384, but round otherwise: one bf16 step
+// in 2 % of dz.)
 constexpr int kBwdEpiThreads = kBwdThreads + 64;
-constexpr int kBwdEpiSmemBytes = 6 * kBwdTile + 8192 /* exchange, constants */ + 512 /* barriers */ + 1024;
+constexpr int kBwdEpiXchg = 3 * kBwdXchg + 2048;  // three exchanges of partial sums, 1 / sigma, constants
+constexpr int kBwdEpiSmemBytes = 6 * kBwdTile + kBwdEpiXchg + 512 /* barriers */ + 1024;
 template <int MODE, int C = 128>
 __global__ void __launch_bounds__(kBwdEpiThreads, 1)
 bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_z,
@@ -223,19 +251,20 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
   constexpr int kZHalves = C / 64;      // 64-channel halves of a [pos][C] tile
   constexpr uint32_t kWHalf = C * 128;  // bytes of one 64-wide k half of a weight matrix with C rows
   constexpr int kBarN = 2, kBarA = 3, kBarS = 4, kBarC = 5, kOne = kBwdThreads + 32, kTwo = kBwdThreads + 64;
+  constexpr int kBarT = 6, kBarZ = 7, kBarQ = 8;  // (kBarQ .. kBarQ + 3: the threads of 32 positions)
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t wo_s = smem_base, wg_s = smem_base + kBwdTile;
   const uint32_t tiles_s = smem_base + 2 * kBwdTile;  // four tile buffers whose roles rotate from tile to tile
-  const uint32_t xchg = smem_base + 6 * kBwdTile;     // float2 [kBwdParts][128]: partial sums of the LayerNorm backward
-  const uint32_t coef_s = xchg + kBwdXchg;        // float [3][128]: d t = a d t_hat + b + c t_hat
-  const uint32_t rstd_s = coef_s + 1536;              // float [128]: 1 / sigma of the output LayerNorm
-  float* const_ptr = reinterpret_cast<float*>(smem + 6 * kBwdTile + kBwdXchg + 2048);  // d_out, d_gate, rowsum(Wo') [3][128]
-  const uint32_t bar_base = smem_base + 6 * kBwdTile + 8192;
+  // float2 [kBwdParts][128] each: partial statistics of t and of z, partial sums of the LayerNorm backward
+  const uint32_t xchg = smem_base + 6 * kBwdTile, xchg_z = xchg + kBwdXchg, xchg_s = xchg_z + kBwdXchg;
+  const uint32_t rstd_s = xchg_s + kBwdXchg;      // float [128]: 1 / sigma of the output LayerNorm
+  float* const_ptr = reinterpret_cast<float*>(smem + 6 * kBwdTile + 3 * kBwdXchg + 512);  // d_out, d_gate [2][128]
+  const uint32_t bar_base = smem_base + 6 * kBwdTile + kBwdEpiXchg;
   const uint32_t w_full = bar_base, t_full = bar_base + 8, z_full = bar_base + 16, dy_full = bar_base + 24;
   const uint32_t pp_full = bar_base + 32, fwd_done = bar_base + 40, d_done = bar_base + 48, grad_done = bar_base + 56;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 6 * kBwdTile + 8192 + 64);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 6 * kBwdTile + kBwdEpiXchg + 64);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -257,7 +286,6 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
   grid_dependency_wait();
   grid_dependents_launch();
   if (threadIdx.x < 256) const_ptr[threadIdx.x] = p.consts[threadIdx.x];
-  else if (threadIdx.x < 384) const_ptr[threadIdx.x] = p.row_sums[threadIdx.x - 256];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -299,18 +327,18 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
       __syncwarp();
       named_bar_sync(kBarA, kTwo);
       if (lane == 0) {
-        // d t_hat^T = Wo'^T dproj^T (0-127, lanes = channels of t, columns = positions), d x_hat = dgate Wg' (128-255, lanes
-        // = positions); Mo += dproj^T t_hat (256-383), Mg += dgate^T x_hat (384-511)
+        // d t_hat = dproj Wo' (0-127), d x_hat = dgate Wg' (128-255; lanes = positions); Mo += dproj^T t_hat (256-383), Mg +=
+        // dgate^T x_hat (384-511)
         tc_fence_after();
-        constexpr uint32_t idesc_d = umma_idesc(128, 128, true, false, kFmtF16, kFmtF16);
+        constexpr uint32_t idesc_d = umma_idesc(128, 128, false, true, kFmtF16, kFmtF16);
         constexpr uint32_t idesc_dx = umma_idesc(128, C, false, true, kFmtF16, kFmtF16);
         constexpr uint32_t idesc_mo = umma_idesc(128, 128, true, false, kFmtF16, kFmtF16);
         constexpr uint32_t idesc_mg = umma_idesc(128, C, true, true, kFmtF16, kFmtF16);
         const uint32_t accum = it != 0 ? 1u : 0u;
 #pragma unroll
-        for (int ks = 0; ks < C / 16; ++ks) {  // K = the C channels of dproj; Wo' [C][128] read MN-major (its k halves are M blocks)
+        for (int ks = 0; ks < C / 16; ++ks) {  // K = the C channels of dproj; Wo' [C][128] read MN-major (its k halves are N blocks)
           const uint64_t kb = static_cast<uint64_t>((ks & 3) * 2);
-          umma_bf16(tmem_base, umma_desc_mnmajor(wo_s + ks * 2048, kWHalf), umma_desc_kmajor(dy_s + (ks >> 2) * 16384) + kb,
+          umma_bf16(tmem_base, umma_desc_kmajor(dy_s + (ks >> 2) * 16384) + kb, umma_desc_mnmajor(wo_s + ks * 2048, kWHalf),
                     idesc_d, ks != 0 ? 1u : 0u);
         }
         if constexpr (MODE != 1) {
@@ -461,133 +489,78 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
       const int j0 = (tile - row * p.tiles_per_row) * 128;
       const int j = j0 + pos;
       const uint32_t t_s = t_buf(it), z_s = t_s + kBwdTile, dy_s = y_buf(it), dg_s = dy_s + kBwdTile;
-      // ---- t normalised in place: a warp takes eight positions (one 16-byte chunk column), a lane four of the 128 channels
-      thread_wait(t_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
-      __syncwarp();
-      {
-        const uint32_t col = t_s + static_cast<uint32_t>(warp >> 3) * 16384;
-        uint32_t addr[4];
-        float2 v[4][4];  // [channel][position pair]
+      if (warp < 8) {
+        // ---- t normalised in place: a thread takes 32 channels (`grp`) of two neighbouring positions, so that a warp reads and
+        // writes a channel's 64 positions in one 128-byte access
+        thread_wait(t_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+        __syncwarp();
+        const int p0 = (warp & 1) * 64 + 2 * lane, grp = warp >> 1;
+        const uint32_t col = t_s + static_cast<uint32_t>(warp & 1) * 16384 + grp * 32 * 128 + (lane & 3) * 4;
+        auto t_addr = [&](int cc) { return col + cc * 128 + (((lane >> 2) ^ (cc & 7)) << 4); };
+        uint32_t x[32];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int c = k * 32 + lane;
-          addr[k] = col + c * 128 + (((warp & 7) ^ (c & 7)) << 4);
-          const uint4 x = ld_chunk(addr[k]);
-          v[k][0] = f16x2_to_float2(x.x), v[k][1] = f16x2_to_float2(x.y);
-          v[k][2] = f16x2_to_float2(x.z), v[k][3] = f16x2_to_float2(x.w);
-        }
-        // sums over the 32 lanes of eight values: three halving exchanges, then two plain ones; the lane ends with the sum
-        // of position `mine` of the eight
-        auto reduce8 = [&](const float2 (&s)[4]) {
-          const bool u16 = (lane & 16) != 0, u8 = (lane & 8) != 0, u4 = (lane & 4) != 0;
-          float2 k0 = u16 ? s[2] : s[0], k1 = u16 ? s[3] : s[1];
-          const float2 g0 = u16 ? s[0] : s[2], g1 = u16 ? s[1] : s[3];
-          k0.x += __shfl_xor_sync(0xFFFFFFFFu, g0.x, 16), k0.y += __shfl_xor_sync(0xFFFFFFFFu, g0.y, 16);
-          k1.x += __shfl_xor_sync(0xFFFFFFFFu, g1.x, 16), k1.y += __shfl_xor_sync(0xFFFFFFFFu, g1.y, 16);
-          float2 m = u8 ? k1 : k0;
-          const float2 h = u8 ? k0 : k1;
-          m.x += __shfl_xor_sync(0xFFFFFFFFu, h.x, 8), m.y += __shfl_xor_sync(0xFFFFFFFFu, h.y, 8);
-          float r = u4 ? m.y : m.x;
-          r += __shfl_xor_sync(0xFFFFFFFFu, u4 ? m.x : m.y, 4);
-          r += __shfl_xor_sync(0xFFFFFFFFu, r, 2);
-          r += __shfl_xor_sync(0xFFFFFFFFu, r, 1);
-          return r;
-        };
-        const int mine = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-        auto owner = [](int e) { return ((e >> 2) & 1) * 16 + ((e >> 1) & 1) * 8 + (e & 1) * 4; };
-        float2 nmean[4], rstd[4];
-        float my_rstd = 0.f;
+        for (int cc = 0; cc < 32; ++cc) x[cc] = ld_word(t_addr(cc));
+        float2 scale, shift;  // t_hat = t scale + shift
         if constexpr (MODE == 0) {
-          float2 s[4];
+          const float2 pv = f16x2_to_float2(x[0]), npv = make_float2(-pv.x, -pv.y);
+          float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) s[e] = __fadd2_rn(__fadd2_rn(v[0][e], v[1][e]), __fadd2_rn(v[2][e], v[3][e]));
-          const float mean = reduce8(s) * (1.0f / 128.0f);
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            nmean[e] = make_float2(-__shfl_sync(0xFFFFFFFFu, mean, owner(2 * e)), -__shfl_sync(0xFFFFFFFFu, mean, owner(2 * e + 1)));
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            s[e] = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              v[k][e] = __fadd2_rn(v[k][e], nmean[e]);
-              s[e] = __ffma2_rn(v[k][e], v[k][e], s[e]);
-            }
+          for (int cc = 0; cc < 32; ++cc) {
+            const float2 d = __fadd2_rn(f16x2_to_float2(x[cc]), npv);
+            s1 = __fadd2_rn(s1, d);
+            s2 = __ffma2_rn(d, d, s2);
           }
-          my_rstd = rsqrtf(reduce8(s) * (1.0f / 128.0f) + p.eps_out);
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            rstd[e] = make_float2(__shfl_sync(0xFFFFFFFFu, my_rstd, owner(2 * e)), __shfl_sync(0xFFFFFFFFu, my_rstd, owner(2 * e + 1)));
+          constexpr float kInv = 1.0f / 32;
+          asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(xchg + (grp * 128 + p0) * 8), "f"(pv.x + s1.x * kInv),
+                       "f"(fmaxf(s2.x - s1.x * s1.x * kInv, 0.f)), "f"(pv.y + s1.y * kInv),
+                       "f"(fmaxf(s2.y - s1.y * s1.y * kInv, 0.f)) : "memory");
+          named_bar_sync(kBarT, 256);
+          float2 mean_a, mean_b;
+          mean_a = merge_partials<32>(xchg, p0, p.eps_out), mean_b = merge_partials<32>(xchg, p0 + 1, p.eps_out);
+          scale = make_float2(mean_a.y, mean_b.y);
+          shift = make_float2(-mean_a.x * mean_a.y, -mean_b.x * mean_b.y);
         } else {
-          const int j8 = j0 + warp * 8;
-          float2 st = make_float2(0.f, 0.f);  // (positions past the end stay zero)
-          if (j8 + mine < p.n) st = p.ext_stats[static_cast<size_t>(row) * p.ld + j8 + mine];
-          my_rstd = st.y;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            nmean[e] = make_float2(-__shfl_sync(0xFFFFFFFFu, st.x, owner(2 * e)), -__shfl_sync(0xFFFFFFFFu, st.x, owner(2 * e + 1)));
-            rstd[e] = make_float2(__shfl_sync(0xFFFFFFFFu, st.y, owner(2 * e)), __shfl_sync(0xFFFFFFFFu, st.y, owner(2 * e + 1)));
-#pragma unroll
-            for (int k = 0; k < 4; ++k) v[k][e] = __fadd2_rn(v[k][e], nmean[e]);
-          }
+          float4 st = make_float4(0.f, 0.f, 0.f, 0.f);  // (positions past the end stay zero)
+          if (j0 + p0 < p.n) st = *reinterpret_cast<const float4*>(p.ext_stats + static_cast<size_t>(row) * p.ld + j0 + p0);
+          if (j0 + p0 + 1 >= p.n) st.z = 0.f, st.w = 0.f;
+          scale = make_float2(st.y, st.w);
+          shift = make_float2(-st.x * st.y, -st.z * st.w);
         }
-        if ((lane & 3) == 0)
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(rstd_s + (warp * 8 + mine) * 4), "f"(my_rstd) : "memory");
+        if (grp == 0)
+          asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(rstd_s + p0 * 4), "f"(scale.x), "f"(scale.y) : "memory");
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          st_chunk(addr[k], pack_f16x2_sat(__fmul2_rn(v[k][0], rstd[0])), pack_f16x2_sat(__fmul2_rn(v[k][1], rstd[1])),
-                   pack_f16x2_sat(__fmul2_rn(v[k][2], rstd[2])), pack_f16x2_sat(__fmul2_rn(v[k][3], rstd[3])));
-      }
-      // ---- z normalised in place: eight lanes per position, 64 positions per pass
-      thread_wait(z_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
-      __syncwarp();
-      {
-        constexpr int kPairs = 4 * kZHalves;  // channel pairs per lane
-        const int sub = threadIdx.x & 7, slot = threadIdx.x >> 3;
-        uint32_t addr[2];
-        float2 v[2][kPairs];
+        for (int cc = 0; cc < 32; ++cc) st_word(t_addr(cc), pack_f16x2_sat(__ffma2_rn(f16x2_to_float2(x[cc]), scale, shift)));
+      } else {
+        // ---- z normalised in place: a thread takes a quarter of the channels of its position, twice
+        thread_wait(z_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
+        __syncwarp();
+        const int zp = threadIdx.x & 127, first = (threadIdx.x >> 7) & 1;  // quarters `first` and `first` + 2
+        uint4 v[2][kZChunks];
 #pragma unroll
-        for (int pass = 0; pass < 2; ++pass) {
-          const int zp = pass * 64 + slot;
-          addr[pass] = z_s + zp * 128 + ((sub ^ (zp & 7)) << 4);
+        for (int h = 0; h < 2; ++h) {
+          const int grp = first + 2 * h;
 #pragma unroll
-          for (int h = 0; h < kZHalves; ++h) {
-            const uint4 x = ld_chunk(addr[pass] + h * 16384);
-            v[pass][4 * h] = bf16x2_to_float2(x.x), v[pass][4 * h + 1] = bf16x2_to_float2(x.y);
-            v[pass][4 * h + 2] = bf16x2_to_float2(x.z), v[pass][4 * h + 3] = bf16x2_to_float2(x.w);
-          }
+          for (int ch = 0; ch < kZChunks; ++ch) v[h][ch] = ld_chunk(z_s + tile_chunk(zp, grp * kZChunks + ch));
+          const float2 m = partial_statistics<kZChunks>(v[h]);
+          asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg_z + (grp * 128 + zp) * 8), "f"(m.x), "f"(m.y) : "memory");
         }
+        named_bar_sync(kBarZ, 256);
+        const float2 st = merge_partials<kZCh>(xchg_z, zp, p.eps_in);
+        if constexpr (MODE != 1) {
+          if (first == 0 && j0 + zp < p.n) p.rstd[static_cast<size_t>(row) * p.ld + j0 + zp] = st.y;
+        }
+        const float2 scale = make_float2(st.y, st.y), shift = make_float2(-st.x * st.y, -st.x * st.y);
 #pragma unroll
-        for (int pass = 0; pass < 2; ++pass) {
-          float2 s = make_float2(0.f, 0.f);
+        for (int h = 0; h < 2; ++h) {
 #pragma unroll
-          for (int i = 0; i < kPairs; ++i) s = __fadd2_rn(s, v[pass][i]);
-          float sum = s.x + s.y;
-          sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
-          sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
-          sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 4);
-          const float mean = sum * (1.0f / C);
-          float2 qs = make_float2(0.f, 0.f);
-#pragma unroll
-          for (int i = 0; i < kPairs; ++i) {
-            v[pass][i] = __fadd2_rn(v[pass][i], make_float2(-mean, -mean));
-            qs = __ffma2_rn(v[pass][i], v[pass][i], qs);
+          for (int ch = 0; ch < kZChunks; ++ch) {
+            const uint4 w = v[h][ch];
+            st_chunk(z_s + tile_chunk(zp, (first + 2 * h) * kZChunks + ch),
+                     pack_f16x2_sat(__ffma2_rn(bf16x2_to_float2(w.x), scale, shift)),
+                     pack_f16x2_sat(__ffma2_rn(bf16x2_to_float2(w.y), scale, shift)),
+                     pack_f16x2_sat(__ffma2_rn(bf16x2_to_float2(w.z), scale, shift)),
+                     pack_f16x2_sat(__ffma2_rn(bf16x2_to_float2(w.w), scale, shift)));
           }
-          float ssq = qs.x + qs.y;
-          ssq += __shfl_xor_sync(0xFFFFFFFFu, ssq, 1);
-          ssq += __shfl_xor_sync(0xFFFFFFFFu, ssq, 2);
-          ssq += __shfl_xor_sync(0xFFFFFFFFu, ssq, 4);
-          const float rs = rsqrtf(ssq * (1.0f / C) + p.eps_in);
-          const float2 rs2 = make_float2(rs, rs);
-          if constexpr (MODE != 1) {
-            const int jz = j0 + pass * 64 + slot;
-            if (sub == 0 && jz < p.n) p.rstd[static_cast<size_t>(row) * p.ld + jz] = rs;
-          }
-#pragma unroll
-          for (int h = 0; h < kZHalves; ++h)
-            st_chunk(addr[pass] + h * 16384, pack_f16x2_sat(__fmul2_rn(v[pass][4 * h], rs2)),
-                     pack_f16x2_sat(__fmul2_rn(v[pass][4 * h + 1], rs2)), pack_f16x2_sat(__fmul2_rn(v[pass][4 * h + 2], rs2)),
-                     pack_f16x2_sat(__fmul2_rn(v[pass][4 * h + 3], rs2)));
         }
       }
       fence_proxy_async_smem();
@@ -604,7 +577,7 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
       }
       float2 other = make_float2(0.f, 0.f);  // MODE 2: the first launch's sums of this position
       if constexpr (MODE == 2) {
-        if (part == 0 && j < p.n) other = p.ln_part[static_cast<size_t>(row) * p.ld + j];
+        if (j < p.n) other = p.ln_part[static_cast<size_t>(row) * p.ld + j];
       }
       thread_wait(dy_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
       if constexpr (MODE == 2) thread_wait(pp_full, it & 1, abort_flag, p.status, kDevTimeoutStats);
@@ -612,8 +585,7 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
       __syncwarp();
       tc_fence_after();
       // ---- dproj = c du gate, dgate = c du proj gate (1 - gate); du = dy (* dropout scale). This thread: one position,
-      // kZCh channels; s = sums over them of dproj rowsum(Wo') and dproj P.
-      float2 sum1 = make_float2(0.f, 0.f), sum2 = make_float2(0.f, 0.f);
+      // kZCh channels.
       {
         const float2 half2 = make_float2(0.5f, 0.5f), gc2 = make_float2(gc, gc);
         uint32_t vp[2][8], vg[2][8];
@@ -637,17 +609,13 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
           uint32_t op[4], og[4];
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
-            const float2 praw = pair_of(vp[ch & 1][2 * t], vp[ch & 1][2 * t + 1]);
-            float2 proj = __fadd2_rn(praw, cp[t]);
+            float2 proj = __fadd2_rn(pair_of(vp[ch & 1][2 * t], vp[ch & 1][2 * t + 1]), cp[t]);
             if constexpr (MODE == 2) proj = __fadd2_rn(proj, f16x2_to_float2(pw[t]));
             const float2 gh = __fmul2_rn(__fadd2_rn(pair_of(vg[ch & 1][2 * t], vg[ch & 1][2 * t + 1]), cp[64 + t]), half2);
             const float2 gate = __ffma2_rn(make_float2(tanh_approx(gh.x), tanh_approx(gh.y)), half2, half2);
             const float2 du = __fmul2_rn(__fmul2_rn(bf16x2_to_float2(dw[t]), bf16x2_to_float2(sw[t])), gc2);
             const float2 dp = __fmul2_rn(du, gate);
             op[t] = pack_f16x2_sat(dp);
-            const float2 dpr = f16x2_to_float2(op[t]);  // what the gradient GEMMs read
-            sum1 = __ffma2_rn(dpr, cp[128 + t], sum1);
-            sum2 = __ffma2_rn(dpr, praw, sum2);
             // MODE 1 hands its part of proj on
             og[t] = pack_f16x2_sat(MODE == 1 ? proj
                                              : __fmul2_rn(dp, __ffma2_rn(make_float2(-proj.x, -proj.y), gate, proj)));
@@ -663,33 +631,21 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
           }
         }
       }
-      asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg + (part * 128 + pos) * 8), "f"(sum1.x + sum1.y),
-                   "f"(sum2.x + sum2.y) : "memory");
       tc_fence_before();
       fence_proxy_async_smem();
       __syncwarp();
       named_bar_sync(kBarA, kTwo);
-      // ---- (under the gradient GEMMs) the position's two means and the coefficients of its LayerNorm backward
-      if (part == 0) {
-        float m1, m2;
-        sum_partials(xchg, pos, m1, m2);
-        if constexpr (MODE == 1) {
-          if (j < p.n) p.ln_part[static_cast<size_t>(row) * p.ld + j] = make_float2(m1, m2);
-        } else {
-          if constexpr (MODE == 2) {
-            m1 = (m1 + other.x) * (1.0f / 256.0f), m2 = (m2 + other.y) * (1.0f / 256.0f);
-            if (j < p.n) p.ln_part[static_cast<size_t>(row) * p.ld + j] = make_float2(m1, m2);
-          } else {
-            m1 *= 1.0f / 128.0f, m2 *= 1.0f / 128.0f;
-          }
-          float rs;
-          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(rs) : "r"(rstd_s + pos * 4));
-          rs *= 0.0625f;  // d / d t of the stored t / 16
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(coef_s + pos * 4), "f"(rs) : "memory");
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(coef_s + 512 + pos * 4), "f"(-rs * m1) : "memory");
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(coef_s + 1024 + pos * 4), "f"(-rs * m2) : "memory");
-        }
+      // ---- (under the gradient GEMMs) this thread's t_hat values, its position's 1 / sigma, column sums
+      uint32_t th[16];  // channels part * 32 + 8 k + i and, in the upper half, + 4 (k, i = 0 .. 3)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          th[k * 4 + i] = ld_half(t_s + tile_off(part * 32 + k * 8 + i, pos)) | (ld_half(t_s + tile_off(part * 32 + k * 8 + i + 4, pos)) << 16);
       }
+      float rs;
+      asm volatile("ld.shared.f32 %0, [%1];" : "=f"(rs) : "r"(rstd_s + pos * 4));
+      rs *= 0.0625f;  // d / d t of the stored t / 16
       if (sum_chunk < C / 8) {  // column sums of the two fp16 tiles the GEMMs are reading
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -714,48 +670,43 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
       }
       __syncwarp();
       named_bar_arrive(kBarS, kOne);
-      if constexpr (MODE != 1) named_bar_sync(1, kBwdThreads);  // the coefficients are there
-      // ---- LayerNorm backward of the output normalisation for this thread's channel and 32 positions; d x_hat of its position
+      // ---- LayerNorm backward of the output normalisation for this thread's position and 32 channels; d x_hat
       thread_wait(d_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
       __syncwarp();
       tc_fence_after();
+      uint32_t dv[32];
+      tmem_ld32(tmem_base + lane_sel + part * 32, dv);
+      tmem_ld_wait();
+      float m1 = 0.f, m2 = 0.f;
+#pragma unroll
+      for (int cc = 0; cc < 32; ++cc) {
+        const float2 t2 = f16x2_to_float2(th[(cc >> 3) * 4 + (cc & 3)]);
+        const float d = __uint_as_float(dv[cc]);
+        m1 += d;
+        m2 = fmaf(d, (cc & 4) ? t2.y : t2.x, m2);
+      }
+      asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xchg_s + (part * 128 + pos) * 8), "f"(m1), "f"(m2) : "memory");
+      named_bar_sync(kBarQ + q, 32 * kBwdParts);  // the threads of these 32 positions
+      if (MODE != 1 || part == 0) sum_partials(xchg_s, pos, m1, m2);
+      if constexpr (MODE == 1) {
+        if (part == 0 && j < p.n) p.ln_part[static_cast<size_t>(row) * p.ld + j] = make_float2(m1, m2);
+      } else if constexpr (MODE == 2) {
+        m1 = (m1 + other.x) * (1.0f / 256.0f), m2 = (m2 + other.y) * (1.0f / 256.0f);
+        if (part == 0 && j < p.n) p.ln_part[static_cast<size_t>(row) * p.ld + j] = make_float2(m1, m2);
+      } else {
+        m1 *= 1.0f / 128.0f, m2 *= 1.0f / 128.0f;
+      }
+      // d t = rs (d t_hat - m1 - t_hat m2). Two neighbouring lanes swap halves, the even one ending with a channel of both
+      // positions and the odd one with the channel four rows on, so that a warp stores two 64-byte runs without a bank conflict
       uint32_t ot[16];
+      const float2 nm1 = make_float2(-m1, -m1), nm2 = make_float2(-m2, -m2), rs2 = make_float2(rs, rs);
 #pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        uint32_t dv[16];
-        tmem_ld16(tmem_base + lane_sel + part * 32 + hf * 16, dv);
-        uint4 th[2];
-        if constexpr (MODE != 1) {
-#pragma unroll
-          for (int k = 0; k < 2; ++k) th[k] = ld_chunk(t_s + tile_chunk(pos, part * 4 + hf * 2 + k));
-        }
-        tmem_ld_wait();
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const uint32_t tw[4] = {th[k].x, th[k].y, th[k].z, th[k].w};
-#pragma unroll
-          for (int t2 = 0; t2 < 2; ++t2) {
-            const uint32_t cpos = static_cast<uint32_t>(part * 32 + hf * 16 + k * 8 + t2 * 4) * 4;
-            float4 ca, cb, cc;  // four positions (the same addresses for the whole warp)
-            if constexpr (MODE != 1) {
-              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(ca.x), "=f"(ca.y), "=f"(ca.z), "=f"(ca.w) : "r"(coef_s + cpos));
-              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(cb.x), "=f"(cb.y), "=f"(cb.z), "=f"(cb.w) : "r"(coef_s + 512 + cpos));
-              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(cc.x), "=f"(cc.y), "=f"(cc.z), "=f"(cc.w) : "r"(coef_s + 1024 + cpos));
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const int t = t2 * 2 + u;
-              float2 d = pair_of(dv[k * 8 + 2 * t], dv[k * 8 + 2 * t + 1]);
-              if constexpr (MODE != 1) {
-                const float2 a2 = u == 0 ? make_float2(ca.x, ca.y) : make_float2(ca.z, ca.w);
-                const float2 b2 = u == 0 ? make_float2(cb.x, cb.y) : make_float2(cb.z, cb.w);
-                const float2 c2 = u == 0 ? make_float2(cc.x, cc.y) : make_float2(cc.z, cc.w);
-                d = __ffma2_rn(d, a2, __ffma2_rn(f16x2_to_float2(tw[t]), c2, b2));
-              }
-              ot[hf * 8 + k * 4 + t] = pack_f16x2_sat(d);  // (MODE 1: finished by bwd_ln_finish_kernel)
-            }
-          }
-        }
+      for (int k = 0; k < 16; ++k) {
+        float2 d = pair_of(dv[(k >> 2) * 8 + (k & 3)], dv[(k >> 2) * 8 + (k & 3) + 4]);
+        if constexpr (MODE != 1) d = __fmul2_rn(rs2, __ffma2_rn(f16x2_to_float2(th[k]), nm2, __fadd2_rn(d, nm1)));
+        const uint32_t o = pack_f16x2_sat(d);  // (MODE 1: finished by bwd_ln_finish_kernel)
+        const uint32_t n = __shfl_xor_sync(0xFFFFFFFFu, o, 1);
+        ot[k] = (lane & 1) ? __byte_perm(n, o, 0x7632) : __byte_perm(o, n, 0x5410);
       }
       uint32_t ox[MODE != 1 ? kZChunks * 4 : 1];
       if constexpr (MODE != 1) {
@@ -772,8 +723,8 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
       thread_wait(grad_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);  // the GEMMs have read t_hat and x_hat
       __syncwarp();
 #pragma unroll
-      for (int k4 = 0; k4 < 4; ++k4)
-        st_chunk(t_s + tile_chunk(pos, part * 4 + k4), ot[k4 * 4], ot[k4 * 4 + 1], ot[k4 * 4 + 2], ot[k4 * 4 + 3]);
+      for (int k = 0; k < 16; ++k)
+        st_word(t_s + tile_off(part * 32 + (k >> 2) * 8 + (k & 3) + (lane & 1) * 4, pos & ~1), ot[k]);
       if constexpr (MODE != 1) {
 #pragma unroll
         for (int ch = 0; ch < kZChunks; ++ch)
@@ -1189,7 +1140,7 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     // dvalue / dgate are formed on the transposed projections (TMEM lanes = contracted channels, columns = positions): a
     // thread owns channel `pos` (its lane) and the position quarter `part`, so its constants and its column sums are
     // scalars and dO, stored [channel][position], is read in 16-byte runs of positions.
-    float2 acc_v2 = make_float2(0.f, 0.f), acc_g2 = make_float2(0.f, 0.f);  // over the even and the odd positions
+    float acc_v = 0.f, acc_g = 0.f;
     const float2 c_value2 = make_float2(c_value, c_value), c_gate_half2 = make_float2(c_gate_half, c_gate_half);
     const float2 half2 = make_float2(0.5f, 0.5f), eight2 = make_float2(8.f, 8.f);
     auto pair_of = [](uint32_t lo, uint32_t hi) { return make_float2(__uint_as_float(lo), __uint_as_float(hi)); };
@@ -1264,8 +1215,9 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
               // the contraction's outputs are stored times 2^-4: 16 sg = 8 tanh + 8
               const float2 dv = __fmul2_rn(d_o, __ffma2_rn(th, eight2, eight2));
               const float2 dg = __fmul2_rn(dv, __ffma2_rn(make_float2(-val.x, -val.y), sg, val));
-              acc_v2 = __fadd2_rn(acc_v2, dv);
-              acc_g2 = __fadd2_rn(acc_g2, dg);
+              // (one chain in the order of the positions)
+              acc_v += dv.x, acc_v += dv.y;
+              acc_g += dg.x, acc_g += dg.y;
               ov[t] = pack_f16x2_sat(dv);
               dg_p[hf * 8 + k4 * 4 + t] = pack_f16x2_sat(dg);
             }
@@ -1397,8 +1349,7 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
     // column sums: the four position quarters of a channel, fixed order (through the running sum's buffer, read by all)
     named_bar_sync(1, kBwdThreads);
-    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dx_s + (part * 128 + pos) * 8), "f"(acc_v2.x + acc_v2.y),
-                 "f"(acc_g2.x + acc_g2.y) : "memory");
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dx_s + (part * 128 + pos) * 8), "f"(acc_v), "f"(acc_g) : "memory");
     named_bar_sync(1, kBwdThreads);
     if (threadIdx.x < 128) {
       float a, b;
@@ -1476,8 +1427,7 @@ __device__ __forceinline__ void amax_and_scale(const uint4* dy, size_t n_chunks,
 // as dense fp16 [128][128] with the LayerNorm gamma of their input folded in, W'[r][k] = W[r][k] gamma[k], and
 // d[m][r] = sum_k W[r][k] beta[k] + bias[m][r] (fp32) behind them. One warp per matrix row.
 constexpr size_t kBwdPackedD = 6 * 32768;
-constexpr size_t kBwdPackedRowSum = kBwdPackedD + 3072;        // float[128]: row sums of W'_out
-constexpr size_t kBwdPackedBytes = kBwdPackedRowSum + 1024;    // 200704, a multiple of 1024
+constexpr size_t kBwdPackedBytes = kBwdPackedD + 3072;  // 199680, a multiple of 1024
 __device__ __forceinline__ void bwd_pack_row(const PackArgs& a, uint8_t* packed, int gw) {  // gw: 0 .. 767
   const int lane = threadIdx.x & 31;
   const int m = gw >> 7, row = gw & 127;
@@ -1499,13 +1449,11 @@ __device__ __forceinline__ void bwd_pack_row(const PackArgs& a, uint8_t* packed,
   const float4 g = active ? reinterpret_cast<const float4*>(gamma)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float4 b = active ? reinterpret_cast<const float4*>(beta)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float gg[4] = {g.x, g.y, g.z, g.w}, bb[4] = {b.x, b.y, b.z, b.w};
-  float d = 0.f, rs = 0.f;
+  float d = 0.f;
   uint16_t o[4];
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
-    const __half r = __float2half_rn(fminf(fmaxf(w[t] * gg[t], -65504.f), 65504.f));
-    o[t] = __half_as_ushort(r);
-    rs += __half2float(r);
+    o[t] = __half_as_ushort(__float2half_rn(fminf(fmaxf(w[t] * gg[t], -65504.f), 65504.f)));
     d = fmaf(w[t], bb[t], d);
   }
   if (active) {
@@ -1515,11 +1463,7 @@ __device__ __forceinline__ void bwd_pack_row(const PackArgs& a, uint8_t* packed,
     reinterpret_cast<uint2*>(packed + static_cast<size_t>(m) * 32768)[row * (k / 4) + lane] = ov;
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    d += __shfl_xor_sync(0xFFFFFFFFu, d, off);
-    rs += __shfl_xor_sync(0xFFFFFFFFu, rs, off);
-  }
-  if (lane == 0 && m == 4) reinterpret_cast<float*>(packed + kBwdPackedRowSum)[row] = rs;
+  for (int off = 16; off > 0; off >>= 1) d += __shfl_xor_sync(0xFFFFFFFFu, d, off);
   if (lane == 0)
     reinterpret_cast<float*>(packed + kBwdPackedD)[m * 128 + row] = d + (a.bias[m] != nullptr ? a.bias[m][row] : 0.f);
 }
@@ -1567,7 +1511,7 @@ struct BwdFinalHalf {
   const float* part_s[6];  // per matrix: [n_parts][2][128]
   float* dw[6];            // fp32 gradient blocks
   int dw_ld[6];            // their leading dimensions
-  float* ln_rows;          // [6][4][2][128]: the terms of dgamma and dbeta from 32 matrix rows each
+  float* ln_rows;          // [6][8][2][128]: the terms of dgamma and dbeta from 16 matrix rows each
   unsigned mask;           // bit m set: matrix m is present in this half
 };
 struct BwdFinalArgs {
@@ -1575,12 +1519,14 @@ struct BwdFinalArgs {
   int n_parts;
   const float* scale;  // [2]
 };
-// Sums over the CTAs, for the block's 32 rows (lanes): four columns of the matrix (`m` points at CTA 0's, matrices
-// `m_stride` floats apart) and the column sum belonging to the row (`col_sum` likewise, or null). Valid in warp 0.
+// Sums over the CTAs, for the block's 32 lanes: four columns of a matrix row (`m` points at the row's columns in CTA 0's
+// matrix, matrices `m_stride` floats apart) and the column sum belonging to the row (`col_sum` likewise, or null). Valid in
+// warp 0. The order of the additions: partial i belongs to chain i mod 16, except that the partials of an incomplete last
+// sixteen are added to chain i mod 4 if it has no partial i mod 4 + 12; then the chains four apart, then the four sums.
 __device__ __forceinline__ void sum_partials_of_rows(const float* m, size_t m_stride, const float* col_sum, size_t s_stride,
-                                                     int n_parts, int group, int row0, float4& mv, float& sv) {
-  __shared__ float4 comb[kFinGroups * 32];
-  __shared__ float comb_s[kFinGroups * 32];
+                                                     int n_parts, float4& mv, float& sv) {
+  __shared__ float4 comb[2][kFinGroups * 32];
+  __shared__ float comb_s[2][kFinGroups * 32];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   float4 v[kFinFlight];
   float c[kFinFlight];
@@ -1588,43 +1534,48 @@ __device__ __forceinline__ void sum_partials_of_rows(const float* m, size_t m_st
   for (int u = 0; u < kFinFlight; ++u) {
     const size_t i = g + u * kFinGroups;
     const bool there = g + u * kFinGroups < n_parts;
-    v[u] = there ? __ldcg(reinterpret_cast<const float4*>(m + i * m_stride) + group * 128 + row0 + lane)
-                 : make_float4(0.f, 0.f, 0.f, 0.f);
-    c[u] = there && col_sum != nullptr ? __ldcg(col_sum + i * s_stride + row0 + lane) : 0.f;
+    v[u] = there ? __ldcg(reinterpret_cast<const float4*>(m + i * m_stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    c[u] = there && col_sum != nullptr ? __ldcg(col_sum + i * s_stride) : 0.f;
   }
-  float4 s = v[0];
-  float t = c[0];
+  // partial i = g + 16 u of an incomplete sixteen that does not stay in its chain
+  const int full = n_parts & ~(kFinGroups - 1);
+  const bool moved = g >= 4 && full + g < n_parts && full + (g & 3) + 12 >= n_parts;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f), tail = s;
+  float t = 0.f, tail_s = 0.f;
 #pragma unroll
-  for (int u = 1; u < kFinFlight; ++u) s.x += v[u].x, s.y += v[u].y, s.z += v[u].z, s.w += v[u].w, t += c[u];
-  comb[g * 32 + lane] = s;
-  comb_s[g * 32 + lane] = t;
+  for (int u = 0; u < kFinFlight; ++u) {
+    if (moved && u * kFinGroups == full) tail = v[u], tail_s = c[u];
+    else s.x += v[u].x, s.y += v[u].y, s.z += v[u].z, s.w += v[u].w, t += c[u];
+  }
+  comb[0][g * 32 + lane] = s, comb[1][g * 32 + lane] = tail;
+  comb_s[0][g * 32 + lane] = t, comb_s[1][g * 32 + lane] = tail_s;
   __syncthreads();
-  mv = make_float4(0.f, 0.f, 0.f, 0.f);
-  sv = 0.f;
-  if (g == 0) {
+  if (g != 0) return;
+  float4 q[4];
+  float qs[4];
 #pragma unroll
-    for (int q = 0; q < kFinGroups; ++q) {
-      const float4 x = comb[q * 32 + lane];
-      mv.x += x.x, mv.y += x.y, mv.z += x.z, mv.w += x.w;
-      sv += comb_s[q * 32 + lane];
+  for (int r = 0; r < 4; ++r) {
+    float4 x[4];
+    float y[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[k] = comb[0][(r + 4 * k) * 32 + lane], y[k] = comb_s[0][(r + 4 * k) * 32 + lane];
+#pragma unroll
+    for (int k = 1; k < 4; ++k) {  // (zeros where nothing moved)
+      const float4 e = comb[1][(r + 4 * k) * 32 + lane];
+      x[0].x += e.x, x[0].y += e.y, x[0].z += e.z, x[0].w += e.w, y[0] += comb_s[1][(r + 4 * k) * 32 + lane];
     }
+    q[r].x = (x[0].x + x[1].x) + (x[2].x + x[3].x), q[r].y = (x[0].y + x[1].y) + (x[2].y + x[3].y);
+    q[r].z = (x[0].z + x[1].z) + (x[2].z + x[3].z), q[r].w = (x[0].w + x[1].w) + (x[2].w + x[3].w);
+    qs[r] = (y[0] + y[1]) + (y[2] + y[3]);
   }
+  mv.x = (q[0].x + q[1].x) + (q[2].x + q[3].x), mv.y = (q[0].y + q[1].y) + (q[2].y + q[3].y);
+  mv.z = (q[0].z + q[1].z) + (q[2].z + q[3].z), mv.w = (q[0].w + q[1].w) + (q[2].w + q[3].w);
+  sv = (qs[0] + qs[1]) + (qs[2] + qs[3]);
 }
-// the sum of a value over the 32 lanes (rows) of a warp
-__device__ __forceinline__ float sum_lanes(float x) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xFFFFFFFFu, x, off);
-  return x;
-}
-// warp 0: one row per lane; w, mv: four columns of the weights and of M / c, sv: S / c. Lane 0 writes the block's terms.
-__device__ __forceinline__ void store_ln_terms(float* dst, const float (&w)[4], const float (&mv)[4], float sv) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    const float a = sum_lanes(w[t] * mv[t]), b = sum_lanes(w[t] * sv);
-    if (lane == 0) dst[t] = a, dst[128 + t] = b;
-  }
-}
+// One row of the terms of dgamma and dbeta: four columns of the weights and of M / c, and S / c.
+struct LnRow {
+  float w[4], mv[4], sv;
+};
 __global__ void __launch_bounds__(512) bwd_finalize_kernel(const __grid_constant__ BwdFinalArgs args) {
   grid_dependency_wait();
   grid_dependents_launch();
@@ -1634,9 +1585,9 @@ __global__ void __launch_bounds__(512) bwd_finalize_kernel(const __grid_constant
   if (((a.mask >> m) & 1u) == 0u || q * 32 >= n_rows || group * 4 >= n_cols) return;
   float4 m4;
   float s1;
-  sum_partials_of_rows(a.part_m[m], 2 * 128 * 128, a.part_s[m], 2 * 128, args.n_parts, group, q * 32, m4, s1);
+  const int r = q * 32 + (threadIdx.x & 31), k0 = group * 4;
+  sum_partials_of_rows(a.part_m[m] + (group * 128 + r) * 4, 2 * 128 * 128, a.part_s[m] + r, 2 * 128, args.n_parts, m4, s1);
   if (threadIdx.x >= 32) return;
-  const int r = q * 32 + threadIdx.x, k0 = group * 4;
   const float cinv = args.scale[1];
   const float sv = s1 * cinv, mv[4] = {m4.x * cinv, m4.y * cinv, m4.z * cinv, m4.w * cinv};
   const float4 gamma = *reinterpret_cast<const float4*>((m == 4 ? a.w.ln_out_w : a.w.ln_in_w) + k0);
@@ -1653,7 +1604,21 @@ __global__ void __launch_bounds__(512) bwd_finalize_kernel(const __grid_constant
   float* dw = a.dw[m] + static_cast<size_t>(r) * a.dw_ld[m] + k0;
   dw[0] = fmaf(mv[0], gamma.x, sv * beta.x), dw[1] = fmaf(mv[1], gamma.y, sv * beta.y);
   dw[2] = fmaf(mv[2], gamma.z, sv * beta.z), dw[3] = fmaf(mv[3], gamma.w, sv * beta.w);
-  store_ln_terms(a.ln_rows + (m * 4 + q) * 256 + k0, w, mv, sv);
+  __shared__ LnRow rows[32];
+  rows[threadIdx.x] = {{w[0], w[1], w[2], w[3]}, {mv[0], mv[1], mv[2], mv[3]}, sv};
+  __syncwarp();
+  if (threadIdx.x < 8) {  // four columns of two groups of 16 rows, in the order of the rows
+    const int t = threadIdx.x & 3, half = threadIdx.x >> 2;
+    float ag = 0.f, ab = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const LnRow& x = rows[half * 16 + i];
+      ag = fmaf(x.w[t], x.mv[t], ag);
+      ab = fmaf(x.w[t], x.sv, ab);
+    }
+    float* dst = a.ln_rows + (m * 8 + q * 2 + half) * 256 + k0 + t;
+    dst[0] = ag, dst[128] = ab;
+  }
 }
 // Adds the LayerNorm terms in a fixed order. Grid 1 + halves: the input LayerNorm, then the output LayerNorm's 128 channels
 // of each half; thread = gamma or beta and channel.
@@ -1676,9 +1641,12 @@ __global__ void __launch_bounds__(256) bwd_finalize_ln_kernel(const BwdLnArgs a)
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
       if ((m == 4) == input || ((a.mask[h] >> m) & 1u) == 0u) continue;
+      float x[8], sm = 0.f;
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (m < 4 || q * 32 < a.c) s += __ldcg(a.ln_rows[h] + (m * 4 + q) * 256 + threadIdx.x);
+      for (int rb = 0; rb < 8; ++rb) x[rb] = m < 4 || rb * 16 < a.c ? __ldcg(a.ln_rows[h] + (m * 8 + rb) * 256 + threadIdx.x) : 0.f;
+#pragma unroll
+      for (int rb = 0; rb < 8; ++rb) sm += x[rb];
+      s += sm;
     }
   }
   (input ? a.d_in[vec] : a.d_out[vec] + 128 * (static_cast<int>(blockIdx.x) - 1))[k] = s;

@@ -548,9 +548,9 @@ __global__ void __launch_bounds__(256) tr_bwd_setup_kernel(const __grid_constant
 //   (column sums in the first 128 entries)
 //   dWa[j*128+r][k] = (Ma_j[r][k] gamma[k] + sa_j[r] beta[k]) / c, dWb likewise, dWs[c][j*128+h] = dWs_j[c][h] / c
 //   dgamma[k] = sum_j sum_r (Wa Ma + Wb Mb) / c,  dbeta[k] = sum_j sum_r (Wa sa + Wb sb) / c
-// Grid (128: group of four columns and quarter of the rows, 3 matrices, 4 blocks j), as bwd_finalize_kernel; the LayerNorm
-// terms [2][4][4][2][128] are added by tr_bwd_final_ln_kernel. (A reduction per launch and a gradient kernel on 4 x 8 blocks
-// were 4 x 5.9 + 22.4 us.)
+// Grid (384, 4 blocks j): 256 blocks (group of four columns, 16 rows) of Ma and Mb, whose LayerNorm terms are one chain over
+// both, and 128 blocks (group of four columns, 32 rows) of dWs; as bwd_finalize_kernel. The terms [4][8][2][128] are added by
+// tr_bwd_final_ln_kernel. (A reduction per launch and a gradient kernel on 4 x 8 blocks were 4 x 5.9 + 22.4 us.)
 struct TrBwdFinalArgs {
   TrBwdPackArgs w;
   const float* part_m;
@@ -560,23 +560,26 @@ struct TrBwdFinalArgs {
   float* d_wa;     // [512][128]
   float* d_wb;     // [512][128]
   float* d_ws;     // [128][512]
-  float* ln_rows;  // [2][4][4][2][128]
+  float* ln_rows;  // [4][8][2][128]
   float* d_ln[2];  // dgamma, dbeta [128]
 };
 __global__ void __launch_bounds__(512) tr_bwd_final_kernel(const __grid_constant__ TrBwdFinalArgs a) {
   grid_dependency_wait();
   grid_dependents_launch();
-  const int group = blockIdx.x >> 2, q = blockIdx.x & 3, m = blockIdx.y, j = blockIdx.z;
-  const float* parts = a.part_m + (static_cast<size_t>(j) * a.n_parts * 3 + m) * 128 * 128;
-  const float* sums = m == 2 ? nullptr : a.part_s + (static_cast<size_t>(j) * a.n_parts * 2 + m) * 512;
+  const bool squeeze = blockIdx.x >= 256;
+  const int lane = threadIdx.x & 31, j = blockIdx.y;
+  const int group = squeeze ? (blockIdx.x - 256) >> 2 : blockIdx.x >> 3, k0 = group * 4;
+  const int rb = blockIdx.x & 7;  // 16 rows of Ma (lanes 0-15) and Mb (lanes 16-31)
+  const int m = squeeze ? 2 : lane >> 4, r = squeeze ? (blockIdx.x & 3) * 32 + lane : rb * 16 + (lane & 15);
+  const float* parts = a.part_m + (static_cast<size_t>(j) * a.n_parts * 3 + m) * 128 * 128 + (group * 128 + r) * 4;
+  const float* sums = squeeze ? nullptr : a.part_s + (static_cast<size_t>(j) * a.n_parts * 2 + m) * 512 + r;
   float4 m4;
   float s1;
-  sum_partials_of_rows(parts, 3 * 128 * 128, sums, 2 * 512, a.n_parts, group, q * 32, m4, s1);
+  sum_partials_of_rows(parts, 3 * 128 * 128, sums, 2 * 512, a.n_parts, m4, s1);
   if (threadIdx.x >= 32) return;
-  const int r = q * 32 + threadIdx.x, k0 = group * 4;
   const float cinv = a.scale[1];
   const float sv = s1 * cinv, mv[4] = {m4.x * cinv, m4.y * cinv, m4.z * cinv, m4.w * cinv};
-  if (m == 2) {
+  if (squeeze) {
     float* dst = a.d_ws + static_cast<size_t>(r) * 512 + j * 128 + k0;
 #pragma unroll
     for (int t = 0; t < 4; ++t) dst[t] = mv[t];
@@ -584,13 +587,26 @@ __global__ void __launch_bounds__(512) tr_bwd_final_kernel(const __grid_constant
   }
   const size_t wi = static_cast<size_t>(j * 128 + r) * 128 + k0;
   float* dst = (m == 0 ? a.d_wa : a.d_wb) + wi;
-  float w[4];
+  __shared__ LnRow rows[32];
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
-    w[t] = tr_load_w(m == 0 ? a.w.w_a : a.w.w_b, wi + t, a.w.f32_weights);
     dst[t] = fmaf(mv[t], a.w.ln_w[k0 + t], sv * a.w.ln_b[k0 + t]);
+    rows[lane].w[t] = tr_load_w(m == 0 ? a.w.w_a : a.w.w_b, wi + t, a.w.f32_weights);
+    rows[lane].mv[t] = mv[t];
   }
-  store_ln_terms(a.ln_rows + ((m * 4 + j) * 4 + q) * 256 + k0, w, mv, sv);
+  rows[lane].sv = sv;
+  __syncwarp();
+  if (lane < 4) {
+    float ag = 0.f, ab = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const LnRow &x = rows[i], &y = rows[16 + i];
+      ag = fmaf(x.w[lane], x.mv[lane], fmaf(y.w[lane], y.mv[lane], ag));
+      ab = fmaf(x.w[lane], x.sv, fmaf(y.w[lane], y.sv, ab));
+    }
+    float* terms = a.ln_rows + (j * 8 + rb) * 256 + k0 + lane;
+    terms[0] = ag, terms[128] = ab;
+  }
 }
 __global__ void __launch_bounds__(256) tr_bwd_final_ln_kernel(const TrBwdFinalArgs a) {
   grid_dependency_wait();
