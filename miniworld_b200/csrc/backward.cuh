@@ -772,65 +772,49 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
 }
 
 // Mean and rstd of the stored t over the 256 channels of two tensors [rows][128][N] (fp16): stats[row][j] = {mean,
-// rsqrt(var + eps)} (eps already scaled like the stored t). A block takes 32 groups of eight columns, a warp 32 of the 256
-// channels of all of them (16-byte loads, 512 bytes per warp and channel, eight in flight); the eight warps' partial means
-// and squared deviations are merged through shared memory. (One thread per group over all 256 channels left the chip idle
-// at small N: 8192 threads at N = 256, 29 us for 34 MB.)
-constexpr int kLnStatsGroups = 32;
+// rsqrt(var + eps)} (eps already scaled like the stored t). The sums of a column are one chain over its 256 channels in
+// order. A block brings eight groups of eight columns into shared memory (128 bytes per channel, all loads in flight at once);
+// then one warp walks the channels, a lane two columns. (One thread per group of eight columns that loaded as it went left
+// the chip idle at small N: 8192 threads at N = 256, 29 us for 34 MB.)
+constexpr int kLnStatsGroups = 8;
 __global__ void __launch_bounds__(256) bwd_ln_stats_kernel(const uint4* t0, const uint4* t1, int n, long long groups, float eps,
                                                            float2* stats) {
   grid_dependency_wait();
   grid_dependents_launch();
-  constexpr int kPerWarp = 32;  // channels
-  __shared__ float2 part[8][8][kLnStatsGroups];  // [warp][column][group]: mean, sum of squared deviations
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  const long long g = blockIdx.x * static_cast<long long>(kLnStatsGroups) + lane;
+  __shared__ uint4 tile[256][kLnStatsGroups];
   const int per_row = n / 8;
-  const long long row = g / per_row;
-  const int jc = static_cast<int>(g - row * per_row);
-  float pv[8], s1[8], s2[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) pv[e] = 0.f, s1[e] = 0.f, s2[e] = 0.f;
-  if (g < groups) {
-    const int c_first = (wp & 3) * kPerWarp;
-    const uint4* src = (wp < 4 ? t0 : t1) + (row * 128 + c_first) * per_row + jc;
-#pragma unroll
-    for (int c0 = 0; c0 < kPerWarp; c0 += 8) {
+  const long long first = blockIdx.x * static_cast<long long>(kLnStatsGroups);
+  {
+    const int k = threadIdx.x & (kLnStatsGroups - 1), c0 = threadIdx.x / kLnStatsGroups;
+    const long long g = first + k;
+    if (g < groups) {
+      const long long row = g / per_row;
+      const long long at = row * 128 * per_row + (g - row * per_row);
       uint4 v[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = __ldg(src + static_cast<long long>(c0 + k) * per_row);
+      for (int u = 0; u < 8; ++u)
+        v[u] = __ldg((u < 4 ? t0 : t1) + at + static_cast<long long>((c0 + 32 * u) & 127) * per_row);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const float2 x = f16x2_to_float2(w[t]);
-          if (c0 == 0 && k == 0) pv[2 * t] = x.x, pv[2 * t + 1] = x.y;
-          const float d0 = x.x - pv[2 * t], d1 = x.y - pv[2 * t + 1];
-          s1[2 * t] += d0, s1[2 * t + 1] += d1;
-          s2[2 * t] = fmaf(d0, d0, s2[2 * t]), s2[2 * t + 1] = fmaf(d1, d1, s2[2 * t + 1]);
-        }
-      }
+      for (int u = 0; u < 8; ++u) tile[c0 + 32 * u][k] = v[u];
     }
   }
-#pragma unroll
-  for (int e = 0; e < 8; ++e)
-    part[wp][e][lane] = make_float2(pv[e] + s1[e] * (1.0f / kPerWarp), fmaxf(s2[e] - s1[e] * s1[e] * (1.0f / kPerWarp), 0.f));
   __syncthreads();
-  if (g >= groups) return;
-  // this thread: column `wp` of group `lane`; equal-sized partials: mean of means, M2 = sum M2_k + n_k sum (mean_k - mean)^2
-  float2 p[8];
-  float mean = 0.f, m2 = 0.f;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    p[k] = part[k][wp][lane];
-    mean += p[k].x;
-    m2 += p[k].y;
+  const long long g = first + (threadIdx.x >> 2);
+  if (threadIdx.x >= 32 || g >= groups) return;
+  const uint32_t* col = reinterpret_cast<const uint32_t*>(tile) + threadIdx.x;  // columns 2 * lane, 2 * lane + 1
+  const float2 pv = f16x2_to_float2(col[0]), npv = make_float2(-pv.x, -pv.y);
+  float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f);
+#pragma unroll 32
+  for (int c = 0; c < 256; ++c) {
+    const float2 d = __fadd2_rn(f16x2_to_float2(col[c * 32]), npv);
+    s1 = __fadd2_rn(s1, d);
+    s2 = __ffma2_rn(d, d, s2);
   }
-  mean *= 0.125f;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) m2 = fmaf(static_cast<float>(kPerWarp) * (p[k].x - mean), p[k].x - mean, m2);
-  stats[row * n + jc * 8 + wp] = make_float2(mean, rsqrtf(m2 * (1.0f / 256.0f) + eps));
+  constexpr float kInv = 1.0f / 256.0f;
+  const float var0 = fmaxf(s2.x - s1.x * s1.x * kInv, 0.f) * kInv, var1 = fmaxf(s2.y - s1.y * s1.y * kInv, 0.f) * kInv;
+  const long long row = g / per_row;
+  reinterpret_cast<float4*>(stats + row * n + (g - row * per_row) * 8)[threadIdx.x & 3] =
+      make_float4(pv.x + s1.x * kInv, rsqrtf(var0 + eps), pv.y + s1.y * kInv, rsqrtf(var1 + eps));
 }
 
 // Finishes the first tensor's gradient of the 256-channel LayerNorm backward, in place over the raw d t_hat the MODE 1

@@ -11,7 +11,7 @@ ALLOWED = {
     ("backward.cuh", "asm volatile(\"ld.global.nc.v8.b32"): "the load of ldg_32B, whose only caller is ldg_chunks",
     ("backward.cuh", "for (int c = 0; c < CHUNKS; ++c) out[c] = __ldg(p + c);"): "ldg_chunks",
     ("backward.cuh", "ldg_chunks(reinterpret_cast<const uint4*>(p.drop_scale"): "an argument; the set-up launch starts after it is written",
-    ("backward.cuh", "__ldg(src + static_cast<long long>(c0 + k) * per_row);"): "the forward's tri; likewise",
+    ("backward.cuh", "__ldg((u < 4 ? t0 : t1) + at"): "the forward's tri; likewise",
     ("backward.cuh", "const float4 st = __ldg(sp + q)"): "statistics, written three launches before",
     ("backward.cuh", "tv[k] = __ldg(t + base"): "the forward's tri",
     ("backward.cuh", "rstd_in = __ldg(p.rstd"): "written by the epilogue's backward, contractions in between",

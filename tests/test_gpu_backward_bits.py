@@ -27,6 +27,9 @@ CASES = {
     "out_n192": (True, 128, 1, 192, "token", True, torch.float32),
     "in_b2_n72": (False, 128, 2, 72, "pair", False, torch.float32),
     "in_n264_bf16": (False, 128, 1, 264, "pair", False, torch.bfloat16),
+    "bidir_b2_n24": (None, 128, 2, 24, "token", False, torch.float32),
+    "bidir_n136": (None, 128, 1, 136, None, False, torch.float32),
+    "bidir_n160_drop": (None, 128, 1, 160, "token", True, torch.float32),
     "narrow_out_n136": (True, 64, 1, 136, "pair", False, torch.float32),
     "narrow_bidir_b2_n88": (None, 64, 2, 88, "token", False, torch.float32),
 }
