@@ -75,19 +75,6 @@ __device__ __forceinline__ void ldg_32B(const void* p, uint4& a, uint4& b) {
                : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
                : "l"(p));
 }
-// The same for a tensor the kernel before this one writes (see grid_dependency_wait), 32-byte aligned: coherent loads.
-template <int CHUNKS>
-__device__ __forceinline__ void ld_chunks_32B(const uint4* p, uint4 (&out)[CHUNKS]) {
-  static_assert(CHUNKS % 2 == 0, "pairs of 16-byte chunks");
-#pragma unroll
-  for (int c = 0; c < CHUNKS; c += 2) {
-    uint4 &a = out[c], &b = out[c + 1];
-    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
-                 : "l"(p + c)
-                 : "memory");
-  }
-}
 // `chunks` 16-byte pieces (an even count) from p: 32-byte requests if the address allows, else 16-byte ones
 template <int CHUNKS>
 __device__ __forceinline__ void ldg_chunks(const uint4* p, bool wide, uint4 (&out)[CHUNKS]) {
@@ -838,7 +825,7 @@ __global__ void __launch_bounds__(256) bwd_ln_finish_kernel(uint4* dt, const uin
     const float4* mp = reinterpret_cast<const float4*>(means + row * n + jc * 8);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const float4 st = __ldg(sp + q), mm = mp[q];  // (the launch before this one writes the means)
+      const float4 st = __ldg(sp + q), mm = __ldcg(mp + q);  // (the launch before this one writes the means)
       mean[2 * q] = st.x, k0[2 * q] = st.y * 0.0625f, k1[2 * q] = st.y * mm.y, m1[2 * q] = mm.x;
       mean[2 * q + 1] = st.z, k0[2 * q + 1] = st.w * 0.0625f, k1[2 * q + 1] = st.w * mm.w, m1[2 * q + 1] = mm.z;
     }

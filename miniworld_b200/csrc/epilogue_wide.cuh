@@ -415,8 +415,7 @@ epilogue_wide_kernel(const __grid_constant__ CUtensorMap map_t0, const __grid_co
         const int bb = row / p.rows_per_sample;
         const int j = j0 + pos < p.n ? j0 + pos : p.n - 1;
         const uint4* sp = reinterpret_cast<const uint4*>(p.drop_scale + (static_cast<size_t>(bb) * p.n + j) * 128 + half * 64);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) sc[c] = sp[c];
+        ld_gpu_chunks(sp, (reinterpret_cast<uintptr_t>(p.drop_scale) & 31u) == 0, sc);
       }
 
       mbar_wait_warp(acc_full(grp), ph, abort_flag, p.status, kDevTimeoutEpilogue);

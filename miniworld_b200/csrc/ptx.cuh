@@ -114,12 +114,34 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
 
 // ------------------------------------------------------------------ dependent launches
 // Waits until the kernel before this one on the stream has completed and its writes are visible (returns at once if the
-// launch does not overlap it). Every thread calls it before it touches global memory. A kernel's life begins before the one
-// before it has ended, so non-coherent loads (ld.global.nc, __ldg: of data that does not change during the kernel's life) must
-// not read what that one may write: a kernel that an entry point launches first reads every operand with plain or .cg loads or
-// through TMA, a later one the operands its direct predecessor writes. Memory written earlier is safe: the predecessor has
-// itself waited before it let this kernel begin.
+// launch does not overlap it). Every thread calls it before it touches global memory.
+//
+// A kernel's life begins before the one before it has ended, so two kinds of loads must not read what that one may write:
+// - non-coherent ones (ld.global.nc, __ldg), which are for data that does not change during the kernel's life;
+// - plain ones, if that kernel has also READ it through its SMs' L1: a line that it left there is found again (measured: the
+//   running d x_hat of the Transition's backward, read with plain loads and stored by TMA in every launch, came back old in
+//   the next launch and put its gradients off by 3e-3). Such data is read through TMA or with ld_gpu_chunks.
+// The first kernel of an entry point may follow any kernel of the caller, the entry point's own last one with its output as
+// this one's input among them. Memory written earlier is safe: the predecessor has itself waited before it let this kernel begin.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// `CHUNKS` 16-byte pieces (an even count) from p at gpu scope, which no line in L1 answers: 32-byte requests if the address allows
+template <int CHUNKS>
+__device__ __forceinline__ void ld_gpu_chunks(const uint4* p, bool wide, uint4 (&out)[CHUNKS]) {
+  static_assert(CHUNKS % 2 == 0, "pairs of 16-byte chunks");
+#pragma unroll
+  for (int c = 0; c < CHUNKS; c += 2) {
+    uint4 &a = out[c], &b = out[c + 1];
+    if (wide) {
+      asm volatile("ld.relaxed.gpu.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                   : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                   : "l"(p + c)
+                   : "memory");
+    } else {
+      asm volatile("ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w) : "l"(p + c) : "memory");
+      asm volatile("ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w) : "l"(p + c + 1) : "memory");
+    }
+  }
+}
 // The next kernel's blocks may be placed as this one's leave their SMs (they wait as above before they touch memory).
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

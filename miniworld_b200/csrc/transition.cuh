@@ -392,8 +392,13 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       const bool in_range = grow < p.positions;
       const uint4* xp = reinterpret_cast<const uint4*>(p.x + (in_range ? grow : 0) * 128);
       uint4 xr[2][2];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) xr[0][c] = (p.residual && in_range) ? xp[c] : make_uint4(0u, 0u, 0u, 0u);
+      // (x may be the output of the launch before this one, even over its own input)
+      const bool wide_x = (reinterpret_cast<uintptr_t>(p.x) & 31u) == 0;
+      auto load_x = [&](int pair, uint4 (&dst)[2]) {
+        dst[0] = dst[1] = make_uint4(0u, 0u, 0u, 0u);
+        if (p.residual && in_range) ld_gpu_chunks(xp + pair * 2, wide_x, dst);
+      };
+      load_x(0, xr[0]);
       {
         const bool got = mbar_wait_warp(d2_full(t & 1), (t >> 1) & 1, abort_flag, p.status, kDevTimeoutEpilogue);
         if (!named_bar_and(1, 128, got)) break;
@@ -403,11 +408,7 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       const uint32_t t_d2 = tmem_base + lane_off + kTrColD2 + (t & 1) * 128;
 #pragma unroll
       for (int ps = 0; ps < 8; ++ps) {
-        if (ps < 7) {
-#pragma unroll
-          for (int c = 0; c < 2; ++c)
-            xr[(ps + 1) & 1][c] = (p.residual && in_range) ? xp[(ps + 1) * 2 + c] : make_uint4(0u, 0u, 0u, 0u);
-        }
+        if (ps < 7) load_x(ps + 1, xr[(ps + 1) & 1]);
         uint32_t v[16];
         tmem_ld16(t_d2 + ps * 16, v);
         tmem_ld_wait();

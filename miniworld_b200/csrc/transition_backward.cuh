@@ -351,7 +351,7 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
       for (int ch = 0; ch < kBwdChunks; ++ch) dx_prev[ch] = make_uint4(0u, 0u, 0u, 0u);
       if constexpr (!FIRST) {
-        if (inside) ld_chunks_32B(reinterpret_cast<const uint4*>(p.dx_in + gp * 128 + part * kBwdCh), dx_prev);
+        if (inside) ld_gpu_chunks(reinterpret_cast<const uint4*>(p.dx_in + gp * 128 + part * kBwdCh), true, dx_prev);
       }
       thread_wait(ra_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
       __syncwarp();
