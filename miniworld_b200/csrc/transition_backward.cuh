@@ -49,8 +49,9 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                       const __grid_constant__ CUtensorMap map_ws, const __grid_constant__ CUtensorMap map_xh,
                       const __grid_constant__ CUtensorMap map_dyc, const __grid_constant__ CUtensorMap map_out,
                       const BwdTransitionParams p) {
-  // named barriers: inputs converted (FIRST), dh read, a read, da / db written, h written and d x_hat read, output written
-  constexpr int kBarN = 2, kBarR1 = 3, kBarR2 = 4, kBarA = 5, kBarH = 6, kBarC = 7;
+  // named barriers: inputs converted (FIRST), dh read, a read, da / db written, column sums taken, h written and d x_hat read,
+  // output written
+  constexpr int kBarN = 2, kBarR1 = 3, kBarR2 = 4, kBarA = 5, kBarS = 8, kBarH = 6, kBarC = 7;
   constexpr int kOne = kBwdThreads + 32, kTwo = kBwdThreads + 64;  // with one or both issuing warps
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -202,6 +203,7 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         }
         __syncwarp();
       }
+      named_bar_sync(kBarS, kOne);  // the column sums have been read off S2
       if (lane == 0 && has_next) {
         thread_wait(ra_done, it & 1, abort_flag, p.status, kDevTimeoutProducer);
         issue_y(next, it + 1);  // into S2
@@ -245,8 +247,10 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
     const float gc = p.grad_scale[0], gc_inv = p.grad_scale[1];
     const float ca = p.consts[p.block * 128 + pos], cb = p.consts[512 + p.block * 128 + pos];
-    // column sums of da and db over this thread's even and odd positions
-    float2 acc_a2 = make_float2(0.f, 0.f), acc_b2 = make_float2(0.f, 0.f);
+    // column sums of da and db as the GEMMs see them (fp16), a chain per group of four positions
+    float acc_a[8], acc_b[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc_a[c] = 0.f, acc_b[c] = 0.f;
     const float2 ca2 = make_float2(ca, ca), cb2 = make_float2(cb, cb), half2 = make_float2(0.5f, 0.5f);
     const float2 one = make_float2(1.f, 1.f), minus1 = make_float2(-1.f, -1.f);
     auto pair_of = [](uint32_t lo, uint32_t hi) { return make_float2(__uint_as_float(lo), __uint_as_float(hi)); };
@@ -312,31 +316,32 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       // ---- da -> S1, db -> S2 ([hidden unit][position]), h packed in registers
       // (packed fp32 pairs: the pass is bound by its instruction count)
       uint32_t h_p[16];
-      uint32_t v[2][8];
-      tmem_ld8(tmem_base + lane_sel + part * 32, v[0]);
+      uint32_t v[2][4];
+      tmem_ld4(tmem_base + lane_sel + part * 32, v[0]);
 #pragma unroll
       for (int k4 = 0; k4 < 4; ++k4) {
-        tmem_ld_wait();
-        if (k4 < 3) tmem_ld8(tmem_base + lane_sel + part * 32 + (k4 + 1) * 8, v[(k4 + 1) & 1]);
         uint32_t da_p[4], db_p[4];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const int i = k4 * 8 + t * 2;
-          const float2 b2 = __fadd2_rn(pair_of(v[k4 & 1][t * 2], v[k4 & 1][t * 2 + 1]), cb2);
-          const float2 a2 = __fadd2_rn(pair_of(av[i], av[i + 1]), ca2);
-          const float2 d2 = pair_of(dh[i], dh[i + 1]);
-          const float2 ah = __fmul2_rn(a2, half2);
-          const float2 sg = __ffma2_rn(make_float2(tanh_approx(ah.x), tanh_approx(ah.y)), half2, half2);
-          const float2 silu = __fmul2_rn(a2, sg);
-          // silu' = sg (1 + a (1 - sg)) = sg + silu (1 - sg)
-          const float2 dsilu = __ffma2_rn(silu, __ffma2_rn(sg, minus1, one), sg);
-          const float2 da = __fmul2_rn(__fmul2_rn(d2, b2), dsilu);
-          const float2 db = __fmul2_rn(d2, silu);
-          acc_a2 = __fadd2_rn(acc_a2, da);
-          acc_b2 = __fadd2_rn(acc_b2, db);
-          da_p[t] = pack_f16x2_sat(da);
-          db_p[t] = pack_f16x2_sat(db);
-          h_p[k4 * 4 + t] = pack_f16x2_sat(__fmul2_rn(silu, b2));
+        for (int hf = 0; hf < 2; ++hf) {
+          tmem_ld_wait();
+          if (k4 * 2 + hf < 7) tmem_ld4(tmem_base + lane_sel + part * 32 + (k4 * 2 + hf + 1) * 4, v[hf ^ 1]);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int t = hf * 2 + u, i = k4 * 8 + t * 2;
+            const float2 b2 = __fadd2_rn(pair_of(v[hf][u * 2], v[hf][u * 2 + 1]), cb2);
+            const float2 a2 = __fadd2_rn(pair_of(av[i], av[i + 1]), ca2);
+            const float2 d2 = pair_of(dh[i], dh[i + 1]);
+            const float2 ah = __fmul2_rn(a2, half2);
+            const float2 sg = __ffma2_rn(make_float2(tanh_approx(ah.x), tanh_approx(ah.y)), half2, half2);
+            const float2 silu = __fmul2_rn(a2, sg);
+            // silu' = sg (1 + a (1 - sg))
+            const float2 dsilu = __fmul2_rn(sg, __ffma2_rn(a2, __ffma2_rn(sg, minus1, one), one));
+            const float2 da = __fmul2_rn(__fmul2_rn(d2, b2), dsilu);
+            const float2 db = __fmul2_rn(d2, silu);
+            da_p[t] = pack_f16x2_sat(da);
+            db_p[t] = pack_f16x2_sat(db);
+            h_p[k4 * 4 + t] = pack_f16x2_sat(__fmul2_rn(silu, b2));
+          }
         }
         const uint32_t off = tile_chunk(pos, part * 4 + k4);
         st_chunk(s1_s + off, da_p[0], da_p[1], da_p[2], da_p[3]);
@@ -353,6 +358,19 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       if constexpr (!FIRST) {
         if (inside) ld_gpu_chunks(reinterpret_cast<const uint4*>(p.dx_in + gp * 128 + part * kBwdCh), true, dx_prev);
       }
+      // (under the GEMM round) the column sums, from the tiles this thread has written
+#pragma unroll
+      for (int k4 = 0; k4 < 4; ++k4) {
+        auto add = [](float& s, uint32_t lo, uint32_t hi) {
+          const float2 x = f16x2_to_float2(lo), y = f16x2_to_float2(hi);
+          s += x.x, s += x.y, s += y.x, s += y.y;
+        };
+        const uint4 a = ld_chunk(s1_s + tile_chunk(pos, part * 4 + k4)), b = ld_chunk(s2_s + tile_chunk(pos, part * 4 + k4));
+        add(acc_a[2 * k4], a.x, a.y), add(acc_a[2 * k4 + 1], a.z, a.w);
+        add(acc_b[2 * k4], b.x, b.y), add(acc_b[2 * k4 + 1], b.z, b.w);
+      }
+      __syncwarp();
+      named_bar_arrive(kBarS, kOne);
       thread_wait(ra_done, it & 1, abort_flag, p.status, kDevTimeoutEpilogue);
       __syncwarp();
       tc_fence_after();
@@ -450,17 +468,18 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         store_partial(pm + m * 128 * 128, pos, part * kBwdChunks + ch, v);
       }
     }
-    // the four position quarters of a hidden unit, fixed order (through the weights' region: every GEMM that reads it has been
-    // waited for, while the store of x_hat of the last tile may still be reading the x_hat buffer)
-    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(wa_s + (part * 128 + pos) * 8), "f"(acc_a2.x + acc_a2.y),
-                 "f"(acc_b2.x + acc_b2.y) : "memory");
+    // the 32 groups of four positions of a hidden unit, in order (through the weights' region, which no GEMM reads any more)
+    float* sc = reinterpret_cast<float*>(smem);  // [32 groups][2][128]
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      sc[((part * 8 + c) * 2 + 0) * 128 + pos] = acc_a[c];
+      sc[((part * 8 + c) * 2 + 1) * 128 + pos] = acc_b[c];
+    }
     named_bar_sync(1, kBwdThreads);
-    if (threadIdx.x < 128) {
-      float a, b;
-      sum_partials(wa_s, threadIdx.x, a, b);
-      float* ps = p.part_s + static_cast<size_t>(blockIdx.x) * 2 * 512;
-      ps[threadIdx.x] = a;
-      ps[512 + threadIdx.x] = b;
+    if (threadIdx.x < 256) {
+      float sum = 0.f;
+      for (int g = 0; g < 32; ++g) sum += sc[g * 256 + threadIdx.x];
+      p.part_s[static_cast<size_t>(blockIdx.x) * 2 * 512 + (threadIdx.x >> 7) * 512 + (threadIdx.x & 127)] = sum;
     }
   }
   tc_fence_before();

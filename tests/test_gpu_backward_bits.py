@@ -32,6 +32,11 @@ CASES = {
     "bidir_n160_drop": (None, 128, 1, 160, "token", True, torch.float32),
     "narrow_out_n136": (True, 64, 1, 136, "pair", False, torch.float32),
     "narrow_bidir_b2_n88": (None, 64, 2, 88, "token", False, torch.float32),
+    "transition_1": ("transition", 128, 1, 1, None, False, torch.float32),
+    "transition_300": ("transition", 128, 1, 300, None, False, torch.float32),
+    "transition_14075": ("transition", 128, 1, 14075, None, False, torch.bfloat16),
+    "transition_37965": ("transition", 128, 1, 37965, None, False, torch.float32),
+    "transition_147456": ("transition", 128, 1, 147456, None, False, torch.float32),
 }
 
 
