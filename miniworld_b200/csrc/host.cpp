@@ -129,25 +129,43 @@ void launch_forward(const TriCall& c, const Tensor& z, at::TensorList p, const O
         "b200_trimul_forward_ex");
 }
 
-// Forward without a graph: (y, workspace used) or None. `workspace` is used if it is large enough and on the device.
-std::optional<std::tuple<Tensor, Tensor>> trimul_forward(const Tensor& z, const std::vector<Tensor>& params,
-                                                         const OptTensor& token_mask, const OptTensor& pair_mask,
-                                                         const OptTensor& workspace, int64_t d_pair, int64_t direction,
-                                                         double eps_in, double eps_out, bool residual, bool any_n) {
+// Scratch memory that a module keeps from one call to the next, with the stream that it may be used on again: the memory of a
+// call belongs to that call's launches, so only a later call on the same stream can take it. A call that is being captured
+// neither takes kept memory (a graph would go on using it after the module has let it go) nor leaves any to be taken: what it
+// allocates belongs to the graph's pool, and kNoStream marks it.
+constexpr int64_t kNoStream = -1;
+using Kept = std::tuple<int64_t, Tensor>;
+int64_t stream_key(const Tensor& like) {
+  const c10::cuda::CUDAGuard guard(like.device());
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return kNoStream;
+  return static_cast<int64_t>(reinterpret_cast<intptr_t>(stream_of(like)));
+}
+bool usable(const Tensor& kept, int64_t kept_stream, int64_t stream, const Tensor& like) {
+  return stream != kNoStream && kept_stream == stream && kept.device() == like.device();
+}
+
+// Forward without a graph: (y, (stream, workspace used)) or None. `kept`: what an earlier call returned, which no other call is
+// using now.
+std::optional<std::tuple<Tensor, Kept>> trimul_forward(const Tensor& z, const std::vector<Tensor>& params,
+                                                       const OptTensor& token_mask, const OptTensor& pair_mask,
+                                                       const std::optional<Kept>& kept, int64_t d_pair, int64_t direction,
+                                                       double eps_in, double eps_out, bool residual, bool any_n) {
   TriCall c;
   if (!fill_call(c, z, params, token_mask, pair_mask, std::nullopt, d_pair, direction, eps_in, eps_out, residual, any_n))
     return std::nullopt;
   const at::NoGradGuard no_grad;
   const size_t need = forward_bytes(c);
+  const int64_t stream = stream_key(z);
   Tensor ws;
-  if (workspace.has_value() && workspace->device() == z.device() && static_cast<size_t>(workspace->numel()) >= need) {
-    ws = *workspace;
+  if (kept.has_value() && usable(std::get<1>(*kept), std::get<0>(*kept), stream, z) &&
+      static_cast<size_t>(std::get<1>(*kept).numel()) >= need) {
+    ws = std::get<1>(*kept);
   } else {
     ws = aligned_empty(need, z);
   }
   Tensor y = at::empty_like(z);
   launch_forward(c, z, params, token_mask, pair_mask, std::nullopt, y, ws);
-  return std::make_tuple(y, ws);
+  return std::make_tuple(y, Kept(stream, ws));
 }
 
 // Saved for the backward: the input and the parameters (as autograd saves them), the masks, the dropout scale and the
@@ -264,15 +282,27 @@ void launch_transition(const Tensor& x, at::TensorList p, double eps, bool resid
         "b200_transition_forward");
 }
 
-// Forward without a graph into a new tensor, or None. packed / status: the module's scratch, on the input's device.
-OptTensor transition_forward(const Tensor& x, const std::vector<Tensor>& params, const Tensor& packed, const Tensor& status,
-                             double eps, bool residual) {
+// Forward without a graph: (y, (stream, scratch used)) or None. The scratch holds the packed weights, then 16 status words, which
+// are cleared when it is allocated. `kept` as in trimul_forward.
+std::optional<std::tuple<Tensor, Kept>> transition_forward(const Tensor& x, const std::vector<Tensor>& params,
+                                                           const std::optional<Kept>& kept, double eps, bool residual) {
   if (!transition_plain(x, params)) return std::nullopt;
   const at::NoGradGuard no_grad;
   const c10::cuda::CUDAGuard guard(x.device());
+  const size_t bytes = b200_transition_packed_bytes();
+  const int64_t stream = stream_key(x);
+  Tensor scratch;
+  if (kept.has_value() && usable(std::get<1>(*kept), std::get<0>(*kept), stream, x)) {
+    scratch = std::get<1>(*kept);
+  } else {
+    scratch = aligned_empty(bytes + 64, x);
+    check(b200_trimul_clear_status(reinterpret_cast<int*>(static_cast<uint8_t*>(scratch.data_ptr()) + bytes), stream_of(x)),
+          "b200_trimul_clear_status");
+  }
+  uint8_t* base = static_cast<uint8_t*>(scratch.data_ptr());
   Tensor y = at::empty_like(x);
-  launch_transition(x, params, eps, residual, packed.data_ptr(), static_cast<int*>(status.data_ptr()), y);
-  return y;
+  launch_transition(x, params, eps, residual, base, reinterpret_cast<int*>(base + bytes), y);
+  return std::make_tuple(y, Kept(stream, scratch));
 }
 
 struct TransitionNode : public torch::autograd::Function<TransitionNode> {

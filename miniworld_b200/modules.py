@@ -84,6 +84,32 @@ def _registered(module: nn.Module, names) -> Optional[list]:
     return out
 
 
+class _Kept:
+    """Scratch memory that a module keeps from one call to the next, as ``(stream, tensor)`` in its attribute ``name``.
+
+    A call takes it out of the module while it launches, so that a call from another thread does not find it, and only if the
+    last call was on the same stream: on another one, that call may still be running. Otherwise the call allocates its own, which
+    replaces the kept one (its memory goes back to the allocator, in the order of the stream it was allocated on). A call that is
+    being captured never takes kept memory, and what it allocates, in the graph's pool, is not taken again (stream -1)."""
+
+    def __init__(self, module: nn.Module, name: str, need: int, device: torch.device, clear=None):
+        self.module, self.name, self.need, self.device, self.clear = module, name, need, device, clear
+
+    def __enter__(self) -> torch.Tensor:
+        kept = self.module.__dict__.pop(self.name, None)
+        with torch.cuda.device(self.device):
+            stream = -1 if torch.cuda.is_current_stream_capturing() else torch.cuda.current_stream().cuda_stream
+        if kept is None or stream < 0 or kept[0] != stream or kept[1].device != self.device or kept[1].numel() < self.need:
+            kept = (stream, F_.aligned_empty(self.need, self.device))
+            if self.clear is not None:
+                self.clear(kept[1])
+        self.kept = kept
+        return kept[1]
+
+    def __exit__(self, *error) -> None:
+        self.module.__dict__[self.name] = self.kept
+
+
 class Fp32LayerNorm(nn.LayerNorm):
     """LayerNorm parameter holder whose affine parameters are pinned to fp32: ``module.to(torch.bfloat16)`` moves them
     between devices but never changes (or rounds) their values, like the reference's fp32-pinned LayerNorm
@@ -165,7 +191,7 @@ class TriangleMultiplication(nn.Module):
         nn.init.zeros_(self.to_gate.weight)
         nn.init.zeros_(self.to_out.weight)
         self._biases: Optional[dict] = None
-        self._workspace: Optional[torch.Tensor] = None
+        self._workspace: Optional[tuple] = None  # (stream, workspace) of the last forward, see _Kept
         self._wcache = None  # (key, validated parameter pointers); the values themselves are re-read every call
 
     # ------------------------------------------------------------------ dtype handling
@@ -212,9 +238,8 @@ class TriangleMultiplication(nn.Module):
     def device_status(self) -> int:
         """Synchronise and return the device status word of the last forward: 0, or the 1xx code of a device-side wait
         that gave up (:func:`miniworld_b200.functional.check_status` raises on it)."""
-        if self._workspace is None:
-            return 0
-        return F_.read_status(self._workspace[:64].view(torch.int32))
+        kept = self.__dict__.get("_workspace")
+        return 0 if kept is None else F_.read_status(kept[1][:64].view(torch.int32))
 
     def _direction(self):
         return None if self._bidirectional else self.outgoing
@@ -226,14 +251,6 @@ class TriangleMultiplication(nn.Module):
         B, N, C = pair.shape[0], pair.shape[2], pair.shape[3]
         keep = torch.rand(B, 1, N, C, device=pair.device) >= p
         return keep.to(torch.bfloat16) / (1.0 - p)
-
-    def _get_workspace(self, B: int, N: int, device: torch.device) -> torch.Tensor:
-        need = F_.workspace_bytes(B, N, self._direction(), self.d_pair)
-        ws = self._workspace
-        if ws is None or ws.device != device or ws.numel() < need:
-            ws = F_.aligned_empty(need, device)
-            self._workspace = ws
-        return ws
 
     def _backward_supported(self) -> bool:
         return True  # every width the constructor accepts has a backward
@@ -279,11 +296,11 @@ class TriangleMultiplication(nn.Module):
                 pair_mask = torch.broadcast_to(pair_mask.to(z.device), (B, N, N))
             if scale is not None:
                 scale = F_.aligned16(torch.broadcast_to(scale, (B, 1, N, self.d_pair)).contiguous())
-        with torch.no_grad():
+        need = F_.workspace_bytes(B, F_._pitch(N) if ragged else N, self._direction(), self.d_pair)
+        with torch.no_grad(), _Kept(self, "_workspace", need, z.device) as workspace:
             y = F_._forward(
                 z, self._params(), token_mask, self._direction(), float(self.ln_pair.eps), float(self.ln_out.eps), pair_mask,
-                self.residual, self._biases, self._get_workspace(B, F_._pitch(N) if ragged else N, z.device), None,
-                self.check_status, self._weights(z.device), scale, ragged,
+                self.residual, self._biases, workspace, None, self.check_status, self._weights(z.device), scale, ragged,
             )
         return y if in_dtype == torch.bfloat16 else y.to(in_dtype)
 
@@ -294,13 +311,15 @@ class TriangleMultiplication(nn.Module):
         params = _registered(self, _TRI_NAMES) if ordinary(pair) and pair.dim() == 4 else None
         if params is None:
             return None
+        kept = self.__dict__.pop("_workspace", None)  # (see _Kept)
         got = _lib.native().trimul_forward(
-            pair, params, token_mask, pair_mask, self._workspace, self.d_pair, F_._direction(self._direction()),
-            self.ln_pair.eps, self.ln_out.eps, self.residual, pair.shape[1] % 8 != 0,
+            pair, params, token_mask, pair_mask, kept, self.d_pair, F_._direction(self._direction()), self.ln_pair.eps,
+            self.ln_out.eps, self.residual, pair.shape[1] % 8 != 0,
         )
         if got is None:
+            self.__dict__["_workspace"] = kept
             return None
-        y, self._workspace = got
+        y, self.__dict__["_workspace"] = got
         return y
 
     def _run_train(self, pair: torch.Tensor, token_mask, pair_mask) -> torch.Tensor:
@@ -406,7 +425,7 @@ class Transition(nn.Module):
         self.expand_b = nn.Linear(d, n * d, bias=False)
         self.squeeze = nn.Linear(n * d, d, bias=False)
         nn.init.zeros_(self.squeeze.weight)  # the reference's final linears start at zero
-        self._scratch = None
+        self._scratch = None  # (stream, packed weights and status words) of the last forward without a graph, see _Kept
 
     def _apply(self, fn, recurse=True):
         super()._apply(fn, recurse)
@@ -414,7 +433,13 @@ class Transition(nn.Module):
         return self
 
     def device_status(self) -> int:
-        return 0 if self._scratch is None else F_.read_status(self._scratch[1])
+        kept = self.__dict__.get("_scratch")
+        return 0 if kept is None else F_.read_status(self._split(kept[1])[1])
+
+    @staticmethod
+    def _split(scratch: torch.Tensor):
+        n = F_.transition_packed_bytes()
+        return scratch[:n], scratch[n : n + 64].view(torch.int32)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         from .training import ordinary, transition_train
@@ -437,17 +462,18 @@ class Transition(nn.Module):
         if xb.dtype != torch.bfloat16:
             xb = xb.to(torch.bfloat16)
         xb = xb.contiguous()
-        if self._scratch is None or self._scratch[0].device != xb.device:
-            self._scratch = (F_.aligned_empty(F_.transition_packed_bytes(), xb.device),
-                             torch.zeros(16, dtype=torch.int32, device=xb.device))
-        packed, status = self._scratch
         if plain is not None and not self.check_status and in_dtype == torch.bfloat16 and ordinary(x):
-            y = _lib.native().transition_forward(xb, plain, packed, status, self.ln_in.eps, self.residual)
-            if y is not None:
+            kept = self.__dict__.pop("_scratch", None)  # (see _Kept)
+            got = _lib.native().transition_forward(xb, plain, kept, self.ln_in.eps, self.residual)
+            if got is not None:
+                y, self.__dict__["_scratch"] = got
                 return y
-        with torch.no_grad():
+            self.__dict__["_scratch"] = kept
+        clear = lambda t: self._split(t)[1].zero_()  # noqa: E731
+        with torch.no_grad(), _Kept(self, "_scratch", F_.transition_packed_bytes() + 64, xb.device, clear) as scratch:
+            packed, status = self._split(scratch)
             F_.transition_pack_weights(params, packed)  # packed in every call: a captured graph replays current weights
             y = F_.transition_forward(xb, packed, status, eps=float(self.ln_in.eps), residual=self.residual)
-        if self.check_status:
-            F_.check_status(status, "b200_transition_forward")
+            if self.check_status:
+                F_.check_status(status, "b200_transition_forward")
         return y if in_dtype == torch.bfloat16 else y.to(in_dtype)
