@@ -13,6 +13,7 @@ CSRC = PKG_DIR / "csrc"
 LIB_NAME = "libb200_trimul.so"
 LIB_PATH = PKG_DIR / LIB_NAME
 NATIVE_PATH = PKG_DIR / "_native.so"
+NATIVE_TAG_PATH = PKG_DIR / "_native.tag"  # what NATIVE_PATH was built against
 HOST_SOURCE = CSRC / "host.cpp"
 HEADER = PKG_DIR.parent / "include" / "b200_trimul.h"
 
@@ -39,11 +40,20 @@ def is_stale() -> bool:
     return any(src.stat().st_mtime > built for src in _sources())
 
 
+def native_tag() -> str:
+    """The interpreter and the PyTorch that ``_native.so`` is bound to: with another one it does not load, or not rightly."""
+    import sysconfig
+
+    import torch
+
+    return f"{sysconfig.get_config_var('SOABI')} torch {torch.__version__} cxx11 abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)}\n"
+
+
 def native_is_stale() -> bool:
-    if not NATIVE_PATH.exists():
+    if not NATIVE_PATH.exists() or not NATIVE_TAG_PATH.exists() or NATIVE_TAG_PATH.read_text() != native_tag():
         return True
     built = NATIVE_PATH.stat().st_mtime
-    return any(src.stat().st_mtime > built for src in (HOST_SOURCE, HEADER))
+    return any(src.stat().st_mtime > built for src in (HOST_SOURCE, HEADER, Path(__file__)))
 
 
 def find_nvcc() -> str:
@@ -77,6 +87,7 @@ def build_native(force: bool = False) -> Path:
           str(HOST_SOURCE), "-o", str(tmp), f"-L{root}/lib", "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda",
           f"-L{PKG_DIR}", f"-l:{LIB_NAME}", "-Wl,-rpath,$ORIGIN"])
     os.replace(tmp, NATIVE_PATH)
+    NATIVE_TAG_PATH.write_text(native_tag())
     return NATIVE_PATH
 
 
