@@ -27,10 +27,9 @@
 
 namespace trimul {
 
-#ifndef TRIMUL_BWD_PARTS
-#define TRIMUL_BWD_PARTS 4
-#endif
-constexpr int kBwdParts = TRIMUL_BWD_PARTS;      // threads per position: each covers 128 / kBwdParts channels
+// threads per position, each covering 128 / kBwdParts channels. Not a knob: 16 warps (four per TMEM lane quarter, eight for each
+// of t and z), 32 positions per thread and 32 groups of four rows are written into the kernels.
+constexpr int kBwdParts = 4;
 constexpr int kBwdThreads = 128 * kBwdParts;
 constexpr int kBwdCh = 128 / kBwdParts;          // channels per thread of a 128-channel tile
 constexpr int kBwdChunks = kBwdCh / 8;           // 16-byte chunks (8 channels) per thread

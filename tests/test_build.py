@@ -38,3 +38,10 @@ def test_a_newer_source_makes_it_stale(built, source):
     newer = os.stat(getattr(built, source)).st_mtime - 10
     os.utime(built.NATIVE_PATH, (newer, newer))
     assert built.native_is_stale()
+
+
+def test_no_knobs_in_the_kernels():
+    """A macro that a build may set to another value than the kernels are written for (four threads per position in the backward,
+    once) would compile and give wrong results: the sources have no such switches."""
+    for source in sorted(build.CSRC.iterdir()):
+        assert not [line for line in source.read_text().splitlines() if line.lstrip().startswith(("#if", "#ifdef", "#ifndef"))], source.name
