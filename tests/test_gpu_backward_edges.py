@@ -66,10 +66,24 @@ def test_transition_last_tile_repeats(positions):
         assert all(torch.equal(a, b) for a, b in zip(first, grads()))
 
 
-@pytest.mark.parametrize("B,N", [(1, 8), (3, 8), (1, 24), (1, 136)])
+def _triangle64(m, z, dy):
+    """Gradients of the bidirectional module in float64."""
+    p = {k: v.detach().double().requires_grad_(True) for k, v in m.named_parameters()}
+    x = z.double().requires_grad_(True)
+    h = F.layer_norm(x, (128,), p["ln_pair.weight"], p["ln_pair.bias"], 1e-5)
+    left = torch.sigmoid(F.linear(h, p["to_left_gate.weight"])) * F.linear(h, p["to_left.weight"])
+    right = torch.sigmoid(F.linear(h, p["to_right_gate.weight"])) * F.linear(h, p["to_right.weight"])
+    t = torch.cat([torch.einsum("bikd,bjkd->bijd", left[..., :128], right[..., :128]),
+                   torch.einsum("bkid,bkjd->bijd", left[..., 128:], right[..., 128:])], -1)
+    t = F.layer_norm(t, (256,), p["ln_out.weight"], p["ln_out.bias"], 1e-5)
+    y = x + torch.sigmoid(F.linear(h, p["to_gate.weight"])) * F.linear(t, p["to_out.weight"])
+    return torch.autograd.grad(y, [x, *p.values()], dy.double())
+
+
+@pytest.mark.parametrize("B,N", [(1, 8), (3, 8), (1, 24), (1, 136), (2, 40)])
 def test_wide_statistics_of_short_rows(B, N):
-    """The bidirectional module's gradients do not depend on the batch they are computed in (its statistics kernel takes 32
-    column groups per block, across rows and samples)."""
+    """The bidirectional module's gradients against float64 where its statistics kernel has edges (a block takes eight groups of
+    eight columns, across rows and samples); and they do not depend on the batch they are computed in."""
     m, g = _module(lambda: mw.BidirectionalTriangleMultiplication(128), 7 * N)
     z = torch.randn(B, N, N, 128, generator=g).to(torch.bfloat16).to(DEV)
     dy = (torch.randn(B, N, N, 128, generator=g) * 0.02).to(torch.bfloat16).to(DEV)
@@ -80,6 +94,7 @@ def test_wide_statistics_of_short_rows(B, N):
         return torch.autograd.grad(m(a), a, b)[0]
 
     whole = grad(z, dy)
+    assert _rel(whole, _triangle64(m, z, dy)[0]) <= TOL
     for i in range(B):
         assert torch.equal(whole[i : i + 1], grad(z[i : i + 1], dy[i : i + 1]))
 
@@ -100,5 +115,9 @@ def test_scale_of_special_gradients(make, shape):
     bad = dy.clone()
     bad.view(-1, 128)[-1, 3] = float("inf")
     out = torch.autograd.grad(m(x), x, bad)[0]
-    if len(shape) == 2:  # (the Transition works position by position)
-        assert torch.equal(out[:-1], a[0][:-1])
+    # the Transition works position by position; the triangle update (outgoing) passes a gradient at (i, j) on to row i through
+    # left and to row j through right, which is the last row twice
+    reached = -1 if len(shape) == 2 else (slice(None), -1)
+    clean = torch.ones_like(out, dtype=torch.bool)
+    clean[reached] = False
+    assert torch.equal(out[clean], a[0][clean]) and bool(torch.isfinite(out[clean]).all())

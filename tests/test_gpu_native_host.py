@@ -1,11 +1,13 @@
 """The native host path of the modules against the general Python path (which ``check_status`` selects): the same kernels on
-the same arguments, so the same bits; and calls the native path leaves to the general one."""
+the same arguments, so the same bits; and calls the native path leaves to the general one. Which path a call took is counted at
+the native entry points."""
 
 import pytest
 import torch
 from torch import nn
 
 import miniworld_b200 as mw
+from miniworld_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -37,38 +39,75 @@ def _input(kind, B=2, N=40, seed=5):
     return z, (torch.rand(B, N, generator=g) > 0.2).to(DEV), (torch.randn(z.shape, generator=g) * 0.02).to(torch.bfloat16).to(DEV)
 
 
+class _Counted:
+    """The native module; ``taken`` and ``left`` count the calls it served and the ones it answered with None."""
+
+    def __init__(self, module):
+        self.module, self.taken, self.left = module, 0, 0
+
+    def __getattr__(self, name):
+        f = getattr(self.module, name)
+
+        def call(*args):
+            out = f(*args)
+            if out is None:
+                self.left += 1
+            else:
+                self.taken += 1
+            return out
+
+        return call
+
+    def __call__(self, f):
+        """(calls served, calls left) by the native module while ``f`` runs."""
+        before = self.taken, self.left
+        f()
+        return self.taken - before[0], self.left - before[1]
+
+
+@pytest.fixture
+def native(monkeypatch):
+    counted = _Counted(_lib.native())
+    monkeypatch.setattr(_lib, "_native", counted)
+    return counted
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("N", [40, 43])
 @pytest.mark.parametrize("kind", list(MAKE))
-def test_same_bits_as_the_general_path(kind, N, dtype):
+def test_same_bits_as_the_general_path(kind, N, dtype, native):
     a, b = _pair(kind, dtype)
     z, mask, dy = _input(kind, N=N)
     args = () if kind == "transition" else (mask,)
     with torch.no_grad():
         assert torch.equal(a.eval()(z, *args), b.eval()(z, *args))
+        assert (native.taken, native.left) == (1, 0)  # a's call; b did not ask
     grads = []
     for m in (a.train(), b.train()):
         zr = z.clone().requires_grad_(True)
         y = m(zr, *args)
         grads.append([y.detach(), *torch.autograd.grad(y, [zr, *m.parameters()], dy)])
+    assert (native.taken, native.left) == (2, 0)
     for x, y in zip(*grads):
         assert x.dtype == y.dtype and torch.equal(x, y)
 
 
-def test_calls_left_to_the_general_path():
+def test_calls_left_to_the_general_path(native):
     a, b = _pair("in", torch.bfloat16)
     z, mask, _ = _input("in")
     with torch.no_grad():
         want = b.eval()(z, mask)
         a = a.eval()
-        assert torch.equal(a(z, mask.to(torch.uint8)), want)
-        assert torch.equal(a(z, mask.float()), want)
-        assert torch.equal(a(z, mask.cpu()), want)
-        assert torch.equal(a(z.float(), mask), want.float())
+        assert native(lambda: a(z, mask)) == (1, 0)
+        for m in (mask.to(torch.uint8), mask.float(), mask.cpu()):
+            assert native(lambda: a(z, m)) == (0, 1)
+            assert torch.equal(a(z, m), want)
+        assert torch.equal(a(z.float(), mask), want.float()) and native(lambda: a(z.float(), mask)) == (0, 1)
         zt = z.transpose(1, 2).contiguous().transpose(1, 2)
-        assert not zt.is_contiguous() and torch.equal(a(zt, mask), want)
+        assert not zt.is_contiguous() and torch.equal(a(zt, mask), want) and native(lambda: a(zt, mask)) == (0, 1)
         pair = (mask[:, :, None] & mask[:, None, :])
         assert torch.equal(a(z, pair), want) and torch.equal(a(z, pair.transpose(1, 2)), want)
+        taken = native.taken
         for bad in (z[:, :-1], z.cpu(), z[..., :64], z[0]):
             with pytest.raises(RuntimeError):
                 a(bad, mask)
@@ -77,9 +116,10 @@ def test_calls_left_to_the_general_path():
         a.to_left.weight.data = a.to_left.weight.data.t().contiguous().t()
         with pytest.raises(RuntimeError):
             a(z, mask)
+        assert native.taken == taken
 
 
-def test_reparametrised_and_swapped_parameters():
+def test_reparametrised_and_swapped_parameters(native):
     a, b = _pair("out", torch.float32)
     z, mask, _ = _input("out")
 
@@ -91,6 +131,7 @@ def test_reparametrised_and_swapped_parameters():
     b.to_left.weight.data.mul_(2.0)
     with torch.no_grad():
         assert torch.equal(a.eval()(z, mask), b.eval()(z, mask))
+        assert native.taken == 0
     c, d = _pair("out", torch.float32)
     new = {"to_gate.weight": torch.randn(128, 128, device=DEV) * 0.1}
     d.to_gate.weight.data.copy_(new["to_gate.weight"])
@@ -98,7 +139,7 @@ def test_reparametrised_and_swapped_parameters():
         assert torch.equal(torch.func.functional_call(c.eval(), new, (z, mask)), d.eval()(z, mask))
 
 
-def test_graph_behaviour():
+def test_graph_behaviour(native):
     a, b = _pair("bidir", torch.float32, p_drop=0.25)
     z, mask, dy = _input("bidir")
     scale = ((torch.rand(2, 1, 40, 128, generator=torch.Generator().manual_seed(1)) > 0.25).float() / 0.75).to(torch.bfloat16).to(DEV)
@@ -106,6 +147,7 @@ def test_graph_behaviour():
     a, b = a.train(), b.train()
     # parameters only, a subset of the gradients, an expanded output gradient
     y = a(z, mask)
+    assert (native.taken, native.left) == (1, 0) and "TriMulFunction" not in type(y.grad_fn).__name__
     got = torch.autograd.grad(y, [a.to_out.weight, a.ln_pair.bias], dy[:1].expand_as(dy))
     want = torch.autograd.grad(b(z, mask), [b.to_out.weight, b.ln_pair.bias], dy[:1].expand_as(dy).contiguous())
     assert all(torch.equal(p, q) for p, q in zip(got, want))
