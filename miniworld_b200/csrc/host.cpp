@@ -126,7 +126,7 @@ void launch_forward(const TriCall& c, const Tensor& z, at::TensorList p, const O
           static_cast<const uint8_t*>(ptr(token_mask)), static_cast<const uint8_t*>(ptr(pair_mask)), ptr(drop_scale),
           y.data_ptr(), ws.data_ptr(), static_cast<size_t>(ws.numel()), c.B, c.N, c.d_pair, c.d_hidden, c.direction, c.eps_in,
           c.eps_out, c.residual ? 1 : 0, stream_of(z)),
-        "b200_trimul_forward_ex");
+        c.any_n ? "b200_trimul_forward_any" : "b200_trimul_forward_ex");
 }
 
 // Scratch memory that a module keeps from one call to the next, with the stream that it may be used on again: the memory of a
@@ -235,7 +235,7 @@ struct TriMul : public torch::autograd::Function<TriMul> {
             ptr(drop_scale), ws.data_ptr(), dz.data_ptr(), dw, gp(kLnInW), gp(kLnInB), gp(kLnOutW), gp(kLnOutB),
             bws.data_ptr(), static_cast<size_t>(bws.numel()), c.B, c.N, c.d_pair, c.d_hidden, c.direction, c.eps_in, c.eps_out,
             c.residual ? 1 : 0, stream_of(z)),
-          "b200_trimul_backward");
+          c.any_n ? "b200_trimul_backward_any" : "b200_trimul_backward");
     d.erase("ws");
 
     variable_list out(1 + kTriParams + 4);  // z, the parameters; call, masks and scale have no gradient

@@ -529,7 +529,7 @@ def _forward(z, params, mask, outgoing, eps_in, eps_out, pair_mask, residual, bi
             int(bool(residual)),
             _stream(dev),
         )
-    _lib.check(rc, "b200_trimul_forward_ex")
+    _lib.check(rc, "b200_trimul_forward_any" if any_n else "b200_trimul_forward_ex")
     if check:
         check_status(workspace[:4].view(torch.int32), "b200_trimul_forward")
     return out
@@ -616,7 +616,7 @@ def _backward(dy, z, params, forward_workspace, mask, outgoing, eps_in, eps_out,
             _ptr(workspace), workspace.numel() * workspace.element_size(), B, N, C, w.d_hidden, _direction(outgoing), float(eps_in),
             float(eps_out), int(bool(residual)), _stream(dev),
         )
-    _lib.check(rc, "b200_trimul_backward")
+    _lib.check(rc, "b200_trimul_backward_any" if any_n else "b200_trimul_backward")
     if check:
         check_status(workspace[:4].view(torch.int32), "b200_trimul_backward")
     grads = dict(zip(WEIGHT_KEYS, dws))

@@ -119,6 +119,16 @@ def test_calls_left_to_the_general_path(native):
         assert native.taken == taken
 
 
+@pytest.mark.parametrize("N,entry", [(40, "b200_trimul_forward_ex"), (43, "b200_trimul_forward_any")])
+def test_an_error_names_the_entry_point(N, entry):
+    """(a weight whose storage starts off 16 bytes is refused by the C entry, on either path)"""
+    for m in _pair("out", torch.float32):
+        w = m.to_gate.weight.detach()
+        m.to_gate.weight.data = torch.empty(w.numel() + 1, device=DEV)[1:].view(w.shape).copy_(w)
+        with torch.no_grad(), pytest.raises(RuntimeError, match=entry + ":"):
+            m.eval()(_input("out", N=N)[0])
+
+
 def test_reparametrised_and_swapped_parameters(native):
     a, b = _pair("out", torch.float32)
     z, mask, _ = _input("out")
