@@ -58,7 +58,7 @@ extern "C" {
 #define B200_TRIMUL_E_NULL (-1)        /* a required pointer is null */
 #define B200_TRIMUL_E_SHAPE (-2)       /* bad B / N / rows / direction */
 #define B200_TRIMUL_E_UNSUPPORTED (-3) /* a width outside the list above, N not a multiple of 8 */
-#define B200_TRIMUL_E_ALIGN (-4)       /* a pointer is not 16-byte aligned (workspace: 1024) */
+#define B200_TRIMUL_E_ALIGN (-4)       /* a pointer (tensor, weight or LayerNorm parameter) is not 16-byte aligned (workspace: 1024) */
 #define B200_TRIMUL_E_WORKSPACE (-5)   /* workspace too small */
 #define B200_TRIMUL_E_CUDA (-6)        /* a CUDA runtime / driver call failed; see b200_trimul_last_cuda_error */
 #define B200_TRIMUL_E_DEVICE (-7)      /* not an sm_100 device */

@@ -494,6 +494,8 @@ static int pack_block(PackLaunch& l, int block, const void* const w[6], const in
                       void* packed, int c = kC) {
   if (!ln_in_w || !ln_in_b || !ln_out_w || !ln_out_b || !packed) return B200_TRIMUL_E_NULL;
   if (weight_dtype != B200_TRIMUL_DTYPE_BF16 && weight_dtype != B200_TRIMUL_DTYPE_F32) return B200_TRIMUL_E_SHAPE;
+  for (const float* v : {ln_in_w, ln_in_b, ln_out_w, ln_out_b})
+    if (!aligned(v, 16)) return B200_TRIMUL_E_ALIGN;  // (read in 16-byte pieces)
   PackArgs& a = l.block[block];
   for (int i = 0; i < 6; ++i) {
     if (!w[i]) return B200_TRIMUL_E_NULL;

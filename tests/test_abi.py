@@ -108,3 +108,18 @@ def test_any_length_entry_points_validate_before_any_cuda_call(lib):
     for n, code in ((0, -2), (-3, -2), (2**31 - 1, -2), (203, -5)):
         assert lib.b200_trimul_forward_any(*head, 8, 1, n, *tail) == code, n
     assert lib.b200_trimul_forward_ex(*head, 8, 1, 203, *tail) == -3
+
+
+@pytest.mark.parametrize("which", range(10))
+def test_misaligned_parameters_are_refused_before_any_cuda_call(lib, which):
+    """Weights and LayerNorm parameters are read in 16-byte pieces: one that starts elsewhere (a slice of a flat buffer) is an error
+    of the call."""
+    buf = ctypes.create_string_buffer(4096)
+    a = (ctypes.addressof(buf) + 1023) // 1024 * 1024  # never read
+    weights, lns = [a] * 6, [a] * 4
+    (weights if which < 6 else lns)[which % 6] += 4
+    assert lib.b200_trimul_pack_weights(*weights, 1, *lns, None, a, None) == -4
+    six = (ctypes.c_void_p * 6)(*[a] * 6)
+    rc = lib.b200_trimul_backward(a, a, *weights, 1, *lns, None, None, None, None, a, a, six, a, a, a, a, a, 1 << 40, 1, 384, 128, 128, 1,
+                                  1e-5, 1e-5, 1, None)
+    assert rc == -4
