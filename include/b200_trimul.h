@@ -324,7 +324,9 @@ int b200_trimul_forward_static(const void* z, const void* w_left, const void* w_
  * the prologue's backward four times (side x half).
  * The result is deterministic (fixed summation order). Workspace: b200_trimul_backward_workspace_bytes, 1024-byte
  * aligned; _layout gives its 17 region offsets + the total (status, packed weights, scale, LayerNorm terms, x_hat and
- * 1 / sigma, per-CTA partials of M and S of every launch, dtri, dleft, dright, d x_hat, then the bidirectional module's extra regions) for tests.
+ * 1 / sigma, per-CTA partials of M and S of every launch, dtri, dleft, dright, d x_hat, then the bidirectional module's extra
+ * regions) for tests. About five pair tensors of 128 16-bit channels (nine for direction 0) and 63 MB of partials (126 MB, at
+ * most 160 CTAs): one direction 253 MB at N = 384 and 821 MB at N = 768, direction 0 280 MB at N = 256 and 1.50 GB at N = 768.
  */
 int b200_trimul_backward_workspace_bytes(int B, int N, int direction, size_t* out_bytes);
 int b200_trimul_backward_workspace_layout(int B, int N, int direction, size_t* offsets18);
@@ -379,7 +381,9 @@ int b200_trimul_read_status(const int* status, void* cuda_stream, int* host_stat
  * non-zero) and, in fp32 and the parameters' shapes, d_expand_a / d_expand_b [512, 128], d_squeeze [128, 512],
  * d_ln_w / d_ln_b [128]. Every output is overwritten. One launch per block of 128 hidden units (four), whose three
  * weight-gradient accumulators stay in tensor memory over all positions; x_hat, the scaled dy (both left by the first
- * launch) and the running d x_hat are carried between the launches in the workspace. Deterministic. Workspace: b200_transition_backward_workspace_bytes, 1024-byte aligned.
+ * launch) and the running d x_hat are carried between the launches in the workspace. Deterministic. Workspace:
+ * b200_transition_backward_workspace_bytes, 1024-byte aligned: 772 bytes per position (x_hat, scaled dy, running d x_hat,
+ * 1 / sigma) and 129 MB of partials (at most 160 CTAs); 243 MB at 384^2 positions, 584 MB at 768^2, 938 MB at 1024^2.
  */
 int b200_transition_backward_workspace_bytes(long long positions, size_t* out_bytes);
 int b200_transition_backward(const void* dy, const void* x, const void* w_expand_a, const void* w_expand_b,
