@@ -84,6 +84,19 @@ def _registered(module: nn.Module, names) -> Optional[list]:
     return out
 
 
+class _Scratch(nn.Module):
+    """A module whose scratch memory and pointer caches (``_scratch_names``) are its own: copies and pickles start without them,
+    whatever a pickle of an earlier version holds."""
+
+    _scratch_names = ()
+
+    def __getstate__(self):
+        return {**self.__dict__, **dict.fromkeys(self._scratch_names)}
+
+    def __setstate__(self, state):
+        super().__setstate__({**state, **dict.fromkeys(self._scratch_names)})
+
+
 class _Kept:
     """Scratch memory that a module keeps from one call to the next, as ``(stream, tensor)`` in its attribute ``name``.
 
@@ -132,7 +145,7 @@ _TRI_NAMES = [tuple(k.split(".")) for k in (
 _TRANSITION_NAMES = [tuple(k.split(".")) for k in F_.TRANSITION_KEYS]
 
 
-class TriangleMultiplication(nn.Module):
+class TriangleMultiplication(_Scratch):
     """Triangle multiplicative update on B200 kernels (forward and backward).
 
     ``forward(pair [B,N,N,d_pair] bf16, mask Bool[B,N] | None) -> pair + update`` (bf16).
@@ -142,6 +155,7 @@ class TriangleMultiplication(nn.Module):
     """
 
     _bidirectional = False
+    _scratch_names = ("_workspace", "_wcache")
 
     def __init__(
         self,
@@ -400,7 +414,7 @@ class BidirectionalTriangleMultiplication(TriangleMultiplication):
                          residual=residual, check_status=check_status)
 
 
-class Transition(nn.Module):
+class Transition(_Scratch):
     """Pair transition ``x + squeeze(SiLU(expand_a(LN x)) * expand_b(LN x))`` on the B200 kernels (forward and backward).
 
     Mirrors ``miniworld_engine.modules.Transition(d, n=4, implementation=...)`` as MiniWorld's blocks build it
@@ -408,6 +422,8 @@ class Transition(nn.Module):
     ``expand_a`` / ``expand_b`` [n d, d], ``squeeze`` [d, n d], all linears bias-free
     (``benchmarks/protenix_finetune/patch_engine.py:35-37``). d = 128 and n = 4 are what the kernel takes.
     """
+
+    _scratch_names = ("_scratch",)
 
     def __init__(self, d: int = D_SUPPORTED, n: int = 4, implementation=None, residual: bool = True, check_status: bool = False):
         super().__init__()

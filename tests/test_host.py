@@ -259,3 +259,22 @@ def test_symmetric_setup_failure_on_one_rank_does_not_split_the_ranks(explicit):
                 assert ret[rank] == ("raised", True), dict(ret)
             else:
                 assert ret[rank] == ("fallback", True, "nccl", "rows", 1), dict(ret)
+
+
+@pytest.mark.parametrize("make", [lambda: mw.TriangleMultiplication(128), lambda: mw.BidirectionalTriangleMultiplication(64), lambda: mw.Transition(128)])
+def test_copies_and_pickles_hold_no_scratch_memory(make):
+    """Two modules must not take the same scratch memory, and a pickle of an earlier version held it as a bare tensor."""
+    import copy
+    import pickle
+
+    m = make()
+    for name in m._scratch_names:
+        m.__dict__[name] = torch.zeros(64, dtype=torch.uint8)
+    old = dict(m.__dict__)
+    for other in (copy.copy(m), copy.deepcopy(m), pickle.loads(pickle.dumps(m))):
+        assert all(other.__dict__[name] is None for name in m._scratch_names)
+        assert all(torch.equal(a, b) for a, b in zip(m.state_dict().values(), other.state_dict().values()))
+    other = make()
+    other.__setstate__(old)
+    assert all(other.__dict__[name] is None for name in m._scratch_names)
+    assert all(isinstance(m.__dict__[name], torch.Tensor) for name in m._scratch_names)  # the module itself keeps its own
