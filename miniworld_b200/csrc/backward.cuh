@@ -287,13 +287,13 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
   // one poll, so that all warps walk through the same barriers to the end)
   if (warp == kBwdThreads / 32) {
     // ------------------------------------------------------------ MMAs
-    if (lane == 0) thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
+    if (elect_one()) thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
     __syncwarp();
     int it = 0;
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
       const uint32_t t_s = t_buf(it), z_s = t_s + kBwdTile, dy_s = y_buf(it), dg_s = dy_s + kBwdTile;
       named_bar_sync(kBarN, kTwo);
-      if (lane == 0) {
+      if (elect_one()) {
         // P = t_hat Wo'^T (columns 0-127), G = x_hat Wg'^T (columns 128-255); lanes = positions
         tc_fence_after();
         constexpr uint32_t idesc_p = umma_idesc(128, C, true, false, kFmtF16, kFmtF16);
@@ -312,7 +312,7 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
       }
       __syncwarp();
       named_bar_sync(kBarA, kTwo);
-      if (lane == 0) {
+      if (elect_one()) {
         // d t_hat = dproj Wo' (0-127), d x_hat = dgate Wg' (128-255; lanes = positions); Mo += dproj^T t_hat (256-383), Mg +=
         // dgate^T x_hat (384-511)
         tc_fence_after();
@@ -969,7 +969,7 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       }
       umma_commit(fwd_done);
     };
-    if (lane == 0) {
+    if (elect_one()) {
       thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
       issue_fwd(0);
     }
@@ -978,7 +978,7 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
       const uint32_t x_s = role(it, 0), dv_s = role(it, 2), dg_s = role(it, 3);
       named_bar_sync(kBarA, kCountA);  // dvalue and dgate are written, value / gate are read
-      if (lane == 0) {
+      if (elect_one()) {
         // d x_hat = dvalue Wv' + dgate Wg' (columns 0-127, lanes = positions); Mv += dvalue^T x_hat (256-383), Mg +=
         // dgate^T x_hat (384-511). dvalue / dgate are [channel][position] tiles: MN-major as the A operand of the first
         // pair of GEMMs (M = positions), K-major as that of the second (M = channels, K = positions).
@@ -1007,7 +1007,7 @@ bwd_prologue_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       }
       __syncwarp();
       named_bar_sync(kBarB, kCountB);  // d x_hat has left tensor memory
-      if (lane == 0 && tile + static_cast<int>(gridDim.x) < p.num_tiles) issue_fwd(it + 1);
+      if (elect_one() && tile + static_cast<int>(gridDim.x) < p.num_tiles) issue_fwd(it + 1);
       __syncwarp();
     }
   } else if (warp == kBwdThreads / 32 + 1) {

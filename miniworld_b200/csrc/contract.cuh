@@ -195,7 +195,7 @@ contract_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc(kBM, BN, A_MN, B_MN, kFmtF16, kFmtF16);
       int s = 0;
       uint32_t ph = 0;

@@ -160,7 +160,7 @@ contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = umma_idesc(256, BN, A_MN, B_MN, kFmtF16, kFmtF16);
       int s = 0;
       uint32_t ph = 0;

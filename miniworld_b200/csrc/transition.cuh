@@ -187,7 +187,7 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     // ------------------------------------------------------------ issuer of G1 (leader CTA only)
     // D1[gb & 1] = x_hat * [W_a ; W_b](block)^T, as soon as the weights are there and the SwiGLU group of that buffer
     // has taken its previous contents into registers.
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = umma_idesc(256, 128, false, false, kFmtF16, kFmtF16);
       const long long total = static_cast<long long>(my_tiles) * kTrBlocks;
       for (long long gb = 0; gb < total; ++gb) {
@@ -215,7 +215,7 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     // ------------------------------------------------------------ issuer of G2 (leader CTA only)
     // D2 += H[gb & 1] * W_s(block)^T once the SwiGLU warps of both CTAs have written h. G1 of the same block completed
     // before h could be computed, so one commit after G2 says that the block's weight stage and its H buffer are free.
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = umma_idesc(256, 128, false, false, kFmtF16, kFmtF16);
       const long long total = static_cast<long long>(my_tiles) * kTrBlocks;
       for (long long gb = 0; gb < total; ++gb) {

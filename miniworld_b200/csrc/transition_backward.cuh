@@ -93,7 +93,7 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
   // one poll, so that all warps walk through the same barriers to the end)
   if (warp == kBwdThreads / 32) {
     // ------------------------------------------------------------ MMAs
-    if (lane == 0) thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
+    if (elect_one()) thread_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
     __syncwarp();
     constexpr uint32_t idesc_kk = umma_idesc(128, 128, false, false, kFmtF16, kFmtF16);
     constexpr uint32_t idesc_mk = umma_idesc(128, 128, true, false, kFmtF16, kFmtF16);
@@ -108,7 +108,7 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       const uint32_t y_s = ring(it, 0), s1_s = ring(it, 1), s2_s = ring(it, 2);
       const uint32_t accum = it != 0 ? 1u : 0u;
       if constexpr (FIRST) named_bar_sync(kBarN, kTwo);
-      if (lane == 0) {
+      if (elect_one()) {
         // dh^T: A = Ws_j [c][hid] read MN-major, B = dy [pos][c]
         if constexpr (!FIRST) thread_wait(y_full, it & 1, abort_flag, p.status, kDevTimeoutMma);
         tc_fence_after();
@@ -118,7 +118,7 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       }
       __syncwarp();
       named_bar_sync(kBarR1, kOne);
-      if (lane == 0) {
+      if (elect_one()) {
         if constexpr (!FIRST) thread_wait(x_full, it & 1, abort_flag, p.status, kDevTimeoutMma);
         tc_fence_after();
 #pragma unroll
@@ -127,7 +127,7 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       }
       __syncwarp();
       named_bar_sync(kBarR2, kOne);
-      if (lane == 0) {
+      if (elect_one()) {
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) umma_bf16(tmem_base, kmaj(wb_s, ks), kmaj(x_s, ks), idesc_kk, ks != 0 ? 1u : 0u);
@@ -135,7 +135,7 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       }
       __syncwarp();
       named_bar_sync(kBarA, kOne);
-      if (lane == 0) {
+      if (elect_one()) {
         // d x_hat (columns 0-127, lanes = positions), Ma (128-255), Mb (256-383; lanes = hidden units)
         tc_fence_after();
 #pragma unroll
@@ -153,7 +153,7 @@ bwd_transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       }
       __syncwarp();
       named_bar_sync(kBarH, kOne);
-      if (lane == 0) {
+      if (elect_one()) {
         // dWs (384-511, lanes = channels c, columns = hidden units): A = dy read MN-major, B = h [hid][pos]
         tc_fence_after();
 #pragma unroll
