@@ -15,28 +15,37 @@
 // positions, which is exactly the row-plane layout [B, rows, H, N] of the outputs (written as fp16; masked
 // cells are exactly zero).
 //
-// The two CTAs of a pair split the OUTPUTS: CTA 0 produces `left`, CTA 1 produces `right`, each holding only
-// its own two matrices (64 KiB), which leaves room for five input stages and two staging buffers. Every MMA
-// spans both CTAs (M = 256: rows 0-127 are CTA 0's matrix, rows 128-255 CTA 1's matrix at the same
-// shared-memory offset; N = 128 positions, of which each CTA loads and normalises 64). So per tile each CTA
-//   * loads and LayerNorms 64 positions,
-//   * receives proj / gate accumulators of ITS output for all 128 positions in its own TMEM (2 x 128 columns,
-//     double-buffered: the MMAs of tile t+1 overlap the epilogue of tile t),
-//   * gates, masks and stores 128 channels x 128 positions of its output.
+// The two CTAs of a pair split the OUTPUTS: CTA 0 produces `left`, CTA 1 `right`, each holding only its own two matrices.
+// These stay in TENSOR MEMORY as the A operand of every MMA (128 columns), so the tensor cores read nothing but the
+// normalised tile from shared memory, which eight input stages and four staging buffers share. A tile is processed as two
+// halves of 64 positions, because the other 384 columns hold three accumulator buffers of a half (value and gate, 64 columns
+// each) but not two of a whole tile. Every MMA spans both CTAs (M = 256: rows 0-127 CTA 0's matrix, rows 128-255 CTA 1's;
+// N = 64 positions, of which each CTA loads and normalises 32). So per half tile each CTA
+//   * loads and LayerNorms 32 positions,
+//   * receives proj / gate accumulators of ITS output for all 64 positions in its own TMEM (the MMAs of the next halves
+//     overlap the epilogue of this one),
+//   * gates, masks and stores 128 channels x 64 positions of its output.
 // Only mbarrier signals cross between the CTAs (statistics-done and accumulator-free arrive on the leader's
 // barriers; the leader's MMA commits release both CTAs' barriers); no tile is broadcast. A single-CTA version
 // of this kernel (all four matrices resident, two input stages) measured 3 % slower at N = 768.
+//
+// What bounds it: per SM the tensor pipe and the MUFU (tanh) are busy for half of the time each, 60 % of the issue slots and
+// 0.75 of the copy rate of HBM are used; the stages of the pipeline take turns at these. With the matrices in shared memory
+// (128-position tiles, two accumulator buffers, five input stages) the MMAs' operand reads held up the other roles: leaving
+// out most MMAs gained 18 us of 95. Now 94.8 -> 91.4 us at N = 768, 28.3 -> 27.4 at N = 384, 84.3 -> 81.2 for 8 x 256 in
+// short runs (whole forwards 1 %; at N = 768 in sustained calls, which run at the power limit, no change). The 64-column
+// MMAs pay only because their issuer runs on an elected lane (113 us otherwise).
 //
 // Outputs leave through a swizzled shared-memory staging tile and TMA stores (full 128-byte rows);
 // direct per-thread 16-byte stores to 128 different channel rows ran the store path at a third of this.
 //
 // Warp roles (864 threads per CTA):
-//   warp 0        TMA producer (input tiles, this CTA's weights once)
+//   warp 0        TMA producer (input tiles)
 //   warp 1        MMA issuer (leader CTA) / TMEM owner
 //   warps 2-9     LayerNorm: 8 threads per position (16 channels each, their gamma / beta in registers), two
 //                 passes of 32 positions computed as independent chains; normalises the tile in place.
-//   warps 10-25   epilogue: two groups of eight warps on alternate tiles (one thread per channel x 64 positions:
-//                 TMEM -> tanh gate -> mask -> staging -> TMA store)
+//   warps 10-25   epilogue: four groups of four warps take half tiles in turn (one thread per channel x 64 positions:
+//                 TMEM -> tanh gate -> mask -> staging -> TMA store); at the start they bring the weights to TMEM
 //   warp 26       validity bitmap of the tile
 #pragma once
 
@@ -53,6 +62,7 @@ struct PrologueParams {
   int num_tiles;       // B * rows * tiles_per_row
   const uint8_t* token_mask;  // [B, N] non-zero = valid, or null
   const uint8_t* pair_mask;   // [B, rows, N] non-zero = valid, or null
+  const uint4* w;             // [4][128][C] fp16 packed matrices: left, left gate, right, right gate
   const float* d1;            // [4][128] additive constants (0.5 * bias): left, left gate, right, right gate
   const float* ln_w;          // [128] LayerNorm gamma
   const float* ln_b;          // [128] LayerNorm beta
@@ -82,44 +92,44 @@ struct OutputMaps {
 };
 
 constexpr int kProThreads = 864;
-constexpr int kProStages = 5;
-constexpr int kProRing = 8;              // mask ring entries (>= stages + 3)
-constexpr int kProRingBytes = 272;       // 64 pair-mask words + 4 ballots
-constexpr int kProStageOutBytes = 2 * 32768;  // two staging buffers of [128 channels][128 positions]
-constexpr int kProBarBytes = 256;
+constexpr int kProStages = 8;
+constexpr int kProRing = kProStages + 4;  // mask ring entries: the input may run so many tiles ahead of an epilogue group
+constexpr int kProRingBytes = 272;        // 64 pair-mask words + 4 ballots
+constexpr int kProStageOutBytes = 4 * 16384;  // per epilogue group a staging buffer of [128 channels][64 positions]
+constexpr int kProBarBytes = 320;
+constexpr int kProAccs = 3;       // accumulator buffers (of a 64-position half tile: value and gate, 64 columns each)
+constexpr int kProGroups = 4;     // epilogue groups
+constexpr int kProAccBase = 128;  // tensor-memory column of the first one, behind the two weight matrices
 // C = d_pair, the channels of the input tensor (128, or 64 for the narrow pair stacks); the outputs always have 128
 // channels. The shared-memory budget is that of C = 128 for both.
-constexpr int kProSmemBytes =
-    2 * 32768 + kProStages * 16384 + kProStageOutBytes + kProRing * kProRingBytes + kProBarBytes + 1024;
+constexpr int kProSmemBytes = kProStages * 16384 + kProStageOutBytes + kProRing * kProRingBytes + kProBarBytes + 1024;
 
 template <bool HAS_BIAS, int C = 128>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProThreads, 1)
-prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_w,
-                const __grid_constant__ OutputMaps out, const PrologueParams p) {
+prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ OutputMaps out, const PrologueParams p) {
   static_assert(C == 128 || C == 64, "d_pair is 128 or 64");
   constexpr int S = kProStages;
   constexpr int kHalves = C / 64;              // 64-channel (128-byte) halves of an input row
-  constexpr int kProWBytes = 2 * 128 * C * 2;  // this CTA's proj and gate matrices, [128, C] fp16 each
   constexpr int kProZBytes = 64 * C * 2;       // 64 positions x C channels, 16-bit
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t w_base = smem_base;
-  const uint32_t z_base = smem_base + kProWBytes;
+  const uint32_t z_base = smem_base;
   const uint32_t stage_out_base = z_base + S * kProZBytes;
   const uint32_t ring_base = stage_out_base + kProStageOutBytes;
   const uint32_t bar_base = ring_base + kProRing * kProRingBytes;
-  uint32_t* ring_ptr = reinterpret_cast<uint32_t*>(smem + kProWBytes + S * kProZBytes + kProStageOutBytes);
-  // barriers: w_full (leader), z_full[S] (own), xn_ready[S] (leader), z_empty[S] (both), acc_full[2] (both),
-  // acc_empty[2] (leader)
+  uint32_t* ring_ptr = reinterpret_cast<uint32_t*>(smem + S * kProZBytes + kProStageOutBytes);
+  // barriers: w_full (leader), z_full[S] (own), xn_ready[S] (leader), z_empty[S] (both), acc_full[4] (both, one per
+  // epilogue group, which so sees every phase of its barrier), acc_empty[3] (leader)
   const uint32_t w_full = bar_base;
   auto z_full = [&](int s) { return bar_base + 8u * (1 + s); };
   auto xn_ready = [&](int s) { return bar_base + 8u * (1 + S + s); };
   auto z_empty = [&](int s) { return bar_base + 8u * (1 + 2 * S + s); };
-  auto acc_full = [&](int a) { return bar_base + 8u * (1 + 3 * S + a); };
-  auto acc_empty = [&](int a) { return bar_base + 8u * (1 + 3 * S + 2 + a); };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kProWBytes + S * kProZBytes + kProStageOutBytes +
-                                                    kProRing * kProRingBytes + 8 * (1 + 3 * S + 4));
+  auto acc_full = [&](int g) { return bar_base + 8u * (1 + 3 * S + g); };
+  auto acc_empty = [&](int a) { return bar_base + 8u * (1 + 3 * S + kProGroups + a); };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + S * kProZBytes + kProStageOutBytes +
+                                                    kProRing * kProRingBytes + 8 * (1 + 3 * S + kProGroups + kProAccs));
+  static_assert(8 * (1 + 3 * S + kProGroups + kProAccs) + 8 <= kProBarBytes, "barriers");
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -129,20 +139,17 @@ prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant
   const int num_pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
-    mbar_init(w_full, 1);
+    mbar_init(w_full, 32);  // the sixteen epilogue warps of each CTA
     for (int s = 0; s < S; ++s) {
       mbar_init(z_full(s), 1);
       mbar_init(xn_ready(s), 18);  // eight LayerNorm warps and the mask warp of each CTA
       mbar_init(z_empty(s), 1);
     }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(acc_full(a), 1);
-      mbar_init(acc_empty(a), 16);  // the eight warps of epilogue group a in each CTA
-    }
+    for (int g = 0; g < kProGroups; ++g) mbar_init(acc_full(g), 1);
+    for (int a = 0; a < kProAccs; ++a) mbar_init(acc_empty(a), 8);  // the four warps of an epilogue group in each CTA
     *abort_flag = 0;
     fence_mbar_init();
     prefetch_tmap(&map_z);
-    prefetch_tmap(&map_w);
     prefetch_tmap(&out.left[0]);
     prefetch_tmap(&out.right[0]);
   }
@@ -161,42 +168,27 @@ prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
     if (lane == 0) {
-      // this CTA's two matrices: packed order is left, left gate, right, right gate
-      if (rank == 0) mbar_arrive_expect_tx(w_full, 2 * kProWBytes);  // bytes of both CTAs
-      const uint32_t lead_w = map_to_cta(w_full, 0);
-#pragma unroll
-      for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int kh = 0; kh < kHalves; ++kh)
-          tma_load_2d_pair(w_base + m * (kProWBytes / 2) + kh * 16384, &map_w, lead_w, kh * 64,
-                           (static_cast<int>(rank) * 2 + m) * 128);
       int s = 0;
       uint32_t ph = 0;
       int issued = 0;
       for (int tile = pair; tile < p.num_tiles; tile += num_pairs) {
         if (!mbar_wait(z_empty(s), ph ^ 1u, abort_flag, p.status, kDevTimeoutProducer)) break;
         const int row = tile / p.tiles_per_row;
-        const int j0 = (tile - row * p.tiles_per_row) * 128 + static_cast<int>(rank) * 64;  // this CTA's 64 positions
+        // this CTA's 64 positions: of each 64-position half of the tile the 32 that are its rows of the B operand
+        const int j0 = (tile - row * p.tiles_per_row) * 128 + static_cast<int>(rank) * 32;
         mbar_arrive_expect_tx(z_full(s), kProZBytes);
 #pragma unroll
-        for (int kh = 0; kh < kHalves; ++kh) tma_load_3d(z_base + s * kProZBytes + kh * 8192, &map_z, z_full(s), kh * 64, j0, row);
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int kh = 0; kh < kHalves; ++kh)
+            tma_load_3d(z_base + s * kProZBytes + kh * 8192 + u * 4096, &map_z, z_full(s), kh * 64, j0 + u * 64, row);
         ++issued;
         if (++s == S) {
           s = 0;
           ph ^= 1u;
         }
       }
-      // Drain every copy this thread started before the CTA may exit (the weights report to the leader, whose
-      // MMA thread waits for them; the closing cluster barrier keeps this CTA alive until then).
-      if (rank == 0) {
-        const long long t0 = clock64();
-        while (!mbar_try_wait(w_full, 0)) {
-          if (clock64() - t0 > kWaitLimitCycles) {
-            atomicCAS(p.status, 0, kDevTimeoutDrain);
-            break;
-          }
-        }
-      }
+      // Drain every copy this thread started before the CTA may exit.
       const int pending = issued < S ? issued : S;
       for (int q = 0; q < pending; ++q) {
         if (s == 0) {
@@ -215,30 +207,39 @@ prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
-      constexpr uint32_t idesc = umma_idesc(256, 128, false, false, kFmtF16, kFmtF16);
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t idesc = umma_idesc(256, 64, false, false, kFmtF16, kFmtF16);
       bool ok = mbar_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);
       int s = 0;
       uint32_t ph = 0;
-      int it = 0;
-      for (int tile = pair; ok && tile < p.num_tiles; tile += num_pairs, ++it) {
-        const int buf = it & 1;
+      int a = 0;  // accumulator buffer of the next half tile
+      uint32_t aph = 1u;
+      int g = 0;  // its epilogue group: 0, 2 before its tile's two halves
+      for (int tile = pair; ok && tile < p.num_tiles; tile += num_pairs, g ^= 2) {
         if (!mbar_wait(xn_ready(s), ph, abort_flag, p.status, kDevTimeoutMma)) break;
-        if (!mbar_wait(acc_empty(buf), ((it >> 1) & 1) ^ 1u, abort_flag, p.status, kDevTimeoutMma)) break;
-        tc_fence_after();
-        const uint32_t zs = z_base + s * kProZBytes;
+        const uint64_t db0 = umma_desc_kmajor(z_base + s * kProZBytes);
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-          const uint32_t d_tmem = tmem_base + buf * 256 + m * 128;
-          const uint32_t wm = w_base + m * (kProWBytes / 2);
+        for (int u = 0; u < 2; ++u) {
+          ok = mbar_wait(acc_empty(a), aph, abort_flag, p.status, kDevTimeoutMma);
+          if (!ok) break;
+          tc_fence_after();
 #pragma unroll
-          for (int ks = 0; ks < C / 16; ++ks) {
-            const uint64_t da = umma_desc_kmajor(wm + (ks >> 2) * 16384) + static_cast<uint64_t>((ks & 3) * 2);
-            const uint64_t db = umma_desc_kmajor(zs + (ks >> 2) * 8192) + static_cast<uint64_t>((ks & 3) * 2);
-            umma_pair(d_tmem, da, db, idesc, ks != 0 ? 1u : 0u);
+          for (int m = 0; m < 2; ++m) {
+            const uint32_t d_tmem = tmem_base + kProAccBase + a * 128 + m * 64;
+            const uint32_t wm = tmem_base + m * (C / 2);
+#pragma unroll
+            for (int ks = 0; ks < C / 16; ++ks) {
+              const uint64_t db = db0 + static_cast<uint64_t>((ks >> 2) * 512 + u * 256 + (ks & 3) * 2);
+              umma_pair_ta(d_tmem, wm + ks * 8, db, idesc, ks != 0 ? 1u : 0u);
+            }
+          }
+          umma_commit_pair(acc_full(g + u));
+          if (++a == kProAccs) {
+            a = 0;
+            aph ^= 1u;
           }
         }
-        umma_commit_pair(acc_full(buf));
+        if (!ok) break;
         umma_commit_pair(z_empty(s));
         if (++s == S) {
           s = 0;

@@ -618,13 +618,13 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
   rc = device_info(&info);
   if (rc != B200_TRIMUL_OK) return rc;
 
-  CUtensorMap map_z, map_w;
+  CUtensorMap map_z;
   OutputMaps out;
   {
     const uint64_t dp = static_cast<uint64_t>(d_pair);
     const uint64_t dims[3] = {dp, static_cast<uint64_t>(N), static_cast<uint64_t>(B) * rows};
     const uint64_t strides[2] = {dp * 2ull, static_cast<uint64_t>(N) * dp * 2ull};
-    const uint32_t box[3] = {64, 64, 1};  // each CTA of a pair loads 64 of a tile's 128 positions
+    const uint32_t box[3] = {64, 32, 1};  // each CTA of a pair loads 32 of the positions of each half tile
     rc = make_map(&map_z, z, 3, dims, strides, box);
     if (rc != B200_TRIMUL_OK) return rc;
   }
@@ -664,14 +664,6 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
       out.warp_store = 1;
     }
   }
-  {
-    // the four left / right matrices [128, d_pair], one after the other at the start of the packed block
-    const uint64_t dims[2] = {static_cast<uint64_t>(d_pair), 4ull * 128};
-    const uint64_t strides[1] = {static_cast<uint64_t>(d_pair) * 2ull};
-    const uint32_t box[2] = {64, 128};
-    rc = make_map(&map_w, packed, 2, dims, strides, box);
-    if (rc != B200_TRIMUL_OK) return rc;
-  }
   PrologueParams p;
   p.batch = B;
   p.rows = rows;
@@ -681,6 +673,7 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
   p.num_tiles = B * rows * p.tiles_per_row;
   p.token_mask = token_mask;
   p.pair_mask = pair_mask;
+  p.w = static_cast<const uint4*>(packed);  // the four left / right matrices, one after the other
   p.d1 = reinterpret_cast<const float*>(static_cast<const uint8_t*>(packed) + kPackedD1Off);
   p.ln_w = reinterpret_cast<const float*>(static_cast<const uint8_t*>(packed) + kPackedLnOff);
   p.ln_b = p.ln_w + 128;
@@ -693,7 +686,7 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
   do {                                                                                               \
     rc = set_smem(prologue_kernel<BIAS, DP>, kProSmemBytes, info.device);                            \
     if (rc != B200_TRIMUL_OK) return rc;                                                             \
-    TRIMUL_CUDA(launch_overlapped(prologue_kernel<BIAS, DP>, grid, kProThreads, kProSmemBytes, stream, map_z, map_w, out, p)); \
+    TRIMUL_CUDA(launch_overlapped(prologue_kernel<BIAS, DP>, grid, kProThreads, kProSmemBytes, stream, map_z, out, p)); \
   } while (0)
   if (d_pair == kC) {
     if (has_bias) TRIMUL_LAUNCH_PROLOGUE(true, 128);
