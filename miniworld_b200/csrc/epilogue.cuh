@@ -34,6 +34,7 @@ struct EpilogueParams {
   float eps_in;
   float eps_out;
   int residual;
+  int early;  // z and the packed weights are older than the kernel before this one
   int* status;
 };
 
@@ -102,8 +103,7 @@ epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant
     prefetch_tmap(&map_wo);
     prefetch_tmap(&map_wg);
   }
-  grid_dependency_wait();
-  grid_dependents_launch();
+  if (!p.early) grid_dependency_wait();
   if (threadIdx.x >= 64 && threadIdx.x < 64 + C / 2) {
     // constants regrouped per channel pair so that one 16-byte load feeds a packed fp32x2 FMA
     const int cp = threadIdx.x - 64;
@@ -120,6 +120,11 @@ epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // (the weights and the first two z tiles land while the contraction ends)
+  if (warp != 0) {
+    grid_dependency_wait();
+    grid_dependents_launch();
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -131,13 +136,26 @@ epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant
 #pragma unroll
       for (int kh = 0; kh < kZHalves; ++kh) tma_load_2d(wg_base + kh * kWoHalf, &map_wg, w_full, kh * 64, 0);
       int it = 0, t_issued = 0, z_issued = 0;
+      auto issue_z = [&](int s, int row, int j0) {
+        mbar_arrive_expect_tx(z_full(s), kZHalves * 16384);
+#pragma unroll
+        for (int kh = 0; kh < kZHalves; ++kh)
+          tma_load_3d(stage_base + s * kEpiStageBytes + 32768 + kh * 16384, &map_z, z_full(s), kh * 64, j0, row);
+        ++z_issued;
+      };
+      if (p.early) {
+        for (int tile = blockIdx.x; tile < p.num_tiles && z_issued < 2; tile += gridDim.x) {
+          const int row = tile / p.tiles_per_row;
+          issue_z(z_issued, row, (tile - row * p.tiles_per_row) * 128);
+        }
+        grid_dependency_wait();
+      }
       for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++it) {
         const int s = it & 1;
         const uint32_t ph = (it >> 1) & 1;
         const int row = tile / p.tiles_per_row;
         const int j0 = (tile - row * p.tiles_per_row) * 128;
         const uint32_t ts = stage_base + s * kEpiStageBytes;
-        const uint32_t zs = ts + 32768;
         if (!mbar_wait(t_empty(s), ph ^ 1u, abort_flag, p.status, kDevTimeoutProducer)) break;
         mbar_arrive_expect_tx(t_full(s), 32768);
         // 4-d map (column, channel in group, channel group, row): one group of 128 channels on one GPU, 128/P
@@ -145,11 +163,9 @@ epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant
         tma_load_4d(ts, &map_t, t_full(s), j0, 0, 0, row);
         tma_load_4d(ts + 16384, &map_t, t_full(s), j0 + 64, 0, 0, row);
         ++t_issued;
+        if (z_issued > it) continue;
         if (!mbar_wait(z_empty(s), ph ^ 1u, abort_flag, p.status, kDevTimeoutProducer)) break;
-        mbar_arrive_expect_tx(z_full(s), kZHalves * 16384);
-#pragma unroll
-        for (int kh = 0; kh < kZHalves; ++kh) tma_load_3d(zs + kh * 16384, &map_z, z_full(s), kh * 64, j0, row);
-        ++z_issued;
+        issue_z(s, row, j0);
       }
       // Drain every copy this thread started before the CTA may exit.
       {

@@ -38,6 +38,7 @@ struct EpilogueWideParams {
   float eps_in;
   float eps_out;
   int residual;
+  int early;  // z, the packed weights and the dropout scale are older than the kernel before this one
   int* status;
 };
 
@@ -109,8 +110,7 @@ epilogue_wide_kernel(const __grid_constant__ CUtensorMap map_t0, const __grid_co
     prefetch_tmap(&map_w0);
     prefetch_tmap(&map_w1);
   }
-  grid_dependency_wait();
-  grid_dependents_launch();
+  if (!p.early) grid_dependency_wait();
   if (threadIdx.x >= 64 && threadIdx.x < 128) {
     // constants regrouped per channel pair so that one 16-byte load feeds a packed fp32x2 FMA
     const int cp = threadIdx.x - 64;
@@ -132,6 +132,11 @@ epilogue_wide_kernel(const __grid_constant__ CUtensorMap map_t0, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // (the weights and the first two z tiles land while the contraction ends)
+  if (warp != 0 && warp < 18) {
+    grid_dependency_wait();
+    grid_dependents_launch();
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------ weights and chunks of t
@@ -146,6 +151,7 @@ epilogue_wide_kernel(const __grid_constant__ CUtensorMap map_t0, const __grid_co
 #pragma unroll
         for (int kh = 0; kh < 2; ++kh) tma_load_2d(wo1_base + kh * 16384, &map_w1, w_full, kh * 64, 4 * 128);
       }
+      grid_dependency_wait();
       int it = 0;
       long long t_issued = 0;
       uint32_t full_par = 0;  // parity of the next use of t_full(g, slot), bit g * R + slot
@@ -263,6 +269,7 @@ epilogue_wide_kernel(const __grid_constant__ CUtensorMap map_t0, const __grid_co
     const int first = static_cast<int>(blockIdx.x) + grp * static_cast<int>(gridDim.x);
     if (lane == 0 && first < p.num_tiles) issue_z(first);
     __syncwarp();
+    grid_dependency_wait();
     for (int tile = first; tile < p.num_tiles; tile += step) {
       named_bar_sync(4 + grp, 288);  // the group has written its y tile
       if (lane == 0 && *abort_flag == 0) {

@@ -67,6 +67,7 @@ struct PrologueParams {
   const float* ln_w;          // [128] LayerNorm gamma
   const float* ln_b;          // [128] LayerNorm beta
   float eps;
+  int early;  // z is older than the kernel before this one
   int* status;
 };
 
@@ -157,12 +158,15 @@ prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant
     tmem_alloc_pair(smem_u32(tmem_slot), 512);
     tmem_relinquish_pair();
   }
-  grid_dependency_wait();
-  grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // barriers of both CTAs are initialised before any signal crosses
   tc_fence_after();
+  // (the first z tiles land while the packing of the weights ends)
+  if (warp != 0 || !p.early) {
+    grid_dependency_wait();
+    grid_dependents_launch();
+  }
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {

@@ -140,6 +140,11 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
 // The first kernel of an entry point may follow any kernel of the caller, the entry point's own last one with its output as
 // this one's input among them. Memory written earlier is safe: the predecessor has itself waited before it let this kernel begin.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A kernel whose launch says that some inputs are older than the kernel before it (`early`: what a module call was given, and
+// what its launches before that one wrote) reads those while that kernel finishes; the threads that read anything else, and
+// all that write, still wait.
+// (N = 203: 40.3 -> 39.0 us, N = 384: 90.6 -> 89.4, bidirectional N = 512: 265.7 -> 264.9, with dropout in training N = 256:
+// 387 -> 380; the prologue's input lands while the weights are packed, the epilogues' weights and z while the contraction ends.)
 // `CHUNKS` 16-byte pieces (an even count) from p at gpu scope, which no line in L1 answers: 32-byte requests if the address allows
 template <int CHUNKS>
 __device__ __forceinline__ void ld_gpu_chunks(const uint4* p, bool wide, uint4 (&out)[CHUNKS]) {

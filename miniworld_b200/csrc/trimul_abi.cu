@@ -604,7 +604,7 @@ enum PrologueMode { kLocal, kGatherRight, kChannels };
 static int prologue_impl(const void* z, const void* packed, const uint8_t* token_mask, const uint8_t* pair_mask,
                          void* const* left_dst, int n_left, void* const* right_dst, int n_right, PrologueMode mode,
                          int B, int N, int row_begin, int rows, float eps_in, int has_bias, int* status,
-                         void* cuda_stream, int d_pair = kC, bool any_n = false) {
+                         void* cuda_stream, int d_pair = kC, bool any_n = false, bool early = false) {
   if (d_pair != kC && d_pair != 64) return B200_TRIMUL_E_UNSUPPORTED;
   if (!z || !packed || !left_dst || !right_dst || !status) return B200_TRIMUL_E_NULL;
   if (n_left < 1 || n_left > kMaxDst || n_right < 1 || n_right > kMaxDst) return B200_TRIMUL_E_SHAPE;
@@ -678,6 +678,7 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
   p.ln_w = reinterpret_cast<const float*>(static_cast<const uint8_t*>(packed) + kPackedLnOff);
   p.ln_b = p.ln_w + 128;
   p.eps = eps_in;
+  p.early = early ? 1 : 0;
   p.status = status;
   const int pairs = p.num_tiles < info.sms / 2 ? p.num_tiles : info.sms / 2;
   const int grid = 2 * pairs;  // clusters of two CTAs: CTA 0 produces `left`, CTA 1 `right`
@@ -940,7 +941,7 @@ int b200_trimul_reduce_partials(void* tri, const void* const* partials, int n_sr
 // in slab g (what the channel-sharded contraction of GPU g stored there).
 static int epilogue_impl(const void* tri, const void* z, const void* packed, void* y, int B, int N, int rows, int groups,
                          float eps_in, float eps_out, int residual, int* status, void* cuda_stream, int d_pair = kC,
-                         bool any_n = false) {
+                         bool any_n = false, bool early = false) {
   if (!tri || !z || !packed || !y || !status) return B200_TRIMUL_E_NULL;
   if (d_pair != kC && d_pair != 64) return B200_TRIMUL_E_UNSUPPORTED;
   if (groups < 1 || groups > 8 || kC % groups != 0 || (groups > 1 && B != 1)) return B200_TRIMUL_E_SHAPE;
@@ -994,6 +995,7 @@ static int epilogue_impl(const void* tri, const void* z, const void* packed, voi
   p.eps_in = eps_in;
   p.eps_out = eps_out * (kTriScale * kTriScale);  // tri arrives scaled by kTriScale
   p.residual = residual;
+  p.early = early ? 1 : 0;
   p.status = status;
   const int grid = p.num_tiles < info.sms ? p.num_tiles : info.sms;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
@@ -1040,7 +1042,8 @@ extern "C" {
 
 static int epilogue_wide_impl(const void* tri, const void* tri_in, const void* z, const void* packed,
                               const void* packed_in, const void* drop_scale, void* y, int B, int N, int rows,
-                              float eps_in, float eps_out, int residual, int* status, void* cuda_stream, bool any_n) {
+                              float eps_in, float eps_out, int residual, int* status, void* cuda_stream, bool any_n,
+                              bool early = false) {
   if (!tri || !z || !packed || !y || !status) return B200_TRIMUL_E_NULL;
   const bool bidir = tri_in != nullptr;
   if (bidir && !packed_in) return B200_TRIMUL_E_NULL;
@@ -1095,6 +1098,7 @@ static int epilogue_wide_impl(const void* tri, const void* tri_in, const void* z
   p.eps_in = eps_in;
   p.eps_out = eps_out * (kTriScale * kTriScale);  // tri arrives scaled by kTriScale
   p.residual = residual;
+  p.early = early ? 1 : 0;
   p.status = status;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   if (bidir) {
@@ -1143,7 +1147,7 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
     void* l[1] = {left};
     void* r[1] = {right};
     return prologue_impl(z, pk, token_mask, pair_mask, l, 1, r, 1, kLocal, B, N, 0, N, eps_in, has_bias, status, cuda_stream,
-                         d_pair, any_n);
+                         d_pair, any_n, true);
   };
   auto contract = [&](void* dst, int dir) {
     return contract_impl(left, right, dst, nullptr, 0, 0, kC, B, N, 0, N, N, dir, status, cuda_stream, 0, any_n);
@@ -1171,7 +1175,7 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
       rc = contract(tri, direction);
     }
     if (rc != B200_TRIMUL_OK) return rc;
-    return epilogue_impl(tri, z, packed, y, B, N, N, 1, eps_in, eps_out, residual, status, cuda_stream, 64, any_n);
+    return epilogue_impl(tri, z, packed, y, B, N, N, 1, eps_in, eps_out, residual, status, cuda_stream, 64, any_n, true);
   }
   if (direction == B200_TRIMUL_BIDIRECTIONAL) {
     // workspace tail: second tri tensor, then the second packed block
@@ -1190,7 +1194,7 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
     rc = contract(tri_in, B200_TRIMUL_INCOMING);
     if (rc != B200_TRIMUL_OK) return rc;
     return epilogue_wide_impl(tri, tri_in, z, packed, packed_in, drop_scale, y, B, N, N, eps_in, eps_out, residual,
-                                     status, cuda_stream, any_n);
+                                     status, cuda_stream, any_n, true);
   }
   rc = pack_one(w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w,
                                 ln_in_b, ln_out_w, ln_out_b, bias_opt, packed, kC, status, cuda_stream);
@@ -1201,8 +1205,8 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
   if (rc != B200_TRIMUL_OK) return rc;
   if (drop_scale != nullptr)
     return epilogue_wide_impl(tri, nullptr, z, packed, nullptr, drop_scale, y, B, N, N, eps_in, eps_out, residual,
-                                     status, cuda_stream, any_n);
-  return epilogue_impl(tri, z, packed, y, B, N, N, 1, eps_in, eps_out, residual, status, cuda_stream, kC, any_n);
+                                     status, cuda_stream, any_n, true);
+  return epilogue_impl(tri, z, packed, y, B, N, N, 1, eps_in, eps_out, residual, status, cuda_stream, kC, any_n, true);
 }
 
 int b200_trimul_forward_ex(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
