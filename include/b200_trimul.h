@@ -73,11 +73,11 @@ const char* b200_trimul_strerror(int code);
 /* Last cudaError_t seen by this thread inside the library (0 if none). */
 int b200_trimul_last_cuda_error(void);
 
-/* Bytes of workspace needed by b200_trimul_forward for a full (unsharded) call. */
+/* Bytes of workspace that serve a full (unsharded) call of any of the forward entry points below. */
 int b200_trimul_workspace_bytes(int B, int N, int d_pair, int d_hidden, int direction, size_t* out_bytes);
 
-/* Offsets (bytes) of the regions inside a workspace: [0] status words, [1] packed weights,
- * [2] left, [3] right, [4] tri. For tests and profilers that want to look at the stages. */
+/* Offsets (bytes) of the regions inside a workspace of b200_trimul_forward / _forward_ex: [0] status words, [1] packed
+ * weights, [2] left, [3] right, [4] tri (dense). For tests and profilers that want to look at the stages. */
 int b200_trimul_workspace_layout(int B, int N, size_t out_offsets[5]);
 
 /* Bytes of the packed-weight block written by b200_trimul_pack_weights. */
@@ -245,7 +245,8 @@ int b200_trimul_forward_ex(const void* z, const void* w_left, const void* w_left
 
 /*
  * b200_trimul_forward_ex for every N >= 1. Nothing is padded: z, y, the masks and drop_scale are dense with N columns,
- * only the intermediates in the workspace have their columns N rounded up to a multiple of 8 apart. Workspace:
+ * only the intermediates in the workspace have their channels N rounded up to a multiple of 64 columns apart (rows of
+ * whole 128-byte lines; the faster form wherever N is not a multiple of 64). Workspace:
  * b200_trimul_workspace_bytes of N rounded up to a multiple of 8. A workspace this call leaves behind is read by
  * b200_trimul_backward_any with the same N.
  */
@@ -323,7 +324,7 @@ int b200_trimul_forward_static(const void* z, const void* w_left, const void* w_
  * prologue once more (left / right of the first half, which the forward overwrote), four contraction gradient launches,
  * the prologue's backward four times (side x half).
  * The result is deterministic (fixed summation order). Workspace: b200_trimul_backward_workspace_bytes, 1024-byte
- * aligned; _layout gives its 17 region offsets + the total (status, packed weights, scale, LayerNorm terms, x_hat and
+ * aligned, which serves this call and b200_trimul_backward_any; _layout gives this call's 17 region offsets + the end (status, packed weights, scale, LayerNorm terms, x_hat and
  * 1 / sigma, per-CTA partials of M and S of every launch, dtri, dleft, dright, d x_hat, then the bidirectional module's extra
  * regions) for tests. About five pair tensors of 128 16-bit channels (nine for direction 0) and 63 MB of partials (126 MB, at
  * most 160 CTAs): one direction 253 MB at N = 384 and 821 MB at N = 768, direction 0 280 MB at N = 256 and 1.50 GB at N = 768.

@@ -758,12 +758,13 @@ bwd_epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_cons
 }
 
 // Mean and rstd of the stored t over the 256 channels of two tensors [rows][128][N] (fp16): stats[row][j] = {mean,
-// rsqrt(var + eps)} (eps already scaled like the stored t). The sums of a column are one chain over its 256 channels in
+// rsqrt(var + eps)} (eps already scaled like the stored t; `n` columns per row of statistics, channels `pitch` 16-byte pieces
+// apart in t). The sums of a column are one chain over its 256 channels in
 // order. A block brings eight groups of eight columns into shared memory (128 bytes per channel, all loads in flight at once);
 // then one warp walks the channels, a lane two columns. (One thread per group of eight columns that loaded as it went left
 // the chip idle at small N: 8192 threads at N = 256, 29 us for 34 MB.)
 constexpr int kLnStatsGroups = 8;
-__global__ void __launch_bounds__(256) bwd_ln_stats_kernel(const uint4* t0, const uint4* t1, int n, long long groups, float eps,
+__global__ void __launch_bounds__(256) bwd_ln_stats_kernel(const uint4* t0, const uint4* t1, int n, int pitch, long long groups, float eps,
                                                            float2* stats) {
   grid_dependency_wait();
   grid_dependents_launch();
@@ -775,11 +776,11 @@ __global__ void __launch_bounds__(256) bwd_ln_stats_kernel(const uint4* t0, cons
     const long long g = first + k;
     if (g < groups) {
       const long long row = g / per_row;
-      const long long at = row * 128 * per_row + (g - row * per_row);
+      const long long at = row * 128 * pitch + (g - row * per_row);
       uint4 v[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u)
-        v[u] = __ldg((u < 4 ? t0 : t1) + at + static_cast<long long>((c0 + 32 * u) & 127) * per_row);
+        v[u] = __ldg((u < 4 ? t0 : t1) + at + static_cast<long long>((c0 + 32 * u) & 127) * pitch);
 #pragma unroll
       for (int u = 0; u < 8; ++u) tile[c0 + 32 * u][k] = v[u];
     }
@@ -808,7 +809,7 @@ __global__ void __launch_bounds__(256) bwd_ln_stats_kernel(const uint4* t0, cons
 // One thread per row, group of eight columns and group of 16 channels: the eight positions' statistics are read once.
 constexpr int kLnFinishChannels = 16;
 __global__ void __launch_bounds__(256) bwd_ln_finish_kernel(uint4* dt, const uint4* t, const float2* stats, const float2* means,
-                                                            int n, long long threads) {
+                                                            int n, int pitch, long long threads) {
   grid_dependency_wait();
   grid_dependents_launch();
   const long long g = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
@@ -829,14 +830,14 @@ __global__ void __launch_bounds__(256) bwd_ln_finish_kernel(uint4* dt, const uin
       mean[2 * q + 1] = st.z, k0[2 * q + 1] = st.w * 0.0625f, k1[2 * q + 1] = st.w * mm.w, m1[2 * q + 1] = mm.z;
     }
   }
-  const long long base = (row * 128 + c_first) * per_row + jc;
+  const long long base = (row * 128 + c_first) * pitch + jc;
 #pragma unroll
   for (int c0 = 0; c0 < kLnFinishChannels; c0 += 4) {
     uint4 dv[4], tv[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      dv[k] = dt[base + static_cast<long long>(c0 + k) * per_row];
-      tv[k] = __ldg(t + base + static_cast<long long>(c0 + k) * per_row);
+      dv[k] = dt[base + static_cast<long long>(c0 + k) * pitch];
+      tv[k] = __ldg(t + base + static_cast<long long>(c0 + k) * pitch);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -850,7 +851,7 @@ __global__ void __launch_bounds__(256) bwd_ln_finish_kernel(uint4* dt, const uin
         const float r1 = k0[2 * q + 1] * (d.y - m1[2 * q + 1] - (x.y - mean[2 * q + 1]) * k1[2 * q + 1]);
         o[q] = pack_f16x2_sat(make_float2(r0, r1));
       }
-      dt[base + static_cast<long long>(c0 + k) * per_row] = make_uint4(o[0], o[1], o[2], o[3]);
+      dt[base + static_cast<long long>(c0 + k) * pitch] = make_uint4(o[0], o[1], o[2], o[3]);
     }
   }
 }

@@ -65,7 +65,9 @@ struct TriCall {
   float eps_in, eps_out;
   bool residual, any_n;
   int dtype;
-  int pitch() const { return any_n ? (N + 7) / 8 * 8 : N; }
+  // The C entry points below are the any-length ones for every N, because their intermediates have aligned rows; any_n says
+  // which lengths and gradients are taken and which entry point of the general path an error names.
+  int sized_n() const { return (N + 7) / 8 * 8; }
 };
 
 bool fill_call(TriCall& c, const Tensor& z, at::TensorList p, const OptTensor& token_mask,
@@ -112,16 +114,15 @@ bool fill_call(TriCall& c, const Tensor& z, at::TensorList p, const OptTensor& t
 
 size_t forward_bytes(const TriCall& c) {
   size_t need = 0;
-  check(b200_trimul_workspace_bytes(c.B, c.pitch(), c.d_pair, c.d_hidden, c.direction, &need), "b200_trimul_workspace_bytes");
+  check(b200_trimul_workspace_bytes(c.B, c.sized_n(), c.d_pair, c.d_hidden, c.direction, &need), "b200_trimul_workspace_bytes");
   return need;
 }
 
 void launch_forward(const TriCall& c, const Tensor& z, at::TensorList p, const OptTensor& token_mask,
                     const OptTensor& pair_mask, const OptTensor& drop_scale, const Tensor& y, const Tensor& ws) {
   const c10::cuda::CUDAGuard guard(z.device());
-  auto* f = c.any_n ? b200_trimul_forward_any : b200_trimul_forward_ex;
   auto fp = [&](int i) { return static_cast<const float*>(p[i].data_ptr()); };
-  check(f(z.data_ptr(), p[kLeft].data_ptr(), p[kLeftGate].data_ptr(), p[kRight].data_ptr(), p[kRightGate].data_ptr(),
+  check(b200_trimul_forward_any(z.data_ptr(), p[kLeft].data_ptr(), p[kLeftGate].data_ptr(), p[kRight].data_ptr(), p[kRightGate].data_ptr(),
           p[kGate].data_ptr(), p[kOut].data_ptr(), c.dtype, fp(kLnInW), fp(kLnInB), fp(kLnOutW), fp(kLnOutB), nullptr,
           static_cast<const uint8_t*>(ptr(token_mask)), static_cast<const uint8_t*>(ptr(pair_mask)), ptr(drop_scale),
           y.data_ptr(), ws.data_ptr(), static_cast<size_t>(ws.numel()), c.B, c.N, c.d_pair, c.d_hidden, c.direction, c.eps_in,
@@ -218,7 +219,7 @@ struct TriMul : public torch::autograd::Function<TriMul> {
 
     const c10::cuda::CUDAGuard guard(z.device());
     size_t need = 0;
-    check(b200_trimul_backward_workspace_bytes(c.B, c.pitch(), c.direction, &need), "b200_trimul_backward_workspace_bytes");
+    check(b200_trimul_backward_workspace_bytes(c.B, c.sized_n(), c.direction, &need), "b200_trimul_backward_workspace_bytes");
     Tensor bws = aligned_empty(need, z);
     Tensor dz = at::empty_like(z);
     const auto f32 = z.options().dtype(at::kFloat).requires_grad(false);
@@ -228,8 +229,7 @@ struct TriMul : public torch::autograd::Function<TriMul> {
                    g[kGate].data_ptr(), g[kOut].data_ptr()};
     auto fp = [&](int i) { return static_cast<const float*>(p[i].data_ptr()); };
     auto gp = [&](int i) { return static_cast<float*>(g[i].data_ptr()); };
-    auto* f = c.any_n ? b200_trimul_backward_any : b200_trimul_backward;
-    check(f(dy.data_ptr(), z.data_ptr(), p[kLeft].data_ptr(), p[kLeftGate].data_ptr(), p[kRight].data_ptr(),
+    check(b200_trimul_backward_any(dy.data_ptr(), z.data_ptr(), p[kLeft].data_ptr(), p[kLeftGate].data_ptr(), p[kRight].data_ptr(),
             p[kRightGate].data_ptr(), p[kGate].data_ptr(), p[kOut].data_ptr(), c.dtype, fp(kLnInW), fp(kLnInB), fp(kLnOutW),
             fp(kLnOutB), nullptr, static_cast<const uint8_t*>(ptr(token_mask)), static_cast<const uint8_t*>(ptr(pair_mask)),
             ptr(drop_scale), ws.data_ptr(), dz.data_ptr(), dw, gp(kLnInW), gp(kLnInB), gp(kLnOutW), gp(kLnOutB),

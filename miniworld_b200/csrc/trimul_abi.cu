@@ -350,15 +350,19 @@ static int check_bn(int B, int N, bool any_n = false) {
 
 static size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Columns from one channel of a pair row to the next in the row-plane intermediates (left, right, tri and their
-// gradients): N rounded up to the 16 bytes a tensor map's strides need. The maps' extents stay N: loads read zeros past
-// it and stores are clipped there, so the columns N .. pitch-1 are never written or used and no input is padded.
-// (N = 203, one sample: copying z, mask and output to and from 208 columns was 43 us of kernels beside the 37 us of the
-// three stages.)
-static int plane_pitch(int N) { return (N + 7) / 8 * 8; }
+// Columns from one channel of a pair row to the next in the row-plane intermediates (left, right, tri and their gradients)
+// of an any-length call: N rounded up to 128 bytes, so that every 64-column piece that the stages copy is one line of L2 and
+// not parts of two. The maps' extents stay N: loads read zeros past it and stores are clipped there, so the columns N ..
+// pitch-1 cost memory but no traffic and are never used, and no input is padded. The stage entry points take dense tensors
+// (pitch N), and so do calls that leave a workspace of the documented layout. Module calls with rows a multiple of 16 bytes
+// before and of 128 bytes now: N = 264 forward 68.1 -> 61.2 us, training step 264 -> 249; 321: 82.4 -> 76.1; 376: 92.9 -> 87.1;
+// 520: 185 -> 166, training step 690 -> 635; 760: 316 -> 287 (768, aligned either way: 288 -> 286).
+static int plane_pitch(int N) { return static_cast<int>((static_cast<unsigned>(N) + 63u) / 64u * 64u); }
+// per-position statistics [rows][N] have their rows this far apart (16-byte pieces of 16-bit columns)
+static int round_up_8(int N) { return static_cast<int>((static_cast<unsigned>(N) + 7u) / 8u * 8u); }
 
-static size_t plane_tensor_bytes(int B, int rows, int N) {
-  return round_up(static_cast<size_t>(B) * rows * kC * N * 2, 1024);
+static size_t plane_tensor_bytes(int B, int rows, int ld) {
+  return round_up(static_cast<size_t>(B) * rows * kC * ld * 2, 1024);
 }
 
 // Column tile width of the contraction: the candidate that wastes the fewest padded columns.
@@ -443,21 +447,25 @@ int b200_trimul_last_cuda_error(void) { return tl_last_cuda_error; }
 
 size_t b200_trimul_packed_bytes(void) { return kPackedBytes; }
 
+// Regions of a workspace whose intermediates have the pitch `ld`.
+static void workspace_offsets(int B, int N, int ld, size_t off[5]) {
+  const size_t t = plane_tensor_bytes(B, N, ld);
+  off[0] = 0;
+  off[1] = kStatusBytes;
+  off[2] = kStatusBytes + kPackedBytes;
+  off[3] = off[2] + t;
+  off[4] = off[3] + t;
+}
+
 int b200_trimul_workspace_layout(int B, int N, size_t out_offsets[5]) {
   if (out_offsets == nullptr) return B200_TRIMUL_E_NULL;
   int rc = check_bn(B, N);
   if (rc != B200_TRIMUL_OK) return rc;
-  const size_t t = plane_tensor_bytes(B, N, N);
-  out_offsets[0] = 0;
-  out_offsets[1] = kStatusBytes;
-  out_offsets[2] = kStatusBytes + kPackedBytes;
-  out_offsets[3] = out_offsets[2] + t;
-  out_offsets[4] = out_offsets[3] + t;
+  workspace_offsets(B, N, N, out_offsets);
   return B200_TRIMUL_OK;
 }
 
-int b200_trimul_workspace_bytes(int B, int N, int d_pair, int d_hidden, int direction, size_t* out_bytes) {
-  if (out_bytes == nullptr) return B200_TRIMUL_E_NULL;
+static int workspace_need(int B, int N, int ld, int d_pair, int d_hidden, int direction, size_t* out_bytes) {
   if (direction != B200_TRIMUL_OUTGOING && direction != B200_TRIMUL_INCOMING && direction != B200_TRIMUL_BIDIRECTIONAL)
     return B200_TRIMUL_E_SHAPE;
   // supported widths: d_pair = d_hidden = 128 (every direction); d_pair = 64 with 128 contracted channels in total,
@@ -465,12 +473,25 @@ int b200_trimul_workspace_bytes(int B, int N, int d_pair, int d_hidden, int dire
   const bool wide = d_pair == kC && d_hidden == kC;
   const bool narrow = d_pair == 64 && d_hidden == (direction == B200_TRIMUL_BIDIRECTIONAL ? 64 : kC);
   if (!wide && !narrow) return B200_TRIMUL_E_UNSUPPORTED;
-  size_t off[5];
-  int rc = b200_trimul_workspace_layout(B, N, off);
+  int rc = check_bn(B, N, true);
+  if (rc == B200_TRIMUL_OK) rc = check_bn(B, round_up_8(N));
   if (rc != B200_TRIMUL_OK) return rc;
-  *out_bytes = off[4] + plane_tensor_bytes(B, N, N);
+  size_t off[5];
+  workspace_offsets(B, N, ld, off);
+  *out_bytes = off[4] + plane_tensor_bytes(B, N, ld);
   // bidirectional: a second packed block and a second tri tensor (left / right are reused by the two halves)
-  if (direction == B200_TRIMUL_BIDIRECTIONAL && wide) *out_bytes += kPackedBytes + plane_tensor_bytes(B, N, N);
+  if (direction == B200_TRIMUL_BIDIRECTIONAL && wide) *out_bytes += kPackedBytes + plane_tensor_bytes(B, N, ld);
+  return B200_TRIMUL_OK;
+}
+
+// (the larger pitch of the any-length calls: enough for both kinds)
+int b200_trimul_workspace_bytes(int B, int N, int d_pair, int d_hidden, int direction, size_t* out_bytes) {
+  if (out_bytes == nullptr) return B200_TRIMUL_E_NULL;
+  size_t need = 0;
+  int rc = workspace_need(B, N, plane_pitch(N), d_pair, d_hidden, direction, &need);
+  if (rc == B200_TRIMUL_OK) rc = check_bn(B, N);
+  if (rc != B200_TRIMUL_OK) return rc;
+  *out_bytes = need;
   return B200_TRIMUL_OK;
 }
 
@@ -604,14 +625,15 @@ enum PrologueMode { kLocal, kGatherRight, kChannels };
 static int prologue_impl(const void* z, const void* packed, const uint8_t* token_mask, const uint8_t* pair_mask,
                          void* const* left_dst, int n_left, void* const* right_dst, int n_right, PrologueMode mode,
                          int B, int N, int row_begin, int rows, float eps_in, int has_bias, int* status,
-                         void* cuda_stream, int d_pair = kC, bool any_n = false, bool early = false) {
+                         void* cuda_stream, int d_pair = kC, int ld = 0, bool early = false) {
   if (d_pair != kC && d_pair != 64) return B200_TRIMUL_E_UNSUPPORTED;
   if (!z || !packed || !left_dst || !right_dst || !status) return B200_TRIMUL_E_NULL;
   if (n_left < 1 || n_left > kMaxDst || n_right < 1 || n_right > kMaxDst) return B200_TRIMUL_E_SHAPE;
   if (mode != kLocal && B != 1) return B200_TRIMUL_E_SHAPE;
   if (mode == kChannels && (n_left != n_right || kC % n_left != 0 || (kC / n_left) % 8 != 0)) return B200_TRIMUL_E_SHAPE;
-  int rc = check_bn(B, N, any_n);
+  int rc = check_bn(B, N, ld != 0);
   if (rc != B200_TRIMUL_OK) return rc;
+  if (ld == 0) ld = N;
   if (rows < 1 || row_begin < 0 || row_begin + rows > N) return B200_TRIMUL_E_SHAPE;
   if (!aligned(z, 16) || !aligned(packed, 1024)) return B200_TRIMUL_E_ALIGN;
   DeviceInfo info;
@@ -632,8 +654,8 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
     // outputs, row-plane: [rows][channels][N columns]
     const uint64_t n64 = static_cast<uint64_t>(N);
     const uint64_t ch = mode == kChannels ? static_cast<uint64_t>(kC / n_left) : static_cast<uint64_t>(kC);
-    const uint64_t ld = static_cast<uint64_t>(plane_pitch(N));
-    const uint64_t strides[2] = {ld * 2ull, ld * ch * 2ull};
+    const uint64_t ld64 = static_cast<uint64_t>(ld);
+    const uint64_t strides[2] = {ld64 * 2ull, ld64 * ch * 2ull};
     const uint32_t box[3] = {64, static_cast<uint32_t>(ch), 1};
     const uint64_t dims_local[3] = {n64, ch, static_cast<uint64_t>(B) * rows};
     const uint64_t dims_all[3] = {n64, ch, n64};
@@ -740,12 +762,12 @@ constexpr int kDirMixed = 3;
 
 static int contract_impl(const void* left, const void* right, void* tri, void* const* owner_dst, int n_owners, int slot,
                          int channels, int B, int N, int row_begin, int rows, int k_rows, int direction, int* status,
-                         void* cuda_stream, int row_channels = 0, bool any_n = false) {
+                         void* cuda_stream, int row_channels = 0, int pitch = 0) {
   if (!left || !right || !status) return B200_TRIMUL_E_NULL;
   if (n_owners == 0 && !tri) return B200_TRIMUL_E_NULL;
   if (n_owners < 0 || n_owners > kMaxOwners || (n_owners > 0 && !owner_dst)) return B200_TRIMUL_E_SHAPE;
   if (channels < 8 || channels > kC || channels % 8 != 0) return B200_TRIMUL_E_SHAPE;
-  int rc = check_bn(B, N, any_n);
+  int rc = check_bn(B, N, pitch != 0);
   if (rc != B200_TRIMUL_OK) return rc;
   if (rows < 1 || row_begin < 0 || row_begin + rows > N) return B200_TRIMUL_E_SHAPE;
   if (k_rows < 1 || k_rows > N) return B200_TRIMUL_E_SHAPE;
@@ -765,7 +787,7 @@ static int contract_impl(const void* left, const void* right, void* tri, void* c
   const bool use_pair = rows >= 256 && (pair_rows - rows) * 4 <= rows;
   const int bn = use_pair ? ((N + 255) / 256 * 256 <= (N + 127) / 128 * 128 ? 256 : 128) : choose_bn(N);
   const uint64_t n64 = static_cast<uint64_t>(N);
-  const uint64_t ld = static_cast<uint64_t>(plane_pitch(N));
+  const uint64_t ld = static_cast<uint64_t>(pitch != 0 ? pitch : N);
   const uint64_t ch64 = static_cast<uint64_t>(channels);
   const uint64_t row_stride = static_cast<uint64_t>(row_channels > 0 ? row_channels : channels) * ld * 2;  // bytes between pair rows
   const uint64_t h_stride = ld * 2;
@@ -851,27 +873,27 @@ int b200_trimul_contract(const void* left, const void* right, void* tri, int B, 
 }
 
 static int contract_backward_impl(const void* dtri, const void* left, const void* right, void* dleft, void* dright, int B,
-                                  int N, int direction, int* status, void* cuda_stream, bool any_n) {
+                                  int N, int direction, int* status, void* cuda_stream, int pitch) {
   if (!dtri || !left || !right || !dleft || !dright) return B200_TRIMUL_E_NULL;
   int rc;
   if (direction == B200_TRIMUL_OUTGOING) {
     // t_ij = sum_k l_ik r_jk:  dl_ik = sum_j dt_ij r_jk (mixed),  dr_jk = sum_i dt_ij l_ik (the incoming form)
-    rc = contract_impl(dtri, right, dleft, nullptr, 0, 0, kC, B, N, 0, N, N, kDirMixed, status, cuda_stream, 0, any_n);
+    rc = contract_impl(dtri, right, dleft, nullptr, 0, 0, kC, B, N, 0, N, N, kDirMixed, status, cuda_stream, 0, pitch);
     if (rc != B200_TRIMUL_OK) return rc;
-    return contract_impl(dtri, left, dright, nullptr, 0, 0, kC, B, N, 0, N, N, B200_TRIMUL_INCOMING, status, cuda_stream, 0, any_n);
+    return contract_impl(dtri, left, dright, nullptr, 0, 0, kC, B, N, 0, N, N, B200_TRIMUL_INCOMING, status, cuda_stream, 0, pitch);
   }
   if (direction == B200_TRIMUL_INCOMING) {
     // t_ij = sum_k l_ki r_kj:  dl_ki = sum_j r_kj dt_ij (the outgoing form),  dr_kj = sum_i l_ki dt_ij (mixed)
-    rc = contract_impl(right, dtri, dleft, nullptr, 0, 0, kC, B, N, 0, N, N, B200_TRIMUL_OUTGOING, status, cuda_stream, 0, any_n);
+    rc = contract_impl(right, dtri, dleft, nullptr, 0, 0, kC, B, N, 0, N, N, B200_TRIMUL_OUTGOING, status, cuda_stream, 0, pitch);
     if (rc != B200_TRIMUL_OK) return rc;
-    return contract_impl(left, dtri, dright, nullptr, 0, 0, kC, B, N, 0, N, N, kDirMixed, status, cuda_stream, 0, any_n);
+    return contract_impl(left, dtri, dright, nullptr, 0, 0, kC, B, N, 0, N, N, kDirMixed, status, cuda_stream, 0, pitch);
   }
   return B200_TRIMUL_E_SHAPE;
 }
 
 int b200_trimul_contract_backward(const void* dtri, const void* left, const void* right, void* dleft, void* dright, int B,
                                   int N, int direction, int* status, void* cuda_stream) {
-  return contract_backward_impl(dtri, left, right, dleft, dright, B, N, direction, status, cuda_stream, false);
+  return contract_backward_impl(dtri, left, right, dleft, dright, B, N, direction, status, cuda_stream, 0);
 }
 
 int b200_trimul_contract_partial(const void* left, const void* right, void* tri_partial, int B, int N, int k_rows,
@@ -941,11 +963,11 @@ int b200_trimul_reduce_partials(void* tri, const void* const* partials, int n_sr
 // in slab g (what the channel-sharded contraction of GPU g stored there).
 static int epilogue_impl(const void* tri, const void* z, const void* packed, void* y, int B, int N, int rows, int groups,
                          float eps_in, float eps_out, int residual, int* status, void* cuda_stream, int d_pair = kC,
-                         bool any_n = false, bool early = false) {
+                         int pitch = 0, bool early = false) {
   if (!tri || !z || !packed || !y || !status) return B200_TRIMUL_E_NULL;
   if (d_pair != kC && d_pair != 64) return B200_TRIMUL_E_UNSUPPORTED;
   if (groups < 1 || groups > 8 || kC % groups != 0 || (groups > 1 && B != 1)) return B200_TRIMUL_E_SHAPE;
-  int rc = check_bn(B, N, any_n);
+  int rc = check_bn(B, N, pitch != 0);
   if (rc != B200_TRIMUL_OK) return rc;
   if (rows < 1 || rows > N) return B200_TRIMUL_E_SHAPE;
   if (!aligned(tri, 16) || !aligned(z, 16) || !aligned(y, 16) || !aligned(packed, 1024)) return B200_TRIMUL_E_ALIGN;
@@ -959,7 +981,7 @@ static int epilogue_impl(const void* tri, const void* z, const void* packed, voi
   {
     const uint64_t cg = static_cast<uint64_t>(kC / groups);
     const uint64_t dims[4] = {n64, cg, static_cast<uint64_t>(groups), nrows};
-    const uint64_t ld = static_cast<uint64_t>(plane_pitch(N));
+    const uint64_t ld = static_cast<uint64_t>(pitch != 0 ? pitch : N);
     const uint64_t strides[3] = {ld * 2, nrows * cg * ld * 2, cg * ld * 2};
     const uint32_t box[4] = {64, static_cast<uint32_t>(cg), static_cast<uint32_t>(groups), 1};
     rc = make_map(&map_t, tri, 4, dims, strides, box);
@@ -1042,12 +1064,12 @@ extern "C" {
 
 static int epilogue_wide_impl(const void* tri, const void* tri_in, const void* z, const void* packed,
                               const void* packed_in, const void* drop_scale, void* y, int B, int N, int rows,
-                              float eps_in, float eps_out, int residual, int* status, void* cuda_stream, bool any_n,
+                              float eps_in, float eps_out, int residual, int* status, void* cuda_stream, int pitch,
                               bool early = false) {
   if (!tri || !z || !packed || !y || !status) return B200_TRIMUL_E_NULL;
   const bool bidir = tri_in != nullptr;
   if (bidir && !packed_in) return B200_TRIMUL_E_NULL;
-  int rc = check_bn(B, N, any_n);
+  int rc = check_bn(B, N, pitch != 0);
   if (rc != B200_TRIMUL_OK) return rc;
   if (rows < 1 || rows > N) return B200_TRIMUL_E_SHAPE;
   if (!aligned(tri, 16) || !aligned(z, 16) || !aligned(y, 16) || !aligned(packed, 1024)) return B200_TRIMUL_E_ALIGN;
@@ -1061,7 +1083,7 @@ static int epilogue_wide_impl(const void* tri, const void* tri_in, const void* z
   CUtensorMap map_t0, map_t1, map_z, map_y, map_w0, map_w1;
   {
     const uint64_t dims[3] = {n64, static_cast<uint64_t>(kC), nrows};
-    const uint64_t ld = static_cast<uint64_t>(plane_pitch(N));
+    const uint64_t ld = static_cast<uint64_t>(pitch != 0 ? pitch : N);
     const uint64_t strides[2] = {ld * 2, static_cast<uint64_t>(kC) * ld * 2};
     const uint32_t box[3] = {64, 64, 1};  // one chunk half: 64 positions of 64 channels
     rc = make_map(&map_t0, tri, 3, dims, strides, box);
@@ -1113,7 +1135,7 @@ int b200_trimul_epilogue_wide(const void* tri, const void* tri_in, const void* z
                               const void* packed_in, const void* drop_scale, void* y, int B, int N, int rows,
                               float eps_in, float eps_out, int residual, int* status, void* cuda_stream) {
   return epilogue_wide_impl(tri, tri_in, z, packed, packed_in, drop_scale, y, B, N, rows, eps_in, eps_out, residual, status,
-                            cuda_stream, false);
+                            cuda_stream, 0);
 }
 
 static int forward_impl(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
@@ -1126,14 +1148,14 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
   if (!z || !y || !workspace) return B200_TRIMUL_E_NULL;
   size_t need = 0;
   if (any_n && (N < 1 || N > 0x7FFFFFFF / 128)) return B200_TRIMUL_E_SHAPE;
-  const int ld = any_n ? plane_pitch(N) : N;  // the workspace is the one of N rounded up to a multiple of 8
-  int rc = b200_trimul_workspace_bytes(B, ld, d_pair, d_hidden, direction, &need);
+  const int ld = any_n ? plane_pitch(N) : N;
+  int rc = workspace_need(B, N, ld, d_pair, d_hidden, direction, &need);
+  if (rc == B200_TRIMUL_OK) rc = check_bn(B, N, any_n);
   if (rc != B200_TRIMUL_OK) return rc;
   if (workspace_bytes < need) return B200_TRIMUL_E_WORKSPACE;
   if (!aligned(workspace, 1024)) return B200_TRIMUL_E_ALIGN;
   size_t off[5];
-  rc = b200_trimul_workspace_layout(B, ld, off);
-  if (rc != B200_TRIMUL_OK) return rc;
+  workspace_offsets(B, N, ld, off);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   int* status = reinterpret_cast<int*>(ws + off[0]);
   void* packed = ws + off[1];
@@ -1147,10 +1169,10 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
     void* l[1] = {left};
     void* r[1] = {right};
     return prologue_impl(z, pk, token_mask, pair_mask, l, 1, r, 1, kLocal, B, N, 0, N, eps_in, has_bias, status, cuda_stream,
-                         d_pair, any_n, true);
+                         d_pair, ld, true);
   };
   auto contract = [&](void* dst, int dir) {
-    return contract_impl(left, right, dst, nullptr, 0, 0, kC, B, N, 0, N, N, dir, status, cuda_stream, 0, any_n);
+    return contract_impl(left, right, dst, nullptr, 0, 0, kC, B, N, 0, N, N, dir, status, cuda_stream, 0, ld);
   };
   if (d_pair == 64) {
     // Narrow pair stacks: 64 input channels, 128 contracted channels in one [rows, 128, N] tensor. The parameter
@@ -1166,20 +1188,20 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
     if (direction == B200_TRIMUL_BIDIRECTIONAL) {
       const size_t half = static_cast<size_t>(64) * ld * 2;  // bytes from channel 0 to channel 64 of a pair row
       rc = contract_impl(left, right, tri, nullptr, 0, 0, 64, B, N, 0, N, N, B200_TRIMUL_OUTGOING, status, cuda_stream, kC,
-                         any_n);
+                         ld);
       if (rc != B200_TRIMUL_OK) return rc;
       rc = contract_impl(static_cast<uint8_t*>(left) + half, static_cast<uint8_t*>(right) + half,
                          static_cast<uint8_t*>(tri) + half, nullptr, 0, 0, 64, B, N, 0, N, N, B200_TRIMUL_INCOMING, status,
-                         cuda_stream, kC, any_n);
+                         cuda_stream, kC, ld);
     } else {
       rc = contract(tri, direction);
     }
     if (rc != B200_TRIMUL_OK) return rc;
-    return epilogue_impl(tri, z, packed, y, B, N, N, 1, eps_in, eps_out, residual, status, cuda_stream, 64, any_n, true);
+    return epilogue_impl(tri, z, packed, y, B, N, N, 1, eps_in, eps_out, residual, status, cuda_stream, 64, ld, true);
   }
   if (direction == B200_TRIMUL_BIDIRECTIONAL) {
     // workspace tail: second tri tensor, then the second packed block
-    const size_t plane = plane_tensor_bytes(B, ld, ld);
+    const size_t plane = plane_tensor_bytes(B, N, ld);
     void* tri_in = ws + off[4] + plane;
     void* packed_in = ws + off[4] + 2 * plane;
     rc = pack_bidir(w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w,
@@ -1194,7 +1216,7 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
     rc = contract(tri_in, B200_TRIMUL_INCOMING);
     if (rc != B200_TRIMUL_OK) return rc;
     return epilogue_wide_impl(tri, tri_in, z, packed, packed_in, drop_scale, y, B, N, N, eps_in, eps_out, residual,
-                                     status, cuda_stream, any_n, true);
+                                     status, cuda_stream, ld, true);
   }
   rc = pack_one(w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w,
                                 ln_in_b, ln_out_w, ln_out_b, bias_opt, packed, kC, status, cuda_stream);
@@ -1205,8 +1227,8 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
   if (rc != B200_TRIMUL_OK) return rc;
   if (drop_scale != nullptr)
     return epilogue_wide_impl(tri, nullptr, z, packed, nullptr, drop_scale, y, B, N, N, eps_in, eps_out, residual,
-                                     status, cuda_stream, any_n, true);
-  return epilogue_impl(tri, z, packed, y, B, N, N, 1, eps_in, eps_out, residual, status, cuda_stream, kC, any_n, true);
+                                     status, cuda_stream, ld, true);
+  return epilogue_impl(tri, z, packed, y, B, N, N, 1, eps_in, eps_out, residual, status, cuda_stream, kC, ld, true);
 }
 
 int b200_trimul_forward_ex(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
@@ -1375,7 +1397,8 @@ extern "C" int b200_trimul_forward_static(const void* z, const void* w_left, con
                                           int** device_status_out, void* cuda_stream) {
   if (!z || !y) return B200_TRIMUL_E_NULL;
   size_t need = 0;
-  int rc = b200_trimul_workspace_bytes(B, N, d_pair, d_hidden, direction, &need);
+  int rc = workspace_need(B, N, N, d_pair, d_hidden, direction, &need);
+  if (rc == B200_TRIMUL_OK) rc = check_bn(B, N);
   if (rc != B200_TRIMUL_OK) return rc;
   if (static_cast<long long>(B) * N * N > kStaticMaxCells || need > kStaticWorkspaceBytes) return B200_TRIMUL_E_TOO_LARGE;
   DeviceInfo info;

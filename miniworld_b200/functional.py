@@ -469,7 +469,7 @@ def trimul_forward(
 
 
 def _pitch(N: int) -> int:
-    """Columns between consecutive channels of a pair row in the intermediates: N rounded up to a multiple of 8."""
+    """The length whose workspace size an any-length call of ``N`` tokens needs: N rounded up to a multiple of 8."""
     return (N + 7) // 8 * 8
 
 
