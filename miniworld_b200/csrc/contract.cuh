@@ -31,6 +31,7 @@ struct ContractParams {
   int a_col_off;  // incoming only: first output row, as a column offset into a's inner dimension
   int n_cols;     // output columns (N)
   int m_rows;     // output rows of this call
+  int bn;         // columns of an output tile (contract_wide_kernel)
   int* status;
 };
 

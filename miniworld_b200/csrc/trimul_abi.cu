@@ -8,6 +8,7 @@
 
 #include "contract.cuh"
 #include "contract_pair.cuh"
+#include "contract_wide.cuh"
 #include "epilogue.cuh"
 #include "epilogue_wide.cuh"
 #include "prologue.cuh"
@@ -410,6 +411,19 @@ static int launch_contract_pair(const CUtensorMap& ma, const CUtensorMap& mb, co
   return B200_TRIMUL_OK;
 }
 
+template <int MODE>
+static int launch_contract_wide(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mt, const ContractParams& p,
+                                const DeviceInfo& info, cudaStream_t stream) {
+  auto kernel = contract_wide_kernel<MODE>;
+  int rc = set_smem(kernel, kWideContractSmem, info.device);
+  if (rc != B200_TRIMUL_OK) return rc;
+  const long long tiles = static_cast<long long>(p.planes) * p.m_tiles * p.n_tiles;
+  const long long pairs = tiles < info.sms / 2 ? tiles : info.sms / 2;
+  // clusters of two CTAs
+  TRIMUL_CUDA(launch_overlapped(kernel, static_cast<int>(2 * pairs), kWideContractThreads, kWideContractSmem, stream, ma, mb, mt, p));
+  return B200_TRIMUL_OK;
+}
+
 }  // namespace trimul
 
 #include "backward.cuh"  // after PackArgs
@@ -786,6 +800,15 @@ static int contract_impl(const void* left, const void* right, void* tri, void* c
   const int pair_rows = (rows + 255) / 256 * 256;
   const bool use_pair = rows >= 256 && (pair_rows - rows) * 4 <= rows;
   const int bn = use_pair ? ((N + 255) / 256 * 256 <= (N + 127) / 128 * 128 ? 256 : 128) : choose_bn(N);
+  // Tiles of up to 512 columns where the other kernels would cut the columns in pieces of 128, or those of one CTA would pad,
+  // and for the largest problems where the width divides them (whole forwards: N = 400 107 -> 106 us and four of 400 346 ->
+  // 330, 640 227 -> 218, 832 431 -> 384, 1100 819 -> 707, 1408 1382 -> 1173, 1920 2990 -> 2515, 1024 551 -> 541). Elsewhere
+  // the exactly fitting 192- and 256-column tiles are ahead: N = 288 63 / 66, 512 131 / 134, 576 182 / 189, 768 292 / 296,
+  // 1792 2045 / 2103 us.
+  const bool use_wide = n_owners == 0 && rows > 384 && N > 384 &&
+                        (use_pair ? bn == 128 || (N > 896 && (N + 127) / 128 % 4 == 0) : bn != 192);
+  const int wide_tiles = (N + 511) / 512;
+  const int wide_bn = ((N + wide_tiles - 1) / wide_tiles + 127) / 128 * 128;
   const uint64_t n64 = static_cast<uint64_t>(N);
   const uint64_t ld = static_cast<uint64_t>(pitch != 0 ? pitch : N);
   const uint64_t ch64 = static_cast<uint64_t>(channels);
@@ -806,7 +829,7 @@ static int contract_impl(const void* left, const void* right, void* tri, void* c
   {
     const uint64_t dims[4] = {n64, right_rows, ch64, static_cast<uint64_t>(B)};
     const uint64_t strides[3] = {row_stride, h_stride, right_rows * row_stride};
-    const uint32_t box_out[4] = {64, static_cast<uint32_t>(use_pair ? bn / 2 : bn), 1, 1};  // a CTA of a pair loads half
+    const uint32_t box_out[4] = {64, static_cast<uint32_t>(use_wide ? 64 : use_pair ? bn / 2 : bn), 1, 1};  // a CTA of a pair loads half
     const uint32_t box_in[4] = {64, 64, 1, 1};
     rc = make_map(&map_b, right, 4, dims, strides, b_mn ? box_in : box_out);
     if (rc != B200_TRIMUL_OK) return rc;
@@ -818,7 +841,7 @@ static int contract_impl(const void* left, const void* right, void* tri, void* c
   if (n_owners == 0) {
     const uint64_t dims[4] = {n64, static_cast<uint64_t>(rows), ch64, static_cast<uint64_t>(B)};
     const uint64_t strides[3] = {row_stride, h_stride, static_cast<uint64_t>(rows) * row_stride};
-    const uint32_t box[4] = {64, 128, 1, 1};
+    const uint32_t box[4] = {64, use_wide ? 32u : 128u, 1, 1};
     rc = make_map(&map_t, tri, 4, dims, strides, box);
     if (rc != B200_TRIMUL_OK) return rc;
   } else {
@@ -843,9 +866,10 @@ static int contract_impl(const void* left, const void* right, void* tri, void* c
   ContractParams p;
   p.H = channels;
   p.planes = B * channels;
-  p.m_tiles = use_pair ? pair_rows / 256 : (rows + kBM - 1) / kBM;
+  p.m_tiles = use_pair || use_wide ? pair_rows / 256 : (rows + kBM - 1) / kBM;
   p.m_rows = rows;
-  p.n_tiles = (N + bn - 1) / bn;
+  p.bn = use_wide ? wide_bn : bn;
+  p.n_tiles = (N + p.bn - 1) / p.bn;
   p.num_kb = ((b_mn ? k_rows : N) + kBK - 1) / kBK;  // rows past k_rows read as zero (TMA out-of-bounds fill)
   p.a_col_off = a_mn ? row_begin : 0;
   p.n_cols = N;
@@ -853,6 +877,7 @@ static int contract_impl(const void* left, const void* right, void* tri, void* c
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
 #define TRIMUL_CONTRACT_MODE(MODE)                                                                       \
   do {                                                                                                   \
+    if (use_wide) return launch_contract_wide<MODE>(map_a, map_b, map_t, p, info, stream);              \
     if (use_pair) {                                                                                      \
       if (bn == 256) return launch_contract_pair<256, MODE>(map_a, map_b, map_t, own, p, info, stream); \
       return launch_contract_pair<128, MODE>(map_a, map_b, map_t, own, p, info, stream);                \
