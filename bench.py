@@ -317,10 +317,11 @@ class Runner:
         return self.parallelism
 
     def launches_per_step(self):
-        """This repository's kernels per step: (pack, prologue, contraction, epilogue) x 2 directions; on several GPUs
-        the barrier kernels between the stages and, row scheme, the reduce kernel of the incoming direction."""
+        """This repository's kernels per step: (prologue, contraction, epilogue) x 2 directions; on several GPUs a packing
+        launch before each, the barrier kernels between the stages and, row scheme, the reduce kernel of the incoming
+        direction."""
         if self.kind != "rows":
-            return 8
+            return 6
         m = self.mods["outgoing"]
         if m.transport != "p2p":
             return 8

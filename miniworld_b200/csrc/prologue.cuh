@@ -49,6 +49,7 @@
 //   warp 26       validity bitmap of the tile
 #pragma once
 
+#include "pack.cuh"
 #include "ptx.cuh"
 
 namespace trimul {
@@ -62,12 +63,16 @@ struct PrologueParams {
   int num_tiles;       // B * rows * tiles_per_row
   const uint8_t* token_mask;  // [B, N] non-zero = valid, or null
   const uint8_t* pair_mask;   // [B, rows, N] non-zero = valid, or null
+  // Where this kernel's matrices come from. raw = 0: `w`, the packed block of an earlier launch. raw = 1: the parameters
+  // themselves (block `raw_block` of the kernel's PackLaunch), which with z, the masks and the LayerNorm parameters below are
+  // older than the kernel before this one; then this launch also packs what the epilogue reads (matrices 4 and 5 of block 0,
+  // matrix 4 of block 1; `pack_blocks` of them) and, if it packs anything, clears the status words of the call.
+  int raw, raw_block, pack_blocks;
   const uint4* w;             // [4][128][C] fp16 packed matrices: left, left gate, right, right gate
   const float* d1;            // [4][128] additive constants (0.5 * bias): left, left gate, right, right gate
   const float* ln_w;          // [128] LayerNorm gamma
   const float* ln_b;          // [128] LayerNorm beta
   float eps;
-  int early;  // z is older than the kernel before this one
   int* status;
 };
 
@@ -107,7 +112,8 @@ constexpr int kProSmemBytes = kProStages * 16384 + kProStageOutBytes + kProRing 
 
 template <bool HAS_BIAS, int C = 128>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProThreads, 1)
-prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ OutputMaps out, const PrologueParams p) {
+prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ OutputMaps out,
+                const __grid_constant__ PackLaunch params, const PrologueParams p) {
   static_assert(C == 128 || C == 64, "d_pair is 128 or 64");
   constexpr int S = kProStages;
   constexpr int kHalves = C / 64;              // 64-channel (128-byte) halves of an input row
@@ -162,8 +168,9 @@ prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant
   __syncthreads();
   cluster_sync_all();  // barriers of both CTAs are initialised before any signal crosses
   tc_fence_after();
-  // (the first z tiles land while the packing of the weights ends)
-  if (warp != 0 || !p.early) {
+  // A call's first launch may follow any kernel. With the call's arguments as the inputs of a later one only the warps that
+  // store wait for the kernel before it, behind their share of the weights.
+  if (!p.raw || p.pack_blocks > 0) {
     grid_dependency_wait();
     grid_dependents_launch();
   }
@@ -211,6 +218,13 @@ prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
+    if (rank != 0 && p.pack_blocks > 0) {
+      // in the other CTA this warp packs what the epilogue reads
+      if (pair == 0 && lane < 16) p.status[lane] = 0;
+#pragma unroll 4
+      for (int r = pair; r < (p.pack_blocks > 1 ? 384 : 256); r += num_pairs)
+        pack_matrix_row(params.block[r >> 8], params.packed[r >> 8], 512 + (r & 255));
+    }
     if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = umma_idesc(256, 64, false, false, kFmtF16, kFmtF16);
       bool ok = mbar_wait(w_full, 0, abort_flag, p.status, kDevTimeoutMma);

@@ -11,6 +11,7 @@
 #include "contract_wide.cuh"
 #include "epilogue.cuh"
 #include "epilogue_wide.cuh"
+#include "pack.cuh"
 #include "prologue.cuh"
 #include "transition.cuh"
 
@@ -18,12 +19,6 @@ namespace trimul {
 
 constexpr int kC = 128;
 constexpr size_t kStatusBytes = 1024;
-constexpr size_t kPackedMatrixBytes = 6 * 32768;
-constexpr size_t kPackedD1Off = kPackedMatrixBytes;            // float[4][128]
-constexpr size_t kPackedC3Off = kPackedMatrixBytes + 2048;     // float4[128]
-constexpr size_t kPackedLnOff = kPackedMatrixBytes + 4096;     // float[2][128]: input LayerNorm gamma, beta
-constexpr size_t kPackedBytes = kPackedMatrixBytes + 5120;     // 201728, a multiple of 1024
-
 static thread_local int tl_last_cuda_error = 0;
 
 #define TRIMUL_CUDA(expr)                             \
@@ -34,116 +29,6 @@ static thread_local int tl_last_cuda_error = 0;
       return B200_TRIMUL_E_CUDA;                      \
     }                                                 \
   } while (0)
-
-// ---------------------------------------------------------------------------------------------
-// Weight packing: one warp per matrix row. C = d_pair (128 or 64); the contracted width is 128 in both cases.
-//   matrices 0..3 (left, left gate, right, right gate) [128, C]: W' = fp16(0.5 W), d = 0.5 bias
-//     (the prologue applies the input LayerNorm affine itself; gamma_in / beta_in are copied alongside)
-//   matrix 4 (out)  [C, 128]: W' = fp16(0.5 W gamma_out), s = rowsum(W'), d = 0.5 (W beta_out + bias)
-//   matrix 5 (gate) [C, C]:   W' = bf16(0.5 W gamma_in),  s = rowsum(W'), d = 0.5 (W beta_in + bias)
-// Packed matrices are dense and follow one another: 0..3 at m * 128 * C * 2 bytes, 4 after them, 5 after 4.
-struct PackArgs {
-  const void* w[6];
-  int ld[6];  // elements between consecutive rows of w[m] (128 for a matrix of its own, more for a column slice)
-  const float* bias[6];
-  const float* ln_in_w;
-  const float* ln_in_b;
-  const float* ln_out_w;
-  const float* ln_out_b;
-  int f32_weights;
-  int c;  // d_pair
-};
-
-__host__ __device__ inline size_t packed_matrix_offset(int m, int c) {
-  return m <= 4 ? static_cast<size_t>(m) * 128 * c * 2 : static_cast<size_t>(4) * 128 * c * 2 + static_cast<size_t>(c) * 128 * 2;
-}
-
-// One launch packs one or two blocks (grid.y) and clears the status words of the call that follows, if given.
-struct PackLaunch {
-  PackArgs block[2];
-  uint8_t* packed[2];
-  int* clear_status;
-};
-__global__ void __launch_bounds__(128) pack_kernel(const __grid_constant__ PackLaunch l) {
-  grid_dependents_launch();
-  const PackArgs& a = l.block[blockIdx.y];
-  uint8_t* packed = l.packed[blockIdx.y];
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 16 && l.clear_status != nullptr) l.clear_status[threadIdx.x] = 0;
-  const int gw = blockIdx.x * 4 + (threadIdx.x >> 5);  // 0 .. 767
-  const int lane = threadIdx.x & 31;
-  const int m = gw >> 7;
-  const int row = gw & 127;
-  const int n_rows = m < 4 ? 128 : a.c;
-  const int k = m == 4 ? 128 : a.c;  // row length
-  if (row >= n_rows) return;
-  const bool active = lane * 4 < k;
-  const float* gamma = (m == 4) ? a.ln_out_w : a.ln_in_w;
-  const float* beta = (m == 4) ? a.ln_out_b : a.ln_in_b;
-  float w[4] = {0.f, 0.f, 0.f, 0.f};
-  if (!active) {
-  } else if (a.f32_weights) {
-    const float4 v = reinterpret_cast<const float4*>(static_cast<const float*>(a.w[m]) + static_cast<size_t>(row) * a.ld[m])[lane];
-    w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
-  } else {
-    const uint2 v = reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(a.w[m]) + static_cast<size_t>(row) * a.ld[m])[lane];
-    w[0] = bf16_lo(v.x), w[1] = bf16_hi(v.x), w[2] = bf16_lo(v.y), w[3] = bf16_hi(v.y);
-  }
-  const float4 g = active ? reinterpret_cast<const float4*>(gamma)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 b = active ? reinterpret_cast<const float4*>(beta)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float gg[4] = {g.x, g.y, g.z, g.w};
-  const float bb[4] = {b.x, b.y, b.z, b.w};
-  float s = 0.f, d = 0.f;
-  uint16_t o[4];
-  // Both operands of an MMA share one 16-bit format. Matrices 0..3 meet the fp16 x_hat and matrix 4 the
-  // fp16 t tile, so they are fp16 (three more mantissa bits than bf16; |0.5 W gamma| is far from 65504).
-  // Matrix 5 meets the module's raw bf16 input, so it is bf16.
-  const bool fold = m >= 4;
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    const float v = fold ? 0.5f * w[t] * gg[t] : 0.5f * w[t];
-    if (m == 5) {
-      const __nv_bfloat16 r = __float2bfloat16_rn(v);
-      o[t] = __bfloat16_as_ushort(r);
-      s += __bfloat162float(r);
-    } else {
-      const __half r = __float2half_rn(fminf(fmaxf(v, -65504.f), 65504.f));
-      o[t] = __half_as_ushort(r);
-      s += __half2float(r);
-    }
-    if (fold) d = fmaf(w[t], bb[t], d);
-  }
-  if (gw == 0 && active) {
-    reinterpret_cast<float4*>(packed + kPackedLnOff)[lane] = g;
-    reinterpret_cast<float4*>(packed + kPackedLnOff + 512)[lane] = b;
-  }
-  if (active) {
-    uint2 ov;
-    ov.x = static_cast<uint32_t>(o[0]) | (static_cast<uint32_t>(o[1]) << 16);
-    ov.y = static_cast<uint32_t>(o[2]) | (static_cast<uint32_t>(o[3]) << 16);
-    reinterpret_cast<uint2*>(packed + packed_matrix_offset(m, a.c))[row * (k / 4) + lane] = ov;
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    s += __shfl_xor_sync(0xFFFFFFFFu, s, off);
-    d += __shfl_xor_sync(0xFFFFFFFFu, d, off);
-  }
-  if (lane == 0) {
-    const float bias = a.bias[m] != nullptr ? a.bias[m][row] : 0.f;
-    d = 0.5f * (d + bias);  // d is the folded W beta term for matrices 4 and 5, zero for the others
-    if (m < 4) {
-      reinterpret_cast<float*>(packed + kPackedD1Off)[m * 128 + row] = d;
-    } else {
-      float* c3 = reinterpret_cast<float*>(packed + kPackedC3Off) + row * 4;
-      if (m == 5) {
-        c3[0] = s;
-        c3[1] = d;
-      } else {
-        c3[2] = s;
-        c3[3] = d;
-      }
-    }
-  }
-}
 
 // Sum of the incoming-direction partial results of several GPUs for the rows one GPU owns:
 // tri[e] = sum_s src[s][e] over `count` 16-byte groups of eight fp16 values, fp32 accumulation in source order,
@@ -320,8 +205,8 @@ static int set_smem(K kernel, int bytes, int device) {
 }
 
 // Launch a kernel whose blocks may be placed while the kernel before it on the stream finishes: it sets itself up and calls
-// grid_dependency_wait before it touches global memory. Every kernel of a call after its first is launched this way, which
-// takes the set-up (barriers, tensor memory, cluster start) and part of the tail off every boundary: the forward takes 26.6 us
+// grid_dependency_wait before it touches global memory. The kernels of a call are launched this way (but a backward's set-up),
+// which takes the set-up (barriers, tensor memory, cluster start) and part of the tail off every boundary: the forward takes 26.6 us
 // without and 21.8 us with it at N = 64, 91.9 / 88.7 us at N = 384, 339.3 / 333.7 us at N = 768 (one box, in turn).
 template <typename... P, typename... A>
 static cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t stream, const A&... args) {
@@ -558,10 +443,9 @@ static int launch_pack(const PackLaunch& l, int blocks, void* cuda_stream) {
   return B200_TRIMUL_OK;
 }
 
-static int pack_one(const void* w_left, const void* w_left_gate, const void* w_right, const void* w_right_gate,
+static int fill_pack(PackLaunch& l, const void* w_left, const void* w_left_gate, const void* w_right, const void* w_right_gate,
                     const void* w_gate, const void* w_out, int weight_dtype, const float* ln_in_w, const float* ln_in_b,
-                    const float* ln_out_w, const float* ln_out_b, const void* const* bias_opt, void* packed, int c,
-                    int* clear_status, void* cuda_stream) {
+                    const float* ln_out_w, const float* ln_out_b, const void* const* bias_opt, void* packed, int c) {
   const void* w[6] = {w_left, w_left_gate, w_right, w_right_gate, w_out, w_gate};
   const int ld[6] = {c, c, c, c, kC, c};
   const float* bias[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -571,19 +455,18 @@ static int pack_one(const void* w_left, const void* w_left_gate, const void* w_r
     bias[5] = static_cast<const float*>(bias_opt[4]);
     bias[4] = static_cast<const float*>(bias_opt[5]);
   }
-  PackLaunch l;
-  l.clear_status = clear_status;
-  int rc = pack_block(l, 0, w, ld, weight_dtype, ln_in_w, ln_in_b, ln_out_w, ln_out_b, bias, packed, c);
-  if (rc != B200_TRIMUL_OK) return rc;
-  return launch_pack(l, 1, cuda_stream);
+  return pack_block(l, 0, w, ld, weight_dtype, ln_in_w, ln_in_b, ln_out_w, ln_out_b, bias, packed, c);
 }
 
 int b200_trimul_pack_weights(const void* w_left, const void* w_left_gate, const void* w_right,
                              const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,
                              const float* ln_in_w, const float* ln_in_b, const float* ln_out_w,
                              const float* ln_out_b, const void* const* bias_opt, void* packed, void* cuda_stream) {
-  return pack_one(w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
-                  ln_out_b, bias_opt, packed, kC, nullptr, cuda_stream);
+  PackLaunch l;
+  int rc = fill_pack(l, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
+                     ln_out_b, bias_opt, packed, kC);
+  if (rc != B200_TRIMUL_OK) return rc;
+  return launch_pack(l, 1, cuda_stream);
 }
 
 // Bidirectional module: the four left / right matrices are [256, 128] (rows 0-127 feed the outgoing contraction, rows
@@ -591,11 +474,11 @@ int b200_trimul_pack_weights(const void* w_left, const void* w_left_gate, const 
 // `packed_out` serves stage 1 of the outgoing half and stage 3 (its matrix 4 is W_out[:, 0:128] folded with
 // gamma_out[0:128]; its constants carry the output bias), `packed_in` serves stage 1 of the incoming half and
 // holds W_out[:, 128:256] as its matrix 4. Stage 3 adds the two blocks' s_out / d_out constants.
-static int pack_bidir(const void* w_left, const void* w_left_gate, const void* w_right,
+static int fill_pack_bidir(PackLaunch& l, const void* w_left, const void* w_left_gate, const void* w_right,
                                    const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,
                                    const float* ln_in_w, const float* ln_in_b, const float* ln_out_w,
                                    const float* ln_out_b, const void* const* bias_opt, void* packed_out,
-                                   void* packed_in, int* clear_status, void* cuda_stream) {
+                                   void* packed_in) {
   if (!w_left || !w_left_gate || !w_right || !w_right_gate || !w_gate || !w_out || !ln_out_w || !ln_out_b)
     return B200_TRIMUL_E_NULL;
   if (weight_dtype != B200_TRIMUL_DTYPE_BF16 && weight_dtype != B200_TRIMUL_DTYPE_F32) return B200_TRIMUL_E_SHAPE;
@@ -605,8 +488,6 @@ static int pack_bidir(const void* w_left, const void* w_left_gate, const void* w
   if (bias_opt != nullptr)
     for (int i = 0; i < 6; ++i) b[i] = static_cast<const float*>(bias_opt[i]);
   const int ld[6] = {kC, kC, kC, kC, 2 * kC, kC};
-  PackLaunch l;
-  l.clear_status = clear_status;
   {
     const void* w[6] = {w_left, w_left_gate, w_right, w_right_gate, w_out, w_gate};
     const float* bias[6] = {b[0], b[1], b[2], b[3], b[5], b[4]};
@@ -617,9 +498,7 @@ static int pack_bidir(const void* w_left, const void* w_left_gate, const void* w
                       static_cast<const uint8_t*>(w_out) + kC * es, w_gate};
   const float* bias[6] = {b[0] ? b[0] + kC : nullptr, b[1] ? b[1] + kC : nullptr, b[2] ? b[2] + kC : nullptr,
                           b[3] ? b[3] + kC : nullptr, nullptr, nullptr};
-  int rc = pack_block(l, 1, w, ld, weight_dtype, ln_in_w, ln_in_b, ln_out_w + kC, ln_out_b + kC, bias, packed_in);
-  if (rc != B200_TRIMUL_OK) return rc;
-  return launch_pack(l, 2, cuda_stream);
+  return pack_block(l, 1, w, ld, weight_dtype, ln_in_w, ln_in_b, ln_out_w + kC, ln_out_b + kC, bias, packed_in);
 }
 
 int b200_trimul_pack_weights_bidir(const void* w_left, const void* w_left_gate, const void* w_right,
@@ -627,8 +506,11 @@ int b200_trimul_pack_weights_bidir(const void* w_left, const void* w_left_gate, 
                                    const float* ln_in_w, const float* ln_in_b, const float* ln_out_w,
                                    const float* ln_out_b, const void* const* bias_opt, void* packed_out,
                                    void* packed_in, void* cuda_stream) {
-  return pack_bidir(w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
-                    ln_out_b, bias_opt, packed_out, packed_in, nullptr, cuda_stream);
+  PackLaunch l;
+  int rc = fill_pack_bidir(l, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
+                           ln_out_b, bias_opt, packed_out, packed_in);
+  if (rc != B200_TRIMUL_OK) return rc;
+  return launch_pack(l, 2, cuda_stream);
 }
 
 // Where stage 1 writes (see OutputMaps): kLocal - left / right are [B, rows, 128, N]; kGatherRight (B = 1) - left is
@@ -639,9 +521,10 @@ enum PrologueMode { kLocal, kGatherRight, kChannels };
 static int prologue_impl(const void* z, const void* packed, const uint8_t* token_mask, const uint8_t* pair_mask,
                          void* const* left_dst, int n_left, void* const* right_dst, int n_right, PrologueMode mode,
                          int B, int N, int row_begin, int rows, float eps_in, int has_bias, int* status,
-                         void* cuda_stream, int d_pair = kC, int ld = 0, bool early = false) {
+                         void* cuda_stream, int d_pair = kC, int ld = 0, const PackLaunch* raw = nullptr, int raw_block = 0,
+                         int pack_blocks = 0) {
   if (d_pair != kC && d_pair != 64) return B200_TRIMUL_E_UNSUPPORTED;
-  if (!z || !packed || !left_dst || !right_dst || !status) return B200_TRIMUL_E_NULL;
+  if (!z || (!packed && !raw) || !left_dst || !right_dst || !status) return B200_TRIMUL_E_NULL;
   if (n_left < 1 || n_left > kMaxDst || n_right < 1 || n_right > kMaxDst) return B200_TRIMUL_E_SHAPE;
   if (mode != kLocal && B != 1) return B200_TRIMUL_E_SHAPE;
   if (mode == kChannels && (n_left != n_right || kC % n_left != 0 || (kC / n_left) % 8 != 0)) return B200_TRIMUL_E_SHAPE;
@@ -649,7 +532,7 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
   if (rc != B200_TRIMUL_OK) return rc;
   if (ld == 0) ld = N;
   if (rows < 1 || row_begin < 0 || row_begin + rows > N) return B200_TRIMUL_E_SHAPE;
-  if (!aligned(z, 16) || !aligned(packed, 1024)) return B200_TRIMUL_E_ALIGN;
+  if (!aligned(z, 16) || (!raw && !aligned(packed, 1024))) return B200_TRIMUL_E_ALIGN;
   DeviceInfo info;
   rc = device_info(&info);
   if (rc != B200_TRIMUL_OK) return rc;
@@ -709,12 +592,23 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
   p.num_tiles = B * rows * p.tiles_per_row;
   p.token_mask = token_mask;
   p.pair_mask = pair_mask;
-  p.w = static_cast<const uint4*>(packed);  // the four left / right matrices, one after the other
-  p.d1 = reinterpret_cast<const float*>(static_cast<const uint8_t*>(packed) + kPackedD1Off);
-  p.ln_w = reinterpret_cast<const float*>(static_cast<const uint8_t*>(packed) + kPackedLnOff);
-  p.ln_b = p.ln_w + 128;
+  p.raw = raw != nullptr ? 1 : 0;
+  p.raw_block = raw_block;
+  p.pack_blocks = pack_blocks;
+  if (raw != nullptr) {
+    p.w = nullptr;
+    p.d1 = nullptr;
+    p.ln_w = raw->block[raw_block].ln_in_w;
+    p.ln_b = raw->block[raw_block].ln_in_b;
+  } else {
+    p.w = static_cast<const uint4*>(packed);  // the four left / right matrices, one after the other
+    p.d1 = reinterpret_cast<const float*>(static_cast<const uint8_t*>(packed) + kPackedD1Off);
+    p.ln_w = reinterpret_cast<const float*>(static_cast<const uint8_t*>(packed) + kPackedLnOff);
+    p.ln_b = p.ln_w + 128;
+  }
+  static const PackLaunch no_params = {};
+  const PackLaunch& params = raw != nullptr ? *raw : no_params;
   p.eps = eps_in;
-  p.early = early ? 1 : 0;
   p.status = status;
   const int pairs = p.num_tiles < info.sms / 2 ? p.num_tiles : info.sms / 2;
   const int grid = 2 * pairs;  // clusters of two CTAs: CTA 0 produces `left`, CTA 1 `right`
@@ -723,7 +617,7 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
   do {                                                                                               \
     rc = set_smem(prologue_kernel<BIAS, DP>, kProSmemBytes, info.device);                            \
     if (rc != B200_TRIMUL_OK) return rc;                                                             \
-    TRIMUL_CUDA(launch_overlapped(prologue_kernel<BIAS, DP>, grid, kProThreads, kProSmemBytes, stream, map_z, out, p)); \
+    TRIMUL_CUDA(launch_overlapped(prologue_kernel<BIAS, DP>, grid, kProThreads, kProSmemBytes, stream, map_z, out, params, p)); \
   } while (0)
   if (d_pair == kC) {
     if (has_bias) TRIMUL_LAUNCH_PROLOGUE(true, 128);
@@ -1190,11 +1084,13 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
   int has_bias = 0;
   if (bias_opt != nullptr)
     for (int i = 0; i < 4; ++i) has_bias |= bias_opt[i] != nullptr;
-  auto prologue = [&](const void* pk) {
+  PackLaunch pk;
+  // stage 1 takes its weights from the parameters; the call's first launch packs those of stage 3 and clears the status words
+  auto prologue = [&](int block, int pack_blocks) {
     void* l[1] = {left};
     void* r[1] = {right};
-    return prologue_impl(z, pk, token_mask, pair_mask, l, 1, r, 1, kLocal, B, N, 0, N, eps_in, has_bias, status, cuda_stream,
-                         d_pair, ld, true);
+    return prologue_impl(z, nullptr, token_mask, pair_mask, l, 1, r, 1, kLocal, B, N, 0, N, eps_in, has_bias, status, cuda_stream,
+                         d_pair, ld, &pk, block, pack_blocks);
   };
   auto contract = [&](void* dst, int dir) {
     return contract_impl(left, right, dst, nullptr, 0, 0, kC, B, N, 0, N, N, dir, status, cuda_stream, 0, ld);
@@ -1205,10 +1101,10 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
     // to_gate [64, 64] for both forms; the bidirectional module contracts channels 0-63 outgoing and 64-127 incoming.
     if (drop_scale != nullptr) return B200_TRIMUL_E_UNSUPPORTED;
     if (!w_left || !w_left_gate || !w_right || !w_right_gate || !w_gate || !w_out) return B200_TRIMUL_E_NULL;
-    rc = pack_one(w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w, ln_out_b,
-                  bias_opt, packed, 64, status, cuda_stream);
+    rc = fill_pack(pk, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
+                   ln_out_b, bias_opt, packed, 64);
     if (rc != B200_TRIMUL_OK) return rc;
-    rc = prologue(packed);
+    rc = prologue(0, 1);
     if (rc != B200_TRIMUL_OK) return rc;
     if (direction == B200_TRIMUL_BIDIRECTIONAL) {
       const size_t half = static_cast<size_t>(64) * ld * 2;  // bytes from channel 0 to channel 64 of a pair row
@@ -1229,24 +1125,24 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
     const size_t plane = plane_tensor_bytes(B, N, ld);
     void* tri_in = ws + off[4] + plane;
     void* packed_in = ws + off[4] + 2 * plane;
-    rc = pack_bidir(w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w,
-                                        ln_in_b, ln_out_w, ln_out_b, bias_opt, packed, packed_in, status, cuda_stream);
+    rc = fill_pack_bidir(pk, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
+                         ln_out_b, bias_opt, packed, packed_in);
     if (rc != B200_TRIMUL_OK) return rc;
-    rc = prologue(packed);
+    rc = prologue(0, 2);
     if (rc != B200_TRIMUL_OK) return rc;
     rc = contract(tri, B200_TRIMUL_OUTGOING);
     if (rc != B200_TRIMUL_OK) return rc;
-    rc = prologue(packed_in);
+    rc = prologue(1, 0);
     if (rc != B200_TRIMUL_OK) return rc;
     rc = contract(tri_in, B200_TRIMUL_INCOMING);
     if (rc != B200_TRIMUL_OK) return rc;
     return epilogue_wide_impl(tri, tri_in, z, packed, packed_in, drop_scale, y, B, N, N, eps_in, eps_out, residual,
                                      status, cuda_stream, ld, true);
   }
-  rc = pack_one(w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w,
-                                ln_in_b, ln_out_w, ln_out_b, bias_opt, packed, kC, status, cuda_stream);
+  rc = fill_pack(pk, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
+                 ln_out_b, bias_opt, packed, kC);
   if (rc != B200_TRIMUL_OK) return rc;
-  rc = prologue(packed);
+  rc = prologue(0, 1);
   if (rc != B200_TRIMUL_OK) return rc;
   rc = contract(tri, direction);
   if (rc != B200_TRIMUL_OK) return rc;

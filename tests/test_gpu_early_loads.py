@@ -47,3 +47,34 @@ def test_stack_of_calls(kind, c, n, graph):
     else:
         got = run(False)
     assert torch.isfinite(want).all() and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+def test_arguments_written_by_the_launch_before(kind):
+    """Parameters, masks and the pair tensor are changed in place right before every call."""
+    g = torch.Generator().manual_seed(5)
+    m = KINDS[kind](128).to(DEV).to(torch.bfloat16).eval()
+    n = 136
+    z = torch.randn(1, n, n, 128, generator=g).to(torch.bfloat16).to(DEV)
+    mask = (torch.rand(1, n, generator=g) >= 0.3).to(DEV)
+    start = {k: v.detach().clone() for k, v in m.named_parameters()}
+    z0, mask0 = z.clone(), mask.clone()
+
+    def run(wait):
+        out = []
+        with torch.no_grad():
+            for k, v in m.named_parameters():
+                v.copy_(start[k])
+            z.copy_(z0), mask.copy_(mask0)
+            for i in range(8):
+                changed = [z, mask, *m.parameters()]
+                for t in changed[i % len(changed) :] + changed[: i % len(changed)]:  # each is the last one once
+                    t.logical_not_() if t.dtype == torch.bool else t.mul_(-0.75)
+                if wait:
+                    torch.cuda.synchronize()
+                out.append(m(z, mask))
+                if wait:
+                    torch.cuda.synchronize()
+        return out
+
+    assert all(torch.equal(a, b) for a, b in zip(run(True), run(False)))
