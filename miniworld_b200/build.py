@@ -84,7 +84,7 @@ def build_native(force: bool = False) -> Path:
     _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native", "-DTORCH_API_INCLUDE_EXTENSION_H",
           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{root}/include",
           f"-I{root}/include/torch/csrc/api/include", f"-I{cuda}/include", f"-I{sysconfig.get_paths()['include']}",
-          str(HOST_SOURCE), "-o", str(tmp), f"-L{root}/lib", "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda",
+          str(HOST_SOURCE), "-o", str(tmp), f"-L{root}/lib", "-ltorch", "-ltorch_cpu", "-ltorch_python", "-ltorch_cuda", "-lc10", "-lc10_cuda",
           f"-L{PKG_DIR}", f"-l:{LIB_NAME}", "-Wl,-rpath,$ORIGIN"])
     os.replace(tmp, NATIVE_PATH)
     NATIVE_TAG_PATH.write_text(native_tag())
