@@ -368,6 +368,12 @@ int b200_transition_pack_weights(const void* w_expand_a, const void* w_expand_b,
                                  const float* ln_w, const float* ln_b, void* packed, void* cuda_stream);
 int b200_transition_forward(const void* x, const void* packed, void* y, long long positions, int d, int n, float eps,
                             int residual, int* status, void* cuda_stream);
+/* Both of these in one call: the first input tiles are read and normalised while the weights are packed. `clear_status`
+ * non-zero zeroes the 16 status words first. */
+int b200_transition_pack_forward(const void* x, const void* w_expand_a, const void* w_expand_b, const void* w_squeeze,
+                                 int weight_dtype, const float* ln_w, const float* ln_b, void* packed, void* y,
+                                 long long positions, int d, int n, float eps, int residual, int* status, int clear_status,
+                                 void* cuda_stream);
 
 /* Zero the status words at the start of a workspace (asynchronous). */
 int b200_trimul_clear_status(int* status, void* cuda_stream);

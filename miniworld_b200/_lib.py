@@ -121,6 +121,10 @@ SIGNATURES = {
         c_int,
         [c_void_p, c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
     ),
+    "b200_transition_pack_forward": (
+        c_int,
+        [c_void_p] * 4 + [c_int] + [c_void_p] * 4 + [ctypes.c_longlong, c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p],
+    ),
     "b200_transition_backward_workspace_bytes": (c_int, [ctypes.c_longlong, POINTER(c_size_t)]),
     "b200_transition_backward": (
         c_int,

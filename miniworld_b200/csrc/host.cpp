@@ -294,14 +294,11 @@ bool transition_plain(const Tensor& x, at::TensorList p) {
 int dtype_code(const Tensor& w) { return w.scalar_type() == at::kBFloat16 ? B200_TRIMUL_DTYPE_BF16 : B200_TRIMUL_DTYPE_F32; }
 
 void launch_transition(const Tensor& x, at::TensorList p, double eps, bool residual, void* packed, int* status,
-                       const Tensor& y) {
-  void* stream = stream_of(x);
-  check(b200_transition_pack_weights(p[kTrA].data_ptr(), p[kTrB].data_ptr(), p[kTrS].data_ptr(), dtype_code(p[kTrA]),
-                                     static_cast<const float*>(p[kTrLnW].data_ptr()),
-                                     static_cast<const float*>(p[kTrLnB].data_ptr()), packed, stream),
-        "b200_transition_pack_weights");
-  check(b200_transition_forward(x.data_ptr(), packed, y.data_ptr(), x.numel() / 128, 128, 4, static_cast<float>(eps),
-                                residual ? 1 : 0, status, stream),
+                       bool clear_status, const Tensor& y) {
+  check(b200_transition_pack_forward(x.data_ptr(), p[kTrA].data_ptr(), p[kTrB].data_ptr(), p[kTrS].data_ptr(), dtype_code(p[kTrA]),
+                        static_cast<const float*>(p[kTrLnW].data_ptr()), static_cast<const float*>(p[kTrLnB].data_ptr()), packed,
+                        y.data_ptr(), x.numel() / 128, 128, 4, static_cast<float>(eps), residual ? 1 : 0, status,
+                        clear_status ? 1 : 0, stream_of(x)),
         "b200_transition_forward");
 }
 
@@ -315,17 +312,11 @@ std::optional<std::tuple<Tensor, Kept>> transition_forward(const Tensor& x, cons
   const c10::cuda::CUDAGuard guard(x.device());
   const size_t bytes = b200_transition_packed_bytes();
   const int64_t stream = stream_key(x);
-  Tensor scratch;
-  if (kept.has_value() && usable(std::get<1>(*kept), std::get<0>(*kept), stream, x)) {
-    scratch = std::get<1>(*kept);
-  } else {
-    scratch = aligned_empty(bytes + 64, x);
-    check(b200_trimul_clear_status(reinterpret_cast<int*>(static_cast<uint8_t*>(scratch.data_ptr()) + bytes), stream_of(x)),
-          "b200_trimul_clear_status");
-  }
+  const bool keep = kept.has_value() && usable(std::get<1>(*kept), std::get<0>(*kept), stream, x);
+  const Tensor scratch = keep ? std::get<1>(*kept) : aligned_empty(bytes + 64, x);
   uint8_t* base = static_cast<uint8_t*>(scratch.data_ptr());
   Tensor y = empty_on(x.sizes(), at::kBFloat16, x);
-  launch_transition(x, params, eps, residual, base, reinterpret_cast<int*>(base + bytes), y);
+  launch_transition(x, params, eps, residual, base, reinterpret_cast<int*>(base + bytes), !keep, y);
   return std::make_tuple(y, Kept(stream, scratch));
 }
 
@@ -336,9 +327,8 @@ struct TransitionNode : public torch::autograd::Function<TransitionNode> {
     const Tensor scratch = scratch_for(bytes + 64, x);  // packed weights, then the status words
     uint8_t* base = aligned_start(scratch);
     int* status = reinterpret_cast<int*>(base + bytes);
-    check(b200_trimul_clear_status(status, stream_of(x)), "b200_trimul_clear_status");
     Tensor y = empty_on(x.sizes(), at::kBFloat16, x);
-    launch_transition(x, params, eps, residual, base, status, y);
+    launch_transition(x, params, eps, residual, base, status, true, y);
     variable_list save;
     save.push_back(x);
     save.insert(save.end(), params.begin(), params.end());

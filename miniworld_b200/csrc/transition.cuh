@@ -31,6 +31,8 @@
 // group. Three input stages let LayerNorm of tile t + 2 run while tile t is still being written out.
 // G1 and G2 have an issuing thread each: issuing one 256 x 128 x 16 MMA costs about as long as it runs, so a single
 // thread that also waits for the SwiGLU warps between the two GEMMs leaves the tensor pipe idle half of the time.
+// In a call that packs the weights itself the first input tiles are read and normalised while it does: 48 x 48 positions, where
+// the launch's latencies count, 16.4 -> 13.4 us, 512 x 512 111.4 -> 109.5.
 // Only mbarrier signals cross between the two CTAs. All waits are bounded.
 #pragma once
 
@@ -46,6 +48,7 @@ struct TransitionParams {
   const __nv_bfloat16* x;  // the input again, for the residual
   float eps;
   int residual;
+  int early;  // x, ln_w and ln_b are older than the kernel before this one
   int* status;
 };
 
@@ -123,12 +126,15 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     tmem_alloc_pair(smem_u32(tmem_slot), 512);
     tmem_relinquish_pair();
   }
-  grid_dependency_wait();
-  grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // barriers of both CTAs are initialised before any signal crosses
   tc_fence_after();
+  // (the first input tiles land and are normalised while the weights are packed)
+  if (!p.early || warp == 0 || warp >= 28) {
+    grid_dependency_wait();
+    grid_dependents_launch();
+  }
   const uint32_t tmem_base = *tmem_slot;
 
   // tiles of this pair: tile index t_local = 0, 1, ... <-> global tile pair + t_local * num_pairs
@@ -137,12 +143,12 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   if (warp == 0) {
     // ------------------------------------------------------------ weight producer (both CTAs): 8 blocks per tile
     if (lane == 0) {
-      const long long total = static_cast<long long>(my_tiles) * kTrBlocks;
-      for (long long gb = 0; gb < total; ++gb) {
-        const int slot = static_cast<int>(gb % WS);
+      const int total = my_tiles * kTrBlocks;
+      for (int gb = 0; gb < total; ++gb) {
+        const int slot = gb % WS;
         const uint32_t ph = static_cast<uint32_t>((gb / WS) & 1);
         if (!mbar_wait(blk_done(slot), ph ^ 1u, abort_flag, p.status, kDevTimeoutProducer)) break;
-        const int hb = static_cast<int>(gb % kTrBlocks);
+        const int hb = gb % kTrBlocks;
         if (rank == 0) mbar_arrive_expect_tx(w_full(slot), 2 * kTrWStageBytes);  // bytes of both CTAs
         const uint32_t bar = map_to_cta(w_full(slot), 0);
         const uint32_t ws = w_base + slot * kTrWStageBytes;
@@ -155,11 +161,11 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       }
       // Drain (leader: its barriers count the bytes of both CTAs; the closing cluster barrier keeps CTA 1 alive).
       if (rank == 0) {
-        const long long pending = total < WS ? total : WS;
-        for (long long back = 1; back <= pending; ++back) {
-          const long long gb = total - back;
+        const int pending = total < WS ? total : WS;
+        for (int back = 1; back <= pending; ++back) {
+          const int gb = total - back;
           const long long t0 = clock64();
-          while (!mbar_try_wait(w_full(static_cast<int>(gb % WS)), static_cast<uint32_t>((gb / WS) & 1))) {
+          while (!mbar_try_wait(w_full(gb % WS), static_cast<uint32_t>((gb / WS) & 1))) {
             if (*abort_flag != 0 || clock64() - t0 > kWaitLimitCycles) {
               atomicCAS(p.status, 0, kDevTimeoutDrain);
               break;
@@ -189,15 +195,15 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     // has taken its previous contents into registers.
     if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = umma_idesc(256, 128, false, false, kFmtF16, kFmtF16);
-      const long long total = static_cast<long long>(my_tiles) * kTrBlocks;
-      for (long long gb = 0; gb < total; ++gb) {
-        const int t = static_cast<int>(gb / kTrBlocks);
-        const int hb = static_cast<int>(gb % kTrBlocks);
+      const int total = my_tiles * kTrBlocks;
+      for (int gb = 0; gb < total; ++gb) {
+        const int t = gb / kTrBlocks;
+        const int hb = gb % kTrBlocks;
         const int s = t % XS;
         if (hb == 0 && !mbar_wait(xn_ready(s), (t / XS) & 1, abort_flag, p.status, kDevTimeoutMma)) break;
-        const int slot = static_cast<int>(gb % WS);
+        const int slot = gb % WS;
         if (!mbar_wait(w_full(slot), static_cast<uint32_t>((gb / WS) & 1), abort_flag, p.status, kDevTimeoutMma)) break;
-        const int b = static_cast<int>(gb & 1);
+        const int b = gb & 1;
         if (!mbar_wait(d1_empty(b), static_cast<uint32_t>(((gb >> 1) & 1) ^ 1), abort_flag, p.status, kDevTimeoutMma)) break;
         tc_fence_after();
         const uint32_t xs = x_base + s * kTrXBytes;
@@ -217,12 +223,12 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     // before h could be computed, so one commit after G2 says that the block's weight stage and its H buffer are free.
     if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = umma_idesc(256, 128, false, false, kFmtF16, kFmtF16);
-      const long long total = static_cast<long long>(my_tiles) * kTrBlocks;
-      for (long long gb = 0; gb < total; ++gb) {
-        const int t = static_cast<int>(gb / kTrBlocks);
-        const int hb = static_cast<int>(gb % kTrBlocks);
-        const int b = static_cast<int>(gb & 1);
-        const int slot = static_cast<int>(gb % WS);
+      const int total = my_tiles * kTrBlocks;
+      for (int gb = 0; gb < total; ++gb) {
+        const int t = gb / kTrBlocks;
+        const int hb = gb % kTrBlocks;
+        const int b = gb & 1;
+        const int slot = gb % WS;
         // D2[t & 1] last held tile t - 2 (and lent its first columns to h during tile t - 1, whose G2s this thread has
         // issued before): wait until the output group has read tile t - 2 out of it
         if (hb == 0 && !mbar_wait(d2_empty(t & 1), ((t >> 1) & 1) ^ 1u, abort_flag, p.status, kDevTimeoutMma)) break;
@@ -322,7 +328,7 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       bool alive = true;
 #pragma unroll 1
       for (int hb = grp; hb < kTrBlocks; hb += 2) {
-        const long long gb = static_cast<long long>(t) * kTrBlocks + hb;
+        const int gb = t * kTrBlocks + hb;
         const uint32_t bph = static_cast<uint32_t>((gb >> 1) & 1);
         if (!mbar_wait_warp(d1_full(grp), bph, abort_flag, p.status, kDevTimeoutEpilogue)) {
           alive = false;
@@ -354,8 +360,8 @@ transition_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         // also waits until this CTA's output group has read tile t - 1 out of the D2 buffer that h borrows
         const uint32_t t_h = t_h0 + ((hb >> 1) & 1) * 64;
         if (gb >= 4) {
-          const long long pb = gb - 4;
-          if (!mbar_wait_warp(blk_done(static_cast<int>(pb % WS)), static_cast<uint32_t>((pb / WS) & 1), abort_flag, p.status,
+          const int pb = gb - 4;
+          if (!mbar_wait_warp(blk_done(pb % WS), static_cast<uint32_t>((pb / WS) & 1), abort_flag, p.status,
                               kDevTimeoutEpilogue)) {
             alive = false;
             break;
@@ -484,8 +490,10 @@ __device__ __forceinline__ float load_weight(const void* w, size_t idx, int f32)
   return f32 ? static_cast<const float*>(w)[idx] : __bfloat162float(static_cast<const __nv_bfloat16*>(w)[idx]);
 }
 
-__global__ void __launch_bounds__(256) transition_pack_kernel(const TransitionPackArgs a, uint8_t* packed) {
+// (clears the status words of the call that follows, if given)
+__global__ void __launch_bounds__(256) transition_pack_kernel(const TransitionPackArgs a, uint8_t* packed, int* clear_status) {
   grid_dependents_launch();
+  if (clear_status != nullptr && blockIdx.x == 0 && threadIdx.x < 16) clear_status[threadIdx.x] = 0;
   const int i = blockIdx.x * 256 + threadIdx.x;  // 0 .. 196607
   __half* ab = reinterpret_cast<__half*>(packed);
   __half* ws = reinterpret_cast<__half*>(packed + kTrPackedAbBytes);

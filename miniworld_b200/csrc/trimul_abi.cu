@@ -1191,8 +1191,8 @@ int b200_trimul_forward(const void* z, const void* w_left, const void* w_left_ga
 // --------------------------------------------------------------------------------------------- pair Transition
 size_t b200_transition_packed_bytes(void) { return kTrPackedBytes; }
 
-int b200_transition_pack_weights(const void* w_expand_a, const void* w_expand_b, const void* w_squeeze, int weight_dtype,
-                                 const float* ln_w, const float* ln_b, void* packed, void* cuda_stream) {
+static int transition_pack_impl(const void* w_expand_a, const void* w_expand_b, const void* w_squeeze, int weight_dtype,
+                                const float* ln_w, const float* ln_b, void* packed, int* clear_status, void* cuda_stream) {
   if (!w_expand_a || !w_expand_b || !w_squeeze || !ln_w || !ln_b || !packed) return B200_TRIMUL_E_NULL;
   if (weight_dtype != B200_TRIMUL_DTYPE_BF16 && weight_dtype != B200_TRIMUL_DTYPE_F32) return B200_TRIMUL_E_SHAPE;
   if (!aligned(packed, 1024)) return B200_TRIMUL_E_ALIGN;
@@ -1204,13 +1204,19 @@ int b200_transition_pack_weights(const void* w_expand_a, const void* w_expand_b,
   a.ln_b = ln_b;
   a.f32_weights = weight_dtype == B200_TRIMUL_DTYPE_F32;
   transition_pack_kernel<<<(1024 * 128 + 128 * 512) / 256, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
-      a, static_cast<uint8_t*>(packed));
+      a, static_cast<uint8_t*>(packed), clear_status);
   TRIMUL_CUDA(cudaGetLastError());
   return B200_TRIMUL_OK;
 }
 
-int b200_transition_forward(const void* x, const void* packed, void* y, long long positions, int d, int n, float eps,
-                            int residual, int* status, void* cuda_stream) {
+int b200_transition_pack_weights(const void* w_expand_a, const void* w_expand_b, const void* w_squeeze, int weight_dtype,
+                                 const float* ln_w, const float* ln_b, void* packed, void* cuda_stream) {
+  return transition_pack_impl(w_expand_a, w_expand_b, w_squeeze, weight_dtype, ln_w, ln_b, packed, nullptr, cuda_stream);
+}
+
+// ln_w, ln_b: the parameters, where the packing is this call's own launch before (and x, the parameters are older than that)
+static int transition_impl(const void* x, const void* packed, void* y, long long positions, int d, int n, float eps,
+                           int residual, const float* ln_w, const float* ln_b, int* status, void* cuda_stream) {
   if (!x || !packed || !y || !status) return B200_TRIMUL_E_NULL;
   if (d != kC || n != 4) return B200_TRIMUL_E_UNSUPPORTED;
   if (positions < 1 || positions > 0x7FFFFFFFll - 512) return B200_TRIMUL_E_SHAPE;
@@ -1245,8 +1251,9 @@ int b200_transition_forward(const void* x, const void* packed, void* y, long lon
   TransitionParams p;
   p.positions = positions;
   p.num_tiles = static_cast<int>((positions + 255) / 256);
-  p.ln_w = reinterpret_cast<const float*>(static_cast<const uint8_t*>(packed) + kTrPackedLnOff);
-  p.ln_b = p.ln_w + 128;
+  p.early = ln_w != nullptr ? 1 : 0;
+  p.ln_w = ln_w != nullptr ? ln_w : reinterpret_cast<const float*>(static_cast<const uint8_t*>(packed) + kTrPackedLnOff);
+  p.ln_b = ln_w != nullptr ? ln_b : p.ln_w + 128;
   p.x = static_cast<const __nv_bfloat16*>(x);
   p.eps = eps;
   p.residual = residual;
@@ -1257,6 +1264,20 @@ int b200_transition_forward(const void* x, const void* packed, void* y, long lon
   TRIMUL_CUDA(launch_overlapped(transition_kernel, 2 * pairs, kTrThreads, kTrSmemBytes, static_cast<cudaStream_t>(cuda_stream),
                                 map_x, map_y, map_wab, map_ws, p));
   return B200_TRIMUL_OK;
+}
+
+int b200_transition_forward(const void* x, const void* packed, void* y, long long positions, int d, int n, float eps,
+                            int residual, int* status, void* cuda_stream) {
+  return transition_impl(x, packed, y, positions, d, n, eps, residual, nullptr, nullptr, status, cuda_stream);
+}
+
+int b200_transition_pack_forward(const void* x, const void* w_expand_a, const void* w_expand_b, const void* w_squeeze, int weight_dtype,
+                    const float* ln_w, const float* ln_b, void* packed, void* y, long long positions, int d, int n, float eps,
+                    int residual, int* status, int clear_status, void* cuda_stream) {
+  int rc = transition_pack_impl(w_expand_a, w_expand_b, w_squeeze, weight_dtype, ln_w, ln_b, packed,
+                                clear_status != 0 ? status : nullptr, cuda_stream);
+  if (rc != B200_TRIMUL_OK) return rc;
+  return transition_impl(x, packed, y, positions, d, n, eps, residual, ln_w, ln_b, status, cuda_stream);
 }
 
 }  // extern "C"
