@@ -78,3 +78,33 @@ def test_arguments_written_by_the_launch_before(kind):
         return out
 
     assert all(torch.equal(a, b) for a, b in zip(run(True), run(False)))
+
+
+@pytest.mark.parametrize("kind", [*KINDS, "transition"])
+@pytest.mark.parametrize("n", [8, 136, 200])
+def test_training_steps_in_a_row(kind, n):
+    """The backward's kernels read what is older than the launch before them while that one finishes: steps without a pause, with
+    z and the output's gradient written by the launches right before the passes, against steps with the device idle in between.
+    (Every order of additions in a step is fixed.)"""
+    g = torch.Generator().manual_seed(n)
+    m = (mw.Transition(128) if kind == "transition" else KINDS[kind](128)).to(DEV).to(torch.bfloat16).train()
+    z0 = torch.randn(1, n, n, 128, generator=g).to(torch.bfloat16).to(DEV)
+    dy0 = torch.randn(1, n, n, 128, generator=g).to(torch.bfloat16).to(DEV)
+    mask = (torch.rand(1, n, generator=g) >= 0.1).to(DEV)
+
+    def run(wait):
+        z, out = z0.clone().requires_grad_(), []
+        pause = torch.cuda.synchronize if wait else lambda: None
+        for i in range(4):
+            with torch.no_grad():
+                z.copy_(z0 * (1 - 0.25 * i))
+            pause()
+            y = m(z) if kind == "transition" else m(z, mask)
+            pause()
+            dy = dy0 * (0.5 + 0.25 * i)
+            pause()
+            out += torch.autograd.grad(y, [z, *m.parameters()], dy)
+            pause()
+        return out
+
+    assert all(torch.equal(a, b) for a, b in zip(run(True), run(False)))
