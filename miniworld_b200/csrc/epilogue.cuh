@@ -107,8 +107,9 @@ epilogue_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant
   if (threadIdx.x >= 64 && threadIdx.x < 64 + C / 2) {
     // constants regrouped per channel pair so that one 16-byte load feeds a packed fp32x2 FMA
     const int cp = threadIdx.x - 64;
-    const float4 a = p.c3[2 * cp];
-    const float4 b = p.c3[2 * cp + 1];
+    // (past L1: the call before may have left other constants of the same workspace in it, see grid_dependency_wait)
+    const float4 a = __ldcg(p.c3 + 2 * cp);
+    const float4 b = __ldcg(p.c3 + 2 * cp + 1);
     const_ptr[2 * cp] = make_float4(a.x, b.x, a.y, b.y);      // s_gate pair, d_gate pair
     const_ptr[2 * cp + 1] = make_float4(a.z, b.z, a.w, b.w);  // s_out pair,  d_out pair
   }

@@ -114,11 +114,12 @@ epilogue_wide_kernel(const __grid_constant__ CUtensorMap map_t0, const __grid_co
   if (threadIdx.x >= 64 && threadIdx.x < 128) {
     // constants regrouped per channel pair so that one 16-byte load feeds a packed fp32x2 FMA
     const int cp = threadIdx.x - 64;
-    float4 a = p.c3_a[2 * cp];
-    float4 b = p.c3_a[2 * cp + 1];
+    // (past L1: the call before may have left other constants of the same workspace in it, see grid_dependency_wait)
+    float4 a = __ldcg(p.c3_a + 2 * cp);
+    float4 b = __ldcg(p.c3_a + 2 * cp + 1);
     if constexpr (KCH == 4) {
-      const float4 a1 = p.c3_b[2 * cp];
-      const float4 b1 = p.c3_b[2 * cp + 1];
+      const float4 a1 = __ldcg(p.c3_b + 2 * cp);
+      const float4 b1 = __ldcg(p.c3_b + 2 * cp + 1);
       a.z += a1.z, a.w += a1.w, b.z += b1.z, b.w += b1.w;
     }
     const_ptr[2 * cp] = make_float4(a.x, b.x, a.y, b.y);      // s_gate pair, d_gate pair

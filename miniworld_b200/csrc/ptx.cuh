@@ -130,21 +130,24 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
 
 // ------------------------------------------------------------------ dependent launches
 // Waits until the kernel before this one on the stream has completed and its writes are visible (returns at once if the
-// launch does not overlap it). Every thread calls it before it touches global memory.
+// launch does not overlap it). What may be touched before it: what is older than the kernel before this one, for reading, and
+// that only where the launch says so (`early`, and the rules at the backward's copies): what a call was given, and what its
+// launches before that one wrote. Threads that read anything else, and all that write, call it first.
+// (Early z and weights: N = 203 40.3 -> 39.0 us, N = 384 90.6 -> 89.4, bidirectional N = 512 265.7 -> 264.9, with dropout in
+// training N = 256 387 -> 380.)
 //
 // A kernel's life begins before the one before it has ended, so two kinds of loads must not read what that one may write:
 // - non-coherent ones (ld.global.nc, __ldg), which are for data that does not change during the kernel's life;
 // - plain ones, if that kernel has also READ it through its SMs' L1: a line that it left there is found again (measured: the
 //   running d x_hat of the Transition's backward, read with plain loads and stored by TMA in every launch, came back old in
-//   the next launch and put its gradients off by 3e-3). Such data is read through TMA or with ld_gpu_chunks.
+//   the next launch and put its gradients off by 3e-3). Such data is read through TMA, with __ldcg or with ld_gpu_chunks.
+// The same holds over a chain of overlapped launches, a whole forward and the next one on the same workspace: the packed weights
+// and constants that one call reads are written again by the next, and no ordinary launch in between empties L1. They are read
+// through TMA or with __ldcg.
 // The first kernel of an entry point may follow any kernel of the caller, the entry point's own last one with its output as
-// this one's input among them. Memory written earlier is safe: the predecessor has itself waited before it let this kernel begin.
+// this one's input among them. Memory written earlier is in L2 by then: the predecessor has itself waited before it let this
+// kernel begin, and what a kernel has written is in L2 when it has ended.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// A kernel whose launch says that some inputs are older than the kernel before it (`early`: what a module call was given, and
-// what its launches before that one wrote) reads those while that kernel finishes; the threads that read anything else, and
-// all that write, still wait.
-// (N = 203: 40.3 -> 39.0 us, N = 384: 90.6 -> 89.4, bidirectional N = 512: 265.7 -> 264.9, with dropout in training N = 256:
-// 387 -> 380; the prologue's input lands while the weights are packed, the epilogues' weights and z while the contraction ends.)
 // `CHUNKS` 16-byte pieces (an even count) from p at gpu scope, which no line in L1 answers: 32-byte requests if the address allows
 template <int CHUNKS>
 __device__ __forceinline__ void ld_gpu_chunks(const uint4* p, bool wide, uint4 (&out)[CHUNKS]) {

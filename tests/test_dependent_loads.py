@@ -33,3 +33,16 @@ def test_non_coherent_loads_are_the_listed_ones():
     assert not unknown, unknown
     unused = [a for a in ALLOWED if not any(f[0] == a[0] and a[1] in f[1] for f in found)]
     assert not unused, unused
+
+
+def test_packed_constants_are_read_past_l1():
+    """What one call of a chain of overlapped launches packs, the next one on the same workspace packs again, with no ordinary launch
+    in between that would empty L1."""
+    reads = []
+    for path in sorted(CSRC.glob("prologue*")) + sorted(CSRC.glob("epilogue*")):
+        for line in path.read_text().splitlines():
+            code = line.split("//")[0]
+            if re.search(r"\bp\.(c3|c3_a|c3_b|d1|ln_w|ln_b)\b", code):
+                reads.append((path.name, code.strip()))
+    assert {name for name, _ in reads} == {"prologue_stats.inc", "prologue_epilogue.inc", "epilogue.cuh", "epilogue_wide.cuh"}
+    assert not [r for r in reads if "__ldcg(" not in r[1]]

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import miniworld_b200 as mw
+from miniworld_b200 import functional as F_
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -108,3 +109,41 @@ def test_training_steps_in_a_row(kind, n):
         return out
 
     assert all(torch.equal(a, b) for a, b in zip(run(True), run(False)))
+
+
+@pytest.mark.parametrize("kind,c,drop", [("outgoing", 128, False), ("incoming", 64, False), ("bidirectional", 128, False),
+                                         ("outgoing", 128, True), ("bidirectional", 128, True)])
+@pytest.mark.parametrize("n", [8, 56, 136])
+def test_two_parameter_sets_on_one_workspace(kind, c, drop, n):
+    """Calls back to back with nothing between them, every one with other weights, LayerNorms and biases than the one before and
+    the same workspace: each packs its own constants where those of the call before were read."""
+    g = torch.Generator().manual_seed(n)
+    module = KINDS[kind](c)
+    outgoing = {"outgoing": True, "incoming": False, "bidirectional": None}[kind]
+    z = torch.randn(1, n, n, c, generator=g).to(torch.bfloat16).to(DEV)
+    scale = (torch.rand(1, n, c, generator=g) + 0.5).to(torch.bfloat16).to(DEV) if drop else None
+    sets = []
+    for _ in range(2):
+        p = {k: (torch.randn(v.shape, generator=g) * (0.3 if v.dim() == 1 else v.shape[-1] ** -0.5) + (v.dim() == 1)).to(DEV)
+             for k, v in module.named_parameters()}
+        b = {k: torch.randn(p[f"{k}.weight"].shape[0], generator=g).to(DEV) for k in ("to_left", "to_right_gate", "to_gate", "to_out")}
+        sets.append((p, F_._Weights(p, b, torch.device(DEV), bidirectional=outgoing is None, d_pair=c)))
+    ws = F_.aligned_empty(F_.workspace_bytes(1, n, outgoing, c), torch.device(DEV))
+
+    def run(out, wait=False):
+        for i, y in enumerate(out):
+            p, w = sets[i % 2]
+            F_.trimul_forward(z, p, outgoing=outgoing, workspace=ws, out=y, weights=w, drop_scale=scale)
+            if wait:
+                torch.cuda.synchronize()
+
+    want, got, replayed = ([torch.zeros_like(z) for _ in range(count)] for count in (2, 40, 40))
+    run(want, wait=True)
+    assert not torch.equal(*want) and all(torch.isfinite(w).all() for w in want)
+    run(got)
+    graph = torch.cuda.CUDAGraph()  # (no host time between the launches)
+    with torch.cuda.graph(graph):
+        run(replayed)
+    for _ in range(3):
+        graph.replay()
+    assert all(torch.equal(y, want[i % 2]) for out in (got, replayed) for i, y in enumerate(out))
