@@ -610,7 +610,11 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
   const PackLaunch& params = raw != nullptr ? *raw : no_params;
   p.eps = eps_in;
   p.status = status;
-  const int pairs = p.num_tiles < info.sms / 2 ? p.num_tiles : info.sms / 2;
+  // A launch that packs takes the whole chip, however few tiles there are: the rows of the epilogue's matrices are shared out to
+  // one warp per pair, and with a pair per tile N = 1 left all 256 of them (bidirectional 384) to a single warp. Device time of a
+  // call (replayed graphs): N = 1 142.5 -> 15.0 us, 8 28.3 -> 15.4, 16 20.1 -> 15.4, 32 16.5 -> 15.8, 64 17.0 -> 17.1;
+  // bidirectional N = 1 217 -> 24.4, 16 35.2 -> 26.5; training step at N = 8 79.8 -> 66.0.
+  const int pairs = pack_blocks == 0 && p.num_tiles < info.sms / 2 ? p.num_tiles : info.sms / 2;
   const int grid = 2 * pairs;  // clusters of two CTAs: CTA 0 produces `left`, CTA 1 `right`
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
 #define TRIMUL_LAUNCH_PROLOGUE(BIAS, DP)                                                              \
