@@ -204,7 +204,8 @@ int b200_trimul_epilogue(const void* tri, const void* z, const void* packed, voi
                          float eps_in, float eps_out, int residual, int* status, void* cuda_stream);
 
 /*
- * Whole forward on one device: pack -> prologue -> contract -> epilogue, all on `cuda_stream`.
+ * Whole forward on one device: prologue -> contract -> epilogue, all on `cuda_stream`. The prologue takes its weights from the
+ * parameters and leaves the block of b200_trimul_pack_weights in the workspace on the way.
  * y = z + update when `residual` is non-zero (the reference module owns its residual,
  * src/miniworld/blocks/msa_module.py:116-117), else the update alone.
  * Mirrors `inference(leaves, flat_mask, flat_scale, direction)` of the reference engine

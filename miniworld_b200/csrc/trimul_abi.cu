@@ -1089,7 +1089,8 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
   if (bias_opt != nullptr)
     for (int i = 0; i < 4; ++i) has_bias |= bias_opt[i] != nullptr;
   PackLaunch pk;
-  // stage 1 takes its weights from the parameters; the call's first launch packs those of stage 3 and clears the status words
+  // stage 1 takes its weights from the parameters; the call's first launch packs those of stage 3, leaves its own beside them and
+  // clears the status words
   auto prologue = [&](int block, int pack_blocks) {
     void* l[1] = {left};
     void* r[1] = {right};

@@ -71,3 +71,31 @@ def test_backward_takes_weights_aligned_to_8_bytes():
     F_.trimul_forward(z, p, None, outgoing=None, workspace=ws)
     (dz0, g0), (dz1, g1) = (F_.trimul_backward(z, z, w, ws, None, outgoing=None, check=True) for w in (p, q))
     assert torch.equal(dz0, dz1) and all(torch.equal(g0[k], g1[k]) for k in g0)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("biased", [False, True])
+@pytest.mark.parametrize("bidir", [False, True])
+@pytest.mark.parametrize("B,n", [(1, 8), (1, 80), (2, 136)])
+def test_workspace_holds_the_packed_block(dtype, biased, bidir, B, n):
+    """The second region of a forward's workspace is the block that a packing launch writes, whole: for a look at the stages it can
+    be given to the first one."""
+    p, biases = _params(dtype, 256 if bidir else 128, n)
+    biases = biases if biased else None
+    z = torch.randn(B, n, n, 128, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
+    outgoing = None if bidir else False
+    ws = F_.aligned_empty(F_.workspace_bytes(B, n, outgoing), torch.device(DEV)).fill_(0xA5)
+    F_.trimul_forward(z, p, None, outgoing=outgoing, biases=biases, workspace=ws, check=True)
+    want, other = (F_.aligned_empty(F_.packed_bytes(), torch.device(DEV)) for _ in range(2))
+    F_.pack_weights_bidir(p, want, other, biases) if bidir else F_.pack_weights(p, want, biases)
+    off = F_.workspace_layout(B, n)
+    packed = ws[off[1] : off[1] + want.numel()]
+    assert torch.equal(packed, want)
+    if not bidir:  # (there the second half's planes are left behind)
+        left, right = (torch.empty(B, n, 128, n, dtype=torch.float16, device=DEV) for _ in range(2))
+        status = torch.zeros(16, dtype=torch.int32, device=DEV)
+        F_.prologue(z, packed, left, right, status, has_bias=biased)
+        F_.check_status(status, "prologue")
+        for k, t in ((2, left), (3, right)):
+            kept = ws[off[k] : off[k] + t.numel() * 2].view(torch.int16).view_as(t)
+            assert torch.equal(kept, t.view(torch.int16))
