@@ -761,7 +761,7 @@ def stage_roofline(r: Runner, steps: int, stream, traffic):
     achieved = fl["contraction"] / (t_contract * 1e-3) / 1e12
     P = synthetic.pass_bytes(B, N)
     roofline = {
-        "kernel": "contract_pair_kernel" if N >= 256 else "contract_kernel", "bound": "tensor", "achieved": achieved,
+        "kernel": " / ".join(dict.fromkeys(F_.contract_kernel(N, out) for out in (True, False))), "bound": "tensor", "achieved": achieved,
         "peak": peaks["bf16_tflops"], "unit": "TFLOP/s", "frac": achieved / peaks["bf16_tflops"],
         "peak_source": peaks["source"] + " (burst)",
         "frac_of_sustained": achieved / peaks["bf16_tflops_sustained"] if peaks["bf16_tflops_sustained"] else None,

@@ -116,6 +116,9 @@ int b200_trimul_prologue(const void* z, const void* packed, const uint8_t* token
 int b200_trimul_contract(const void* left, const void* right, void* tri, int B, int N, int row_begin, int rows,
                          int direction, int* status, void* cuda_stream);
 
+/* Name of the kernel that stage 2 launches for these sizes (for profilers; "" where rows are not within N). */
+const char* b200_trimul_contract_kernel(int N, int rows, int direction);
+
 /*
  * Gradients of stage 2 with respect to its operands (the reference's backward runs these four products as cuBLAS
  * calls, "B5-B6" in docs/kernels/trimul/TRIMUL_STATUS.md:47): given dtri = d loss / d tri in the layout of `tri`

@@ -37,6 +37,7 @@ SIGNATURES = {
         c_int,
         [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     ),
+    "b200_trimul_contract_kernel": (c_char_p, [c_int, c_int, c_int]),
     "b200_trimul_contract_backward": (
         c_int,
         [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],

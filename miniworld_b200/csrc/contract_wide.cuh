@@ -8,7 +8,7 @@
 // they have them in registers; the four stages that load meanwhile cover that gap (two accumulators for tiles of 256 columns
 // measured the same). What bounds it: DRAM and L2 up to N = 1024, the tensor pipe at the power limit from there on.
 // Contraction alone (before, 256- or 128-column pair tiles or 128 x 256 ones of one CTA -> these): N = 640 88 -> 82 us,
-// 896 217 -> 180, 1152 423 -> 336, 1408 740 -> 579, 1920 1775 -> 1490, 2048 1542 -> 1541 (incoming 1570 -> 1508).
+// 896 217 -> 180, 1152 423 -> 336, 1408 740 -> 579, 1920 1775 -> 1490, 2048 incoming 1570 -> 1508 (outgoing it is slower there, see contract_plan).
 #pragma once
 
 #include "contract_pair.cuh"

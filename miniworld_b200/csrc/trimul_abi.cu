@@ -672,6 +672,39 @@ int b200_trimul_prologue_channels(const void* z, const void* packed, const uint8
 // internal third operand form of contract_impl (not a module direction): t[i][j] = sum_k a[i][k] b[k][j] per plane
 constexpr int kDirMixed = 3;
 
+// Which kernel a contraction of `rows` rows and N columns takes, and its tiles.
+struct ContractPlan {
+  int pair_rows;  // rows in whole tiles of a CTA pair
+  bool use_pair;  // contract_pair_kernel, tiles of 256 x bn; otherwise contract_kernel, 128 x bn
+  bool use_wide;  // contract_wide_kernel before either
+  int bn;
+};
+static ContractPlan contract_plan(int N, int rows, int direction, int n_owners) {
+  ContractPlan c;
+  // CTA pairs work on 256-row tiles: used when that pads the rows by at most a quarter.
+  c.pair_rows = (rows + 255) / 256 * 256;
+  c.use_pair = rows >= 256 && (c.pair_rows - rows) * 4 <= rows;
+  c.bn = c.use_pair ? ((N + 255) / 256 * 256 <= (N + 127) / 128 * 128 ? 256 : 128) : choose_bn(N);
+  // Tiles of up to 512 columns where the other kernels would cut the columns in pieces of 128, or those of one CTA would pad
+  // (whole forwards: N = 400 107 -> 106 us and four of 400 346 -> 330, 640 227 -> 218, 832 431 -> 384, 1100 819 -> 707, 1408
+  // 1382 -> 1173, 1920 2990 -> 2515). Elsewhere the exactly fitting 192- and 256-column tiles are ahead: N = 288 63 / 66, 512
+  // 131 / 134, 576 182 / 189, 768 292 / 296, 1792 2045 / 2103 us. But where 512 divides the columns in tiles of 128 and N is
+  // above 896, the incoming form, whose operands are both MN-major, is 2 to 4 % faster with the wide ones, and the outgoing
+  // and mixed forms are slower (contraction alone, 256- / up to 512-column tiles): incoming N = 960 249 / 243 us, 1024 267 / 260,
+  // 1472 777 / 758, 1536 839 / 825, 1984 1769 / 1722, 2048 1868 / 1816, 2560 3589 / 3479; outgoing 960 234 / 274, 1024 258 / 297,
+  // 1472 737 / 823, 1536 786 / 889, 1984 1720 / 1835, 2048 1821 / 1960, 2560 3682 / 3829; mixed (after taking the incoming one
+  // off both contractions of a backward) 1024 320 / 331, 2048 2071 / 2236.
+  c.use_wide = n_owners == 0 && rows > 384 && N > 384 &&
+               (c.use_pair ? c.bn == 128 || (direction == B200_TRIMUL_INCOMING && N > 896 && (N + 127) / 128 % 4 == 0) : c.bn != 192);
+  return c;
+}
+
+const char* b200_trimul_contract_kernel(int N, int rows, int direction) {
+  if (N < 1 || rows < 1 || rows > N) return "";
+  const ContractPlan c = contract_plan(N, rows, direction, 0);
+  return c.use_wide ? "contract_wide_kernel" : c.use_pair ? "contract_pair_kernel" : "contract_kernel";
+}
+
 static int contract_impl(const void* left, const void* right, void* tri, void* const* owner_dst, int n_owners, int slot,
                          int channels, int B, int N, int row_begin, int rows, int k_rows, int direction, int* status,
                          void* cuda_stream, int row_channels = 0, int pitch = 0) {
@@ -694,17 +727,9 @@ static int contract_impl(const void* left, const void* right, void* tri, void* c
   // incoming and the mixed one
   const bool a_mn = direction == B200_TRIMUL_INCOMING;
   const bool b_mn = direction != B200_TRIMUL_OUTGOING;
-  // CTA pairs work on 256-row tiles: used when that pads the rows by at most a quarter.
-  const int pair_rows = (rows + 255) / 256 * 256;
-  const bool use_pair = rows >= 256 && (pair_rows - rows) * 4 <= rows;
-  const int bn = use_pair ? ((N + 255) / 256 * 256 <= (N + 127) / 128 * 128 ? 256 : 128) : choose_bn(N);
-  // Tiles of up to 512 columns where the other kernels would cut the columns in pieces of 128, or those of one CTA would pad,
-  // and for the largest problems where the width divides them (whole forwards: N = 400 107 -> 106 us and four of 400 346 ->
-  // 330, 640 227 -> 218, 832 431 -> 384, 1100 819 -> 707, 1408 1382 -> 1173, 1920 2990 -> 2515, 1024 551 -> 541). Elsewhere
-  // the exactly fitting 192- and 256-column tiles are ahead: N = 288 63 / 66, 512 131 / 134, 576 182 / 189, 768 292 / 296,
-  // 1792 2045 / 2103 us.
-  const bool use_wide = n_owners == 0 && rows > 384 && N > 384 &&
-                        (use_pair ? bn == 128 || (N > 896 && (N + 127) / 128 % 4 == 0) : bn != 192);
+  const ContractPlan plan = contract_plan(N, rows, direction, n_owners);
+  const bool use_pair = plan.use_pair, use_wide = plan.use_wide;
+  const int pair_rows = plan.pair_rows, bn = plan.bn;
   const int wide_tiles = (N + 511) / 512;
   const int wide_bn = ((N + wide_tiles - 1) / wide_tiles + 127) / 128 * 128;
   const uint64_t n64 = static_cast<uint64_t>(N);

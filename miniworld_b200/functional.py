@@ -53,6 +53,11 @@ def _direction(outgoing: Optional[bool]) -> int:
     return _lib.OUTGOING if outgoing else _lib.INCOMING
 
 
+def contract_kernel(N: int, outgoing: bool = True) -> str:
+    """Name of the kernel that contracts a whole pair tensor of ``N`` tokens."""
+    return _lib.load().b200_trimul_contract_kernel(N, N, _direction(outgoing)).decode()
+
+
 def workspace_bytes(B: int, N: int, outgoing: Optional[bool] = True, d_pair: int = D) -> int:
     out = c_size_t(0)
     d_hidden = D if (d_pair == D or outgoing is not None) else 64
