@@ -73,11 +73,14 @@ const char* b200_trimul_strerror(int code);
 /* Last cudaError_t seen by this thread inside the library (0 if none). */
 int b200_trimul_last_cuda_error(void);
 
-/* Bytes of workspace that serve a full (unsharded) call of any of the forward entry points below. */
+/* Bytes of workspace that serve a full (unsharded) call of any of the forward entry points below. Sized for the padded rows of
+ * b200_trimul_forward_lines; the others take less (the end of `tri` in b200_trimul_workspace_layout; direction 0 of 128-wide
+ * pairs: one more such tensor and one more packed block). */
 int b200_trimul_workspace_bytes(int B, int N, int d_pair, int d_hidden, int direction, size_t* out_bytes);
 
-/* Offsets (bytes) of the regions inside a workspace of b200_trimul_forward / _forward_ex: [0] status words, [1] packed
- * weights, [2] left, [3] right, [4] tri (dense). For tests and profilers that want to look at the stages. */
+/* Offsets (bytes) of the regions inside a workspace: [0] status words, [1] packed weights, [2] left, [3] right, [4] tri. For tests
+ * and profilers that want to look at the stages of b200_trimul_forward / _forward_ex, or of b200_trimul_forward_any with N
+ * rounded up to a multiple of 8 (b200_trimul_forward_lines lays its workspace out in another way). */
 int b200_trimul_workspace_layout(int B, int N, size_t out_offsets[5]);
 
 /* Bytes of the packed-weight block written by b200_trimul_pack_weights. */
@@ -249,8 +252,7 @@ int b200_trimul_forward_ex(const void* z, const void* w_left, const void* w_left
 
 /*
  * b200_trimul_forward_ex for every N >= 1. Nothing is padded: z, y, the masks and drop_scale are dense with N columns,
- * only the intermediates in the workspace have their channels N rounded up to a multiple of 64 columns apart (rows of
- * whole 128-byte lines; the faster form wherever N is not a multiple of 64). Workspace:
+ * only the intermediates in the workspace have their columns N rounded up to a multiple of 8 apart. Workspace:
  * b200_trimul_workspace_bytes of N rounded up to a multiple of 8. A workspace this call leaves behind is read by
  * b200_trimul_backward_any with the same N.
  */
@@ -261,6 +263,20 @@ int b200_trimul_forward_any(const void* z, const void* w_left, const void* w_lef
                             const void* drop_scale, void* y, void* workspace, size_t workspace_bytes, int B, int N,
                             int d_pair, int d_hidden, int direction, float eps_in, float eps_out, int residual,
                             void* cuda_stream);
+
+/*
+ * b200_trimul_forward_any with the intermediates' channels N rounded up to a multiple of 64 columns apart: rows of whole
+ * 128-byte lines, the faster form wherever N is not a multiple of 64 (what the modules call). Workspace:
+ * b200_trimul_workspace_bytes of N rounded up to a multiple of 8. What it leaves there is for b200_trimul_backward_lines with
+ * the same N only; the other entry points leave and read other layouts.
+ */
+int b200_trimul_forward_lines(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
+                              const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,
+                              const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
+                              const void* const* bias_opt, const uint8_t* token_mask, const uint8_t* pair_mask,
+                              const void* drop_scale, void* y, void* workspace, size_t workspace_bytes, int B, int N,
+                              int d_pair, int d_hidden, int direction, float eps_in, float eps_out, int residual,
+                              void* cuda_stream);
 
 /*
  * Weight packing of the bidirectional module (shapes as in b200_trimul_forward_ex): two blocks of
@@ -328,7 +344,8 @@ int b200_trimul_forward_static(const void* z, const void* w_left, const void* w_
  * prologue once more (left / right of the first half, which the forward overwrote), four contraction gradient launches,
  * the prologue's backward four times (side x half).
  * The result is deterministic (fixed summation order). Workspace: b200_trimul_backward_workspace_bytes, 1024-byte
- * aligned, which serves this call and b200_trimul_backward_any; _layout gives this call's 17 region offsets + the end (status, packed weights, scale, LayerNorm terms, x_hat and
+ * aligned, which serves this call, b200_trimul_backward_any and b200_trimul_backward_lines (the first two take less, the end that
+ * _layout gives); _layout gives this call's 17 region offsets + the end (status, packed weights, scale, LayerNorm terms, x_hat and
  * 1 / sigma, per-CTA partials of M and S of every launch, dtri, dleft, dright, d x_hat, then the bidirectional module's extra
  * regions) for tests. About five pair tensors of 128 16-bit channels (nine for direction 0) and 63 MB of partials (126 MB, at
  * most 160 CTAs): one direction 253 MB at N = 384 and 821 MB at N = 768, direction 0 280 MB at N = 256 and 1.50 GB at N = 768.
@@ -356,6 +373,16 @@ int b200_trimul_backward_any(const void* dy, const void* z, const void* w_left, 
                              float* d_ln_in_w, float* d_ln_in_b, float* d_ln_out_w, float* d_ln_out_b, void* workspace,
                              size_t workspace_bytes, int B, int N, int d_pair, int d_hidden, int direction, float eps_in,
                              float eps_out, int residual, void* cuda_stream);
+
+/* The same after b200_trimul_forward_lines. */
+int b200_trimul_backward_lines(const void* dy, const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
+                               const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,
+                               const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
+                               const void* const* bias_opt, const uint8_t* token_mask, const uint8_t* pair_mask,
+                               const void* drop_scale, const void* forward_workspace, void* dz, void* const* dw,
+                               float* d_ln_in_w, float* d_ln_in_b, float* d_ln_out_w, float* d_ln_out_b, void* workspace,
+                               size_t workspace_bytes, int B, int N, int d_pair, int d_hidden, int direction, float eps_in,
+                               float eps_out, int residual, void* cuda_stream);
 
 /*
  * Pair Transition, the operator on the other side of the triangle update in every block

@@ -138,6 +138,8 @@ SIGNATURES = {
 # the same arguments, every N
 SIGNATURES["b200_trimul_forward_any"] = SIGNATURES["b200_trimul_forward_ex"]
 SIGNATURES["b200_trimul_backward_any"] = SIGNATURES["b200_trimul_backward"]
+SIGNATURES["b200_trimul_forward_lines"] = SIGNATURES["b200_trimul_forward_ex"]
+SIGNATURES["b200_trimul_backward_lines"] = SIGNATURES["b200_trimul_backward"]
 
 _lib = None
 

@@ -87,8 +87,8 @@ struct TriCall {
   float eps_in, eps_out;
   bool residual, any_n;
   int dtype;
-  // The C entry points below are the any-length ones for every N, because their intermediates have aligned rows; any_n says
-  // which lengths and gradients are taken and which entry point of the general path an error names.
+  // The C entry points below are the ones whose intermediates have rows of whole lines, for every N; any_n says which lengths and
+  // gradients are taken and which entry point of the general path refuses what they refuse.
   int sized_n() const { return (N + 7) / 8 * 8; }
 };
 
@@ -144,12 +144,12 @@ void launch_forward(const TriCall& c, const Tensor& z, at::TensorList p, const O
                     const OptTensor& pair_mask, const OptTensor& drop_scale, const Tensor& y, void* ws, size_t ws_bytes) {
   const c10::cuda::CUDAGuard guard(z.device());
   auto fp = [&](int i) { return static_cast<const float*>(p[i].data_ptr()); };
-  check(b200_trimul_forward_any(z.data_ptr(), p[kLeft].data_ptr(), p[kLeftGate].data_ptr(), p[kRight].data_ptr(), p[kRightGate].data_ptr(),
+  check(b200_trimul_forward_lines(z.data_ptr(), p[kLeft].data_ptr(), p[kLeftGate].data_ptr(), p[kRight].data_ptr(), p[kRightGate].data_ptr(),
           p[kGate].data_ptr(), p[kOut].data_ptr(), c.dtype, fp(kLnInW), fp(kLnInB), fp(kLnOutW), fp(kLnOutB), nullptr,
           static_cast<const uint8_t*>(ptr(token_mask)), static_cast<const uint8_t*>(ptr(pair_mask)), ptr(drop_scale),
           y.data_ptr(), ws, ws_bytes, c.B, c.N, c.d_pair, c.d_hidden, c.direction, c.eps_in,
           c.eps_out, c.residual ? 1 : 0, stream_of(z)),
-        c.any_n ? "b200_trimul_forward_any" : "b200_trimul_forward_ex");
+        c.any_n ? "b200_trimul_forward_lines, for b200_trimul_forward_any" : "b200_trimul_forward_lines, for b200_trimul_forward_ex");
 }
 
 // Scratch memory that a module keeps from one call to the next, with the stream that it may be used on again: the memory of a
@@ -251,13 +251,13 @@ struct TriMul : public torch::autograd::Function<TriMul> {
                    g[kGate].data_ptr(), g[kOut].data_ptr()};
     auto fp = [&](int i) { return static_cast<const float*>(p[i].data_ptr()); };
     auto gp = [&](int i) { return static_cast<float*>(g[i].data_ptr()); };
-    check(b200_trimul_backward_any(dy.data_ptr(), z.data_ptr(), p[kLeft].data_ptr(), p[kLeftGate].data_ptr(), p[kRight].data_ptr(),
+    check(b200_trimul_backward_lines(dy.data_ptr(), z.data_ptr(), p[kLeft].data_ptr(), p[kLeftGate].data_ptr(), p[kRight].data_ptr(),
             p[kRightGate].data_ptr(), p[kGate].data_ptr(), p[kOut].data_ptr(), c.dtype, fp(kLnInW), fp(kLnInB), fp(kLnOutW),
             fp(kLnOutB), nullptr, static_cast<const uint8_t*>(ptr(token_mask)), static_cast<const uint8_t*>(ptr(pair_mask)),
             ptr(drop_scale), aligned_start(ws), dz.data_ptr(), dw, gp(kLnInW), gp(kLnInB), gp(kLnOutW), gp(kLnOutB),
             aligned_start(bws), scratch_bytes(bws), c.B, c.N, c.d_pair, c.d_hidden, c.direction, c.eps_in, c.eps_out,
             c.residual ? 1 : 0, stream_of(z)),
-          c.any_n ? "b200_trimul_backward_any" : "b200_trimul_backward");
+          c.any_n ? "b200_trimul_backward_lines, for b200_trimul_backward_any" : "b200_trimul_backward_lines, for b200_trimul_backward");
     d.erase("ws");
 
     variable_list out(1 + kTriParams + 4);  // z, the parameters; call, masks and scale have no gradient
@@ -299,7 +299,7 @@ void launch_transition(const Tensor& x, at::TensorList p, double eps, bool resid
                         static_cast<const float*>(p[kTrLnW].data_ptr()), static_cast<const float*>(p[kTrLnB].data_ptr()), packed,
                         y.data_ptr(), x.numel() / 128, 128, 4, static_cast<float>(eps), residual ? 1 : 0, status,
                         clear_status ? 1 : 0, stream_of(x)),
-        "b200_transition_forward");
+        "b200_transition_pack_forward");
 }
 
 // Forward without a graph: (y, (stream, scratch used)) or None. The scratch holds the packed weights, then 16 status words, which

@@ -236,16 +236,30 @@ static int check_bn(int B, int N, bool any_n = false) {
 
 static size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Columns from one channel of a pair row to the next in the row-plane intermediates (left, right, tri and their gradients)
-// of an any-length call: N rounded up to 128 bytes, so that every 64-column piece that the stages copy is one line of L2 and
-// not parts of two. The maps' extents stay N: loads read zeros past it and stores are clipped there, so the columns N ..
-// pitch-1 cost memory but no traffic and are never used, and no input is padded. The stage entry points take dense tensors
-// (pitch N), and so do calls that leave a workspace of the documented layout. Module calls with rows a multiple of 16 bytes
-// before and of 128 bytes now: N = 264 forward 68.1 -> 61.2 us, training step 264 -> 249; 321: 82.4 -> 76.1; 376: 92.9 -> 87.1;
-// 520: 185 -> 166, training step 690 -> 635; 760: 316 -> 287 (768, aligned either way: 288 -> 286).
+// How the row-plane intermediates (left, right, tri and their gradients) of a whole call lie in its workspace:
+// - kDense: [B, N, 128, N], N a multiple of 8 (the documented layout; the stage entry points take such tensors).
+// - kAny: every N >= 1, channels N rounded up to a multiple of 8 columns apart (the 16 bytes a tensor map's strides need) in
+//   regions of the rounded length: for a multiple of 8 the same as kDense, so that forwards and backwards of the two mix.
+// - kLines: every N >= 1, channels N rounded up to 128 bytes apart, so that every 64-column piece that the stages copy is one line
+//   of L2 and not parts of two. Module calls with kAny / kDense before and kLines now: N = 264 forward 68.1 -> 61.2 us, training
+//   step 264 -> 249; 321: 82.4 -> 76.1; 376: 92.9 -> 87.1; 520: 185 -> 166, training step 690 -> 635; 760: 316 -> 287 (768, aligned
+//   either way: 288 -> 286).
+// The maps' extents stay N: loads read zeros past it and stores are clipped there, so the columns N .. pitch-1 cost memory but
+// no traffic and are never used, and no input is padded.
+enum class Planes { kDense, kAny, kLines };
 static int plane_pitch(int N) { return static_cast<int>((static_cast<unsigned>(N) + 63u) / 64u * 64u); }
 // per-position statistics [rows][N] have their rows this far apart (16-byte pieces of 16-bit columns)
 static int round_up_8(int N) { return static_cast<int>((static_cast<unsigned>(N) + 7u) / 8u * 8u); }
+
+// the pitch `ld` and the rows per sample that the regions of a workspace are sized for
+struct PlaneShape {
+  int rows, ld;
+};
+static PlaneShape plane_shape(Planes planes, int N) {
+  if (planes == Planes::kLines) return {N, plane_pitch(N)};
+  const int ld = planes == Planes::kAny ? round_up_8(N) : N;
+  return {ld, ld};
+}
 
 static size_t plane_tensor_bytes(int B, int rows, int ld) {
   return round_up(static_cast<size_t>(B) * rows * kC * ld * 2, 1024);
@@ -346,9 +360,9 @@ int b200_trimul_last_cuda_error(void) { return tl_last_cuda_error; }
 
 size_t b200_trimul_packed_bytes(void) { return kPackedBytes; }
 
-// Regions of a workspace whose intermediates have the pitch `ld`.
-static void workspace_offsets(int B, int N, int ld, size_t off[5]) {
-  const size_t t = plane_tensor_bytes(B, N, ld);
+// Regions of a workspace whose intermediates have the shape `ps`.
+static void workspace_offsets(int B, PlaneShape ps, size_t off[5]) {
+  const size_t t = plane_tensor_bytes(B, ps.rows, ps.ld);
   off[0] = 0;
   off[1] = kStatusBytes;
   off[2] = kStatusBytes + kPackedBytes;
@@ -360,11 +374,11 @@ int b200_trimul_workspace_layout(int B, int N, size_t out_offsets[5]) {
   if (out_offsets == nullptr) return B200_TRIMUL_E_NULL;
   int rc = check_bn(B, N);
   if (rc != B200_TRIMUL_OK) return rc;
-  workspace_offsets(B, N, N, out_offsets);
+  workspace_offsets(B, plane_shape(Planes::kDense, N), out_offsets);
   return B200_TRIMUL_OK;
 }
 
-static int workspace_need(int B, int N, int ld, int d_pair, int d_hidden, int direction, size_t* out_bytes) {
+static int workspace_need(int B, int N, Planes planes, int d_pair, int d_hidden, int direction, size_t* out_bytes) {
   if (direction != B200_TRIMUL_OUTGOING && direction != B200_TRIMUL_INCOMING && direction != B200_TRIMUL_BIDIRECTIONAL)
     return B200_TRIMUL_E_SHAPE;
   // supported widths: d_pair = d_hidden = 128 (every direction); d_pair = 64 with 128 contracted channels in total,
@@ -375,19 +389,21 @@ static int workspace_need(int B, int N, int ld, int d_pair, int d_hidden, int di
   int rc = check_bn(B, N, true);
   if (rc == B200_TRIMUL_OK) rc = check_bn(B, round_up_8(N));
   if (rc != B200_TRIMUL_OK) return rc;
+  const PlaneShape ps = plane_shape(planes, N);
+  const size_t plane = plane_tensor_bytes(B, ps.rows, ps.ld);
   size_t off[5];
-  workspace_offsets(B, N, ld, off);
-  *out_bytes = off[4] + plane_tensor_bytes(B, N, ld);
+  workspace_offsets(B, ps, off);
+  *out_bytes = off[4] + plane;
   // bidirectional: a second packed block and a second tri tensor (left / right are reused by the two halves)
-  if (direction == B200_TRIMUL_BIDIRECTIONAL && wide) *out_bytes += kPackedBytes + plane_tensor_bytes(B, N, ld);
+  if (direction == B200_TRIMUL_BIDIRECTIONAL && wide) *out_bytes += kPackedBytes + plane;
   return B200_TRIMUL_OK;
 }
 
-// (the larger pitch of the any-length calls: enough for both kinds)
+// (of the form with the largest pitch: enough for every kind of call)
 int b200_trimul_workspace_bytes(int B, int N, int d_pair, int d_hidden, int direction, size_t* out_bytes) {
   if (out_bytes == nullptr) return B200_TRIMUL_E_NULL;
   size_t need = 0;
-  int rc = workspace_need(B, N, plane_pitch(N), d_pair, d_hidden, direction, &need);
+  int rc = workspace_need(B, N, Planes::kLines, d_pair, d_hidden, direction, &need);
   if (rc == B200_TRIMUL_OK) rc = check_bn(B, N);
   if (rc != B200_TRIMUL_OK) return rc;
   *out_bytes = need;
@@ -1092,18 +1108,20 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
                            const void* const* bias_opt, const uint8_t* token_mask, const uint8_t* pair_mask,
                            const void* drop_scale, void* y, void* workspace, size_t workspace_bytes, int B, int N,
                            int d_pair, int d_hidden, int direction, float eps_in, float eps_out, int residual,
-                           void* cuda_stream, bool any_n) {
+                           void* cuda_stream, Planes planes) {
   if (!z || !y || !workspace) return B200_TRIMUL_E_NULL;
   size_t need = 0;
+  const bool any_n = planes != Planes::kDense;
   if (any_n && (N < 1 || N > 0x7FFFFFFF / 128)) return B200_TRIMUL_E_SHAPE;
-  const int ld = any_n ? plane_pitch(N) : N;
-  int rc = workspace_need(B, N, ld, d_pair, d_hidden, direction, &need);
+  const PlaneShape ps = plane_shape(planes, N);
+  const int ld = ps.ld;
+  int rc = workspace_need(B, N, planes, d_pair, d_hidden, direction, &need);
   if (rc == B200_TRIMUL_OK) rc = check_bn(B, N, any_n);
   if (rc != B200_TRIMUL_OK) return rc;
   if (workspace_bytes < need) return B200_TRIMUL_E_WORKSPACE;
   if (!aligned(workspace, 1024)) return B200_TRIMUL_E_ALIGN;
   size_t off[5];
-  workspace_offsets(B, N, ld, off);
+  workspace_offsets(B, ps, off);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   int* status = reinterpret_cast<int*>(ws + off[0]);
   void* packed = ws + off[1];
@@ -1152,7 +1170,7 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
   }
   if (direction == B200_TRIMUL_BIDIRECTIONAL) {
     // workspace tail: second tri tensor, then the second packed block
-    const size_t plane = plane_tensor_bytes(B, N, ld);
+    const size_t plane = plane_tensor_bytes(B, ps.rows, ld);
     void* tri_in = ws + off[4] + plane;
     void* packed_in = ws + off[4] + 2 * plane;
     rc = fill_pack_bidir(pk, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
@@ -1191,7 +1209,7 @@ int b200_trimul_forward_ex(const void* z, const void* w_left, const void* w_left
                            void* cuda_stream) {
   return forward_impl(z, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
                       ln_out_b, bias_opt, token_mask, pair_mask, drop_scale, y, workspace, workspace_bytes, B, N, d_pair,
-                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, false);
+                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, Planes::kDense);
 }
 
 int b200_trimul_forward_any(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
@@ -1203,7 +1221,19 @@ int b200_trimul_forward_any(const void* z, const void* w_left, const void* w_lef
                            void* cuda_stream) {
   return forward_impl(z, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
                       ln_out_b, bias_opt, token_mask, pair_mask, drop_scale, y, workspace, workspace_bytes, B, N, d_pair,
-                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, true);
+                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, Planes::kAny);
+}
+
+int b200_trimul_forward_lines(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
+                           const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,
+                           const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
+                           const void* const* bias_opt, const uint8_t* token_mask, const uint8_t* pair_mask,
+                           const void* drop_scale, void* y, void* workspace, size_t workspace_bytes, int B, int N,
+                           int d_pair, int d_hidden, int direction, float eps_in, float eps_out, int residual,
+                           void* cuda_stream) {
+  return forward_impl(z, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
+                      ln_out_b, bias_opt, token_mask, pair_mask, drop_scale, y, workspace, workspace_bytes, B, N, d_pair,
+                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, Planes::kLines);
 }
 
 int b200_trimul_forward(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
@@ -1369,7 +1399,7 @@ extern "C" int b200_trimul_forward_static(const void* z, const void* w_left, con
                                           int** device_status_out, void* cuda_stream) {
   if (!z || !y) return B200_TRIMUL_E_NULL;
   size_t need = 0;
-  int rc = workspace_need(B, N, N, d_pair, d_hidden, direction, &need);
+  int rc = workspace_need(B, N, Planes::kDense, d_pair, d_hidden, direction, &need);
   if (rc == B200_TRIMUL_OK) rc = check_bn(B, N);
   if (rc != B200_TRIMUL_OK) return rc;
   if (static_cast<long long>(B) * N * N > kStaticMaxCells || need > kStaticWorkspaceBytes) return B200_TRIMUL_E_TOO_LARGE;

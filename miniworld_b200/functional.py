@@ -474,8 +474,24 @@ def trimul_forward(
 
 
 def _pitch(N: int) -> int:
-    """The length whose workspace size an any-length call of ``N`` tokens needs: N rounded up to a multiple of 8."""
+    """Columns between consecutive channels of a pair row in the intermediates of an any-length call: N rounded up to a multiple
+    of 8. Its workspaces are those of that length."""
     return (N + 7) // 8 * 8
+
+
+def _forward_need(B: int, N: int, outgoing: Optional[bool], d_pair: int) -> int:
+    """Bytes of workspace that a forward through the entry points with dense planes needs (``N`` a multiple of 8); what
+    :func:`workspace_bytes` gives also serves the native calls, whose planes have padded rows."""
+    off = workspace_layout(B, N)
+    plane = off[4] - off[3]
+    return off[4] + plane + (packed_bytes() + plane if outgoing is None and d_pair == D else 0)
+
+
+def _backward_need(B: int, N: int, outgoing: Optional[bool]) -> int:
+    """:func:`_forward_need` of the backward's own workspace."""
+    off = (c_size_t * 18)()
+    _lib.check(_lib.load().b200_trimul_backward_workspace_layout(B, N, _direction(outgoing), off), "b200_trimul_backward_workspace_layout")
+    return int(off[17])
 
 
 def _forward(z, params, mask, outgoing, eps_in, eps_out, pair_mask, residual, biases, workspace, out, check, weights,
@@ -497,7 +513,7 @@ def _forward(z, params, mask, outgoing, eps_in, eps_out, pair_mask, residual, bi
         if drop_scale.numel() != B * N * D or drop_scale.shape[-1] != D or drop_scale.shape[0] != B:  # d_pair = 128 here
             raise RuntimeError(f"drop_scale must be [B, 1, N, {D}] = ({B}, 1, {N}, {D}), got {tuple(drop_scale.shape)}")
         ds = drop_scale.detach().to(torch.bfloat16).contiguous()
-    need = workspace_bytes(B, _pitch(N) if any_n else N, outgoing, C)
+    need = _forward_need(B, _pitch(N) if any_n else N, outgoing, C)
     if workspace is None:
         workspace = aligned_empty(need, dev)
     elif workspace.numel() * workspace.element_size() < need:
@@ -598,12 +614,12 @@ def _backward(dy, z, params, forward_workspace, mask, outgoing, eps_in, eps_out,
         if drop_scale.numel() != B * N * D or drop_scale.shape[-1] != D or drop_scale.shape[0] != B:
             raise RuntimeError(f"drop_scale must be [B, 1, N, {D}], got {tuple(drop_scale.shape)}")
         ds = drop_scale.detach().to(device=dev, dtype=torch.bfloat16).contiguous()
-    need = backward_workspace_bytes(B, _pitch(N) if any_n else N, outgoing)
+    need = _backward_need(B, _pitch(N) if any_n else N, outgoing)
     if workspace is None:
         workspace = aligned_empty(need, dev)
     elif workspace.numel() * workspace.element_size() < need:
         raise RuntimeError(f"workspace too small: {workspace.numel() * workspace.element_size()} < {need}")
-    if forward_workspace.numel() * forward_workspace.element_size() < workspace_bytes(B, _pitch(N) if any_n else N, outgoing, C):
+    if forward_workspace.numel() * forward_workspace.element_size() < _forward_need(B, _pitch(N) if any_n else N, outgoing, C):
         raise RuntimeError("forward_workspace is smaller than the forward's workspace for this shape")
     tm = as_mask_u8(mask, dev)
     pm = as_mask_u8(pair_mask, dev)

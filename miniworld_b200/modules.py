@@ -310,7 +310,7 @@ class TriangleMultiplication(_Scratch):
                 pair_mask = torch.broadcast_to(pair_mask.to(z.device), (B, N, N))
             if scale is not None:
                 scale = F_.aligned16(torch.broadcast_to(scale, (B, 1, N, self.d_pair)).contiguous())
-        need = F_.workspace_bytes(B, F_._pitch(N) if ragged else N, self._direction(), self.d_pair)
+        need = F_._forward_need(B, F_._pitch(N) if ragged else N, self._direction(), self.d_pair)
         with torch.no_grad(), _Kept(self, "_workspace", need, z.device) as workspace:
             y = F_._forward(
                 z, self._params(), token_mask, self._direction(), float(self.ln_pair.eps), float(self.ln_out.eps), pair_mask,

@@ -49,7 +49,7 @@ class TriMulFunction(torch.autograd.Function):
         B, N = int(z.shape[0]), int(z.shape[1])
         p = {k: v.detach() for k, v in zip(_PARAM_KEYS, params)}
         any_n = cfg["any_n"]
-        ws = F_.aligned_empty(F_.workspace_bytes(B, F_._pitch(N) if any_n else N, cfg["outgoing"], int(z.shape[3])),
+        ws = F_.aligned_empty(F_._forward_need(B, F_._pitch(N) if any_n else N, cfg["outgoing"], int(z.shape[3])),
                               z.device)  # kept until the backward
         y = F_._forward(z.detach(), p, token_mask, cfg["outgoing"], cfg["eps_in"], cfg["eps_out"], pair_mask, cfg["residual"],
                         cfg["biases"], ws, None, cfg["check"], None, drop_scale, any_n)
