@@ -147,3 +147,139 @@ def test_two_parameter_sets_on_one_workspace(kind, c, drop, n):
     for _ in range(3):
         graph.replay()
     assert all(torch.equal(y, want[i % 2]) for out in (got, replayed) for i, y in enumerate(out))
+
+
+def _filled(kind, seed):
+    """A module whose parameters are all non-zero (the default output gate and projection are zeros, behind which nothing shows)."""
+    g = torch.Generator().manual_seed(seed)
+    m = mw.Transition(128) if kind == "transition" else KINDS[kind](128)
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_((1.0 if p.dim() == 1 else 0.0) + torch.randn(p.shape, generator=g) * (0.1 if p.dim() == 1 else p.shape[-1] ** -0.5))
+    return m.to(DEV)
+
+
+@pytest.mark.parametrize("kind", [*KINDS, "transition"])
+@pytest.mark.parametrize("n", [8, 136])
+def test_every_argument_written_by_the_launch_before(kind, n):
+    """test_arguments_written_by_the_launch_before where each argument shows in the result: one of them is changed before every call,
+    and every call gives another result."""
+    g = torch.Generator().manual_seed(5)
+    m = _filled(kind, n).to(torch.bfloat16).eval()
+    z = torch.randn(1, n, n, 128, generator=g).to(torch.bfloat16).to(DEV)
+    mask = torch.ones(1, n, dtype=torch.bool, device=DEV)
+    mask[:, n // 3] = False
+    args = (z,) if kind == "transition" else (z, mask)
+    changed = [*args, *m.parameters()]
+    start = [t.detach().clone() for t in changed]
+
+    def run(wait):
+        out = []
+        with torch.no_grad():
+            for t, s in zip(changed, start):
+                t.copy_(s)
+            for t in changed:
+                t.logical_not_() if t.dtype == torch.bool else t.add_(0.25)
+                if wait:
+                    torch.cuda.synchronize()
+                out.append(m(*args))
+                if wait:
+                    torch.cuda.synchronize()
+                if t.dtype == torch.bool:
+                    t.logical_not_()
+        return out
+
+    want, got = run(True), run(False)
+    assert all(torch.isfinite(w).all() and not torch.equal(w, z) for w in want)
+    assert all(not torch.equal(a, b) for i, a in enumerate(want) for b in want[:i])
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+@pytest.mark.parametrize("kind", [*KINDS, "transition"])
+@pytest.mark.parametrize("n", [8, 136, 200])
+def test_training_steps_with_every_gradient(kind, n):
+    """test_training_steps_in_a_row where no gradient is zero: other parameters, input and output gradient in each step."""
+    g = torch.Generator().manual_seed(n)
+    m = _filled(kind, n + 1).to(torch.bfloat16).train()
+    start = [p.detach().clone() for p in m.parameters()]
+    z0 = torch.randn(1, n, n, 128, generator=g).to(torch.bfloat16).to(DEV)
+    dy0 = torch.randn(1, n, n, 128, generator=g).to(torch.bfloat16).to(DEV)
+    mask = (torch.rand(1, n, generator=g) >= 0.1).to(DEV)
+
+    def run(wait):
+        z, out = z0.clone().requires_grad_(), []
+        pause = torch.cuda.synchronize if wait else lambda: None
+        for i in range(4):
+            with torch.no_grad():
+                for p, s in zip(m.parameters(), start):
+                    p.copy_(s * (1 + 0.125 * i))
+                z.copy_(z0 * (1 - 0.25 * i))
+            pause()
+            y = m(z) if kind == "transition" else m(z, mask)
+            pause()
+            dy = dy0 * (0.5 + 0.25 * i)
+            pause()
+            out.append([y.detach(), *torch.autograd.grad(y, [z, *m.parameters()], dy)])
+            pause()
+        return out
+
+    want, got = run(True), run(False)
+    for i, step in enumerate(want):
+        assert all(torch.isfinite(t).all() and bool((t != 0).any()) for t in step)
+        assert all(not torch.equal(a, b) for before in want[:i] for a, b in zip(step, before))
+    assert all(torch.equal(a, b) for x, y in zip(want, got) for a, b in zip(x, y))
+
+
+@pytest.mark.parametrize("kind", [*KINDS, "transition"])
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("before", ["copy", "memset", "other stream", "both streams"])
+def test_what_may_come_before_a_call(kind, graph, before):
+    """A call's first launch may overlap the kernel before it; what comes before it may also be a copy, a memset or another stream's
+    work, eager and captured."""
+    n = 72
+    g = torch.Generator().manual_seed(3)
+    m = _filled(kind, 4).to(torch.bfloat16).eval()
+    src = [torch.randn(1, n, n, 128, generator=g).to(torch.bfloat16).to(DEV) for _ in range(3)]
+    src[1].zero_()
+    heavy = torch.randn(2048, 2048, device=DEV)
+    z = torch.empty_like(src[0])
+    side = torch.cuda.Stream()
+
+    def fill(t):
+        t.zero_() if before == "memset" else t.copy_(src[0])
+
+    def run(wait):
+        main = torch.cuda.current_stream()
+        z.fill_(5.0)
+        pause = torch.cuda.synchronize if wait else lambda: None
+        if "stream" in before:
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                h = heavy @ heavy @ heavy  # (so that z comes late)
+                fill(z)
+            if before == "both streams":
+                _ = src[2] * 2.0
+            pause()
+            main.wait_stream(side)
+            h.record_stream(main)
+        else:
+            fill(z)
+        pause()
+        with torch.no_grad():
+            y = m(z)
+        pause()
+        return y
+
+    want = run(True).clone()
+    for _ in range(5):
+        if graph:
+            torch.cuda.synchronize()
+            recorded = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(recorded):
+                got = run(False)
+            z.fill_(5.0)
+            recorded.replay()
+        else:
+            got = run(False)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want) and not torch.equal(want, z)
