@@ -268,7 +268,8 @@ int b200_trimul_forward_any(const void* z, const void* w_left, const void* w_lef
  * b200_trimul_forward_any with the intermediates' channels N rounded up to a multiple of 64 columns apart: rows of whole
  * 128-byte lines, the faster form wherever N is not a multiple of 64 (what the modules call). Workspace:
  * b200_trimul_workspace_bytes of N rounded up to a multiple of 8. What it leaves there is for b200_trimul_backward_lines with
- * the same N only; the other entry points leave and read other layouts.
+ * the same N only; the other entry points leave and read other layouts. Of the packed weights there is only what its
+ * last stage reads.
  */
 int b200_trimul_forward_lines(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
                               const void* w_right_gate, const void* w_gate, const void* w_out, int weight_dtype,

@@ -66,8 +66,8 @@ struct PrologueParams {
   // Where this kernel's matrices come from. raw = 0: `w`, the packed block of an earlier launch. raw = 1: the parameters
   // themselves (block `raw_block` of the kernel's PackLaunch), which with z, the masks and the LayerNorm parameters below are
   // older than the kernel before this one; then this launch also packs what the epilogue reads (matrices 4 and 5 of block 0,
-  // matrix 4 of block 1; `pack_blocks` of them) and, if it packs anything, fills the rest of block 0 and clears the status
-  // words of the call.
+  // matrix 4 of block 1; `pack_blocks` of them) and, if it packs anything, clears the status words of the call. The kernel with
+  // LEAVES, for launches that pack, fills the rest of block 0.
   int raw, raw_block, pack_blocks;
   const uint4* w;             // [4][128][C] fp16 packed matrices: left, left gate, right, right gate
   const float* d1;            // [4][128] additive constants (0.5 * bias): left, left gate, right, right gate
@@ -111,7 +111,7 @@ constexpr int kProAccBase = 128;  // tensor-memory column of the first one, behi
 // channels. The shared-memory budget is that of C = 128 for both.
 constexpr int kProSmemBytes = kProStages * 16384 + kProStageOutBytes + kProRing * kProRingBytes + kProBarBytes + 1024;
 
-template <bool HAS_BIAS, int C = 128>
+template <bool HAS_BIAS, int C = 128, bool LEAVES = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProThreads, 1)
 prologue_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ OutputMaps out,
                 const __grid_constant__ PackLaunch params, const PrologueParams p) {

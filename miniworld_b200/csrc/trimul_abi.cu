@@ -538,7 +538,7 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
                          void* const* left_dst, int n_left, void* const* right_dst, int n_right, PrologueMode mode,
                          int B, int N, int row_begin, int rows, float eps_in, int has_bias, int* status,
                          void* cuda_stream, int d_pair = kC, int ld = 0, const PackLaunch* raw = nullptr, int raw_block = 0,
-                         int pack_blocks = 0) {
+                         int pack_blocks = 0, bool leaves = false) {
   if (d_pair != kC && d_pair != 64) return B200_TRIMUL_E_UNSUPPORTED;
   if (!z || (!packed && !raw) || !left_dst || !right_dst || !status) return B200_TRIMUL_E_NULL;
   if (n_left < 1 || n_left > kMaxDst || n_right < 1 || n_right > kMaxDst) return B200_TRIMUL_E_SHAPE;
@@ -633,13 +633,18 @@ static int prologue_impl(const void* z, const void* packed, const uint8_t* token
   const int pairs = pack_blocks == 0 && p.num_tiles < info.sms / 2 ? p.num_tiles : info.sms / 2;
   const int grid = 2 * pairs;  // clusters of two CTAs: CTA 0 produces `left`, CTA 1 `right`
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-#define TRIMUL_LAUNCH_PROLOGUE(BIAS, DP)                                                              \
+#define TRIMUL_LAUNCH_PROLOGUE(...)                                                                  \
   do {                                                                                               \
-    rc = set_smem(prologue_kernel<BIAS, DP>, kProSmemBytes, info.device);                            \
+    rc = set_smem(prologue_kernel<__VA_ARGS__>, kProSmemBytes, info.device);                         \
     if (rc != B200_TRIMUL_OK) return rc;                                                             \
-    TRIMUL_CUDA(launch_overlapped(prologue_kernel<BIAS, DP>, grid, kProThreads, kProSmemBytes, stream, map_z, out, params, p)); \
+    TRIMUL_CUDA(launch_overlapped(prologue_kernel<__VA_ARGS__>, grid, kProThreads, kProSmemBytes, stream, map_z, out, params, p)); \
   } while (0)
-  if (d_pair == kC) {
+  if (leaves) {
+    if (d_pair == kC && has_bias) TRIMUL_LAUNCH_PROLOGUE(true, 128, true);
+    else if (d_pair == kC) TRIMUL_LAUNCH_PROLOGUE(false, 128, true);
+    else if (has_bias) TRIMUL_LAUNCH_PROLOGUE(true, 64, true);
+    else TRIMUL_LAUNCH_PROLOGUE(false, 64, true);
+  } else if (d_pair == kC) {
     if (has_bias) TRIMUL_LAUNCH_PROLOGUE(true, 128);
     else TRIMUL_LAUNCH_PROLOGUE(false, 128);
   } else {
@@ -1108,7 +1113,7 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
                            const void* const* bias_opt, const uint8_t* token_mask, const uint8_t* pair_mask,
                            const void* drop_scale, void* y, void* workspace, size_t workspace_bytes, int B, int N,
                            int d_pair, int d_hidden, int direction, float eps_in, float eps_out, int residual,
-                           void* cuda_stream, Planes planes) {
+                           void* cuda_stream, Planes planes, bool whole_block) {
   if (!z || !y || !workspace) return B200_TRIMUL_E_NULL;
   size_t need = 0;
   const bool any_n = planes != Planes::kDense;
@@ -1132,13 +1137,13 @@ static int forward_impl(const void* z, const void* w_left, const void* w_left_ga
   if (bias_opt != nullptr)
     for (int i = 0; i < 4; ++i) has_bias |= bias_opt[i] != nullptr;
   PackLaunch pk;
-  // stage 1 takes its weights from the parameters; the call's first launch packs those of stage 3, leaves its own beside them and
-  // clears the status words
+  // stage 1 takes its weights from the parameters; the call's first launch packs those of stage 3, leaves its own beside them where
+  // the workspace's layout is a documented one, and clears the status words
   auto prologue = [&](int block, int pack_blocks) {
     void* l[1] = {left};
     void* r[1] = {right};
     return prologue_impl(z, nullptr, token_mask, pair_mask, l, 1, r, 1, kLocal, B, N, 0, N, eps_in, has_bias, status, cuda_stream,
-                         d_pair, ld, &pk, block, pack_blocks);
+                         d_pair, ld, &pk, block, pack_blocks, pack_blocks > 0 && whole_block);
   };
   auto contract = [&](void* dst, int dir) {
     return contract_impl(left, right, dst, nullptr, 0, 0, kC, B, N, 0, N, N, dir, status, cuda_stream, 0, ld);
@@ -1209,7 +1214,7 @@ int b200_trimul_forward_ex(const void* z, const void* w_left, const void* w_left
                            void* cuda_stream) {
   return forward_impl(z, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
                       ln_out_b, bias_opt, token_mask, pair_mask, drop_scale, y, workspace, workspace_bytes, B, N, d_pair,
-                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, Planes::kDense);
+                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, Planes::kDense, true);
 }
 
 int b200_trimul_forward_any(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
@@ -1221,7 +1226,7 @@ int b200_trimul_forward_any(const void* z, const void* w_left, const void* w_lef
                            void* cuda_stream) {
   return forward_impl(z, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
                       ln_out_b, bias_opt, token_mask, pair_mask, drop_scale, y, workspace, workspace_bytes, B, N, d_pair,
-                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, Planes::kAny);
+                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, Planes::kAny, true);
 }
 
 int b200_trimul_forward_lines(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
@@ -1233,7 +1238,7 @@ int b200_trimul_forward_lines(const void* z, const void* w_left, const void* w_l
                            void* cuda_stream) {
   return forward_impl(z, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
                       ln_out_b, bias_opt, token_mask, pair_mask, drop_scale, y, workspace, workspace_bytes, B, N, d_pair,
-                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, Planes::kLines);
+                      d_hidden, direction, eps_in, eps_out, residual, cuda_stream, Planes::kLines, false);
 }
 
 int b200_trimul_forward(const void* z, const void* w_left, const void* w_left_gate, const void* w_right,
@@ -1410,10 +1415,9 @@ extern "C" int b200_trimul_forward_static(const void* z, const void* w_left, con
   rc = static_scratch(&scratch);
   if (rc != B200_TRIMUL_OK) return rc;
   if (device_status_out != nullptr) *device_status_out = static_cast<int*>(scratch);
-  return b200_trimul_forward(z, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w,
-                             ln_in_b, ln_out_w, ln_out_b, bias_opt, token_mask, pair_mask, y, scratch,
-                             kStaticWorkspaceBytes, B, N, d_pair, d_hidden, direction, eps_in, eps_out, residual,
-                             cuda_stream);
+  return forward_impl(z, w_left, w_left_gate, w_right, w_right_gate, w_gate, w_out, weight_dtype, ln_in_w, ln_in_b, ln_out_w,
+                      ln_out_b, bias_opt, token_mask, pair_mask, nullptr, y, scratch, kStaticWorkspaceBytes, B, N, d_pair, d_hidden,
+                      direction, eps_in, eps_out, residual, cuda_stream, Planes::kDense, false);
 }
 
 #include "backward_host.inc"
