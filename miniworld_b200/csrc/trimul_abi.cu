@@ -440,8 +440,6 @@ static int pack_block(PackLaunch& l, int block, const void* const w[6], const in
     a.ld[i] = ld[i];
     a.bias[i] = bias[i];
   }
-  if (!aligned(ln_in_w, 16) || !aligned(ln_in_b, 16) || !aligned(ln_out_w, 16) || !aligned(ln_out_b, 16))
-    return B200_TRIMUL_E_ALIGN;
   if (!aligned(packed, 1024)) return B200_TRIMUL_E_ALIGN;
   a.ln_in_w = ln_in_w;
   a.ln_in_b = ln_in_b;
