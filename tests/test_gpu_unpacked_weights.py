@@ -99,3 +99,25 @@ def test_workspace_holds_the_packed_block(dtype, biased, bidir, B, n):
         for k, t in ((2, left), (3, right)):
             kept = ws[off[k] : off[k] + t.numel() * 2].view(torch.int16).view_as(t)
             assert torch.equal(kept, t.view(torch.int16))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("outgoing", [True, None])
+@pytest.mark.parametrize("n", [8, 80])
+def test_workspace_holds_the_matrices_of_64_wide_pairs(dtype, outgoing, n):
+    """(no packing entry point for these: the stored values are half the weights in fp16, the LayerNorm parameters as they are)"""
+    g = torch.Generator().manual_seed(n)
+    names = ("to_left", "to_left_gate", "to_right", "to_right_gate")
+    p = {f"{k}.weight": (torch.randn(128, 64, generator=g) * 0.125).to(dtype).to(DEV) for k in names}
+    p["to_gate.weight"], p["to_out.weight"] = ((torch.randn(64, k, generator=g) * k**-0.5).to(dtype).to(DEV) for k in (64, 128))
+    for k, c in (("ln_pair", 64), ("ln_out", 128)):
+        p[f"{k}.weight"], p[f"{k}.bias"] = torch.randn(c, generator=g).to(DEV), torch.randn(c, generator=g).to(DEV)
+    z = torch.randn(1, n, n, 64, generator=g).to(torch.bfloat16).to(DEV)
+    ws = F_.aligned_empty(F_.workspace_bytes(1, n, outgoing, 64), torch.device(DEV)).fill_(0xA5)
+    F_.trimul_forward(z, p, None, outgoing=outgoing, workspace=ws, check=True)
+    start = F_.workspace_layout(1, n)[1]
+    got = ws[start : start + 4 * 128 * 64 * 2].view(torch.float16).view(4, 128, 64)
+    assert torch.equal(got, torch.stack([(0.5 * p[f"{k}.weight"].float()).half() for k in names]))
+    tail = ws[start + 6 * 32768 : start + F_.packed_bytes()].view(torch.float32)  # d [4][128], s / d of the epilogue, LayerNorm [2][128]
+    assert bool((tail[:512] == 0).all())
+    assert torch.equal(tail[1024 : 1024 + 64], p["ln_pair.weight"]) and torch.equal(tail[1152 : 1152 + 64], p["ln_pair.bias"])
