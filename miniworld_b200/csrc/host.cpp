@@ -11,6 +11,7 @@
 // on one device, boolean masks). If it is not, it answers None and changes nothing: the caller then takes the general
 // Python path, which converts what can be converted and says what is wrong with the rest.
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -58,8 +59,10 @@ bool plain_on(const Tensor& t, const Tensor& like, c10::ScalarType type, at::Int
 bool aligned16(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
 
 // Memory for a result or scratch on the device of `like`, from the caching allocator without the dispatcher (0.7 instead of 1.5
-// us each; a forward allocates one tensor, a backward twelve). All of it is overwritten.
+// us each; a forward allocates one tensor, a backward twelve). All of it is overwritten. A dispatch mode sees its allocations: under
+// one that hands out tensors without memory (fake tensors) a call has to fail at the C entry and not run for real.
 Tensor empty_on(at::IntArrayRef shape, c10::ScalarType type, const Tensor& like) {
+  if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return at::empty(shape, at::device(like.device()).dtype(type));
   return Tensor(at::detail::empty_cuda(shape, type, like.device(), std::nullopt));
 }
 Tensor aligned_empty(size_t bytes, const Tensor& like) {

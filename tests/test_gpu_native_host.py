@@ -192,3 +192,32 @@ def test_graph_behaviour(native):
     torch.cuda.current_stream().wait_stream(s)
     zr = z.clone().requires_grad_(True)
     assert torch.equal(g, torch.autograd.grad(b(zr, mask), zr, dy)[0])
+
+
+@pytest.mark.parametrize("kind", ["triangle", "transition"])
+@pytest.mark.parametrize("train", [False, True])
+def test_dispatch_modes_see_the_allocations(kind, train):
+    """Under a mode whose tensors have no memory a call is refused and nothing runs; a mode that only looks on changes nothing."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Count(TorchDispatchMode):
+        empties = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.empties += "empty" in str(func)
+            return func(*args, **(kwargs or {}))
+
+    m = mw.Transition(128) if kind == "transition" else mw.TriangleMultiplication(128, 128, outgoing=True)
+    m = m.to(DEV).to(torch.bfloat16).train(train)
+    z = torch.randn(1, 40, 40, 128, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
+    mask = torch.ones(1, 40, dtype=torch.bool, device=DEV)
+    args = (z,) if kind == "transition" else (z, mask)
+    with torch.set_grad_enabled(train):
+        want = m(*args)
+        with Count() as count:
+            got = m(*args)
+        assert torch.equal(got, want) and count.empties > 0
+        with FakeTensorMode(allow_non_fake_inputs=True), pytest.raises(RuntimeError):
+            m(*args)
+        assert torch.equal(m(*args), want)
